@@ -728,10 +728,8 @@ int launch_attention_fp32(const AttnArgs& a, cudaStream_t st) {
 // 3. Merge the partials of a row, normalise, un-rotate, store.
 //    Also serves tq4_combine_partials (cross-GPU shards) through the "dense" mode.
 // ======================================================================================
-constexpr int kCombHeads = 8;
-
 struct CombineArgs {
-  // sparse mode (plan != null): slots of row r are slot_base[r]..slot_base[r+1], x TPC
+  // sparse mode (slot_base != null): the partials of row r are slot_base[r]..slot_base[r+1], x TPC
   const int* slot_base;
   int TPC;
   const float* part_o;
@@ -749,229 +747,243 @@ struct CombineArgs {
   int out_rotated;
 };
 
-constexpr int kCombMaxParts = 64;  // partials of one row merged per pass
+// Merge kernel: eight warps, VB = 8 / WPV (row, head) vectors per pass.
+//   1. WPV warps merge the partials of one vector: warp w takes partials w, w + WPV, ..., a lane holds
+//      the maximum and sum of one of them and four (D = 256: eight) of the accumulator's coordinates, so
+//      the loads of eight partials are in flight at a time whatever their number.
+//   2. out[v][c] = sum_j x[v][j] * Pi[j][c]: a lane owns 4 columns x 4 vectors, the j range is cut over
+//      the warps (JP parts) and summed in shared memory.
+// Pi is copied to shared memory while the kernel in front is still running.  At head_dim 256 it does
+// not fit: a block owns 64 of the columns and the merge is repeated by the four blocks of a vector.
+// Bound by latency (a chain of three memory round trips), so the split follows the number of
+// vectors: few vectors get all eight warps each, many share a pass.  Measured on whole decode steps
+// against a merge with one thread per coordinate and eight vectors per block: batch 1 x 1024 tokens
+// (28 vectors of 64 partials) 73.8 -> 29.7 us, 16 ragged rows 74 -> 50.6 us, batch 64 x 4096 97.6 -> 92.7 us.
+template <int D, int WPV>
+struct CombineCfg {
+  static constexpr int VB = 8 / WPV;                  // vectors per pass
+  static constexpr int DC = D == 256 ? 64 : D;        // output columns of a block
+  static constexpr int NSPLIT = D / DC;
+  static constexpr int LC = DC / 4;                   // lanes that cover the columns
+  static constexpr int UPW = 32 / LC;                 // units (column sets) per warp: 2 if 16 lanes cover them
+  static constexpr int VPT = VB < 4 ? VB : 4;         // vectors per lane
+  static constexpr int NVG = VB / VPT;
+  static constexpr int JP = 8 * UPW / NVG;            // parts of the j range
+  static constexpr int JN = D / JP;
+  static constexpr int XP = D + 4;                    // pitch of a merged vector
+  static constexpr size_t kOffX = (size_t)D * DC * 4;
+  static constexpr size_t kOffRed = kOffX + (size_t)VB * XP * 4;
+  static constexpr size_t kRed = (size_t)JP * VB * DC * 4, kParts = (size_t)8 * D * 4;  // (the two uses of the area)
+  static constexpr size_t kSmem = kOffRed + (kRed > kParts ? kRed : kParts);
+  static_assert(JN % 4 == 0 && JP * JN == D, "a part of the j range is a multiple of four");
+};
 
-constexpr int kCombFastParts = 8;   // up to this many partials per vector take the one-round-trip path
-
-// Batches of 8 consecutive (row, head) vectors, D threads, a block walks batches grid-stride.
-// Pi is copied to shared memory asynchronously at kernel entry (once per block) and overlaps the
-// merge of the partials.  Typical decode rows have at most 8 partials: then every load of a batch
-// (8 x 8 accumulator elements per thread, the 64 maxima and sums by the first 64 threads) is issued
-// before anything is consumed, so a batch costs two dependent memory round trips.  Rows with more
-// partials go through passes of 64 partials with the merge weights staged in shared memory.
-template <int D>
-__global__ void __launch_bounds__(D) combine_kernel(const CombineArgs a) {
-  static_assert(D >= kCombHeads * kCombFastParts, "the fast path loads one (vector, partial) pair per thread");
+template <int D, int WPV>
+__global__ void __launch_bounds__(256) combine_kernel(const CombineArgs a) {
+  using C = CombineCfg<D, WPV>;
+  constexpr int VB = C::VB, R = D == 256 ? 2 : 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  float* s_pi = reinterpret_cast<float*>(smem_raw);            // [D][D] (D <= 128 only)
-  float* s_o = s_pi + (D <= 128 ? D * D : 0);                   // [D][kCombHeads]
-  float* s_w = s_o + kCombHeads * D;                            // [kCombMaxParts][kCombHeads]
-  float* s_m = s_w + kCombMaxParts * kCombHeads;                // [kCombHeads] running max
-  float* s_l = s_m + kCombHeads;                                // [kCombHeads] running sum
-  __shared__ long long s_p0[kCombHeads];                        // first partial of the vector's row
-  __shared__ int s_np[kCombHeads], s_row[kCombHeads], s_head[kCombHeads];
-  const int d = threadIdx.x;
-  const int64_t n_vec = (int64_t)a.rows * a.Hq;
-  const int64_t n_batches = (n_vec + kCombHeads - 1) / kCombHeads;
-  constexpr float kLn2 = 0.6931471805599453f, kLog2e = 1.4426950408889634f;
-  constexpr bool kStagePi = D <= 128;  // a 256 x 256 fp32 Pi does not fit in shared memory
-  if (kStagePi && !a.out_rotated) {
+  float* s_pi = reinterpret_cast<float*>(smem_raw);                 // [D][DC]
+  float* s_x = reinterpret_cast<float*>(smem_raw + C::kOffX);       // [VB][XP] merged, normalised vectors
+  float* s_red = reinterpret_cast<float*>(smem_raw + C::kOffRed);   // [8][D] partial merges, then [JP][VB][DC] partial products
+  __shared__ float s_m[8], s_l[8];
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int split = blockIdx.x % C::NSPLIT;
+  const int n_vec = a.rows * a.Hq;
+  if (!a.out_rotated) {
     const uint32_t dst = (uint32_t)__cvta_generic_to_shared(s_pi);
-    for (int i = d; i < D * D / 4; i += D)
+    for (int i = tid; i < D * C::LC; i += 256) {
+      const int j = i / C::LC, c4 = i - j * C::LC;
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst + i * 16),
-                   "l"(a.rotation + (size_t)i * 4) : "memory");
+                   "l"(a.rotation + (size_t)j * D + split * C::DC + 4 * c4) : "memory");
+    }
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
   pdl_wait();  // the partials and the plan come from the kernels before this one
   const bool sparse = a.slot_base != nullptr;
-  const float mscale = sparse ? 1.f : kLog2e;  // dense partials carry a natural-log LSE
-  const int64_t pstride = (sparse ? (int64_t)1 : (int64_t)a.rows) * a.Hq * D;
+  const float mscale = sparse ? 1.f : 1.4426950408889634f;  // dense partials carry a natural-log LSE
+  const int64_t pstride = sparse ? (int64_t)a.Hq : (int64_t)a.rows * a.Hq;  // vectors between two partials
 
-  for (int64_t batch = blockIdx.x; batch < n_batches; batch += gridDim.x) {
-    const int64_t v0 = batch * kCombHeads;
-    const int nh = (int)min((int64_t)kCombHeads, n_vec - v0);
-    if (d < kCombHeads) {
-      const int64_t v = v0 + d;
-      const int r = d < nh ? (int)(v / a.Hq) : 0;
-      s_row[d] = r;
-      s_head[d] = d < nh ? (int)(v - (int64_t)r * a.Hq) : 0;
-      // partials of row r: sparse = slot-major list [p0, p0 + np), dense = index w * rows + r
-      s_p0[d] = sparse ? (long long)a.slot_base[r] * a.TPC : (long long)r;
-      s_np[d] = d >= nh ? 0 : (sparse ? (a.slot_base[r + 1] - a.slot_base[r]) * a.TPC : a.world);
-      s_m[d] = -CUDART_INF_F;
-      s_l[d] = 0.f;
-    }
-    __syncthreads();
-    int np = 0;
+  for (int v0 = (int)(blockIdx.x / C::NSPLIT) * VB; v0 < n_vec; v0 += (int)(gridDim.x / C::NSPLIT) * VB) {
+    // ---- merge ------------------------------------------------------------------------------------
+    {
+      const int v = warp / WPV, sub = warp % WPV, vec = v0 + v;
+      float M = -CUDART_INF_F, L = 0.f;
+      float o[R][4];
 #pragma unroll
-    for (int hh = 0; hh < kCombHeads; ++hh) np = max(np, s_np[hh]);
-    auto pidx = [&](int hh, int i) -> int64_t {
-      return sparse ? (int64_t)s_p0[hh] + i : (int64_t)i * a.rows + s_p0[hh];
-    };
-    const float* po[kCombHeads];  // this thread's element of partial 0 of each vector
+      for (int r = 0; r < R; ++r) o[r][0] = o[r][1] = o[r][2] = o[r][3] = 0.f;
+      if (vec < n_vec) {
+        const int row = vec / a.Hq, head = vec - row * a.Hq;
+        const int p0 = sparse ? a.slot_base[row] * a.TPC : 0;
+        const int np = sparse ? a.slot_base[row + 1] * a.TPC - p0 : a.world;
+        const int64_t first = (sparse ? (int64_t)p0 * a.Hq : (int64_t)row * a.Hq) + head + (int64_t)sub * pstride;
+        const int nk = np > sub ? (np - sub + WPV - 1) / WPV : 0;  // partials of this warp
+        for (int k0 = 0; k0 < nk; k0 += 32) {
+          const int kk = min(32, nk - k0);
+          float m = -CUDART_INF_F, l = 0.f;
+          if (lane < kk) {
+            const int64_t idx = first + (int64_t)(k0 + lane) * WPV * pstride;
+            m = __ldg(a.part_m + idx) * mscale;
+            l = sparse ? __ldg(a.part_l + idx) : 1.f;
+          }
+          const float M2 = fmaxf(M, warp_max(m));
+          const float m_use = M2 == -CUDART_INF_F ? 0.f : M2;
+          const float resc = exp2f(M - m_use);   // (0 the first time)
+          const float w = exp2f(m - m_use);      // 0 for empty partials
+          L = L * resc + warp_sum(w * l);
+          M = M2;
 #pragma unroll
-    for (int hh = 0; hh < kCombHeads; ++hh)
-      po[hh] = a.part_o + ((int64_t)s_p0[hh] * a.Hq + s_head[hh]) * D + d;
-
-    if (np <= kCombFastParts) {
-      // ---- every load of the batch in flight at once --------------------------------------------
-      float ov[kCombHeads][kCombFastParts];
+          for (int r = 0; r < R; ++r)
 #pragma unroll
-      for (int hh = 0; hh < kCombHeads; ++hh)
+            for (int e = 0; e < 4; ++e) o[r][e] *= resc;
+          const float* po = a.part_o + (first + (int64_t)k0 * WPV * pstride) * D + 4 * lane;
+          for (int k = 0; k < kk; k += 8) {  // eight partials in flight
+            float4 x[8][R];
+            float wk[8];
 #pragma unroll
-        for (int i = 0; i < kCombFastParts; ++i)
-          ov[hh][i] = i < s_np[hh] ? __ldg(po[hh] + (int64_t)i * pstride) : 0.f;
-      if (d < kCombHeads * kCombFastParts) {
-        const int i = d / kCombHeads, hh = d - i * kCombHeads;
-        const bool valid = i < s_np[hh];
-        const int64_t idx = valid ? pidx(hh, i) * a.Hq + s_head[hh] : 0;
-        s_w[d] = valid ? __ldg(a.part_m + idx) * mscale : -CUDART_INF_F;              // [i][hh]
-        s_w[kCombHeads * kCombFastParts + d] = valid ? (sparse ? __ldg(a.part_l + idx) : 1.f) : 0.f;
+            for (int u = 0; u < 8; ++u) {
+              wk[u] = __shfl_sync(0xffffffffu, w, (k + u) & 31);
+              const bool use = k + u < kk && wk[u] > 0.f;  // (an empty partial's accumulator is never read)
+#pragma unroll
+              for (int r = 0; r < R; ++r) {
+                x[u][r] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (use && 4 * lane + 128 * r < D)
+                  x[u][r] = __ldg(reinterpret_cast<const float4*>(po + (int64_t)(k + u) * WPV * pstride * D + 128 * r));
+              }
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+#pragma unroll
+              for (int r = 0; r < R; ++r) {
+                o[r][0] = fmaf(x[u][r].x, wk[u], o[r][0]);
+                o[r][1] = fmaf(x[u][r].y, wk[u], o[r][1]);
+                o[r][2] = fmaf(x[u][r].z, wk[u], o[r][2]);
+                o[r][3] = fmaf(x[u][r].w, wk[u], o[r][3]);
+              }
+          }
+        }
       }
-      __syncthreads();
-      float res[kCombHeads];
+      if (WPV > 1) {
+        if (lane == 0) { s_m[warp] = M; s_l[warp] = L; }
 #pragma unroll
-      for (int hh = 0; hh < kCombHeads; ++hh) {
-        float M = -CUDART_INF_F;
+        for (int r = 0; r < R; ++r)
+          if (4 * lane + 128 * r < D)
+            *reinterpret_cast<float4*>(s_red + warp * D + 4 * lane + 128 * r) = make_float4(o[r][0], o[r][1], o[r][2], o[r][3]);
+        __syncthreads();
+        M = -CUDART_INF_F;
+        L = 0.f;
 #pragma unroll
-        for (int i = 0; i < kCombFastParts; ++i) M = fmaxf(M, s_w[i * kCombHeads + hh]);
+        for (int u = 0; u < WPV; ++u) M = fmaxf(M, s_m[v * WPV + u]);
         const float m_use = M == -CUDART_INF_F ? 0.f : M;
-        float L = 0.f, o = 0.f;
+        float wu[WPV];
 #pragma unroll
-        for (int i = 0; i < kCombFastParts; ++i) {
-          const float w = exp2f(s_w[i * kCombHeads + hh] - m_use);  // 0 for empty partials
-          L = fmaf(s_w[kCombHeads * kCombFastParts + i * kCombHeads + hh], w, L);
-          o = fmaf(ov[hh][i], w, o);
+        for (int u = 0; u < WPV; ++u) {
+          wu[u] = exp2f(s_m[v * WPV + u] - m_use);
+          L = fmaf(s_l[v * WPV + u], wu[u], L);
         }
-        res[hh] = (hh < nh && L > 0.f) ? o / L : 0.f;
-        if (d == hh && hh < nh && a.lse_out)
-          a.lse_out[(int64_t)(s_row[hh] + a.row_offset) * a.Hq + s_head[hh]] =
-              L > 0.f ? (M + log2f(L)) * kLn2 : -CUDART_INF_F;
+        const float inv = L > 0.f ? 1.f / L : 0.f;
+        // the warps of a vector share its coordinates
+        for (int d = sub * 32 + lane; d < D; d += 32 * WPV) {
+          float x = 0.f;
+#pragma unroll
+          for (int u = 0; u < WPV; ++u) x = fmaf(s_red[(v * WPV + u) * D + d], wu[u], x);
+          s_x[v * C::XP + d] = x * inv;
+        }
+      } else {
+        const float inv = L > 0.f ? 1.f / L : 0.f;
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+          if (4 * lane + 128 * r < D)
+            *reinterpret_cast<float4*>(s_x + v * C::XP + 4 * lane + 128 * r) =
+                make_float4(o[r][0] * inv, o[r][1] * inv, o[r][2] * inv, o[r][3] * inv);
       }
-      float4* so4 = reinterpret_cast<float4*>(s_o + d * kCombHeads);  // s_o is [D][8 vectors]
-      so4[0] = make_float4(res[0], res[1], res[2], res[3]);
-      so4[1] = make_float4(res[4], res[5], res[6], res[7]);
-    } else {
-      float o[kCombHeads];
-#pragma unroll
-      for (int hh = 0; hh < kCombHeads; ++hh) o[hh] = 0.f;
-      for (int c0 = 0; c0 < np; c0 += kCombMaxParts) {
-        const int nc = min(kCombMaxParts, np - c0);
-        __syncthreads();
-        for (int t = d; t < nc * kCombHeads; t += D) {  // (partial, vector) -> log2-domain maximum
-          const int i = t / kCombHeads, hh = t - i * kCombHeads;
-          s_w[t] = c0 + i < s_np[hh] ? __ldg(a.part_m + pidx(hh, c0 + i) * a.Hq + s_head[hh]) * mscale
-                                     : -CUDART_INF_F;
-        }
-        __syncthreads();
-        if (d < kCombHeads) {  // new running max of vector d; rescale what was accumulated so far
-          float M = s_m[d];
-          for (int i = 0; i < nc; ++i) M = fmaxf(M, s_w[i * kCombHeads + d]);
-          const float m_use = M == -CUDART_INF_F ? 0.f : M;
-          const float resc = s_m[d] == -CUDART_INF_F ? 0.f : exp2f(s_m[d] - m_use);
-          s_l[d] *= resc;
-          s_o[d] = resc;  // s_o[0..7] publishes the rescale factors
-          s_m[d] = M;
-        }
-        __syncthreads();
-#pragma unroll
-        for (int hh = 0; hh < kCombHeads; ++hh) o[hh] *= s_o[hh];
-        __syncthreads();
-        for (int t = d; t < nc * kCombHeads; t += D) {
-          const int hh = t % kCombHeads;
-          const float M = s_m[hh];
-          s_w[t] = exp2f(s_w[t] - (M == -CUDART_INF_F ? 0.f : M));  // 0 for empty partials
-        }
-        __syncthreads();
-        if (d < nh) {  // running sum of vector d
-          float L = s_l[d];
-          for (int i = 0; i < nc; ++i) {
-            const float w = s_w[i * kCombHeads + d];
-            if (w > 0.f) L = fmaf(sparse ? __ldg(a.part_l + pidx(d, c0 + i) * a.Hq + s_head[d]) : 1.f, w, L);
-          }
-          s_l[d] = L;
-        }
-#pragma unroll 8
-        for (int i = 0; i < nc; ++i) {  // accumulate: independent loads, eight partials (64 loads) in flight
-#pragma unroll
-          for (int hh = 0; hh < kCombHeads; ++hh) {
-            const float w = s_w[i * kCombHeads + hh];
-            if (w > 0.f) o[hh] = fmaf(__ldg(po[hh] + (int64_t)(c0 + i) * pstride), w, o[hh]);
-          }
-        }
-      }
-      __syncthreads();
-#pragma unroll
-      for (int hh = 0; hh < kCombHeads; ++hh) {
-        const float L = s_l[hh];
-        o[hh] = (hh < nh && L > 0.f) ? o[hh] / L : 0.f;
-      }
-      float4* so4 = reinterpret_cast<float4*>(s_o + d * kCombHeads);
-      so4[0] = make_float4(o[0], o[1], o[2], o[3]);
-      so4[1] = make_float4(o[4], o[5], o[6], o[7]);
-      if (d < nh && a.lse_out) {
-        const float L = s_l[d], M = s_m[d];
-        a.lse_out[(int64_t)(s_row[d] + a.row_offset) * a.Hq + s_head[d]] =
-            L > 0.f ? (M + log2f(L)) * kLn2 : -CUDART_INF_F;
-      }
+      if (a.lse_out && split == 0 && sub == 0 && lane == 0 && vec < n_vec)
+        a.lse_out[(int64_t)a.row_offset * a.Hq + vec] =
+            L > 0.f ? (M + log2f(L)) * 0.6931471805599453f : -CUDART_INF_F;
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
-    float acc[kCombHeads];
-    if (a.out_rotated) {
+    // ---- un-rotate --------------------------------------------------------------------------------
+    if (!a.out_rotated) {
+      const int unit = warp * C::UPW + lane / C::LC, cl = lane % C::LC;
+      const int vg = unit % C::NVG, jp = unit / C::NVG;
+      if (jp < C::JP) {  // (D = 96: lanes 24 .. 31 idle)
+        float acc[C::VPT][4];
 #pragma unroll
-      for (int hh = 0; hh < kCombHeads; ++hh) acc[hh] = s_o[d * kCombHeads + hh];
-    } else {
+        for (int v = 0; v < C::VPT; ++v) acc[v][0] = acc[v][1] = acc[v][2] = acc[v][3] = 0.f;
+        const float4* xp = reinterpret_cast<const float4*>(s_x + vg * C::VPT * C::XP + jp * C::JN);
+        const float4* pp = reinterpret_cast<const float4*>(s_pi + (size_t)jp * C::JN * C::DC) + cl;
+#pragma unroll 2
+        for (int j4 = 0; j4 < C::JN / 4; ++j4) {
+          float4 x[C::VPT];
 #pragma unroll
-      for (int hh = 0; hh < kCombHeads; ++hh) acc[hh] = 0.f;
-      if (kStagePi) {
-#pragma unroll 8
-        for (int j = 0; j < D; ++j) {
-          const float pv = s_pi[j * D + d];
-          const float4 oa = *reinterpret_cast<const float4*>(s_o + j * kCombHeads);
-          const float4 ob = *reinterpret_cast<const float4*>(s_o + j * kCombHeads + 4);
-          acc[0] = fmaf(oa.x, pv, acc[0]); acc[1] = fmaf(oa.y, pv, acc[1]);
-          acc[2] = fmaf(oa.z, pv, acc[2]); acc[3] = fmaf(oa.w, pv, acc[3]);
-          acc[4] = fmaf(ob.x, pv, acc[4]); acc[5] = fmaf(ob.y, pv, acc[5]);
-          acc[6] = fmaf(ob.z, pv, acc[6]); acc[7] = fmaf(ob.w, pv, acc[7]);
+          for (int v = 0; v < C::VPT; ++v) x[v] = xp[v * (C::XP / 4) + j4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float4 p = pp[(4 * j4 + e) * C::LC];
+#pragma unroll
+            for (int v = 0; v < C::VPT; ++v) {
+              const float xe = e == 0 ? x[v].x : e == 1 ? x[v].y : e == 2 ? x[v].z : x[v].w;
+              acc[v][0] = fmaf(xe, p.x, acc[v][0]);
+              acc[v][1] = fmaf(xe, p.y, acc[v][1]);
+              acc[v][2] = fmaf(xe, p.z, acc[v][2]);
+              acc[v][3] = fmaf(xe, p.w, acc[v][3]);
+            }
+          }
         }
+        if (lane < C::UPW * C::LC)
+#pragma unroll
+          for (int v = 0; v < C::VPT; ++v)
+            *reinterpret_cast<float4*>(s_red + ((size_t)jp * VB + vg * C::VPT + v) * C::DC + 4 * cl) =
+                make_float4(acc[v][0], acc[v][1], acc[v][2], acc[v][3]);
+      }
+      __syncthreads();
+    }
+    // ---- sum the parts, cast, store ---------------------------------------------------------------
+    for (int i = tid; i < VB * C::LC; i += 256) {
+      const int v = i / C::LC, c = 4 * (i - v * C::LC), vec = v0 + v;
+      if (vec >= n_vec) continue;
+      float y[4] = {0.f, 0.f, 0.f, 0.f};
+      if (a.out_rotated) {
+        const float4 t = *reinterpret_cast<const float4*>(s_x + v * C::XP + split * C::DC + c);
+        y[0] = t.x; y[1] = t.y; y[2] = t.z; y[3] = t.w;
       } else {
-        for (int j0 = 0; j0 < D; j0 += 16) {  // column d of Pi from L2, 16 loads in flight
-          float pv[16];
 #pragma unroll
-          for (int u = 0; u < 16; ++u) pv[u] = __ldg(a.rotation + (size_t)(j0 + u) * D + d);
-#pragma unroll
-          for (int u = 0; u < 16; ++u)
-#pragma unroll
-            for (int hh = 0; hh < kCombHeads; ++hh)
-              acc[hh] = fmaf(s_o[(j0 + u) * kCombHeads + hh], pv[u], acc[hh]);
+        for (int jp = 0; jp < C::JP; ++jp) {
+          const float4 t = *reinterpret_cast<const float4*>(s_red + ((size_t)jp * VB + v) * C::DC + c);
+          y[0] += t.x; y[1] += t.y; y[2] += t.z; y[3] += t.w;
         }
       }
+      const int row = vec / a.Hq, head = vec - row * a.Hq;
+      store4(a.out, a.out_dtype, (int64_t)(row + a.row_offset) * a.out_token_stride + (int64_t)head * a.out_head_stride +
+                                     split * C::DC + c, y);
     }
-#pragma unroll
-    for (int hh = 0; hh < kCombHeads; ++hh)
-      if (hh < nh)
-        store_from_float(a.out, a.out_dtype,
-                         (int64_t)(s_row[hh] + a.row_offset) * a.out_token_stride +
-                             (int64_t)s_head[hh] * a.out_head_stride + d,
-                         acc[hh]);
-    __syncthreads();  // s_o, s_w and the per-vector entries are rewritten by the next batch
+    __syncthreads();  // s_x and s_red are rewritten by the next pass
   }
 }
 
-template <int D>
-int launch_combine_t(const CombineArgs& c, cudaStream_t st, bool pdl) {
-  constexpr size_t smem = ((size_t)(D <= 128 ? D * D : 0) + kCombHeads * D +
-                           kCombMaxParts * kCombHeads + 2 * kCombHeads) * sizeof(float);
+template <int D, int WPV>
+int launch_combine_w(const CombineArgs& c, cudaStream_t st, bool pdl) {
+  using C = CombineCfg<D, WPV>;
   // (same shared-memory carve-out as the attention kernel it follows: no reconfiguration between them)
-  if (!ensure_dynamic_smem<combine_kernel<D>>((int)smem, true)) return TQ4_ERR_CUDA;
-  const int64_t n_vec = (int64_t)c.rows * c.Hq;
-  int64_t grid = (n_vec + kCombHeads - 1) / kCombHeads;
-  if (grid > 3 * (int64_t)sm_count()) grid = 3 * (int64_t)sm_count();
-  if (launch_kernel(combine_kernel<D>, dim3((unsigned)grid), dim3(D), smem, st, pdl, c) != cudaSuccess)
+  if (!ensure_dynamic_smem<combine_kernel<D, WPV>>((int)C::kSmem, true)) return TQ4_ERR_CUDA;
+  const int64_t passes = ((int64_t)c.rows * c.Hq + C::VB - 1) / C::VB;
+  const int64_t most = 2 * (int64_t)sm_count() / C::NSPLIT;
+  if (launch_kernel(combine_kernel<D, WPV>, dim3((unsigned)((passes < most ? passes : most) * C::NSPLIT)), dim3(256),
+                    C::kSmem, st, pdl, c) != cudaSuccess)
     return TQ4_ERR_CUDA;
   TQ4_CHECK_LAUNCH();
   return TQ4_OK;
+}
+
+// Warps per vector: as many as leave every vector a block of its own in one wave of two blocks per SM
+// (the partials of a vector are then read in one round trip), fewer when the vectors fill the GPU anyway.
+template <int D>
+int launch_combine_t(const CombineArgs& c, cudaStream_t st, bool pdl) {
+  const int64_t n_vec = (int64_t)c.rows * c.Hq, wave = 2 * (int64_t)sm_count() / (D == 256 ? 4 : 1);
+  if (n_vec <= wave) return launch_combine_w<D, 8>(c, st, pdl);
+  if (n_vec <= 4 * wave) return launch_combine_w<D, 2>(c, st, pdl);
+  return launch_combine_w<D, 1>(c, st, pdl);
 }
 
 // pdl: the launch follows another kernel of the same entry point (false for the stand-alone merge,

@@ -106,6 +106,28 @@ __device__ __forceinline__ void store_from_float(void* p, int dtype, int64_t i, 
   else if (dtype == TQ4_F16) reinterpret_cast<__half*>(p)[i] = __float2half_rn(v);
   else reinterpret_cast<__nv_bfloat16*>(p)[i] = __float2bfloat16_rn(v);
 }
+// four consecutive elements i .. i + 3: one store where the address allows it
+__device__ __forceinline__ void store4(void* p, int dtype, int64_t i, const float (&v)[4]) {
+  if (dtype == TQ4_F32) {
+    float* d = reinterpret_cast<float*>(p) + i;
+    if (((uintptr_t)d & 15) == 0) {
+      *reinterpret_cast<float4*>(d) = make_float4(v[0], v[1], v[2], v[3]);
+    } else {
+      d[0] = v[0]; d[1] = v[1]; d[2] = v[2]; d[3] = v[3];
+    }
+    return;
+  }
+  uint16_t h[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e)
+    h[e] = dtype == TQ4_F16 ? __half_as_ushort(__float2half_rn(v[e])) : __bfloat16_as_ushort(__float2bfloat16_rn(v[e]));
+  uint16_t* d = reinterpret_cast<uint16_t*>(p) + i;
+  if (((uintptr_t)d & 7) == 0) {
+    *reinterpret_cast<uint2*>(d) = make_uint2(h[0] | ((uint32_t)h[1] << 16), h[2] | ((uint32_t)h[3] << 16));
+  } else {
+    d[0] = h[0]; d[1] = h[1]; d[2] = h[2]; d[3] = h[3];
+  }
+}
 
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
