@@ -188,23 +188,21 @@ int tq4_paged_attention(const void* q, int q_dtype, int64_t num_rows, int num_se
 
 /*
  * One decode step of a layer: tq4_write_paged of the new tokens followed by tq4_paged_attention,
- * with the cache write folded into the attention's first kernel, so the step costs two or three
- * launches instead of four.  Arguments are the union of the two calls
+ * with the cache write folded into the attention's first kernel, so the step costs three launches
+ * instead of four.  Arguments are the union of the two calls
  * (same meaning and checks); the cache must be block-major contiguous
  * (cache_block_stride == block_size * cache_token_stride), which makes the flat slot
  * s = block * block_size + offset of slot_mapping address row s at cache + s * cache_token_stride.
  * n_tokens == 0 reduces to tq4_paged_attention, num_rows == 0 to tq4_write_paged.
- * Decode calls (query_start_loc == NULL) of up to 512 rows at head_dim <= 128 with more than 512
- * (row, KV head) pairs run as TWO launches (smaller ones too with TQ4_FUSED_PROLOGUE=1 in the
- * environment; =0 turns the form off): the
- * attention kernel plans its tiles, rotates the queries and compresses the new tokens itself, then
+ * With TQ4_FUSED_PROLOGUE=1 in the environment, decode calls (query_start_loc == NULL) of up to 512
+ * rows at head_dim <= 128 run as TWO launches: the attention kernel plans its tiles, rotates the queries and compresses the new tokens itself, then
  * the merge kernel.  There token i must be the newest token of sequence i, i.e.
  * slot_mapping[i] addresses position seq_lens[i] - 1 through block_table (what a decode step of a
  * serving engine passes): the CTA that reads a sequence's last tile is the one that writes the
  * token into it.  A token whose slot is elsewhere is still written, and TQ4_DEV_WRITE_ORDER is
  * raised because this call's attention may have read that slot before the write; a token of a
- * sequence with seq_lens[i] == 0 must have a negative slot.  Other calls (chunked prefill, more
- * rows, head_dim 256) run the write kernel first, then prologue, attention and merge.
+ * sequence with seq_lens[i] == 0 must have a negative slot.  Writes of more than 8192 vectors run as
+ * their own kernel first.
  * Replaces: the body of TQ4AttentionImpl.forward for a decode batch,
  *           src/turboquant_vllm/vllm/tq4_backend.py (_compress_and_store + _fused_decode_path).
  */

@@ -133,6 +133,9 @@ __device__ void build_plan(const AttnArgs& a, int* s_work) {
     p.tile_prefix[r] = s_tiles[r];
     p.slot_base[r] = run;
     run += s_slots[r];
+    // the spans whose first tile is one of this row's
+    const int b = s_tiles[r], e = r + 1 < rows ? s_tiles[r + 1] : total;
+    for (int s = (b + tps - 1) / tps; s * tps < e; ++s) p.span_row[s] = r;
   }
   if (threadIdx.x == 0) {
     p.tile_prefix[rows] = total;
@@ -142,150 +145,49 @@ __device__ void build_plan(const AttnArgs& a, int* s_work) {
   }
 }
 
-template <int D>
-struct QrotCfg {
-  static constexpr int DC = D < 128 ? D : 128;          // columns of Pi staged per pass
-  static constexpr int G = 256 / D >= 1 ? 256 / D : 1;  // thread groups (one output column each)
-  static constexpr int VPG = 4;                         // vectors per group (small: many blocks)
-  static constexpr int VB = G * VPG;                    // (row, head) vectors per block
-  static constexpr int THREADS = G * D;
-  static constexpr size_t rot_bytes = ((size_t)D * (DC + 1) + (size_t)D * VB) * sizeof(float);
-  static constexpr size_t plan_bytes = 2 * (size_t)kMaxRowsPerLaunch * sizeof(int);  // planning block
-  static constexpr size_t smem_bytes = rot_bytes > plan_bytes ? rot_bytes : plan_bytes;
-};
-
-// q_rot[v][j] = sum_d q[v][d] * Pi[j][d].  Pi is staged once per block, transposed into a padded
-// shared array so that thread j walks its own row without bank conflicts; the block's vectors sit
-// in shared memory as [d][v] (swizzled) so that one 16-byte broadcast load feeds four FMAs.
-template <int D>
-__global__ void __launch_bounds__(QrotCfg<D>::THREADS) qrot_plan_kernel(const AttnArgs a) {
-  using Q = QrotCfg<D>;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  pdl_trigger();
-  if (blockIdx.x == gridDim.x - 1) {  // the planning block
-    build_plan(a, reinterpret_cast<int*>(smem_raw));
-    return;
-  }
-  constexpr int DC = Q::DC, VB = Q::VB, VPG = Q::VPG, PITCH = DC + 1;
-  float* s_pi = reinterpret_cast<float*>(smem_raw);  // [D][DC + 1]
-  float* s_q = s_pi + D * PITCH;                     // [D][VB], v swizzled by d
-  const AttnShape& sh = a.sh;
-  const int64_t n_vec = (int64_t)sh.rows * sh.Hq;
-  const int64_t v0 = (int64_t)blockIdx.x * VB;
-  const int tid = threadIdx.x, grp = tid / D, j = tid - grp * D;
-  auto swz = [](int d) { return ((d & 7) << 2) & (VB - 1); };
-
-  // the block's vectors (coalesced over d), converted to fp32
-  for (int i0 = 0; i0 < VB * D; i0 += Q::THREADS * 8) {
-    float x[8];
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int i = i0 + u * Q::THREADS + tid;
-      const int v = i / D, d = i - v * D;
-      const int64_t vec = v0 + v;
-      x[u] = 0.f;
-      if (i < VB * D && vec < n_vec) {
-        const int64_t row = vec / sh.Hq + sh.row_offset;
-        const int h = (int)(vec % sh.Hq);
-        x[u] = load_as_float(a.q, a.q_dtype, row * a.q_token_stride + h * a.q_head_stride + d);
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int i = i0 + u * Q::THREADS + tid;
-      const int v = i / D, d = i - v * D;
-      if (i < VB * D) s_q[d * VB + (v ^ swz(d))] = x[u];
-    }
-  }
-
-  float acc[VPG];
-#pragma unroll
-  for (int v = 0; v < VPG; ++v) acc[v] = 0.f;
-  for (int d0 = 0; d0 < D; d0 += DC) {
-    __syncthreads();
-    // stage Pi[:, d0 : d0 + DC] with 16-byte loads, eight in flight per thread
-    constexpr int N4 = D * DC / 4;
-    for (int i0 = 0; i0 < N4; i0 += Q::THREADS * 8) {
-      float4 x[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int i = i0 + u * Q::THREADS + tid;
-        if (i < N4) {
-          const int jj = i / (DC / 4), c4 = i - jj * (DC / 4);
-          x[u] = __ldg(reinterpret_cast<const float4*>(a.rotation + (size_t)jj * D + d0) + c4);
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < 8; ++u) {
-        const int i = i0 + u * Q::THREADS + tid;
-        if (i < N4) {
-          const int jj = i / (DC / 4), c4 = i - jj * (DC / 4);
-          float* dst = s_pi + jj * PITCH + 4 * c4;
-          dst[0] = x[u].x; dst[1] = x[u].y; dst[2] = x[u].z; dst[3] = x[u].w;
-        }
-      }
-    }
-    __syncthreads();
-#pragma unroll 4
-    for (int dd = 0; dd < DC; ++dd) {
-      const float pv = s_pi[j * PITCH + dd];
-      const int d = d0 + dd;
-      const float* qrow = s_q + d * VB;
-#pragma unroll
-      for (int v4 = 0; v4 < VPG / 4; ++v4) {
-        const float4 qv = *reinterpret_cast<const float4*>(qrow + ((grp * VPG + 4 * v4) ^ swz(d)));
-        acc[4 * v4] = fmaf(qv.x, pv, acc[4 * v4]);
-        acc[4 * v4 + 1] = fmaf(qv.y, pv, acc[4 * v4 + 1]);
-        acc[4 * v4 + 2] = fmaf(qv.z, pv, acc[4 * v4 + 2]);
-        acc[4 * v4 + 3] = fmaf(qv.w, pv, acc[4 * v4 + 3]);
-      }
-    }
-  }
-  pdl_wait();  // the scratch may still be read by the attention kernel of the previous call
-#pragma unroll
-  for (int v = 0; v < VPG; ++v) {
-    const int64_t vec = v0 + grp * VPG + v;
-    if (vec < n_vec) a.plan.q_rot[vec * D + j] = acc[v];
-  }
-}
-
 // --------------------------------------------------------------------------------------
-// Fused prologue (head_dim <= 128): ONE launch rotates every query vector of the call and, when
-// the call carries new tokens, compresses their K and V vectors into the paged cache; an extra
-// block builds the tile plan.  Pi^T is staged once per block into shared memory ([d][j]); one WARP
-// handles four vectors at a time as a 4 x D strip of the product X * Pi^T, each lane a 4 x 4
-// register tile (four vectors x four consecutive output coordinates), so a step of the reduction
-// is two 16-byte shared loads and 16 FMAs, and nothing but warp-level synchronisation is needed.
+// Prologue: ONE launch rotates every query vector of the call and, when the call carries a few new
+// tokens, compresses their K and V vectors into the paged cache; block 0 builds the tile plan.  A
+// block owns JC output coordinates: its slice of Pi^T sits in shared memory ([d][j]), one WARP takes
+// four vectors at a time, and a lane owns NJ consecutive outputs of each, so a step of the reduction
+// is one broadcast load of the four vectors' elements and one load of NJ entries of Pi for 4 NJ FMAs.
+//
+// Latency bound: a decode step waits for this kernel, which is a chain of load Pi, load vectors,
+// reduce, store.  While the vectors do not fill the GPU a block therefore takes 32 of the coordinates
+// (head_dim 128: 16 KB of Pi to fetch and transpose instead of 64, four times the blocks; kernel time at
+// batch 1 11.5 -> 7.8 us, at batch 16 13.4 -> 8.6 us); with many vectors it takes all of them (fewer
+// shared-memory reads per FMA).
 //
 // The write part keeps the arithmetic contract of the compress kernels bit for bit
 // (tq4_compress.cu): squared norm by lane-strided FMAs + butterfly reduction, IEEE division by
 // (norm + 1e-10), four quarter-length FMA chains in ascending k combined as (s0 + s1) + (s2 + s3).
 // --------------------------------------------------------------------------------------
-template <int D>
+template <int D, int JC>
 struct PrologueCfg {
   static constexpr int WARPS = 8;
   static constexpr int THREADS = WARPS * 32;
-  static constexpr int VC = 4;            // vectors per warp per pass
-  static constexpr size_t rot_bytes = ((size_t)D * D + (size_t)WARPS * D * VC) * sizeof(float);
-  static constexpr size_t plan_bytes = 2 * (size_t)kMaxRowsPerLaunch * sizeof(int);
-  static constexpr size_t smem_bytes = rot_bytes > plan_bytes ? rot_bytes : plan_bytes;
+  static constexpr int VC = 4;                          // vectors per warp per pass
+  static constexpr int NJ = JC == 96 ? 4 : JC / 32;     // outputs per lane (JC = 96: lanes 24 .. 31 idle)
+  static constexpr int NSPLIT = D / JC;
+  static constexpr size_t rot_bytes = ((size_t)D * JC + (size_t)WARPS * D * VC) * sizeof(float);
 };
 
-template <int D>
-__global__ void __launch_bounds__(PrologueCfg<D>::THREADS)
+template <int D, int JC>
+__global__ void __launch_bounds__(256)
 prologue_kernel(const AttnArgs a, const CompressArgs w, const int has_attn, const int has_write) {
-  using P = PrologueCfg<D>;
-  constexpr int VC = P::VC, HALF = D / 2, KQ = D / 4, XPL = D / 32;
-  static_assert(D % 32 == 0 && D <= 128 && KQ % 8 == 0, "head_dim must be a multiple of 32, at most 128");
+  using P = PrologueCfg<D, JC>;
+  constexpr int VC = P::VC, NJ = P::NJ, HALF = D / 2, KQ = D / 4, XPL = D / 32;
+  static_assert(D % 32 == 0 && KQ % 8 == 0 && D % JC == 0, "head_dim and column block must be multiples of 32");
   extern __shared__ __align__(16) unsigned char smem_raw[];
   pdl_trigger();
-  if (has_attn && blockIdx.x == gridDim.x - 1) {  // the planning block
+  if (has_attn && blockIdx.x == 0) {  // the planning block
     build_plan(a, reinterpret_cast<int*>(smem_raw));
     return;
   }
-  const int n_rot_blocks = (int)gridDim.x - (has_attn ? 1 : 0);
-  float* s_pit = reinterpret_cast<float*>(smem_raw);                    // [D][D]: s_pit[d][j] = Pi[j][d]
-  float4* s_x = reinterpret_cast<float4*>(s_pit + D * D);               // [WARPS][D] four vectors per entry
+  const int bid = (int)blockIdx.x - (has_attn ? 1 : 0), n_blocks = ((int)gridDim.x - (has_attn ? 1 : 0)) / P::NSPLIT;
+  const int j0 = (bid % P::NSPLIT) * JC;
+  float* s_pit = reinterpret_cast<float*>(smem_raw);                    // [D][JC]: s_pit[d][j] = Pi[j0 + j][d]
+  float4* s_x = reinterpret_cast<float4*>(s_pit + D * JC);              // [WARPS][D] four vectors per entry
   __shared__ float s_bounds[2][16];  // sorted boundaries of K and V, padded with +inf
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (has_write && tid < 32) {
@@ -293,33 +195,33 @@ prologue_kernel(const AttnArgs a, const CompressArgs w, const int has_attn, cons
     s_bounds[src][i] = (src < w.n_sources && i < w.n_bounds[src]) ? w.bounds[src][i] : CUDART_INF_F;
   }
 
-  // ---- stage Pi^T ------------------------------------------------------------------------------
+  // ---- stage the slice of Pi^T --------------------------------------------------------------------
   if (has_attn) {
     // thread -> (4 consecutive d of row j), consecutive threads = consecutive j: conflict-free stores
-    constexpr int N4 = D * D / 4;
-    for (int i0 = 0; i0 < N4; i0 += P::THREADS * 8) {
-      float4 x[8];
+    constexpr int N4 = D * JC / 4, NB = N4 / P::THREADS < 8 ? (N4 + P::THREADS - 1) / P::THREADS : 8;
+    for (int i0 = 0; i0 < N4; i0 += P::THREADS * NB) {
+      float4 x[NB];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
+      for (int u = 0; u < NB; ++u) {
         const int i = i0 + u * P::THREADS + tid;
-        const int c4 = i / D, jj = i - c4 * D;
-        if (i < N4) x[u] = __ldg(reinterpret_cast<const float4*>(a.rotation + (size_t)jj * D) + c4);
+        const int c4 = i / JC, jj = i - c4 * JC;
+        if (i < N4) x[u] = __ldg(reinterpret_cast<const float4*>(a.rotation + (size_t)(j0 + jj) * D) + c4);
       }
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
+      for (int u = 0; u < NB; ++u) {
         const int i = i0 + u * P::THREADS + tid;
-        const int c4 = i / D, jj = i - c4 * D;
+        const int c4 = i / JC, jj = i - c4 * JC;
         if (i < N4) {
-          float* dst = s_pit + (4 * c4) * D + jj;
-          dst[0] = x[u].x; dst[D] = x[u].y; dst[2 * D] = x[u].z; dst[3 * D] = x[u].w;
+          float* dst = s_pit + (4 * c4) * JC + jj;
+          dst[0] = x[u].x; dst[JC] = x[u].y; dst[2 * JC] = x[u].z; dst[3 * JC] = x[u].w;
         }
       }
     }
   } else {  // write only: the caller gave Pi^T split into even / odd output columns
-    for (int i = tid; i < D * HALF; i += P::THREADS) {
-      const int k = i / HALF, pp = i - k * HALF;
-      s_pit[k * D + 2 * pp] = __ldg(w.rot_even + i);
-      s_pit[k * D + 2 * pp + 1] = __ldg(w.rot_odd + i);
+    for (int i = tid; i < D * JC / 2; i += P::THREADS) {
+      const int k = i / (JC / 2), pp = i - k * (JC / 2);
+      s_pit[k * JC + 2 * pp] = __ldg(w.rot_even + k * HALF + j0 / 2 + pp);
+      s_pit[k * JC + 2 * pp + 1] = __ldg(w.rot_odd + k * HALF + j0 / 2 + pp);
     }
   }
   __syncthreads();
@@ -330,8 +232,8 @@ prologue_kernel(const AttnArgs a, const CompressArgs w, const int has_attn, cons
   const int n_w = rows_per_src * (has_write ? w.n_sources : 0);
   const int cq = (n_q + VC - 1) / VC, cw = (n_w + VC - 1) / VC;
   float4* gx = s_x + warp * D;
-  const bool jact = 4 * lane < D;                       // this lane owns outputs 4*lane .. 4*lane+3
-  const float4* pcol = reinterpret_cast<const float4*>(s_pit) + (jact ? lane : 0);  // + d * (D/4)
+  const bool jact = NJ * lane < JC;                     // this lane owns outputs j0 + NJ * lane .. + NJ - 1
+  const float* pcol = s_pit + (jact ? NJ * lane : 0);   // + d * JC
   // (source, token, head) of write vector `vec`
   auto w_coords = [&](int vec, int& src, int& tok, int& h) {
     src = vec >= rows_per_src ? 1 : 0;
@@ -340,7 +242,7 @@ prologue_kernel(const AttnArgs a, const CompressArgs w, const int has_attn, cons
     h = (int)(rem - (unsigned)tok * (unsigned)w.num_heads);
   };
 
-  for (int c = (int)blockIdx.x * P::WARPS + warp; c < cq + cw; c += n_rot_blocks * P::WARPS) {
+  for (int c = (bid / P::NSPLIT) * P::WARPS + warp; c < cq + cw; c += n_blocks * P::WARPS) {
     const bool is_w = c >= cq;
     const int v0 = (is_w ? c - cq : c) * VC;
     const int nv = is_w ? n_w : n_q;
@@ -387,29 +289,31 @@ prologue_kernel(const AttnArgs a, const CompressArgs w, const int has_attn, cons
     for (int i = 0; i < XPL; ++i) gx[lane + 32 * i] = make_float4(xr[i][0], xr[i][1], xr[i][2], xr[i][3]);
     __syncwarp();
 
-    // ---- y[v][4*lane + jj] = sum_d x[v][d] * Pi[4*lane + jj][d] as (s0 + s1) + (s2 + s3): the two
-    // quarter chains of a half advance together (32 independent accumulators); loops stay rolled,
+    // ---- y[v][jj] = sum_d x[v][d] * Pi[j0 + NJ*lane + jj][d] as (s0 + s1) + (s2 + s3): the two
+    // quarter chains of a half advance together (8 NJ independent accumulators); loops stay rolled,
     // a launch of a few thousand vectors runs this code once per warp and pays for its size
-    float y[VC][4];
+    float y[VC][NJ];
 #pragma unroll 1
     for (int hf = 0; hf < 2; ++hf) {
-      float sa[VC][4], sb[VC][4];
+      float sa[VC][NJ], sb[VC][NJ];
 #pragma unroll
       for (int v = 0; v < VC; ++v)
 #pragma unroll
-        for (int jj = 0; jj < 4; ++jj) sa[v][jj] = sb[v][jj] = 0.f;
-      const float4* pa = pcol + (2 * hf) * KQ * (D / 4);
+        for (int jj = 0; jj < NJ; ++jj) sa[v][jj] = sb[v][jj] = 0.f;
+      const float* pa = pcol + (2 * hf) * KQ * JC;
       const float4* xa = gx + (2 * hf) * KQ;
 #pragma unroll 4
       for (int dd = 0; dd < KQ; ++dd) {
-        const float4 p0 = pa[dd * (D / 4)], x0 = xa[dd];
-        const float4 p1 = pa[(KQ + dd) * (D / 4)], x1 = xa[KQ + dd];
-        const float xs0[VC] = {x0.x, x0.y, x0.z, x0.w}, ps0[4] = {p0.x, p0.y, p0.z, p0.w};
-        const float xs1[VC] = {x1.x, x1.y, x1.z, x1.w}, ps1[4] = {p1.x, p1.y, p1.z, p1.w};
+        float ps0[NJ], ps1[NJ];
+        load_n<NJ>(pa + dd * JC, ps0);
+        load_n<NJ>(pa + (KQ + dd) * JC, ps1);
+        const float4 x0 = xa[dd], x1 = xa[KQ + dd];
+        const float xs0[VC] = {x0.x, x0.y, x0.z, x0.w};
+        const float xs1[VC] = {x1.x, x1.y, x1.z, x1.w};
 #pragma unroll
         for (int v = 0; v < VC; ++v)
 #pragma unroll
-          for (int jj = 0; jj < 4; ++jj) {
+          for (int jj = 0; jj < NJ; ++jj) {
             sa[v][jj] = fmaf(xs0[v], ps0[jj], sa[v][jj]);
             sb[v][jj] = fmaf(xs1[v], ps1[jj], sb[v][jj]);
           }
@@ -417,17 +321,14 @@ prologue_kernel(const AttnArgs a, const CompressArgs w, const int has_attn, cons
 #pragma unroll
       for (int v = 0; v < VC; ++v)
 #pragma unroll
-        for (int jj = 0; jj < 4; ++jj)
+        for (int jj = 0; jj < NJ; ++jj)
           y[v][jj] = hf == 0 ? sa[v][jj] + sb[v][jj] : y[v][jj] + (sa[v][jj] + sb[v][jj]);
     }
 
-    pdl_wait();  // nothing before this point wrote global memory
     if (!is_w) {
 #pragma unroll
       for (int v = 0; v < VC; ++v)
-        if (v0 + v < nv && jact)
-          *reinterpret_cast<float4*>(a.plan.q_rot + (int64_t)(v0 + v) * D + 4 * lane) =
-              make_float4(y[v][0], y[v][1], y[v][2], y[v][3]);
+        if (v0 + v < nv && jact) store_n<NJ>(a.plan.q_rot + (int64_t)(v0 + v) * D + j0 + NJ * lane, y[v]);
     } else {
       const RowLayout lay = row_layout(w.num_heads, D);
 #pragma unroll
@@ -437,8 +338,15 @@ prologue_kernel(const AttnArgs a, const CompressArgs w, const int has_attn, cons
         int src, tok, h;
         w_coords(vec, src, tok, h);
         const float* bd = s_bounds[src];
-        const unsigned b0 = (unsigned)((bucketize_sorted16(y[v][0], bd) << 4) | bucketize_sorted16(y[v][1], bd));
-        const unsigned b1 = (unsigned)((bucketize_sorted16(y[v][2], bd) << 4) | bucketize_sorted16(y[v][3], bd));
+        // eight outputs make a word: the lanes that share it OR their nibbles together
+        uint32_t word = 0;
+#pragma unroll
+        for (int jj = 0; jj < NJ; ++jj) {
+          const int p = (NJ * lane + jj) & 7;
+          word |= (uint32_t)bucketize_sorted16(y[v][jj], bd) << (8 * (p >> 1) + ((p & 1) ? 0 : 4));
+        }
+#pragma unroll
+        for (int o = 1; o < 8 / NJ; o <<= 1) word |= __shfl_xor_sync(0xffffffffu, word, o);
         uint8_t* dst_idx;
         float* dst_norm;
         if (w.cache != nullptr) {
@@ -456,35 +364,46 @@ prologue_kernel(const AttnArgs a, const CompressArgs w, const int has_attn, cons
           dst_idx = w.packed_out + (int64_t)vec * HALF;
           dst_norm = w.norms_out + vec;
         }
-        // bytes 2*lane, 2*lane+1 of the head's packed row (2-byte aligned: rows start on 4 bytes)
-        if (jact) *reinterpret_cast<uint16_t*>(dst_idx + 2 * lane) = (uint16_t)(b0 | (b1 << 8));
-        if (lane == 0) *dst_norm = nrm[v];
+        const int jo = j0 + NJ * lane;  // (rows start on 4 bytes)
+        if (jact && (jo & 7) == 0) *reinterpret_cast<uint32_t*>(dst_idx + jo / 2) = word;
+        if (lane == 0 && j0 == 0) *dst_norm = nrm[v];
       }
     }
   }
-  pdl_wait();
 }
 
-template <int D>
-int launch_prologue_t(const AttnArgs* a, const CompressArgs* w, cudaStream_t st) {
-  using P = PrologueCfg<D>;
-  if (!ensure_dynamic_smem<prologue_kernel<D>>((int)P::smem_bytes, true)) return TQ4_ERR_CUDA;
-  const int64_t n_q = a ? (int64_t)a->sh.rows * a->sh.Hq : 0;
-  const int64_t n_w = w ? w->n_tokens * w->num_heads * w->n_sources : 0;
-  const int64_t chunks = (n_q + P::VC - 1) / P::VC + (n_w + P::VC - 1) / P::VC;
-  int64_t blocks = (chunks + P::WARPS - 1) / P::WARPS;
-  if (blocks > 2 * (int64_t)sm_count()) blocks = 2 * (int64_t)sm_count();
+template <int D, int JC>
+int launch_prologue_jc(const AttnArgs* a, const CompressArgs* w, cudaStream_t st, int64_t blocks) {
+  using P = PrologueCfg<D, JC>;
+  const size_t plan = a ? 2 * (size_t)a->sh.rows * sizeof(int) : 0;  // planning block
+  const size_t smem = P::rot_bytes > plan ? P::rot_bytes : plan;
+  if (!ensure_dynamic_smem<prologue_kernel<D, JC>>((int)smem, true)) return TQ4_ERR_CUDA;
+  const int64_t most = 2 * (int64_t)sm_count() / P::NSPLIT;
+  if (JC != 32 && blocks > most) blocks = most;
   if (blocks < 1) blocks = 1;
   static const AttnArgs no_attn{};
   static const CompressArgs no_write{};
   // First kernel of an entry point: a plain stream-ordered launch.  It reads tensors the caller's
   // preceding kernel may have produced (q, key, value, seq_lens), so it must not start before that
   // kernel has completed, whatever launch style the caller's kernels use.
-  if (launch_kernel(prologue_kernel<D>, dim3((unsigned)blocks + (a ? 1 : 0)), dim3(P::THREADS), P::smem_bytes,
+  if (launch_kernel(prologue_kernel<D, JC>, dim3((unsigned)(blocks * P::NSPLIT) + (a ? 1 : 0)), dim3(P::THREADS), smem,
                     st, false, a ? *a : no_attn, w ? *w : no_write, a ? 1 : 0, w ? 1 : 0) != cudaSuccess)
     return TQ4_ERR_CUDA;
   TQ4_CHECK_LAUNCH();
   return TQ4_OK;
+}
+
+// Column blocks of 32 while they all fit the GPU at once (about three resident blocks an SM), of the
+// whole head_dim (64 at head_dim 256: Pi does not fit) above.
+template <int D>
+int launch_prologue_t(const AttnArgs* a, const CompressArgs* w, cudaStream_t st) {
+  constexpr int VC = 4, WARPS = 8;
+  const int64_t n_q = a ? (int64_t)a->sh.rows * a->sh.Hq : 0;
+  const int64_t n_w = w ? w->n_tokens * w->num_heads * w->n_sources : 0;
+  const int64_t chunks = (n_q + VC - 1) / VC + (n_w + VC - 1) / VC;
+  const int64_t blocks = (chunks + WARPS - 1) / WARPS;
+  if (blocks * (D / 32) <= 3 * (int64_t)sm_count()) return launch_prologue_jc<D, 32>(a, w, st, blocks);
+  return launch_prologue_jc<D, (D <= 128 ? D : 64)>(a, w, st, blocks);
 }
 
 // ======================================================================================
@@ -531,17 +450,7 @@ attention_fp32_kernel(const AttnArgs a) {
   if (t_begin >= t_end) return;
   const RowLayout lay = row_layout(sh.Hkv, D);
 
-  // first row r with tile_prefix[r] <= t_begin < tile_prefix[r+1]
-  int r;
-  {
-    int lo = 0, hi = sh.rows - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (p.tile_prefix[mid] <= t_begin) lo = mid; else hi = mid - 1;
-    }
-    r = lo;
-    while (p.tile_prefix[r + 1] <= t_begin) ++r;  // skip rows without tiles
-  }
+  int r = p.span_row[c];
   const int tok = lane & 15, half = lane >> 4;
 
   int t = t_begin;
@@ -999,25 +908,10 @@ int launch_combine(const CombineArgs& c, int D, cudaStream_t st, bool pdl) {
   return TQ4_ERR_UNSUPPORTED;
 }
 
-template <int D>
-int launch_qrot_plan_t(const AttnArgs& a, cudaStream_t st) {
-  using Q = QrotCfg<D>;
-  if (!ensure_dynamic_smem<qrot_plan_kernel<D>>((int)Q::smem_bytes, true)) return TQ4_ERR_CUDA;
-  const int64_t n_vec = (int64_t)a.sh.rows * a.sh.Hq;
-  const unsigned grid = (unsigned)((n_vec + Q::VB - 1) / Q::VB) + 1;
-  // (first kernel of an entry point: plain stream-ordered launch, see launch_prologue_t)
-  if (launch_kernel(qrot_plan_kernel<D>, dim3(grid), dim3(Q::THREADS), Q::smem_bytes, st, false, a) !=
-      cudaSuccess)
-    return TQ4_ERR_CUDA;
-  TQ4_CHECK_LAUNCH();
-  return TQ4_OK;
-}
-
 // Prologue of an attention call (a != nullptr) and / or cache write of a few new tokens
-// (w != nullptr) in one launch; head_dim 256 (Pi does not fit in shared memory) and large writes
-// use the separate kernels.
+// (w != nullptr) in one launch; large writes use the compress kernels.
 int launch_prologue(const AttnArgs* a, const CompressArgs* w, int head_dim, cudaStream_t st) {
-  if (w && (head_dim > 128 || w->n_tokens * w->num_heads * w->n_sources > kSmallRows)) {
+  if (w && w->n_tokens * w->num_heads * w->n_sources > kSmallRows) {
     const int rc = dispatch_compress(*w, head_dim, w->x_dtype, st);
     if (rc != TQ4_OK) return rc;
     w = nullptr;
@@ -1027,7 +921,7 @@ int launch_prologue(const AttnArgs* a, const CompressArgs* w, int head_dim, cuda
     case 64: return launch_prologue_t<64>(a, w, st);
     case 96: return launch_prologue_t<96>(a, w, st);
     case 128: return launch_prologue_t<128>(a, w, st);
-    case 256: return launch_qrot_plan_t<256>(*a, st);
+    case 256: return launch_prologue_t<256>(a, w, st);
   }
   return TQ4_ERR_UNSUPPORTED;
 }
@@ -1162,17 +1056,12 @@ static int attention_impl(
   a.sh.span_ctas = use_mma ? ctas * a.sh.TPC : ctas;
   a.sh.part_tpc = part_tpc;
   cudaStream_t st = (cudaStream_t)stream;
-  // Decode calls of up to kFusedMaxRows rows can plan, rotate and write inside the attention kernel
-  // (two launches per step) or in a prologue kernel in front of it (three).  Measured on B200, graph
-  // replays, head_dim 128, GQA 4: the prologue kernel wins while rows x KV heads <= 512 (8 KV heads:
-  // 92.5 against 92.7 us at batch 64 x 4096, 50.1 against 53.4 at batch 16; 4 / 2 / 1 KV heads with
-  // batch 128 / 256 / 512: 93.9 against 94.9, 100.5 against 103.0, 123.6 against 132.9 us), the fused
-  // form above (8 KV heads: 155.7 against 160.4 us at batch 128, 173.9 against 177.4 at batch 256 x
-  // 2048).  TQ4_FUSED_PROLOGUE=1 / 0 forces it.
-  int force_fused = -1;
-  if (const char* e = getenv("TQ4_FUSED_PROLOGUE")) force_fused = atoi(e) != 0;
-  if (getenv("TQ4_NO_FUSED_PROLOGUE") != nullptr) force_fused = 0;
-  const bool want_fused = force_fused >= 0 ? force_fused != 0 : num_rows * num_kv_heads > kFusedMinRowHeads;
+  // TQ4_FUSED_PROLOGUE=1: decode calls of up to kFusedMaxRows rows plan, rotate and write inside the
+  // attention kernel (two launches per step instead of three).  Never faster than the prologue kernel in
+  // front (B200, graph replays, 32 / 8 heads, head_dim 128: 86.3 against 81.7 us at 64 x 4096, 92.9 / 92.5 at
+  // 128 x 2048, 161.2 / 158.9 at 256 x 2048, 192.2 / 188.9 at 512 x 1024), so only the environment selects it.
+  const char* fused_env = getenv("TQ4_FUSED_PROLOGUE");
+  const bool want_fused = fused_env != nullptr && atoi(fused_env) != 0;
   a.fused = use_mma && !use_prefill && query_start_loc == nullptr && num_rows <= kFusedMaxRows &&
             head_dim <= 128 && want_fused;
 

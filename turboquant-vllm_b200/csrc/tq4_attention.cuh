@@ -24,7 +24,7 @@ constexpr int kMmaWarpsPerCta = 16;    // tensor-core LUT kernel (one CTA per SM
 constexpr int kMaxCtasPerSlice = 148 * 4;  // upper bound used for workspace sizing (fp32 kernel)
 constexpr int kMaxSms = 160;               // tensor-core kernel: one CTA per SM, one span per warp phase
 constexpr int kMaxRowsPerLaunch = 4096;    // larger query batches are processed in pieces
-constexpr int kFusedMaxRows = 512;         // decode calls up to this size plan and rotate inside the attention kernel
+constexpr int kFusedMaxRows = 512;         // decode calls up to this size can plan and rotate inside the attention kernel
 // A row is cut into at most this many spans (= partials the merge kernel has to fold for it): a call of
 // a few long rows would otherwise hand the merge kernel hundreds of partials per row on a handful of
 // CTAs (batch 1 x 8192 tokens: merge 55 us against 16 us for the attention kernel itself).
@@ -35,7 +35,6 @@ __host__ __device__ __forceinline__ int tiles_per_span(int total_tiles, int span
   const int t = even > capped ? even : capped;
   return t > 1 ? t : 1;
 }
-constexpr int kFusedMinRowHeads = 512;     // ... when rows x KV heads exceeds this (else the separate prologue kernel is faster)
 
 struct AttnPlan {
   float* q_rot;      // [rows][Hq][D] fp32, q * Pi^T
@@ -44,6 +43,7 @@ struct AttnPlan {
   int* row_seq;      // [rows]   block-table row of the sequence that owns the query row
   int* tile_prefix;  // [rows+1] exclusive prefix sum of tiles per row
   int* slot_base;    // [rows+1] exclusive prefix sum of segments per row
+  int* span_row;     // [spans]  row that holds the first tile of a span (spans without tiles: unset)
   int* scalars;      // [0] total tiles, [1] tiles per span
   float* part_o;     // [slots][TPC][Hq][D]  un-normalised, rotated space
   float* part_m;     // [slots][TPC][Hq]     running max (log2 domain), -inf if empty
@@ -142,6 +142,7 @@ inline size_t carve_plan(AttnPlan& p, void* ws, int64_t rows, int Hq, int D, int
   p.row_seq = reinterpret_cast<int*>(take((size_t)rows * 4));
   p.tile_prefix = reinterpret_cast<int*>(take((size_t)(rows + 1) * 4));
   p.slot_base = reinterpret_cast<int*>(take((size_t)(rows + 1) * 4));
+  p.span_row = reinterpret_cast<int*>(take((size_t)max_spans * 4));
   p.scalars = reinterpret_cast<int*>(take(64));
   p.part_o = reinterpret_cast<float*>(take((size_t)slots * TPC * Hq * D * 4));
   p.part_m = reinterpret_cast<float*>(take((size_t)slots * TPC * Hq * 4));

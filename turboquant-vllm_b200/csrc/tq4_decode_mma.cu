@@ -719,7 +719,7 @@ __device__ __forceinline__ int v_byte_of_mblock(int g, int i) {
 // 1 = the same with a 16-byte wider V box (V region not 16-byte aligned), 2 = two 4-D boxes per
 // tile: the K and V halves of a token row have the same shape a fixed distance apart, so one box
 // with an extra "half" dimension fetches both index tiles, and one both norm tiles.
-template <int D, int NB, bool ALIGNED, bool PAGE16, int WARPS, bool TMA, int BOX>
+template <int D, int NB, bool ALIGNED, bool PAGE16, int WARPS, bool TMA, int BOX, bool FUSED>
 __global__ void __launch_bounds__(WARPS * 32, 1)
 attention_mma_kernel(const AttnArgs a, const CompressArgs w, const int has_write, const uint32_t smem_total,
                      const __grid_constant__ CUtensorMap tm_data,
@@ -879,8 +879,8 @@ attention_mma_kernel(const AttnArgs a, const CompressArgs w, const int has_write
   int pre_pos = 0, pre_ba = 0, pre_bb = 0;
 
   // ---- fused prologue: tile plan, query rotation and the step's cache write ------------------------
-  if (a.fused) {
-    if constexpr (D <= 128) {
+  if constexpr (FUSED) {
+    {
       const int n_warps = blockDim.x >> 5;
       const bool pi_one_batch = D * D / 4 <= kPiBatch * (int)blockDim.x;
       float4 pi_regs[kPiBatch];
@@ -986,38 +986,19 @@ attention_mma_kernel(const AttnArgs a, const CompressArgs w, const int has_write
   pdl_trigger();
   pdl_wait();
   TQ4_STAMP(4);
-  if (!a.fused) {
+  if constexpr (!FUSED) {
     total = p.scalars[0];
     tps = p.scalars[1];
     t_begin = (int)min((long long)span * tps, (long long)total);
     t_end = min(total, t_begin + tps);
   }
   if (t_begin >= t_end) return;
-
-  // first row of the span: the largest r with tile_prefix[r] <= t_begin (the array is
-  // non-decreasing).  Two levels of 32-way search: two dependent memory round trips instead of
-  // log2(rows) of a binary search.
-  if (!a.fused) {
-    const int rows = sh.rows;
-    const int stride = (rows + 31) / 32;
-    const int v1 = __ldg(p.tile_prefix + min(lane * stride, rows));
-    const unsigned m1 = __ballot_sync(0xffffffffu, v1 <= t_begin);  // a prefix of the lanes (entry 0 is 0)
-    const int base_i = (31 - __clz(m1 | 1u)) * stride;
-    int best = base_i;
-    for (int jj = lane; jj < stride; jj += 32) {
-      const int i = base_i + jj;
-      if (i < rows && __ldg(p.tile_prefix + i) <= t_begin) best = i;
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
-    r = min(best, rows - 1);
-    while (p.tile_prefix[r + 1] <= t_begin) ++r;
-  }
+  if constexpr (!FUSED) r = __ldg(p.span_row + span);
 
   int t = t_begin;
   while (t < t_end) {
     int row_t0, row_t1, kv_start, kv_end, row_seq;
-    if (a.fused) {  // from the sequence length: the plan arrays are not read back
+    if constexpr (FUSED) {  // from the sequence length: the plan arrays are not read back
       decode_row_range(a, r, row_seq, kv_start, kv_end);
       row_t0 = f_t0;
       row_t1 = f_t0 + row_tiles(kv_start, kv_end);
@@ -1503,7 +1484,7 @@ attention_mma_kernel(const AttnArgs a, const CompressArgs w, const int has_write
 
     TQ4_STAMP(6);
     // ---- write this warp's partial for the segment ---------------------------------------------
-    const int slot = (a.fused ? f_slot : p.slot_base[r]) + (span - row_t0 / tps);
+    const int slot = (FUSED ? f_slot : p.slot_base[r]) + (span - row_t0 / tps);
     const int64_t pidx = slot;
     const float inv_av = 1.f / a.lut_scale_v;
 #pragma unroll
@@ -1530,7 +1511,7 @@ attention_mma_kernel(const AttnArgs a, const CompressArgs w, const int has_write
     }
     t = seg_end;
     if (t < t_end) {
-      if (a.fused) {  // next row that has tiles; its first tile and first partial slot follow from this row's
+      if constexpr (FUSED) {  // next row that has tiles; its first tile and first partial slot follow from this row's
         f_slot += (row_t1 - 1) / tps - row_t0 / tps + 1;
         f_t0 = row_t1;
         for (++r; r < sh.rows - 1; ++r) {
@@ -1596,15 +1577,15 @@ bool make_cache_map_halves(CUtensorMap* m, const AttnArgs& a, uint32_t box_bytes
 
 constexpr int kErrNoHalvesMap = -1000;  // internal: the 4-D map could not be encoded, use 3-D boxes
 
-template <int D, int NB, bool ALIGNED, bool PAGE16, bool TMA, int BOX>
-int launch_mma_t(const AttnArgs& a, cudaStream_t st) {
+template <int D, int NB, bool ALIGNED, bool PAGE16, bool TMA, int BOX, bool FUSED>
+int launch_mma_f(const AttnArgs& a, cudaStream_t st) {
   constexpr bool VWIDE = BOX == 1;
   constexpr int kRowPitch = (D + 8 + 15) & ~15;
   constexpr int WARPS = (D * NB <= 128) ? 16 : 8;  // upper bound; the launch uses HPC * TPC warps
   using C = MmaCfg<D, ALIGNED>;
   // All opt-in shared memory of the SM (one CTA per SM by design): the 64 KB table sits on a
   // 64 KB boundary of the shared window and whole rings are packed on both sides of it.
-  constexpr auto kern = attention_mma_kernel<D, NB, ALIGNED, PAGE16, WARPS, TMA, BOX>;
+  constexpr auto kern = attention_mma_kernel<D, NB, ALIGNED, PAGE16, WARPS, TMA, BOX, FUSED>;
   static int smem_avail[kMaxDevices];  // opt-in limit minus the kernel's static shared memory, per device
   const int dev = device_ordinal();
   if (dev < 0) return TQ4_ERR_CUDA;
@@ -1636,12 +1617,19 @@ int launch_mma_t(const AttnArgs& a, cudaStream_t st) {
   const int warps = a.sh.HPC * a.sh.TPC;
   static const CompressArgs no_write{};
   // with the fused prologue this is the first kernel to read the caller's tensors: a plain launch
-  if (launch_kernel(kern, dim3(a.sh.ctas * a.sh.n_slices), dim3(warps * 32), (size_t)smem_total, st, !a.fused, a,
-                    a.fused && a.fused_write ? *a.fused_write : no_write, a.fused && a.fused_write ? 1 : 0,
+  if (launch_kernel(kern, dim3(a.sh.ctas * a.sh.n_slices), dim3(warps * 32), (size_t)smem_total, st, !FUSED, a,
+                    FUSED && a.fused_write ? *a.fused_write : no_write, FUSED && a.fused_write ? 1 : 0,
                     (uint32_t)smem_total, tm_data, tm_v, tm_norm) != cudaSuccess)
     return TQ4_ERR_CUDA;
   TQ4_CHECK_LAUNCH();
   return TQ4_OK;
+}
+
+template <int D, int NB, bool ALIGNED, bool PAGE16, bool TMA, int BOX>
+int launch_mma_t(const AttnArgs& a, cudaStream_t st) {
+  if constexpr (D <= 128)
+    if (a.fused) return launch_mma_f<D, NB, ALIGNED, PAGE16, TMA, BOX, true>(a, st);
+  return launch_mma_f<D, NB, ALIGNED, PAGE16, TMA, BOX, false>(a, st);
 }
 
 bool cache_aligned(const AttnShape& sh, const uint8_t* cache, int64_t bs, int64_t ts) {
