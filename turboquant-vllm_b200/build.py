@@ -1,22 +1,27 @@
-"""Build libtq4_sm100a.so (the C-ABI CUDA library) in-tree with nvcc for sm_100a.
+"""Build libtq4_sm100a.so (the C-ABI CUDA library) and _tq4_host.so (its CPython binding) in-tree.
 
 Usage:  python turboquant-vllm_b200/build.py [--force] [--verbose]
-The library lands in turboquant-vllm_b200/turboquant_vllm/lib/ where the Python host code
-loads it with ctypes.  No torch headers are involved: the ABI is plain C (include/tq4.h).
+Both land in turboquant-vllm_b200/turboquant_vllm/lib/.  The CUDA library is compiled with nvcc for
+sm_100a and has a plain C ABI (include/tq4.h, no torch headers); the binding (csrc/tq4_host.cpp) is
+compiled with g++ against the headers of the installed torch and links to it.
 """
 from __future__ import annotations
 
 import argparse
 import glob
+import importlib.util
 import os
 import subprocess
 import sys
+import sysconfig
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 OUT_DIR = os.path.join(HERE, "turboquant_vllm", "lib")
 OUT = os.path.join(OUT_DIR, "libtq4_sm100a.so")
+HOST_SRC = os.path.join(CSRC, "tq4_host.cpp")
+HOST_OUT = os.path.join(OUT_DIR, "_tq4_host.so")
 
 
 def sources() -> list[str]:
@@ -29,10 +34,29 @@ def _deps() -> list[str]:
 
 
 def needs_build() -> bool:
-    if not os.path.exists(OUT):
+    if not os.path.exists(OUT) or host_needs_build():
         return True
     t = os.path.getmtime(OUT)
     return any(os.path.getmtime(d) > t for d in sources() + _deps())
+
+
+def host_needs_build() -> bool:
+    if not os.path.exists(HOST_OUT):
+        return True
+    t = os.path.getmtime(HOST_OUT)
+    return any(os.path.getmtime(d) > t for d in (HOST_SRC, os.path.join(ROOT, "include", "tq4.h")))
+
+
+def host_command() -> list[str]:
+    """g++ command line of the CPython binding (linked to the CUDA library beside it)."""
+    torch_dir = os.path.dirname(importlib.util.find_spec("torch").origin)
+    inc = os.path.join(torch_dir, "include")
+    cuda = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+    return [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-shared", "-fPIC", "-o", HOST_OUT, HOST_SRC,
+            "-I", inc, "-I", os.path.join(inc, "torch", "csrc", "api", "include"), "-I", os.path.join(cuda, "include"),
+            "-I", sysconfig.get_paths()["include"], "-I", os.path.join(ROOT, "include"),
+            "-L", os.path.join(torch_dir, "lib"), "-ltorch_python", "-ltorch", "-ltorch_cpu", "-lc10", "-lc10_cuda",
+            "-L", OUT_DIR, "-l:libtq4_sm100a.so", "-Wl,-rpath,$ORIGIN"]
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -61,7 +85,12 @@ def build(force: bool = False, verbose: bool = False) -> str:
     failed = [src for src, p in jobs if p.wait() != 0]
     if failed:
         raise subprocess.CalledProcessError(1, f"nvcc -c {' '.join(failed)}")
-    subprocess.run([nvcc, "-shared", "-gencode", "arch=compute_100a,code=sm_100a", "-o", OUT, *objs], check=True)
+    if jobs or not os.path.exists(OUT):
+        subprocess.run([nvcc, "-shared", "-gencode", "arch=compute_100a,code=sm_100a", "-o", OUT, *objs], check=True)
+    else:
+        os.utime(OUT)
+    if force or host_needs_build():
+        subprocess.run(host_command(), check=True)
     return OUT
 
 

@@ -1,0 +1,310 @@
+// Python entry points of the hot calls, as a CPython extension over the C interface (include/tq4.h).
+//
+// A decode step of a small batch takes 15 - 30 us on the GPU; going through ctypes with some fifty
+// arguments, and asking every tensor for its pointer, strides and type from Python, took 43 us of host
+// time a call and bounded it.  Here the tensors are unpacked, checked and passed on in native code
+// (about a tenth of that; what is left is the kernel launches).  The checks, their exceptions and the results are
+// those of the Python wrappers in turboquant_vllm/kernels/ops.py, which only forward to this module.
+#include <Python.h>
+
+#include <ATen/core/Tensor.h>
+#include <ATen/ops/empty.h>
+#include <ATen/ops/empty_strided.h>
+#include <ATen/ops/zeros.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Dtype.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <cmath>
+#include <stdexcept>
+#include <string>
+
+#include "tq4.h"
+
+namespace {
+
+constexpr int kMaxDevices = 64;
+
+// thrown with the Python exception already set
+struct PyError {};
+
+[[noreturn]] void fail(PyObject* type, const std::string& msg) {
+  PyErr_SetString(type, msg.c_str());
+  throw PyError{};
+}
+#define TQ4_ASSERT(cond, msg) \
+  do {                        \
+    if (!(cond)) fail(PyExc_AssertionError, msg); \
+  } while (0)
+
+const at::Tensor& tensor(PyObject* o, const char* name) {
+  if (!THPVariable_Check(o)) fail(PyExc_TypeError, std::string(name) + " must be a torch.Tensor");
+  return THPVariable_Unpack(o);
+}
+const at::Tensor& cuda_tensor(PyObject* o, const char* name) {
+  const at::Tensor& t = tensor(o, name);
+  if (!t.is_cuda())
+    fail(PyExc_RuntimeError, "TQ4 kernels run on CUDA tensors only (sm_100a); got a tensor on " + t.device().str() +
+                                 ". There is no CPU fallback in this package.");
+  return t;
+}
+int dtype_code(at::ScalarType t) {
+  switch (t) {
+    case at::kFloat: return TQ4_F32;
+    case at::kHalf: return TQ4_F16;
+    case at::kBFloat16: return TQ4_BF16;
+    default:
+      fail(PyExc_TypeError, std::string("TQ4 kernels support float32/float16/bfloat16, got ") + c10::toString(t));
+  }
+}
+int64_t as_int(PyObject* o) {
+  const long long v = PyLong_AsLongLong(o);
+  if (v == -1 && PyErr_Occurred()) throw PyError{};
+  return v;
+}
+double as_double(PyObject* o) {
+  const double v = PyFloat_AsDouble(o);
+  if (v == -1.0 && PyErr_Occurred()) throw PyError{};
+  return v;
+}
+bool truth(PyObject* o) {
+  const int v = PyObject_IsTrue(o);
+  if (v < 0) throw PyError{};
+  return v != 0;
+}
+at::ScalarType as_dtype(PyObject* o) {
+  if (!THPDtype_Check(o)) fail(PyExc_TypeError, "dtype must be a torch.dtype");
+  return reinterpret_cast<THPDtype*>(o)->scalar_type;
+}
+at::Tensor inner_contiguous(const at::Tensor& t) { return t.stride(-1) == 1 ? t : t.contiguous(); }
+
+void check(int status, const char* what) {
+  if (status == TQ4_OK) return;
+  const std::string msg = std::string(what) + ": " + tq4_status_string(status);
+  if (status == TQ4_ERR_UNSUPPORTED) fail(PyExc_NotImplementedError, msg);
+  if (status == TQ4_ERR_STATIC_SCRATCH) fail(PyExc_ValueError, msg);
+  fail(PyExc_RuntimeError, msg + " (tq4 status " + std::to_string(status) + ")");
+}
+
+// Per-device error flag and attention scratch (grown on demand).  Never destroyed: the CUDA context may
+// be gone by the time static objects are.  Reached with the GIL held only.
+at::Tensor* g_flag[kMaxDevices];
+at::Tensor* g_workspace[kMaxDevices];
+
+int device_index(const at::Tensor& t) {
+  const int i = t.get_device();
+  if (i < 0 || i >= kMaxDevices) fail(PyExc_RuntimeError, "CUDA device index out of range");
+  return i;
+}
+at::Tensor& flag_of(int dev) {
+  if (!g_flag[dev])
+    g_flag[dev] = new at::Tensor(at::zeros({1}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, dev)));
+  return *g_flag[dev];
+}
+at::Tensor& workspace_of(int dev, int64_t bytes) {
+  if (!g_workspace[dev]) g_workspace[dev] = new at::Tensor();
+  at::Tensor& w = *g_workspace[dev];
+  if (!w.defined() || w.numel() < bytes)
+    w = at::empty({bytes}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, dev));
+  return w;
+}
+
+// The device's stream, with the device current for the duration of a call: the C entry points launch on
+// the current device.
+struct Launch {
+  c10::cuda::OptionalCUDAGuard guard;
+  void* stream;
+  explicit Launch(int dev) {
+    guard.set_index((c10::DeviceIndex)dev);
+    stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
+  }
+};
+
+template <typename F>
+PyObject* guarded(F&& body) {
+  try {
+    return body();
+  } catch (const PyError&) {
+    return nullptr;
+  } catch (const std::exception& e) {
+    PyErr_SetString(PyExc_RuntimeError, e.what());
+    return nullptr;
+  }
+}
+
+bool expect(const char* name, Py_ssize_t got, Py_ssize_t want) {
+  if (got == want) return true;
+  PyErr_Format(PyExc_TypeError, "%s takes %zd arguments, got %zd", name, want, got);
+  return false;
+}
+
+// Slot mapping as contiguous int64.
+at::Tensor slots64(const at::Tensor& s) {
+  at::Tensor t = s.scalar_type() == at::kLong ? s : s.to(at::kLong);
+  return t.is_contiguous() ? t : t.contiguous();
+}
+
+// attention(q, kv_cache, block_table, seq_lens, k_centroids, v_centroids, rotation, num_kv_heads, block_size,
+//           sm_scale, query_start_loc, causal, sliding_window, out, out_dtype, lse_out, out_rotated, workspace,
+//           mode, write)
+PyObject* attention(PyObject*, PyObject* const* p, Py_ssize_t n) {
+  if (!expect("attention", n, 20)) return nullptr;
+  return guarded([&]() -> PyObject* {
+    at::Tensor q = cuda_tensor(p[0], "q");
+    const at::Tensor& cache = cuda_tensor(p[1], "kv_cache");
+    const at::Tensor& bt = cuda_tensor(p[2], "block_table");
+    const at::Tensor& lens = cuda_tensor(p[3], "seq_lens");
+    const at::Tensor& kc = cuda_tensor(p[4], "k_centroids");
+    const at::Tensor& vc = cuda_tensor(p[5], "v_centroids");
+    at::Tensor rot = cuda_tensor(p[6], "rotation");
+    const int64_t hkv = as_int(p[7]), block = as_int(p[8]);
+    TQ4_ASSERT(q.dim() == 3, "q must have three dimensions");
+    const int64_t t = q.size(0), hq = q.size(1), d = q.size(2);
+    TQ4_ASSERT(hkv > 0 && hq % hkv == 0, "query heads must be a multiple of the KV heads");
+    TQ4_ASSERT(cache.scalar_type() == at::kByte && cache.dim() == 3 && cache.stride(2) == 1,
+               "kv_cache must be uint8 [blocks, tokens, bytes] with contiguous rows");
+    TQ4_ASSERT(bt.scalar_type() == at::kInt && bt.dim() == 2 && bt.stride(1) == 1, "block_table must be int32 with contiguous rows");
+    TQ4_ASSERT(lens.scalar_type() == at::kInt && lens.is_contiguous(), "seq_lens must be contiguous int32");
+    TQ4_ASSERT(rot.scalar_type() == at::kFloat, "rotation must be float32");
+    if (!rot.is_contiguous()) rot = rot.contiguous();  // e.g. the column-major Q factor of a QR
+    const at::Tensor* qsl = nullptr;
+    if (p[10] != Py_None) {
+      qsl = &cuda_tensor(p[10], "query_start_loc");
+      TQ4_ASSERT(qsl->scalar_type() == at::kInt && qsl->is_contiguous(), "query_start_loc must be contiguous int32");
+    }
+    q = inner_contiguous(q);
+    const float scale = p[9] == Py_None ? (float)(1.0 / std::sqrt((double)d)) : (float)as_double(p[9]);
+    const int dev = device_index(q);
+    Launch launch(dev);
+    at::Tensor out;
+    const bool own_out = p[13] == Py_None;
+    if (own_out) {
+      const at::ScalarType dt = p[14] == Py_None ? q.scalar_type() : as_dtype(p[14]);
+      out = at::empty({t, hq, d}, q.options().dtype(dt).requires_grad(false));
+    } else {
+      out = cuda_tensor(p[13], "out");
+      TQ4_ASSERT(out.dim() == 3 && out.size(0) == t && out.size(1) == hq && out.size(2) == d && out.stride(2) == 1,
+                 "out must have q's shape and contiguous rows");
+    }
+    float* lse = nullptr;
+    if (p[15] != Py_None) {
+      const at::Tensor& l = cuda_tensor(p[15], "lse_out");
+      TQ4_ASSERT(l.scalar_type() == at::kFloat && l.is_contiguous() && l.numel() >= t * hq,
+                 "lse_out must be contiguous float32 of rows x heads");
+      lse = (float*)l.data_ptr();
+    }
+    const size_t need = tq4_attention_workspace_bytes(t > 1 ? t : 1, (int)hq, (int)hkv, (int)d);
+    if (need == 0)
+      fail(PyExc_ValueError, "unsupported attention shape: Hq=" + std::to_string(hq) + ", Hkv=" + std::to_string(hkv) +
+                                 ", D=" + std::to_string(d));
+    const at::Tensor& ws = p[17] == Py_None ? workspace_of(dev, (int64_t)need) : cuda_tensor(p[17], "workspace");
+    const size_t have = (size_t)ws.numel() * ws.element_size();
+    if (have < need)
+      fail(PyExc_ValueError, "workspace has " + std::to_string(have) + " bytes, " + std::to_string(need) + " needed");
+    const int causal = truth(p[11]) ? 1 : 0, window = p[12] == Py_None ? 0 : (int)as_int(p[12]);
+    const int rotated = truth(p[16]) ? 1 : 0, mode = (int)as_int(p[18]);
+    int* flag = (int*)flag_of(dev).data_ptr();
+    const int q_dt = dtype_code(q.scalar_type()), out_dt = dtype_code(out.scalar_type());
+    int st;
+    if (p[19] == Py_None) {
+      Py_BEGIN_ALLOW_THREADS
+      st = tq4_paged_attention(
+          q.data_ptr(), q_dt, t, (int)lens.numel(), (int)hq, (int)hkv, (int)d, q.stride(0),
+          q.stride(1), (const uint8_t*)cache.data_ptr(), cache.stride(0), cache.stride(1), cache.size(0), (int)block,
+          (const int32_t*)bt.data_ptr(), bt.stride(0), (const int32_t*)lens.data_ptr(),
+          qsl ? (const int32_t*)qsl->data_ptr() : nullptr, (const float*)kc.data_ptr(), (int)kc.numel(),
+          (const float*)vc.data_ptr(), (int)vc.numel(), (const float*)rot.data_ptr(), scale, causal, window,
+          out.data_ptr(), out_dt, out.stride(0), out.stride(1), lse, rotated, ws.data_ptr(), have,
+          mode, flag, launch.stream);
+      Py_END_ALLOW_THREADS
+    } else {
+      TQ4_ASSERT(PyTuple_Check(p[19]) && PyTuple_GET_SIZE(p[19]) == 7, "write must be a tuple of seven tensors");
+      auto item = [&](int i, const char* name) -> const at::Tensor& { return cuda_tensor(PyTuple_GET_ITEM(p[19], i), name); };
+      at::Tensor key = item(0, "key"), value = item(1, "value");
+      const at::Tensor slots = slots64(item(2, "slot_mapping"));
+      const at::Tensor &even = item(3, "rotation_T_even"), &odd = item(4, "rotation_T_odd");
+      const at::Tensor &kb = item(5, "k_boundaries"), &vb = item(6, "v_boundaries");
+      TQ4_ASSERT(cache.is_contiguous(), "the fused write addresses flat slots: block-major contiguous cache");
+      TQ4_ASSERT(key.sizes() == value.sizes() && key.scalar_type() == value.scalar_type() && key.dim() == 3 &&
+                     key.size(1) == hkv && key.size(2) == d,
+                 "key and value must be [tokens, KV heads, head_dim] of one type");
+      key = inner_contiguous(key);
+      value = inner_contiguous(value);
+      const int kv_dt = dtype_code(key.scalar_type());
+      Py_BEGIN_ALLOW_THREADS
+      st = tq4_write_and_attention(
+          key.data_ptr(), value.data_ptr(), kv_dt, key.size(0), key.stride(0), key.stride(1),
+          value.stride(0), value.stride(1), (const int64_t*)slots.data_ptr(), slots.numel(), (const float*)even.data_ptr(),
+          (const float*)odd.data_ptr(), (const float*)kb.data_ptr(), (int)kb.numel(), (const float*)vb.data_ptr(),
+          (int)vb.numel(), q.data_ptr(), q_dt, t, (int)lens.numel(), (int)hq, (int)hkv, (int)d,
+          q.stride(0), q.stride(1), (uint8_t*)cache.data_ptr(), cache.stride(0), cache.stride(1), cache.size(0), (int)block,
+          (const int32_t*)bt.data_ptr(), bt.stride(0), (const int32_t*)lens.data_ptr(),
+          qsl ? (const int32_t*)qsl->data_ptr() : nullptr, (const float*)kc.data_ptr(), (int)kc.numel(),
+          (const float*)vc.data_ptr(), (int)vc.numel(), (const float*)rot.data_ptr(), scale, causal, window,
+          out.data_ptr(), out_dt, out.stride(0), out.stride(1), lse, rotated, ws.data_ptr(), have,
+          mode, flag, launch.stream);
+      Py_END_ALLOW_THREADS
+    }
+    check(st, "paged_tq4_attention");
+    if (!own_out) {
+      Py_INCREF(p[13]);
+      return p[13];
+    }
+    return THPVariable_Wrap(std::move(out));
+  });
+}
+
+// write_paged(key, value, kv_cache, slot_mapping, rotation_T_even, rotation_T_odd, k_boundaries, v_boundaries)
+PyObject* write_paged(PyObject*, PyObject* const* p, Py_ssize_t n) {
+  if (!expect("write_paged", n, 8)) return nullptr;
+  return guarded([&]() -> PyObject* {
+    at::Tensor key = cuda_tensor(p[0], "key"), value = cuda_tensor(p[1], "value");
+    const at::Tensor& cache = cuda_tensor(p[2], "kv_cache");
+    const at::Tensor& slot_mapping = cuda_tensor(p[3], "slot_mapping");
+    const at::Tensor &even = cuda_tensor(p[4], "rotation_T_even"), &odd = cuda_tensor(p[5], "rotation_T_odd");
+    const at::Tensor &kb = cuda_tensor(p[6], "k_boundaries"), &vb = cuda_tensor(p[7], "v_boundaries");
+    TQ4_ASSERT(cache.scalar_type() == at::kByte && cache.dim() == 3 && cache.is_contiguous(), "kv_cache must be contiguous uint8");
+    TQ4_ASSERT(key.dim() == 3 && key.sizes() == value.sizes() && key.scalar_type() == value.scalar_type(),
+               "key and value must be [tokens, KV heads, head_dim] of one type");
+    key = inner_contiguous(key);
+    value = inner_contiguous(value);
+    const at::Tensor slots = slots64(slot_mapping);
+    const int dev = device_index(key);
+    Launch launch(dev);
+    int* flag = (int*)flag_of(dev).data_ptr();
+    const int kv_dt = dtype_code(key.scalar_type());
+    int st;
+    Py_BEGIN_ALLOW_THREADS
+    st = tq4_write_paged(key.data_ptr(), value.data_ptr(), kv_dt, key.size(0), (int)key.size(1),
+                         (int)key.size(2), key.stride(0), key.stride(1), value.stride(0), value.stride(1),
+                         (const int64_t*)slots.data_ptr(), slots.numel(), (const float*)even.data_ptr(),
+                         (const float*)odd.data_ptr(), (const float*)kb.data_ptr(), (int)kb.numel(),
+                         (const float*)vb.data_ptr(), (int)vb.numel(), (uint8_t*)cache.data_ptr(), cache.size(2),
+                         cache.size(0) * cache.size(1), flag, launch.stream);
+    Py_END_ALLOW_THREADS
+    check(st, "tq4_write_paged");
+    Py_RETURN_NONE;
+  });
+}
+
+// error_flag(device_index) -> the device's int32 flag tensor
+PyObject* error_flag(PyObject*, PyObject* const* p, Py_ssize_t n) {
+  if (!expect("error_flag", n, 1)) return nullptr;
+  return guarded([&]() -> PyObject* {
+    const int64_t dev = as_int(p[0]);
+    if (dev < 0 || dev >= kMaxDevices) fail(PyExc_RuntimeError, "CUDA device index out of range");
+    return THPVariable_Wrap(flag_of((int)dev));
+  });
+}
+
+PyMethodDef kMethods[] = {
+    {"attention", (PyCFunction)(void (*)(void))attention, METH_FASTCALL, "Paged TQ4 attention, optionally with a cache write."},
+    {"write_paged", (PyCFunction)(void (*)(void))write_paged, METH_FASTCALL, "Compress K and V into the paged cache."},
+    {"error_flag", (PyCFunction)(void (*)(void))error_flag, METH_FASTCALL, "Device error flag."},
+    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_tq4_host", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__tq4_host(void) { return PyModule_Create(&kModule); }

@@ -1,4 +1,7 @@
-"""ctypes binding of libtq4_sm100a.so (the C ABI declared in include/tq4.h).
+"""Bindings of libtq4_sm100a.so (the C ABI declared in include/tq4.h).
+
+:func:`lib` is the complete ctypes binding; :func:`host` is the CPython extension that the hot calls go
+through (csrc/tq4_host.cpp: the same entry points, called with tensors).
 
 There is no CPU or Triton fallback: if the library is missing, or a tensor is not on a CUDA
 device, the call raises.  The library is built in-tree by ``turboquant-vllm_b200/build.py``.
@@ -8,13 +11,17 @@ from __future__ import annotations
 
 import contextlib
 import ctypes
+import importlib.machinery
+import importlib.util
 import os
 from ctypes import c_char_p, c_float, c_int, c_int64, c_size_t, c_void_p
 
 import torch
 
 _LIB_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "lib", "libtq4_sm100a.so")
+_HOST_PATH = os.path.join(os.path.dirname(_LIB_PATH), "_tq4_host.so")
 _lib = None
+_host = None
 
 F32, F16, BF16 = 0, 1, 2
 _DTYPE_CODE = {torch.float32: F32, torch.float16: F16, torch.bfloat16: BF16}
@@ -108,6 +115,21 @@ def lib() -> ctypes.CDLL:
             fn.argtypes = args
         _lib = handle
     return _lib
+
+
+def host():
+    """The CPython extension over the CUDA library, loaded once; raises like :func:`lib` when missing."""
+    global _host
+    if _host is None:
+        lib()
+        if not os.path.exists(_HOST_PATH):
+            raise RuntimeError(f"TQ4 host extension not found at {_HOST_PATH}. Build it with "
+                               "`python turboquant-vllm_b200/build.py`.")
+        loader = importlib.machinery.ExtensionFileLoader("_tq4_host", _HOST_PATH)
+        mod = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_tq4_host", _HOST_PATH, loader=loader))
+        loader.exec_module(mod)
+        _host = mod
+    return _host
 
 
 def check(status: int, what: str) -> None:

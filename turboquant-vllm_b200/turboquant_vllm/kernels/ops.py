@@ -22,12 +22,8 @@ import torch
 from turboquant_vllm import _native as nv
 
 # --------------------------------------------------------------------------------------
-# per-device scratch: attention workspace (grown on demand, reused) and the error flag
+# per-device scratch (attention workspace, error flag) is kept by the native host module
 # --------------------------------------------------------------------------------------
-_workspaces: dict[int, torch.Tensor] = {}
-_err_flags: dict[int, torch.Tensor] = {}
-
-
 def attention_workspace_bytes(max_query_rows: int, num_q_heads: int, num_kv_heads: int, head_dim: int) -> int:
     """Bytes of scratch ``paged_tq4_attention`` needs for up to ``max_query_rows`` rows."""
     n = nv.lib().tq4_attention_workspace_bytes(max_query_rows, num_q_heads, num_kv_heads, head_dim)
@@ -38,23 +34,10 @@ def attention_workspace_bytes(max_query_rows: int, num_q_heads: int, num_kv_head
     return int(n)
 
 
-def _workspace(device: torch.device, nbytes: int) -> torch.Tensor:
-    idx = device.index if device.index is not None else torch.cuda.current_device()
-    ws = _workspaces.get(idx)
-    if ws is None or ws.numel() < nbytes:
-        ws = torch.empty(nbytes, dtype=torch.uint8, device=device)
-        _workspaces[idx] = ws
-    return ws
-
-
 def error_flag(device: torch.device) -> torch.Tensor:
     """Device int32 that kernels OR with TQ4_DEV_* bits (bad slot / bad block id)."""
     idx = device.index if device.index is not None else torch.cuda.current_device()
-    f = _err_flags.get(idx)
-    if f is None:
-        f = torch.zeros(1, dtype=torch.int32, device=device)
-        _err_flags[idx] = f
-    return f
+    return nv.host().error_flag(idx)
 
 
 def read_and_clear_errors(device: torch.device) -> int:
@@ -223,28 +206,8 @@ def tq4_write_paged(
 ) -> None:
     """Compress ``key``/``value`` ``[N, H, D]`` and scatter the packed rows into ``kv_cache``
     ``(NB, BS, >= H*(D+8))`` at ``slot_mapping`` in one launch (negative slots are skipped)."""
-    nv.require_cuda(key, value, kv_cache, slot_mapping, rotation_T_even, rotation_T_odd,
-                    k_boundaries, v_boundaries)
-    assert kv_cache.dtype == torch.uint8 and kv_cache.is_contiguous()
-    assert key.shape == value.shape and key.dtype == value.dtype
-    n, h, d = key.shape
-    key = _inner_contiguous(key)
-    value = _inner_contiguous(value)
-    if slot_mapping.dtype != torch.int64:
-        slot_mapping = slot_mapping.to(torch.int64)
-    slot_mapping = slot_mapping.contiguous()
-    nb, bs, width = kv_cache.shape
-    st = nv.call(key.device, "tq4_write_paged",
-        key.data_ptr(), value.data_ptr(), nv.dtype_code(key.dtype), n, h, d,
-        key.stride(0), key.stride(1), value.stride(0), value.stride(1),
-        slot_mapping.data_ptr(), slot_mapping.numel(),
-        rotation_T_even.data_ptr(), rotation_T_odd.data_ptr(),
-        k_boundaries.data_ptr(), k_boundaries.numel(),
-        v_boundaries.data_ptr(), v_boundaries.numel(),
-        kv_cache.data_ptr(), width, nb * bs,
-        error_flag(key.device).data_ptr(), nv.stream_ptr(key.device),
-    )
-    nv.check(st, "tq4_write_paged")
+    nv.host().write_paged(key, value, kv_cache, slot_mapping, rotation_T_even, rotation_T_odd,
+                          k_boundaries, v_boundaries)
 
 
 # --------------------------------------------------------------------------------------
@@ -285,63 +248,9 @@ def paged_tq4_attention(
     3 chunked-prefill tcgen05 kernel (head_dim 128 only), 4 the same with single fp16 terms for
     queries and probabilities (faster, about 1e-3 absolute error; never picked automatically).
     """
-    nv.require_cuda(q, kv_cache, block_table, seq_lens, k_centroids, v_centroids, rotation)
-    t, hq, d = q.shape
-    assert hq % num_kv_heads == 0
-    assert kv_cache.dtype == torch.uint8 and kv_cache.stride(2) == 1
-    assert block_table.dtype == torch.int32 and block_table.stride(1) == 1
-    assert seq_lens.dtype == torch.int32 and seq_lens.is_contiguous()
-    assert rotation.dtype == torch.float32
-    if not rotation.is_contiguous():  # e.g. the column-major Q factor of torch.linalg.qr
-        rotation = rotation.contiguous()
-    if query_start_loc is not None:
-        assert query_start_loc.dtype == torch.int32 and query_start_loc.is_contiguous()
-        nv.require_cuda(query_start_loc)
-    q = _inner_contiguous(q)
-    if sm_scale is None:
-        sm_scale = 1.0 / math.sqrt(d)
-    if out is None:
-        out = torch.empty(t, hq, d, dtype=out_dtype or q.dtype, device=q.device)
-    else:
-        nv.require_cuda(out)
-        assert out.shape == (t, hq, d) and out.stride(2) == 1
-    if lse_out is not None:
-        assert lse_out.dtype == torch.float32 and lse_out.is_contiguous() and lse_out.numel() >= t * hq
-    need = attention_workspace_bytes(max(t, 1), hq, num_kv_heads, d)
-    ws = workspace if workspace is not None else _workspace(q.device, need)
-    if ws.numel() * ws.element_size() < need:
-        raise ValueError(f"workspace has {ws.numel() * ws.element_size()} bytes, {need} needed")
-    wargs: tuple = ()
-    if write is not None:
-        key, value, slot_mapping, rot_even, rot_odd, k_bounds, v_bounds = write
-        nv.require_cuda(key, value, slot_mapping, rot_even, rot_odd, k_bounds, v_bounds)
-        assert kv_cache.is_contiguous(), "the fused write addresses flat slots: block-major contiguous cache"
-        assert key.shape == value.shape and key.dtype == value.dtype and key.shape[1:] == (num_kv_heads, d)
-        key = _inner_contiguous(key)
-        value = _inner_contiguous(value)
-        if slot_mapping.dtype != torch.int64:
-            slot_mapping = slot_mapping.to(torch.int64)
-        slot_mapping = slot_mapping.contiguous()
-        wargs = (key.data_ptr(), value.data_ptr(), nv.dtype_code(key.dtype), key.shape[0],
-                 key.stride(0), key.stride(1), value.stride(0), value.stride(1),
-                 slot_mapping.data_ptr(), slot_mapping.numel(), rot_even.data_ptr(), rot_odd.data_ptr(),
-                 k_bounds.data_ptr(), k_bounds.numel(), v_bounds.data_ptr(), v_bounds.numel())
-    st = nv.call(
-        q.device, "tq4_write_and_attention" if write is not None else "tq4_paged_attention",
-        *wargs,
-        q.data_ptr(), nv.dtype_code(q.dtype), t, seq_lens.numel(), hq, num_kv_heads, d,
-        q.stride(0), q.stride(1),
-        kv_cache.data_ptr(), kv_cache.stride(0), kv_cache.stride(1), kv_cache.shape[0], block_size,
-        block_table.data_ptr(), block_table.stride(0), seq_lens.data_ptr(), nv.ptr(query_start_loc),
-        k_centroids.data_ptr(), k_centroids.numel(), v_centroids.data_ptr(), v_centroids.numel(),
-        rotation.data_ptr(), float(sm_scale), int(bool(causal)), int(sliding_window or 0),
-        out.data_ptr(), nv.dtype_code(out.dtype), out.stride(0), out.stride(1),
-        nv.ptr(lse_out), int(bool(out_rotated)),
-        ws.data_ptr(), ws.numel() * ws.element_size(), mode,
-        error_flag(q.device).data_ptr(), nv.stream_ptr(q.device),
-    )
-    nv.check(st, "paged_tq4_attention")
-    return out
+    return nv.host().attention(
+        q, kv_cache, block_table, seq_lens, k_centroids, v_centroids, rotation, num_kv_heads, block_size, sm_scale,
+        query_start_loc, causal, sliding_window, out, out_dtype, lse_out, out_rotated, workspace, mode, write)
 
 
 def tq4_write_and_attention(
