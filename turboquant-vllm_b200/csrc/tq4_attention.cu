@@ -123,7 +123,6 @@ __device__ void build_plan(const AttnArgs& a, int* s_work) {
   run = block_exclusive_scan(local);
   const int total_slots = s_total;
 
-  pdl_wait();
   for (int r = r_lo; r < r_hi; ++r) {
     int seq, start, end;
     row_range(r, seq, start, end);
@@ -132,16 +131,48 @@ __device__ void build_plan(const AttnArgs& a, int* s_work) {
     p.row_seq[r] = seq;
     p.tile_prefix[r] = s_tiles[r];
     p.slot_base[r] = run;
-    run += s_slots[r];
-    // the spans whose first tile is one of this row's
-    const int b = s_tiles[r], e = r + 1 < rows ? s_tiles[r + 1] : total;
-    for (int s = (b + tps - 1) / tps; s * tps < e; ++s) p.span_row[s] = r;
+    if (a.plan_records) {
+      int4* rec = reinterpret_cast<int4*>(p.row_rec + 8 * (int64_t)r);
+      rec[0] = make_int4(s_tiles[r], r + 1 < rows ? s_tiles[r + 1] : total, start, end);
+      rec[1] = make_int4(seq, run, 0, 0);
+    }
+    const int n = s_slots[r];
+    s_slots[r] = run;
+    run += n;
   }
   if (threadIdx.x == 0) {
     p.tile_prefix[rows] = total;
     p.scalars[0] = total;
     p.scalars[1] = tps;
     p.slot_base[rows] = total_slots;
+  }
+  __syncthreads();
+  for (int s = threadIdx.x; s < sh.span_ctas; s += blockDim.x) {
+    const long long T = (long long)s * tps;
+    int r = -1;
+    if (T < total) {
+      int lo = 0, hi = rows - 1;  // the largest r with s_tiles[r] <= T is the row that holds tile T
+      while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (s_tiles[mid] <= T) lo = mid; else hi = mid - 1;
+      }
+      r = lo;
+    }
+    p.span_row[s] = r;
+    if (a.plan_records) {
+      int4* rec = reinterpret_cast<int4*>(p.span_rec + 12 * (int64_t)s);
+      int4 x = make_int4(r, total, tps, 0), y = make_int4(0, 0, 0, 0), z = make_int4(0, 0, 0, 0);
+      if (r >= 0) {
+        int seq, start, end;
+        row_range(r, seq, start, end);
+        y = make_int4(s_tiles[r], r + 1 < rows ? s_tiles[r + 1] : total, start, end);
+        z.x = seq;
+        z.y = s_slots[r];
+      }
+      rec[0] = x;
+      rec[1] = y;
+      rec[2] = z;
+    }
   }
 }
 
@@ -1036,6 +1067,7 @@ static int attention_impl(
   a.lse_out = lse_out;
   a.out_rotated = out_rotated;
   a.err_flag = err_flag;
+  a.plan_records = use_mma;
 
   // chunked prefill (several query rows per sequence) at head_dim 128: tensor-core kernel, one
   // dequantisation of a key tile serves a whole block of query rows

@@ -43,7 +43,10 @@ struct AttnPlan {
   int* row_seq;      // [rows]   block-table row of the sequence that owns the query row
   int* tile_prefix;  // [rows+1] exclusive prefix sum of tiles per row
   int* slot_base;    // [rows+1] exclusive prefix sum of segments per row
-  int* span_row;     // [spans]  row that holds the first tile of a span (spans without tiles: unset)
+  int* span_row;     // [spans]  row that holds the first tile of a span (-1: the span has no tiles)
+  // tensor-core kernel: everything a warp needs to know of a row, and of its span's first row, in one read
+  int* row_rec;      // [rows][8]   tiles [t0, t1), keys [start, end), sequence, first partial slot
+  int* span_rec;     // [spans][12] row, total tiles, tiles per span, -, then the words of the row's record
   int* scalars;      // [0] total tiles, [1] tiles per span
   float* part_o;     // [slots][TPC][Hq][D]  un-normalised, rotated space
   float* part_m;     // [slots][TPC][Hq]     running max (log2 domain), -inf if empty
@@ -91,6 +94,7 @@ struct AttnArgs {
   float* lse_out;
   int out_rotated;
   int* err_flag;
+  int plan_records;  // the plan writes row_rec and span_rec (tensor-core kernel)
   int fused;  // tensor-core kernel: compute the tile plan and rotate the queries inside the kernel
   const CompressArgs* fused_write;  // host side only: the step's cache write, done inside the fused kernel
 };
@@ -143,6 +147,8 @@ inline size_t carve_plan(AttnPlan& p, void* ws, int64_t rows, int Hq, int D, int
   p.tile_prefix = reinterpret_cast<int*>(take((size_t)(rows + 1) * 4));
   p.slot_base = reinterpret_cast<int*>(take((size_t)(rows + 1) * 4));
   p.span_row = reinterpret_cast<int*>(take((size_t)max_spans * 4));
+  p.row_rec = reinterpret_cast<int*>(take((size_t)rows * 32));
+  p.span_rec = reinterpret_cast<int*>(take((size_t)max_spans * 48));
   p.scalars = reinterpret_cast<int*>(take(64));
   p.part_o = reinterpret_cast<float*>(take((size_t)slots * TPC * Hq * D * 4));
   p.part_m = reinterpret_cast<float*>(take((size_t)slots * TPC * Hq * 4));

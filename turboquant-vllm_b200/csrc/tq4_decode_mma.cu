@@ -980,34 +980,51 @@ attention_mma_kernel(const AttnArgs a, const CompressArgs w, const int has_write
     }
   }
   __syncthreads();
-  // everything above used only caller inputs and shared memory (a launch with the fused prologue is
-  // a plain one); without it the kernel now reads the plan and the rotated queries of the prologue
-  // kernel and the cache the write kernel filled
   pdl_trigger();
   pdl_wait();
-  TQ4_STAMP(4);
+  // everything above used only caller inputs and shared memory (with the fused prologue: what this kernel
+  // wrote); the plan, the rotated queries and the written tokens come from the prologue kernel.  One read
+  // of the span's record, one of its page ids, and the first tile pair is in flight while the queries load.
+  int rec = 0;  // lane i < 12: word i of the span's record; later lane i < 8: word i of the next row's record
+  auto rec_word = [&](int i) { return __shfl_sync(0xffffffffu, rec, i); };
   if constexpr (!FUSED) {
-    total = p.scalars[0];
-    tps = p.scalars[1];
+    if (lane < 12) rec = p.span_rec[12 * (int64_t)span + lane];
+    total = rec_word(1);
+    tps = rec_word(2);
     t_begin = (int)min((long long)span * tps, (long long)total);
     t_end = min(total, t_begin + tps);
+    r = rec_word(0);
+    if constexpr (TMA) {
+      if (t_begin < t_end) {
+        const int t0 = rec_word(4), ks = rec_word(6);
+        const int pos = (ks / kTileTokens + (t_begin - t0)) * kTileTokens;
+        pre_two = t_begin + 1 < min(rec_word(5), t_end);
+        const int32_t* bt = a.block_table + (int64_t)rec_word(8) * a.bt_stride;
+        const int ba = __ldg(bt + (pos >> bs_shift)), bb = pre_two ? __ldg(bt + ((pos + kTileTokens) >> bs_shift)) : ba;
+        pre_ok = tma_issue_pair(0, pos, ba, bb, pre_two);
+        pre_issued = true;
+      }
+    }
   }
+  TQ4_STAMP(4);
   if (t_begin >= t_end) return;
-  if constexpr (!FUSED) r = __ldg(p.span_row + span);
 
+  // the row the warp is in: its tiles, keys, sequence and first partial slot
+  int row_t0 = 0, row_t1 = 0, kv_start = 0, kv_end = 0, row_seq = 0, row_slot = 0;
+  if constexpr (!FUSED) {
+    row_t0 = rec_word(4); row_t1 = rec_word(5);
+    kv_start = rec_word(6); kv_end = rec_word(7);
+    row_seq = rec_word(8); row_slot = rec_word(9);
+  }
   int t = t_begin;
   while (t < t_end) {
-    int row_t0, row_t1, kv_start, kv_end, row_seq;
     if constexpr (FUSED) {  // from the sequence length: the plan arrays are not read back
       decode_row_range(a, r, row_seq, kv_start, kv_end);
       row_t0 = f_t0;
       row_t1 = f_t0 + row_tiles(kv_start, kv_end);
-    } else {
-      row_t0 = p.tile_prefix[r];
-      row_t1 = p.tile_prefix[r + 1];
-      kv_start = p.kv_start[r];
-      kv_end = p.kv_end[r];
-      row_seq = p.row_seq[r];
+      row_slot = f_slot;
+    } else if (row_t1 < t_end && lane < 8) {  // the span goes on into the next row: fetch its record now
+      rec = p.row_rec[8 * (int64_t)(r + 1) + lane];
     }
     const int seg_end = min(row_t1, t_end);
     const int32_t* bt = a.block_table + (int64_t)row_seq * a.bt_stride;
@@ -1365,9 +1382,14 @@ attention_mma_kernel(const AttnArgs a, const CompressArgs w, const int has_write
         };
         uint32_t st = gk & 1u, ph = (gk >> 1) & 1u;  // stage and barrier parity of the current pair
         int pos_i = pos0_of(first), pos_c = pos_i;
-        int blk_a = load_blk(pos_i), blk_b = load_blk(pos_i + kTileTokens);
-        __syncwarp();
-        uint32_t ok_cur = pre_issued ? pre_ok : issue(st, pos_i, blk_a, blk_b);  // (pre-issued: stage 0, gk == 0)
+        int blk_a, blk_b;
+        uint32_t ok_cur = pre_ok;
+        if (!pre_issued) {  // (else the pair is in flight in stage gk & 1)
+          blk_a = load_blk(pos_i);
+          blk_b = load_blk(pos_i + kTileTokens);
+          __syncwarp();
+          ok_cur = issue(st, pos_i, blk_a, blk_b);
+        }
         pre_issued = false;
         pos_i += step_tok;
         blk_a = load_blk(pos_i);
@@ -1483,8 +1505,33 @@ attention_mma_kernel(const AttnArgs a, const CompressArgs w, const int has_write
     }
 
     TQ4_STAMP(6);
+    const int slot = row_slot + (span - row_t0 / tps);
+    t = seg_end;
+    if constexpr (!FUSED) {
+      // the next row's first pair goes into flight before this row's partial is stored
+      if (t < t_end) {
+        ++r;
+        while (rec_word(1) <= t) {  // rows without tiles
+          ++r;
+          if (lane < 8) rec = p.row_rec[8 * (int64_t)r + lane];
+        }
+        row_t0 = rec_word(0); row_t1 = rec_word(1);
+        kv_start = rec_word(2); kv_end = rec_word(3);
+        row_seq = rec_word(4); row_slot = rec_word(5);
+        if constexpr (TMA) {
+          if (!dead) {
+            const int pos = kv_start / kTileTokens * kTileTokens;
+            pre_two = row_t0 + 1 < min(row_t1, t_end);
+            const int32_t* nbt = a.block_table + (int64_t)row_seq * a.bt_stride;
+            const int ba = __ldg(nbt + (pos >> bs_shift)), bb = pre_two ? __ldg(nbt + ((pos + kTileTokens) >> bs_shift)) : ba;
+            __syncwarp();
+            pre_ok = tma_issue_pair(gk & 1u, pos, ba, bb, pre_two);
+            pre_issued = true;
+          }
+        }
+      }
+    }
     // ---- write this warp's partial for the segment ---------------------------------------------
-    const int slot = (FUSED ? f_slot : p.slot_base[r]) + (span - row_t0 / tps);
     const int64_t pidx = slot;
     const float inv_av = 1.f / a.lut_scale_v;
 #pragma unroll
@@ -1509,9 +1556,8 @@ attention_mma_kernel(const AttnArgs a, const CompressArgs w, const int has_write
         }
       }
     }
-    t = seg_end;
-    if (t < t_end) {
-      if constexpr (FUSED) {  // next row that has tiles; its first tile and first partial slot follow from this row's
+    if constexpr (FUSED) {
+      if (t < t_end) {  // next row that has tiles; its first tile and first partial slot follow from this row's
         f_slot += (row_t1 - 1) / tps - row_t0 / tps + 1;
         f_t0 = row_t1;
         for (++r; r < sh.rows - 1; ++r) {
@@ -1519,9 +1565,6 @@ attention_mma_kernel(const AttnArgs a, const CompressArgs w, const int has_write
           decode_row_range(a, r, sq, st_, en_);
           if (en_ > st_) break;
         }
-      } else {
-        ++r;
-        while (p.tile_prefix[r + 1] <= t) ++r;
       }
     }
   }

@@ -4,19 +4,19 @@
     python turboquant-vllm_b200/kernel_timeline.py prefill    # tcgen05 chunked prefill, 8 x 2048 on 8192
     python turboquant-vllm_b200/kernel_timeline.py compress   # tcgen05 cache write, 16 384 tokens x 8 heads
 
-Builds `turboquant_vllm/lib/libtq4_sm100a_trace.so`: the same sources with `-DTQ4_TRACE`, which compiles
+Builds `turboquant_vllm/lib/trace/libtq4_sm100a.so`: the same sources with `-DTQ4_TRACE`, which compiles
 time stamps into `attention_mma_kernel` (`%globaltimer` at its phases, lane 0 of every warp of every
 CTA), `prefill_tc_kernel` (SM clock at points of the tile loop, four warps of one CTA) and
 `compress_tc16_kernel` (SM clock at the hand-overs of its tile pipeline, four warps of CTA 0) and
 exports the functions that read them back.  The shipped library has neither.  The workloads are the ones
-`bench.py` times; the decode timeline is taken with the prologue inside the attention kernel
-(`TQ4_FUSED_PROLOGUE=1`), the form whose single kernel shows every phase of a step.
+`bench.py` times; with `TQ4_FUSED_PROLOGUE=1` the decode timeline has the prologue's phases too.
 """
 from __future__ import annotations
 
 import ctypes
 import glob
 import os
+import shutil
 import subprocess
 import sys
 
@@ -25,7 +25,8 @@ import numpy as np
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
-TRACE_LIB = os.path.join(HERE, "turboquant_vllm", "lib", "libtq4_sm100a_trace.so")
+LIB_DIR = os.path.join(HERE, "turboquant_vllm", "lib")
+TRACE_LIB = os.path.join(LIB_DIR, "trace", "libtq4_sm100a.so")  # (the name the host extension is linked to)
 
 
 def build_trace_library() -> str:
@@ -48,6 +49,7 @@ def build_trace_library() -> str:
             raise SystemExit(f"nvcc failed on {src}")
     if jobs or not os.path.exists(TRACE_LIB):
         subprocess.check_call([nvcc, "-shared", "-gencode", "arch=compute_100a,code=sm_100a", "-o", TRACE_LIB, *objs])
+    shutil.copy(os.path.join(LIB_DIR, "_tq4_host.so"), os.path.dirname(TRACE_LIB))
     return TRACE_LIB
 
 
@@ -59,13 +61,13 @@ def _load(kind: str):
     from turboquant_vllm import _native as nv
 
     nv._LIB_PATH = build_trace_library()
+    nv._HOST_PATH = os.path.join(os.path.dirname(TRACE_LIB), "_tq4_host.so")
     reader = {"decode": "tq4_trace_read", "prefill": "tq4_prefill_trace_read", "compress": "tq4_compress_trace_read"}[kind]
     nv._SIGNATURES[reader] = (ctypes.c_int, [ctypes.c_void_p])
     return nv, reader
 
 
 def decode_timeline() -> None:
-    os.environ["TQ4_FUSED_PROLOGUE"] = "1"
     nv, reader = _load("decode")
     import torch
 
