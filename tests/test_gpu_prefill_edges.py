@@ -1,0 +1,65 @@
+"""The tcgen05 prefill kernel at the edges of its row blocks, tiles, key splits and row layouts."""
+
+import numpy as np
+import pytest
+import torch
+
+from oracle import tq4_oracle as O
+from tests.helpers import Prims, build_paged_case, cosine
+
+pytestmark = pytest.mark.gpu
+
+CASES = [  # head_dim, q heads, KV heads, lengths, new rows, mode, window, causal, padded rows
+    (128, 4, 4, [64], [16], 3, None, True, True),            # one row block, one full tile
+    (128, 8, 2, [300, 90], [120, 90], 3, None, True, True),  # a last CTA with one of its two blocks in use
+    (128, 28, 4, [150], [150], 3, None, True, True),         # groups of 7: 126 of 128 lanes
+    (128, 8, 4, [65], [65], 0, None, True, True),            # one key in the second tile
+    (128, 32, 8, [3000], [40], 0, None, True, True),         # cut along the keys
+    (128, 4, 1, [700], [333], 3, None, False, False),        # 136-byte rows: 4-byte loads; not causal
+    (64, 14, 2, [333], [200], 3, None, True, True),
+    (96, 4, 4, [300, 41], [100, 9], 3, None, True, False),
+    (256, 8, 4, [300, 90], [120, 90], 3, 64, True, True),
+    (256, 2, 2, [700], [9], 3, None, True, True),
+    (128, 8, 2, [300, 90, 50, 77], [120, 1, 7, 77], 0, None, True, True),   # long and short sequences
+    (256, 8, 4, [900, 90, 8], [12, 1, 8], 0, None, True, True),
+]
+
+
+@pytest.mark.parametrize("d,hq,hkv,lens,new,mode,window,causal,padded", CASES)
+def test_prefill_edges(cuda_lib, d, hq, hkv, lens, new, mode, window, causal, padded):
+    from turboquant_vllm.kernels import ops
+
+    pr = Prims(d)
+    p = pr.cuda()
+    case = build_paged_case(lens, hkv, d, 16, pr, seed=5, padded=padded)
+    q = torch.randn(sum(new), hq, d, generator=torch.Generator().manual_seed(1)).bfloat16()
+    qsl = torch.tensor(np.concatenate([[0], np.cumsum(new)]), dtype=torch.int32)
+    lse = torch.empty(sum(new), hq, device="cuda")
+    out = ops.paged_tq4_attention(
+        q.cuda(), case["cache"].cuda(), case["block_table"].cuda(), case["seq_lens"].cuda(), p["kc"], p["vc"], p["rot"],
+        hkv, 16, query_start_loc=qsl.cuda(), causal=causal, sliding_window=window, out_dtype=torch.float32, mode=mode,
+        lse_out=lse).cpu()
+    ref, ref_lse = O.paged_attention_fp32(q, case["cache"], case["block_table"], lens, qsl, pr.kc, pr.vc, pr.rot, hkv, None,
+                                          causal, window, return_lse=True)
+    assert cosine(out, ref) >= 0.9999 and (out - ref).abs().max() <= 2e-3
+    assert torch.allclose(lse.cpu(), ref_lse.reshape(lse.shape), atol=1e-3, rtol=1e-4)
+    assert ops.read_and_clear_errors(torch.device("cuda")) == 0
+
+
+def test_prefill_hides_and_reports_bad_pages(cuda_lib):
+    from turboquant_vllm import _native as nv
+    from turboquant_vllm.kernels import ops
+
+    pr = Prims(128)
+    p = pr.cuda()
+    case = build_paged_case([100], 4, 128, 16, pr, seed=5, padded=True)
+    q = torch.randn(30, 8, 128, generator=torch.Generator().manual_seed(1)).bfloat16()
+    qsl = torch.tensor([0, 30], dtype=torch.int32)
+    bt = case["block_table"].clone()
+    bt[0, 1] = 10_000  # keys 16 .. 31 are not there
+    args = (case["seq_lens"].cuda(), p["kc"], p["vc"], p["rot"], 4, 16)
+    out = [ops.paged_tq4_attention(q.cuda(), case["cache"].cuda(), bt.cuda(), *args, query_start_loc=qsl.cuda(),
+                                   out_dtype=torch.float32, mode=m) for m in (2, 3)]
+    torch.cuda.synchronize()
+    assert ops.read_and_clear_errors(torch.device("cuda")) == nv.DEV_BAD_BLOCK
+    assert (out[0] - out[1]).abs().max() <= 2e-3

@@ -21,7 +21,8 @@ __device__ void build_plan(const AttnArgs& a, int* s_work) {
   __shared__ int s_part[32];
   __shared__ int s_total;
   __shared__ int s_max_tiles;  // tiles of the longest row
-  if (threadIdx.x == 0) s_max_tiles = 0;
+  __shared__ int s_active;     // rows up to the last one that is streamed
+  if (threadIdx.x == 0) s_max_tiles = s_active = 0;
   __syncthreads();
   const int rows = sh.rows;
   int* s_tiles = s_work;        // [rows] tile count, then exclusive prefix
@@ -52,6 +53,10 @@ __device__ void build_plan(const AttnArgs& a, int* s_work) {
       seq = lo;
       if (seq < sh.num_seqs && gr < a.query_start_loc[sh.num_seqs]) {
         const int q0 = a.query_start_loc[seq], q1 = a.query_start_loc[seq + 1];
+        if (a.skip_long > 0 && q1 - q0 >= a.skip_long) {  // (an empty range that no key can have: not merged either)
+          end = -1;
+          return;
+        }
         const int len = clamp_seq_len(a, max(0, a.seq_lens[seq]));
         const int pos = len - (q1 - q0) + (gr - q0);
         end = a.causal ? pos + 1 : len;
@@ -97,6 +102,7 @@ __device__ void build_plan(const AttnArgs& a, int* s_work) {
     int seq, start, end;
     row_range(r, seq, start, end);
     const int nt = end > start ? (end + kTileTokens - 1) / kTileTokens - start / kTileTokens : 0;
+    if (end >= 0) atomicMax(&s_active, r + 1);
     s_tiles[r] = nt;
     local += nt;
     row_max = max(row_max, nt);
@@ -144,6 +150,7 @@ __device__ void build_plan(const AttnArgs& a, int* s_work) {
     p.tile_prefix[rows] = total;
     p.scalars[0] = total;
     p.scalars[1] = tps;
+    p.scalars[2] = s_active;
     p.slot_base[rows] = total_slots;
   }
   __syncthreads();
@@ -220,10 +227,21 @@ prologue_kernel(const AttnArgs a, const CompressArgs w, const int has_attn, cons
   float* s_pit = reinterpret_cast<float*>(smem_raw);                    // [D][JC]: s_pit[d][j] = Pi[j0 + j][d]
   float4* s_x = reinterpret_cast<float4*>(s_pit + D * JC);              // [WARPS][D] four vectors per entry
   __shared__ float s_bounds[2][16];  // sorted boundaries of K and V, padded with +inf
+  __shared__ int s_active;           // rows up to the last one that is streamed (mixed calls)
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (has_write && tid < 32) {
     const int src = tid >> 4, i = tid & 15;
     s_bounds[src][i] = (src < w.n_sources && i < w.n_bounds[src]) ? w.bounds[src][i] : CUDART_INF_F;
+  }
+  if (has_attn && a.skip_long > 0) {
+    if (tid == 0) s_active = 0;
+    __syncthreads();
+    int last = 0;
+    for (int s = tid; s < a.sh.num_seqs; s += P::THREADS) {
+      const int q0 = a.query_start_loc[s], q1 = a.query_start_loc[s + 1];
+      if (q1 > q0 && q1 - q0 < a.skip_long) last = max(last, q1 - a.sh.row_offset);
+    }
+    if (last > 0) atomicMax(&s_active, min(last, a.sh.rows));
   }
 
   // ---- stage the slice of Pi^T --------------------------------------------------------------------
@@ -258,7 +276,7 @@ prologue_kernel(const AttnArgs a, const CompressArgs w, const int has_attn, cons
   __syncthreads();
 
   // vector counts fit 32 bits (rows <= kMaxRowsPerLaunch, writes <= kSmallRows): no 64-bit divisions
-  const int n_q = has_attn ? a.sh.rows * a.sh.Hq : 0;
+  const int n_q = has_attn ? (a.skip_long > 0 ? s_active : a.sh.rows) * a.sh.Hq : 0;
   const int rows_per_src = has_write ? (int)w.n_tokens * w.num_heads : 0;
   const int n_w = rows_per_src * (has_write ? w.n_sources : 0);
   const int cq = (n_q + VC - 1) / VC, cw = (n_w + VC - 1) / VC;
@@ -433,7 +451,10 @@ int launch_prologue_t(const AttnArgs* a, const CompressArgs* w, cudaStream_t st)
   const int64_t n_w = w ? w->n_tokens * w->num_heads * w->n_sources : 0;
   const int64_t chunks = (n_q + VC - 1) / VC + (n_w + VC - 1) / VC;
   const int64_t blocks = (chunks + WARPS - 1) / WARPS;
-  if (blocks * (D / 32) <= 3 * (int64_t)sm_count()) return launch_prologue_jc<D, 32>(a, w, st, blocks);
+  const int64_t wave = 3 * (int64_t)sm_count() / (D / 32);
+  if (blocks <= wave) return launch_prologue_jc<D, 32>(a, w, st, blocks);
+  // a mixed call streams few of its rows (the kernel finds out how many)
+  if (a && a->skip_long > 0) return launch_prologue_jc<D, 32>(a, w, st, wave);
   return launch_prologue_jc<D, (D <= 128 ? D : 64)>(a, w, st, blocks);
 }
 
@@ -669,6 +690,9 @@ int launch_attention_fp32(const AttnArgs& a, cudaStream_t st) {
 //    Also serves tq4_combine_partials (cross-GPU shards) through the "dense" mode.
 // ======================================================================================
 struct CombineArgs {
+  const int* active_rows;  // (optional) device count: only the first so many rows are merged ...
+  const int* row_end;      // (optional) last visible key of the rows: -1 = a row of the prefill kernel
+  int rows_long;           // with row_end: merge the prefill kernel's rows (1) or the others (0)
   // sparse mode (slot_base != null): the partials of row r are slot_base[r]..slot_base[r+1], x TPC
   const int* slot_base;
   int TPC;
@@ -729,7 +753,7 @@ __global__ void __launch_bounds__(256) combine_kernel(const CombineArgs a) {
   __shared__ float s_m[8], s_l[8];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int split = blockIdx.x % C::NSPLIT;
-  const int n_vec = a.rows * a.Hq;
+  int n_vec = a.rows * a.Hq;
   if (!a.out_rotated) {
     const uint32_t dst = (uint32_t)__cvta_generic_to_shared(s_pi);
     for (int i = tid; i < D * C::LC; i += 256) {
@@ -740,6 +764,8 @@ __global__ void __launch_bounds__(256) combine_kernel(const CombineArgs a) {
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
   pdl_wait();  // the partials and the plan come from the kernels before this one
+  auto row_mine = [&](int row) { return !a.row_end || (a.row_end[row] < 0) == (a.rows_long != 0); };
+  if (a.active_rows) n_vec = min(n_vec, *a.active_rows * a.Hq);
   const bool sparse = a.slot_base != nullptr;
   const float mscale = sparse ? 1.f : 1.4426950408889634f;  // dense partials carry a natural-log LSE
   const int64_t pstride = sparse ? (int64_t)a.Hq : (int64_t)a.rows * a.Hq;  // vectors between two partials
@@ -837,7 +863,7 @@ __global__ void __launch_bounds__(256) combine_kernel(const CombineArgs a) {
             *reinterpret_cast<float4*>(s_x + v * C::XP + 4 * lane + 128 * r) =
                 make_float4(o[r][0] * inv, o[r][1] * inv, o[r][2] * inv, o[r][3] * inv);
       }
-      if (a.lse_out && split == 0 && sub == 0 && lane == 0 && vec < n_vec)
+      if (a.lse_out && split == 0 && sub == 0 && lane == 0 && vec < n_vec && row_mine(vec / a.Hq))
         a.lse_out[(int64_t)a.row_offset * a.Hq + vec] =
             L > 0.f ? (M + log2f(L)) * 0.6931471805599453f : -CUDART_INF_F;
     }
@@ -895,6 +921,7 @@ __global__ void __launch_bounds__(256) combine_kernel(const CombineArgs a) {
         }
       }
       const int row = vec / a.Hq, head = vec - row * a.Hq;
+      if (!row_mine(row)) continue;
       store4(a.out, a.out_dtype, (int64_t)(row + a.row_offset) * a.out_token_stride + (int64_t)head * a.out_head_stride +
                                      split * C::DC + c, y);
     }
@@ -978,8 +1005,8 @@ extern "C" const char* tq4_status_string(int status) {
   return "unknown status";
 }
 
-extern "C" size_t tq4_attention_workspace_bytes(int64_t max_query_rows, int num_q_heads,
-                                                int num_kv_heads, int head_dim) {
+// What a call of up to so many rows cannot do without.
+static size_t workspace_min(int64_t max_query_rows, int num_q_heads, int num_kv_heads, int head_dim) {
   tq4::AttnShape sh{};
   if (max_query_rows <= 0 || !tq4::make_shape(sh, num_q_heads, num_kv_heads, head_dim)) return 0;
   const int64_t rows = max_query_rows < tq4::kMaxRowsPerLaunch ? max_query_rows : tq4::kMaxRowsPerLaunch;
@@ -988,6 +1015,17 @@ extern "C" size_t tq4_attention_workspace_bytes(int64_t max_query_rows, int num_
   tq4::make_shape(sh, num_q_heads, num_kv_heads, head_dim, tq4::kMmaWarpsPerCta);
   const size_t b = tq4::carve_plan(p, nullptr, rows, num_q_heads, head_dim, 1, (int64_t)tq4::kMaxSms * sh.TPC);
   return a > b ? a : b;
+}
+
+// ... plus room for the partials of prefill calls that are cut along the keys: up to eight parts of the
+// rows, as long as the row blocks alone do not fill the GPU.
+extern "C" size_t tq4_attention_workspace_bytes(int64_t max_query_rows, int num_q_heads,
+                                                int num_kv_heads, int head_dim) {
+  const size_t least = workspace_min(max_query_rows, num_q_heads, num_kv_heads, head_dim);
+  if (least == 0) return 0;
+  int64_t vectors = 8 * max_query_rows * num_q_heads;
+  if (vectors > tq4::kPrefillSplitVectors) vectors = tq4::kPrefillSplitVectors;
+  return max_query_rows < tq4::kPrefillMinRows ? least : least + (size_t)vectors * (head_dim + 1) * 4;
 }
 
 // Shared body of tq4_paged_attention and tq4_write_and_attention: `wr` (optional) is a cache write
@@ -1069,15 +1107,17 @@ static int attention_impl(
   a.err_flag = err_flag;
   a.plan_records = use_mma;
 
-  // chunked prefill (several query rows per sequence) at head_dim 128: tensor-core kernel, one
-  // dequantisation of a key tile serves a whole block of query rows
+  // Chunked prefill: the tcgen05 kernel takes the sequences with at least kPrefillMinRows new rows (a tile
+  // costs it the same for 1 row as for 128 / G, and about as much as the streaming kernel's pass for six of
+  // them), the streaming kernel the others.  The lengths are on the device, so a call that may hold both kinds
+  // launches both; one sequence, or many rows per sequence (where the odd short one costs less than the
+  // streaming kernels' launches), takes one kernel.
   const bool prefill_ok = prefill_tc_supported(a);
   if ((mode == 3 || mode == 4) && !prefill_ok) return TQ4_ERR_UNSUPPORTED;
-  // (automatic only when the query blocks fill the GPU: a CTA owns a (row block, KV head) pair, a
-  // small chunk is spread wider by the streaming kernel)
-  const int64_t prefill_ctas = (num_rows * a.sh.G / 128) * num_kv_heads;
-  const bool use_prefill = mode == 3 || mode == 4 || (mode == 0 && prefill_ok && num_rows >= 8 * (int64_t)num_seqs &&
-                                         2 * prefill_ctas >= sm_count());
+  const bool all_long = mode == 3 || mode == 4 || (num_seqs == 1 && num_rows >= kPrefillMinRows) || num_rows >= 256 * (int64_t)num_seqs;
+  const bool use_prefill = prefill_ok && (mode == 3 || mode == 4 || (mode == 0 && num_rows >= kPrefillMinRows && (num_seqs > 1 || all_long)));
+  const bool use_stream = !use_prefill || !all_long;
+  a.skip_long = use_prefill && use_stream ? kPrefillMinRows : 0;
 
   const int sms = sm_count();
   int ctas = (use_mma ? 1 : 4) * sms / a.sh.n_slices;
@@ -1094,10 +1134,10 @@ static int attention_impl(
   // 128 x 2048, 161.2 / 158.9 at 256 x 2048, 192.2 / 188.9 at 512 x 1024), so only the environment selects it.
   const char* fused_env = getenv("TQ4_FUSED_PROLOGUE");
   const bool want_fused = fused_env != nullptr && atoi(fused_env) != 0;
-  a.fused = use_mma && !use_prefill && query_start_loc == nullptr && num_rows <= kFusedMaxRows &&
+  a.fused = use_mma && query_start_loc == nullptr && num_rows <= kFusedMaxRows &&
             head_dim <= 128 && want_fused;
 
-  for (int64_t r0 = 0; r0 < num_rows; r0 += kMaxRowsPerLaunch) {
+  for (int64_t r0 = 0; use_stream && r0 < num_rows; r0 += kMaxRowsPerLaunch) {
     a.sh.rows = (int)((num_rows - r0) < kMaxRowsPerLaunch ? (num_rows - r0) : kMaxRowsPerLaunch);
     a.sh.row_offset = (int)r0;
     int rc;
@@ -1118,13 +1158,15 @@ static int attention_impl(
       if (rc != TQ4_OK) return rc;
     }
     prof_begin(TQ4_PROF_ATTENTION, st);
-    rc = use_prefill ? launch_prefill_tc(a, st, mode == 4)
-                     : (use_mma ? launch_attention_mma(a, st) : launch_attention_fp32(a, st));
+    rc = use_mma ? launch_attention_mma(a, st) : launch_attention_fp32(a, st);
     prof_end(TQ4_PROF_ATTENTION, st);
     if (rc != TQ4_OK) return rc;
     CombineArgs c{};
-    c.slot_base = use_prefill ? nullptr : a.plan.slot_base;  // prefill: one dense partial per row
-    c.world = 1;
+    c.slot_base = a.plan.slot_base;
+    if (a.skip_long > 0) {
+      c.active_rows = a.plan.scalars + 2;
+      c.row_end = a.plan.kv_end;
+    }
     c.TPC = a.sh.part_tpc;
     c.part_o = a.plan.part_o;
     c.part_m = a.plan.part_m;
@@ -1144,7 +1186,50 @@ static int attention_impl(
     prof_end(TQ4_PROF_COMBINE, st);
     if (rc != TQ4_OK) return rc;
   }
-  return TQ4_OK;
+  if (!use_prefill) return TQ4_OK;
+
+  // ---- the prefill kernel: all its sequences in one launch; the scratch of the streaming part is free again ----
+  a.sh.rows = (int)num_rows;
+  a.sh.row_offset = 0;
+  if (wr && !use_stream) {
+    prof_begin(TQ4_PROF_WRITE, st);
+    const int rc = dispatch_compress(*wr, head_dim, wr->x_dtype, st);
+    prof_end(TQ4_PROF_WRITE, st);
+    if (rc != TQ4_OK) return rc;
+  }
+  // scratch: Pi's image, then the partials of a call cut along the keys; behind the plan where that is still
+  // needed (the merge kernel tells by its ranges which rows are the prefill kernel's)
+  const uintptr_t at = use_stream ? (uintptr_t)a.plan.part_o : (uintptr_t)workspace;
+  uint8_t* image = reinterpret_cast<uint8_t*>((at + 127) & ~(uintptr_t)127);
+  float* part_o = reinterpret_cast<float*>(image + prefill_tc_image_bytes(head_dim));
+  const int64_t room = (int64_t)((uintptr_t)workspace + workspace_bytes) - (int64_t)(uintptr_t)part_o;
+  const int splits = use_stream && num_rows > kMaxRowsPerLaunch
+                         ? 1 : prefill_tc_splits(a, room / ((int64_t)num_q_heads * (head_dim + 1) * 4) - 1);
+  const bool to_parts = splits > 1;
+  float* part_m = part_o + (size_t)splits * num_rows * num_q_heads * head_dim;
+  prof_begin(TQ4_PROF_ATTENTION, st);
+  int rc = launch_prefill_tc(a, st, mode == 4, use_stream ? kPrefillMinRows : 1, splits, to_parts, image, part_o, part_m);
+  prof_end(TQ4_PROF_ATTENTION, st);
+  if (rc != TQ4_OK || !to_parts) return rc;
+  CombineArgs c{};
+  c.world = splits;
+  c.part_o = part_o;
+  c.part_m = part_m;
+  c.rows = (int)num_rows;
+  c.row_end = use_stream ? a.plan.kv_end : nullptr;
+  c.rows_long = 1;
+  c.Hq = num_q_heads;
+  c.rotation = rotation;
+  c.out = out;
+  c.out_dtype = out_dtype;
+  c.out_token_stride = out_token_stride;
+  c.out_head_stride = out_head_stride;
+  c.lse_out = lse_out;
+  c.out_rotated = out_rotated;
+  prof_begin(TQ4_PROF_COMBINE, st);
+  rc = launch_combine(c, head_dim, st, true);
+  prof_end(TQ4_PROF_COMBINE, st);
+  return rc;
 }
 
 extern "C" int tq4_paged_attention(
@@ -1289,7 +1374,7 @@ extern "C" int tq4_paged_attention_static(
     int mode, int* err_flag, void* stream) {
   if (num_rows < 0) return TQ4_ERR_INVALID_ARG;
   if (num_rows == 0) return TQ4_OK;
-  const size_t need = tq4_attention_workspace_bytes(num_rows, num_q_heads, num_kv_heads, head_dim);
+  const size_t need = workspace_min(num_rows, num_q_heads, num_kv_heads, head_dim);
   if (need == 0) return TQ4_ERR_UNSUPPORTED;
   if (need > (size_t)TQ4_STATIC_SCRATCH_BYTES) return TQ4_ERR_STATIC_SCRATCH;
   void* scratch = nullptr;

@@ -24,6 +24,7 @@ constexpr int kMmaWarpsPerCta = 16;    // tensor-core LUT kernel (one CTA per SM
 constexpr int kMaxCtasPerSlice = 148 * 4;  // upper bound used for workspace sizing (fp32 kernel)
 constexpr int kMaxSms = 160;               // tensor-core kernel: one CTA per SM, one span per warp phase
 constexpr int kMaxRowsPerLaunch = 4096;    // larger query batches are processed in pieces
+constexpr int kPrefillSplitVectors = 2 * 148 * 256;  // (row, head) partials of a prefill call cut along the keys
 constexpr int kFusedMaxRows = 512;         // decode calls up to this size can plan and rotate inside the attention kernel
 // A row is cut into at most this many spans (= partials the merge kernel has to fold for it): a call of
 // a few long rows would otherwise hand the merge kernel hundreds of partials per row on a handful of
@@ -47,7 +48,7 @@ struct AttnPlan {
   // tensor-core kernel: everything a warp needs to know of a row, and of its span's first row, in one read
   int* row_rec;      // [rows][8]   tiles [t0, t1), keys [start, end), sequence, first partial slot
   int* span_rec;     // [spans][12] row, total tiles, tiles per span, -, then the words of the row's record
-  int* scalars;      // [0] total tiles, [1] tiles per span
+  int* scalars;      // [0] total tiles, [1] tiles per span, [2] rows up to the last one that is streamed
   float* part_o;     // [slots][TPC][Hq][D]  un-normalised, rotated space
   float* part_m;     // [slots][TPC][Hq]     running max (log2 domain), -inf if empty
   float* part_l;     // [slots][TPC][Hq]     running sum
@@ -94,6 +95,7 @@ struct AttnArgs {
   float* lse_out;
   int out_rotated;
   int* err_flag;
+  int skip_long;     // > 0: sequences with at least this many new rows are left to the prefill kernel
   int plan_records;  // the plan writes row_rec and span_rec (tensor-core kernel)
   int fused;  // tensor-core kernel: compute the tile plan and rotate the queries inside the kernel
   const CompressArgs* fused_write;  // host side only: the step's cache write, done inside the fused kernel
@@ -159,10 +161,15 @@ inline size_t carve_plan(AttnPlan& p, void* ws, int64_t rows, int Hq, int D, int
 // Launchers implemented in tq4_attention.cu / tq4_decode_mma.cu.
 int launch_attention_fp32(const AttnArgs& a, cudaStream_t st);
 int launch_attention_mma(const AttnArgs& a, cudaStream_t st);  // returns TQ4_ERR_UNSUPPORTED if shape not covered
-// tensor-core (tcgen05) chunked-prefill kernel (tq4_prefill_tc.cu): writes one dense partial per row
-// (normalised rotated output in plan.part_o [rows][Hq][D], natural-log LSE in plan.part_m [rows][Hq])
+// tensor-core (tcgen05) chunked-prefill kernel (tq4_prefill_tc.cu) over the sequences with at least `min_rows`
+// new rows: rotates, attends, un-rotates and writes the output, or leaves `splits` dense partials per row
+// (normalised rotated output in part_o [splits][rows][Hq][D], natural-log LSE in part_m [splits][rows][Hq])
 bool prefill_tc_supported(const AttnArgs& a);
-int launch_prefill_tc(const AttnArgs& a, cudaStream_t st, bool fast);
+int prefill_tc_splits(const AttnArgs& a, int64_t slots);
+size_t prefill_tc_image_bytes(int D);
+int launch_prefill_tc(const AttnArgs& a, cudaStream_t st, bool fast, int min_rows, int splits, bool to_parts,
+                      uint8_t* image, float* part_o, float* part_m);
+constexpr int kPrefillMinRows = 8;  // new rows of a sequence from which the prefill kernel is the faster one
 int mma_warps_per_cta(int D, int GC, int Hkv, int64_t token_stride = 0);
 bool attention_mma_supported(const AttnShape& sh, int block_size, const uint8_t* cache,
                              int64_t block_stride, int64_t token_stride);

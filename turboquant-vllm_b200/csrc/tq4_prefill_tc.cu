@@ -1,118 +1,146 @@
-// Chunked-prefill attention over the packed TQ4 cache on the 5th-generation tensor cores
-// (head_dim 128).  A CTA owns a block of 128 / G query rows of one sequence and one KV head: the
-// M = 128 rows of the MMAs are the (query row, query head of the GQA group) pairs, so a key/value
-// tile is dequantised ONCE per CTA and serves all of them (the streaming kernel dequantises it per
-// query row).  Everything happens in rotated space on the queries the prologue kernel rotated.
+// Chunked-prefill attention over the packed TQ4 cache on the 5th-generation tensor cores, head_dim 64 to
+// 256.  A CTA owns one KV head and one or two blocks of 128 / G query rows of a sequence: the M = 128
+// rows of the MMAs are the (query row, query head of the GQA group) pairs, so a key/value tile is
+// dequantised ONCE per CTA and serves all of them (the streaming kernel dequantises it per query row).
 //
-// Per 64-token tile:
-//   TMA boxes (K+V index rows and norm columns of 4 pages)                      -> shared memory
-//   dequantise through a 256-entry byte -> half2 table: K~ [64 tok][128 d] and V~ as fp16,
-//     stored in the swizzled layouts the MMA descriptors expect                  CUDA cores
-//   S = Qhi K~^T + Qlo K~^T   (tcgen05.mma kind::f16, 128 x 64 x 16, fp32 in TMEM, two S buffers)
-//   tcgen05.ld S, x knorm, mask, lazy online softmax, P = p * vnorm as fp16 hi + lo   CUDA cores
-//   O += Plo V~ + Phi V~      (tcgen05.mma 128 x 128 x 16, V~ as an MN-major B operand)
-// The A operands of both products live in TENSOR MEMORY, not in shared memory: the block's queries
-// are written there once (tcgen05.st, two fp16 per 32-bit column), the probabilities once per tile by
-// the threads that computed them.  The loop is bound by shared-memory bandwidth (the tensor pipe
-// fetches its shared-memory operands again for every instruction, beside the dequantisation's own
-// loads and stores): with Q and P in shared memory the MMAs alone read 224 KB per tile, now 96 KB.
-// At the end the normalised rows (still rotated) and their log-sum-exp go to the scratch in the
-// layout of one dense partial per row; the merge kernel un-rotates and stores them.
-// The first 4 * kTPR warps own the S / O rows, kTPR threads per row (softmax, rescale, epilogue; kTPR = 2:
-// with four threads per row the softmax part shortens but the 24 warps slow the dequantisation down
-// more); the next eight warps dequantise the following tile into the other K~ / V~ buffer meanwhile
-// (keys first, so that the next scores can be issued early; then the values).  One thread of the first
-// of them issues the MMAs; one thread of each of the last four issues the TMA copies of one page.
-// (A warp for the issuing alone was tried: five warps on one scheduler cut the register budget to 96
-// and the loop ran no faster.)  Every wait is bounded.
-#include <cuda.h>
+// Phases of a CTA:
+//   1. rotate the block's queries: raw rows, scaled by a power of two, as fp16 hi (+ lo) in tensor memory
+//      times Pi (2^8 Pi as fp16 hi + lo, an operand image in shared memory)         tcgen05.mma
+//   2. per 64-token tile
+//        packed bytes and norms, prefetched into registers a tile ahead             global loads
+//        byte -> half2 table lookups, K~ and V~ into the swizzled operand layouts   dequantising warps
+//        S = Qhi K~^T + Qlo K~^T                        (fp32 in tensor memory)     tcgen05.mma
+//        x knorm, mask, lazy online softmax, P = p * vnorm as fp16 hi + lo          softmax warps
+//        O += Plo V~ + Phi V~                                                       tcgen05.mma
+//   3. un-rotate: O / l as fp16 hi + lo times the same image of Pi (read as the other operand major), and
+//      store the caller's output.  Nothing but queries, cache and outputs touches global memory.
+//
+// Why this shape: a tile costs the tensor pipe 2 x 528 cycles per 128 rows (head_dim 128, two terms), the
+// softmax about 1 500 cycles of latency-bound CUDA-core work and the dequantisation about 600 of
+// shared-memory traffic.  With one row block per CTA these formed one chain of 3 550 cycles a tile; with
+// two blocks the tensor pipe works on one while the other is in its softmax, and a dequantised tile serves
+// 256 rows.  Everything meets at mbarriers only: softmax warps (a thread per row; two at head_dim 256),
+// eight dequantising warps and one issuing thread.
+//   Tensor memory, per block: [S | P in place][Q hi][Q lo][O]: 64 + 64 + 128 columns at head_dim 128, where
+//   Q lo does not fit and sits in shared memory; at head_dim 256 there is one block of 448 columns and the 64 left
+//   hold a second S, so that the scores of the next tile are computed during the softmax of this one.
+//   P overwrites S half by half: the columns of tokens 32 h .. + 31 become P hi and P lo of those tokens.
+//
+// A block with few CTAs is cut along the keys (gridDim.z): each part leaves its normalised rotated rows and
+// their log-sum-exp in the scratch, and the merge kernel folds and un-rotates them.
+// Every wait is bounded; a wait that gives up marks the CTA dead, all roles drain, TQ4_DEV_TIMEOUT is raised.
 #include <math_constants.h>
 
 #include <cstdlib>
-#include <cstring>
 #include <type_traits>
 
 #include "tq4_attention.cuh"
 
 namespace tq4 {
 #ifdef TQ4_TRACE
-// Tuning builds only (-DTQ4_TRACE): the SM clock at points of the tile loop, for four warps of one
-// CTA, read back with tq4_prefill_trace_read.  Compiled out of the shipped library.
-__device__ long long g_ptrace[4][64][16];
-#define PF_STAMP(j, e)                                                                              \
-  do {                                                                                              \
-    if (blockIdx.x == 40 && blockIdx.y == 3 && lane == 0 && (j) < 64 &&                             \
-        (warp == 0 || warp == 4 || warp == TQ4_PREFILL_TPR * 4 || warp == TQ4_PREFILL_TPR * 4 + 7))       \
-      g_ptrace[warp == 0 ? 0 : warp == 4 ? 1 : warp == TQ4_PREFILL_TPR * 4 ? 2 : 3][j][e] = clock64();  \
+// Tuning builds only (-DTQ4_TRACE): the SM clock at points of the tile loop for four warps of one CTA, read
+// back with tq4_prefill_trace_read.  Compiled out of the shipped library.
+__device__ long long g_ptrace[4][64][8];
+#define PF_STAMP(role, j, e)                                                                            \
+  do {                                                                                                  \
+    if (blockIdx.x == gridDim.x / 2 && blockIdx.y == 0 && blockIdx.z == 0 && (role) >= 0 && (j) < 64)   \
+      g_ptrace[(role) & 3][j][e] = clock64();                                                           \
   } while (0)
 #else
-#define PF_STAMP(j, e) do {} while (0)
+#define PF_STAMP(role, j, e) do {} while (0)
 #endif
 namespace {
 
-constexpr int kD = 128;
-constexpr int kBN = 64;                 // tokens per tile
-#ifndef TQ4_PREFILL_TPR
-#define TQ4_PREFILL_TPR 2
-#endif
-constexpr int kTPR = TQ4_PREFILL_TPR;     // softmax threads per row (2 or 4)
-constexpr int kCols = kBN / kTPR;         // score columns per softmax thread
-constexpr int kOCols = kD / kTPR;         // output columns per softmax thread
-constexpr int kSmx = 128 * kTPR;          // softmax warps 0 .. 4 kTPR - 1
-constexpr int kDeq = 256;                 // then eight warps that dequantise
-constexpr int kThreads = kSmx + kDeq;
-constexpr int kIssueWarp = kSmx / 32;     // one thread of warp 8 also issues the MMAs,
-constexpr int kCopyWarp = kThreads / 32 - 1;  // the last four warps issue the TMA copies, one page each
-// tensor memory (all 512 columns: one CTA per SM): S (two buffers) [0, 64) and [64, 128), O [128, 256),
-// Q hi [256, 320) and lo [320, 384) (128 dims, two per column), P hi [384, 416) and lo [416, 448)
-constexpr uint32_t kTmemCols = 512;
-constexpr uint32_t kColS = 0, kColO = 128, kColQ = 256, kColQlo = 320, kColP = 384, kColPlo = 416;
+constexpr int kBN = 64;         // tokens per tile
+constexpr int kSmx = 256;       // warps 0-7: softmax, prologue and epilogue of the rows
+constexpr int kDeq = 256;       // warps 8-15: dequantisation
+constexpr int kThreads = kSmx + kDeq + 32;
+constexpr int kIssueWarp = (kSmx + kDeq) / 32;
+constexpr int kNormBufs = 4;
 
-// shared-memory map (offsets from a 1024-byte aligned base)
-constexpr uint32_t kOffK = 0;                         // 2 buffers x 2 K-blocks x [64 tok][128 B]
-constexpr uint32_t kOffV = kOffK + 32768;             // 2 buffers x 2 MN-blocks x [64 tok][128 B]
-constexpr uint32_t kOffStage = kOffV + 32768;         // 2 x (4 pages x 2048 B indices + 4 x 512 B norms)
-constexpr uint32_t kStageBytes = 4 * 2048 + 4 * 512;
-// byte -> half2 tables of K and V, 32 copies of every entry side by side: lane l reads copy l, so a
-// warp's 32 lookups always hit 32 different banks (with 16 copies 43 % of the kernel's shared-memory
-// wavefronts were conflicts of these lookups)
-constexpr int kLutCopies = 32;
-constexpr uint32_t kOffLut = kOffStage + 2 * kStageBytes;   // 2 tables x 256 entries x 16 copies x 4 B
-constexpr uint32_t kOffNorm = kOffLut + 2 * 256 * kLutCopies * 4;  // 2 buffers x (kn[64], vn[64], lg[64])
-constexpr uint32_t kOffXchg = kOffNorm + 2 * 3 * 64 * 4;     // [4][128 rows] floats exchanged by the threads of a row
-constexpr uint32_t kSmemBytes = kOffXchg + 4 * 128 * 4;
-static_assert(2 * (kSmemBytes + 1024) > 227 * 1024, "one CTA per SM: it allocates the whole tensor memory");
+template <int D>
+struct Cfg {
+  static constexpr int NBLK = D == 256 ? 1 : 2;            // row blocks per CTA
+  static constexpr int TPR = D == 256 ? 2 : 1;             // softmax threads per row
+  static constexpr int CPT = kBN / TPR;                    // score columns per softmax thread
+  static constexpr int DPT = D / TPR;                      // coordinates per softmax thread
+  static constexpr int NC = (D + 63) / 64;                 // 64-coordinate blocks of a row
+  static constexpr int NS = D / 32;                        // 16-byte segments of a packed row
+  static constexpr int NKB = D == 256 ? 1 : 2;             // K~ and V~ buffers
+  static constexpr int NIT = (kBN * NS + kDeq - 1) / kDeq;  // segments per dequantising thread
+  static constexpr bool QLO_SMEM = D >= 128;               // Q lo in shared memory
+  // tensor-memory columns of a block (two S at head_dim 256)
+  static constexpr uint32_t kNS = D == 256 ? 2 : 1;
+  static constexpr uint32_t kColS = 0, kColQ = 64 * kNS, kColQlo = kColQ + D / 2;
+  static constexpr uint32_t kColO = kColQ + (QLO_SMEM ? D / 2 : D);
+  static constexpr uint32_t kBlkCols = kColO + D;
+  static_assert(NBLK * kBlkCols <= 512, "tensor memory");
+  // shared memory, from a 1024-byte boundary
+  static constexpr uint32_t kKvBuf = NC * kBN * 128;       // one K~ or V~ buffer
+  static constexpr uint32_t kImgPart = (D == 256 ? 64 : D) * 128;  // a column block of one chunk of Pi's image
+  static constexpr int kChunks = D == 256 ? 4 : 1;         // chunks of 64 (D = 256) or all of the output coordinates
+  static constexpr uint32_t kOffK = 0;
+  static constexpr uint32_t kOffV = kOffK + NKB * kKvBuf;
+  static constexpr uint32_t kKvEnd = kOffV + NKB * kKvBuf;
+  static constexpr uint32_t kImg = 2 * NC * kImgPart;      // the image (chunk) shares the K~ / V~ buffers
+  static constexpr uint32_t kOffQlo = kKvEnd > kImg ? kKvEnd : kImg;
+  static constexpr uint32_t kOffLut = kOffQlo + (QLO_SMEM ? NBLK * NC * 128 * 128 : 0);
+  static constexpr int kLutCopies = D == 256 ? 16 : 32;    // (16: room; every lookup is then a two-way conflict)
+  static constexpr uint32_t kOffNorm = kOffLut + 2 * 256 * kLutCopies * 4;
+  static constexpr uint32_t kOffXchg = kOffNorm + kNormBufs * 3 * kBN * 4;
+  static constexpr uint32_t kSmem = kOffXchg + (TPR == 2 ? 2 * 2 * 128 * 4 : 0);
+  __host__ __device__ static constexpr uint32_t idesc(uint32_t n, bool b_mn) {  // kind::f16: fp16 operands, fp32 accumulator, M = 128
+    return (1u << 4) | (b_mn ? 1u << 16 : 0u) | ((n >> 3) << 17) | ((128u >> 4) << 24);
+  }
+};
 
-// instruction descriptors (kind::f16, fp16 operands, fp32 accumulator, M = 128)
-constexpr uint32_t kDescS = (1u << 4) | ((64u >> 3) << 17) | ((128u >> 4) << 24);                // N = 64, B K-major
-constexpr uint32_t kDescO = (1u << 4) | (1u << 16) | ((128u >> 3) << 17) | ((128u >> 4) << 24);  // N = 128, B MN-major
+struct PrefillArgs {
+  const uint8_t* image;  // Pi's operand image (pi_image_kernel)
+  int min_rows;          // sequences with fewer new rows are left to the streaming kernel
+  int splits;            // parts of the key range
+  int to_parts;          // leave partials for the merge kernel instead of writing the output
+  float* part_o;         // [splits][rows][Hq][D] normalised, rotated
+  float* part_m;         // [splits][rows][Hq] natural-log LSE
+};
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+// 16-byte chunk c of row `row` inside a [rows][128 B] block, 128-byte swizzle
 __device__ __forceinline__ uint32_t swz(int row, int c) { return (uint32_t)(row * 128 + ((c ^ (row & 7)) << 4)); }
-
-// K-major operand, 128-byte swizzle: 8-row groups 1024 bytes apart
-__device__ __forceinline__ uint64_t desc_kmajor(uint32_t saddr) {
-  return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) |
+// operand descriptor, 128-byte swizzle, 8-row groups 1024 bytes apart; `lbo`: distance of the 64-element blocks
+// of an MN-major operand (K-major: unused)
+__device__ __forceinline__ uint64_t make_desc(uint32_t saddr, uint32_t lbo) {
+  return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo ? lbo >> 4 : 1) << 16) | ((uint64_t)(1024 >> 4) << 32) |
          ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
-// MN-major operand, 128-byte swizzle: 64-element MN blocks `lbo` bytes apart, 8-row K groups 1024 bytes apart
-__device__ __forceinline__ uint64_t desc_mnmajor(uint32_t saddr, uint32_t lbo) {
-  return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)(lbo >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) |
-         ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
-}
-// D (tensor memory) (+)= A * B with the A operand (128 rows x 16 fp16 = 8 columns) read from tensor memory
-__device__ __forceinline__ void mma_f16_ta(uint32_t tmem_d, uint32_t tmem_a, uint64_t db, uint32_t idesc, uint32_t acc) {
+// D (tensor memory) (+)= A * B, A (128 rows x 16 fp16 = 8 columns) from tensor memory
+__device__ __forceinline__ void mma_ta(uint32_t d, uint32_t a, uint64_t b, uint32_t idesc, bool acc) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %6, %7, %8}, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(db), "r"(idesc), "r"(acc), "r"(0u), "r"(0u), "r"(0u), "r"(0u)
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
+      ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(acc ? 1u : 0u), "r"(0u)
+      : "memory");
+}
+// the same with A from shared memory
+__device__ __forceinline__ void mma_sa(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, bool acc) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}"
+      ::"r"(d), "l"(a), "l"(b), "r"(idesc), "r"(acc ? 1u : 0u), "r"(0u)
       : "memory");
 }
 __device__ __forceinline__ void mma_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
-__device__ __forceinline__ bool bar_wait_bounded(uint32_t bar, uint32_t parity) {
+__device__ __forceinline__ void bar_init(uint32_t bar, uint32_t count) {
+  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count) : "memory");
+}
+__device__ __forceinline__ void bar_arrive(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+// Bounded wait that also gives up as soon as another role has marked the CTA dead; marks it itself otherwise.
+__device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, volatile int* dead) {
   for (int it = 0; it < (1 << 22); ++it) {
     uint32_t done;
     asm volatile(
@@ -121,8 +149,17 @@ __device__ __forceinline__ bool bar_wait_bounded(uint32_t bar, uint32_t parity) 
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(done) : "r"(bar), "r"(parity) : "memory");
     if (done) return true;
+    if ((it & 1023) == 1023 && *dead) return false;
   }
+  *dead = 1;
   return false;
+}
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
+}
+__device__ __forceinline__ void expect_tx(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ bool elect_one_sync() {
   uint32_t pred;
@@ -133,14 +170,11 @@ __device__ __forceinline__ bool elect_one_sync() {
       : "=r"(pred));
   return pred != 0;
 }
-__device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap* map, int x, int y, int z, int w,
-                                            uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
-      ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(w), "r"(bar)
-      : "memory");
-}
-// 32 consecutive fp32 columns of this thread's TMEM lane
+__device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void fence_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
+// 32 consecutive 32-bit columns of this thread's tensor-memory lane (with the wait)
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
@@ -153,51 +187,26 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
       : "memory");
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
-// 16 consecutive fp32 columns of this thread's TMEM lane
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
-      "%14, %15}, [%16];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-        "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-      : "r"(taddr)
-      : "memory");
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-// 8 consecutive 32-bit columns of this thread's TMEM lane (no wait: the caller waits once)
-__device__ __forceinline__ void tmem_ld16_nowait(uint32_t taddr, uint32_t (&v)[16]) {  // the caller waits
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
-      "%14, %15}, [%16];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-        "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-      : "r"(taddr)
-      : "memory");
-}
-// wait for the loads in flight; the registers are named so that no use of them moves above the wait
-__device__ __forceinline__ void tmem_ld_wait16(uint32_t (&v)[16]) {
-  asm volatile("tcgen05.wait::ld.sync.aligned;"
-               : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]),
-                 "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15])
-               :
-               : "memory");
-}
-__device__ __forceinline__ void tmem_st8_nowait(uint32_t taddr, const uint32_t (&v)[8]) {
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
-      ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
-      : "memory");
-}
-__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {  // (no wait)
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
       "%15, %16};"
       ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
         "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
       : "memory");
-  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 }
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32]) {  // (no wait)
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
+      "%15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
+      ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
+        "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]),
+        "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]),
+        "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
+      : "memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+
 __device__ __forceinline__ float ex2_approx(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -208,575 +217,932 @@ __device__ __forceinline__ float lg2_approx(float x) {
   asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float y;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(y) : "f"(a), "f"(b), "f"(c));
+  return y;
+}
+// pairs of fp32 values in one 64-bit register: one instruction does both
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 pack2(float lo, float hi) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ f2 mul2(f2 a, f2 b) {
+  f2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+  f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
 __device__ __forceinline__ uint32_t pack_h2(float lo, float hi) {
   __half2 h = __floats2half2_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&h);
 }
-
-// G = query heads per KV head (1, 2, 4 or 8); a block holds RB = 128 / G query rows.
-// FAST: the queries and the probabilities enter the MMAs as ONE fp16 term each instead of hi + lo
-// (half the tensor work and no remainder arithmetic; their rounding, 2^-11 relative, then reaches
-// the output: about 1e-3 absolute instead of 1e-5).
-template <int G, bool FAST>
-__global__ void __launch_bounds__(kThreads, 1)
-prefill_tc_kernel(const AttnArgs a, const __grid_constant__ CUtensorMap tm_idx,
-                  const __grid_constant__ CUtensorMap tm_norm) {
-  constexpr int RB = 128 / G;
-  extern __shared__ __align__(1024) unsigned char smem_raw[];
-  __shared__ __align__(8) uint64_t s_bar[5];  // [0], [1]: tile stages (TMA), [2], [3]: S buffer ready, [4]: PV done
-  __shared__ uint32_t s_tmem;
-  __shared__ int s_info[4];                   // sequence, first local row, rows in block, dead flag
-  const AttnShape& sh = a.sh;
-  const AttnPlan& p = a.plan;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int kvh = blockIdx.y;
-
-  pdl_trigger();
-  pdl_wait();  // plan and rotated queries come from the prologue kernel, the cache from the write
-
-  // ---- which (sequence, row block) is this CTA's? ----------------------------------------------
-  if (tid == 0) {
-    const int lo_all = sh.row_offset, hi_all = sh.row_offset + sh.rows;
-    int acc = 0, found = -1, first = 0, nrows = 0;
-    for (int s = 0; s < sh.num_seqs && found < 0; ++s) {
-      const int q0 = max(a.query_start_loc[s], lo_all), q1 = min(a.query_start_loc[s + 1], hi_all);
-      if (q1 <= q0) continue;
-      const int nb = (q1 - q0 + RB - 1) / RB;
-      if ((int)blockIdx.x < acc + nb) {
-        found = s;
-        first = q0 + ((int)blockIdx.x - acc) * RB;
-        nrows = min(RB, q1 - first);
-      }
-      acc += nb;
-    }
-    s_info[0] = found;
-    s_info[1] = first - sh.row_offset;
-    s_info[2] = nrows;
-    s_info[3] = 0;
+// two values -> fp16 hi pair and fp16 pair of what the rounding left
+__device__ __forceinline__ void split2(float x0, float x1, uint32_t& hi, uint32_t& lo) {
+  const __half2 h = __floats2half2_rn(x0, x1);
+  const float2 f = __half22float2(h);
+  hi = *reinterpret_cast<const uint32_t*>(&h);
+  lo = pack_h2(x0 - f.x, x1 - f.y);
+}
+// power of two that brings a value into [1, 2), and its inverse
+__device__ __forceinline__ void pow2_scale(float amax, float& sc, float& isc) {
+  sc = isc = 1.f;
+  if (amax > 0.f && amax < CUDART_INF_F) {
+    const int e = min(max((int)((__float_as_uint(amax) >> 23) & 0xFFu) - 127, -100), 100);
+    sc = __uint_as_float((uint32_t)(127 - e) << 23);
+    isc = __uint_as_float((uint32_t)(127 + e) << 23);
   }
-  __syncthreads();
-  const int seq = s_info[0], lr0 = s_info[1], nrows = s_info[2];
-  if (seq < 0) return;  // grid is an upper bound on the number of blocks
+}
 
+// 32 consecutive elements i .. i + 31 of a typed tensor
+__device__ __forceinline__ void load32(const void* q, int dtype, int64_t i, bool vec_ok, float (&x)[32]) {
+  if (!vec_ok) {
+#pragma unroll
+    for (int e = 0; e < 32; ++e) x[e] = load_as_float(q, dtype, i + e);
+    return;
+  }
+  if (dtype == TQ4_F32) {
+    const float4* p = reinterpret_cast<const float4*>(reinterpret_cast<const float*>(q) + i);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      const float4 v = __ldg(p + e);
+      x[4 * e] = v.x; x[4 * e + 1] = v.y; x[4 * e + 2] = v.z; x[4 * e + 3] = v.w;
+    }
+    return;
+  }
+  const uint4* p = reinterpret_cast<const uint4*>(reinterpret_cast<const uint16_t*>(q) + i);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const uint4 v = __ldg(p + e);
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      if (dtype == TQ4_F16) {
+        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[k]));
+        x[8 * e + 2 * k] = f.x; x[8 * e + 2 * k + 1] = f.y;
+      } else {
+        x[8 * e + 2 * k] = __uint_as_float(w[k] << 16);
+        x[8 * e + 2 * k + 1] = __uint_as_float(w[k] & 0xFFFF0000u);
+      }
+    }
+  }
+}
+
+// Pi's operand image: [term: fp16 hi, lo of 2^8 Pi][64-column block][row of Pi][128 B, swizzled].  As a K-major
+// operand its rows are output coordinates (rotation), as an MN-major one they are input coordinates
+// (un-rotation).  Columns past head_dim (D = 96) are zero.
+template <int D>
+__global__ void __launch_bounds__(256) pi_image_kernel(const float* __restrict__ rotation, uint8_t* __restrict__ image) {
+  constexpr int NC = (D + 63) / 64;
+  pdl_trigger();
+  const int i = (int)(blockIdx.x * 256 + threadIdx.x);  // (row, 8-column chunk)
+  if (i >= D * NC * 8) return;
+  const int r = i / (NC * 8), k8 = i - r * (NC * 8), c = k8 >> 3;
+  uint32_t hi[4], lo[4];
+#pragma unroll
+  for (int e = 0; e < 4; ++e) {
+    const int col = 8 * k8 + 2 * e;
+    const float x0 = col < D ? 256.f * __ldg(rotation + (size_t)r * D + col) : 0.f;
+    const float x1 = col < D ? 256.f * __ldg(rotation + (size_t)r * D + col + 1) : 0.f;
+    split2(x0, x1, hi[e], lo[e]);
+  }
+  uint8_t* dst = image + (size_t)c * D * 128 + swz(r, k8 & 7);
+  *reinterpret_cast<uint4*>(dst) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+  *reinterpret_cast<uint4*>(dst + (size_t)NC * D * 128) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+}
+
+struct Bars {
+  uint64_t kready[2], vready[2];  // dequantising warps -> issuer: K~ / V~ buffer written
+  uint64_t kfree[2], vfree[2];    // MMAs -> dequantising warps: buffer read
+  uint64_t sready[2];             // MMAs -> softmax: scores of the block (head_dim 256: of the tile's S buffer) complete
+  uint64_t pready[2];             // softmax warps -> issuer: P written
+  uint64_t pvd;                   // MMAs -> softmax: O updated (head_dim 256; elsewhere sready implies it)
+  uint64_t img, cdone;            // image chunk landed / used
+  uint64_t aready, rot;           // A operand of a rotation staged / rotation complete
+  uint64_t pair[4];               // the two warps of a row quadrant (head_dim 256)
+  uint64_t qready, odone;         // queries in place / last MMA of the tile loop complete
+};
+
+template <int D, bool FAST>
+__global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs a, const PrefillArgs pa) {
+  using C = Cfg<D>;
+  constexpr int NBLK = C::NBLK, TPR = C::TPR, CPT = C::CPT, DPT = C::DPT, NC = C::NC, NKB = C::NKB, NIT = C::NIT;
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  __shared__ __align__(8) Bars s_bars;
+  __shared__ uint32_t s_tmem;
+  __shared__ int s_info[4];      // sequence, first row, rows, - of the CTA
+  __shared__ int s_dead, s_bad;  // a wait gave up / some page id is out of range
+  const AttnShape& sh = a.sh;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int kvh = blockIdx.y, G = sh.G, RB = 128 / G;
+  volatile int* dead = &s_dead;
+  auto bar = [](const uint64_t& b) { return smem_addr(&b); };
   const uint32_t base = (smem_addr(smem_raw) + 1023u) & ~1023u;
   unsigned char* sm = smem_raw + (base - smem_addr(smem_raw));
-  const uint32_t bar_t0 = smem_addr(&s_bar[0]), bar_s0 = smem_addr(&s_bar[2]), bar_o = smem_addr(&s_bar[4]);
-  if (tid == 0) {
-#pragma unroll
-    for (int i = 0; i < 5; ++i)
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar_t0 + 8 * i) : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  }
+
+  // ---- which rows are this CTA's?  Sequences in order, a sequence's last rows (the longest) first --------
   if (warp == 0) {
-    __syncwarp();
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&s_tmem)),
-                 "r"(kTmemCols) : "memory");
+    int acc = 0, found = -1, first = 0, nrows = 0;
+    for (int s0 = 0; s0 < sh.num_seqs && found < 0; s0 += 32) {
+      const int s = s0 + lane;
+      int q0 = 0, q1 = 0;
+      if (s < sh.num_seqs) {
+        q0 = max(a.query_start_loc[s], 0);
+        q1 = min(a.query_start_loc[s + 1], sh.rows);
+      }
+      const int n = q1 - q0 >= max(pa.min_rows, 1) ? (q1 - q0 + NBLK * RB - 1) / (NBLK * RB) : 0;
+      int incl = n;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int up = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += up;
+      }
+      const int x = (int)blockIdx.x - acc;
+      const unsigned m = __ballot_sync(0xffffffffu, x < incl);
+      if (m) {
+        const int w = __ffs(m) - 1;
+        const int b = n - 1 - (x - (incl - n));  // (lane w: its block, counted from the end)
+        found = s0 + w;
+        first = __shfl_sync(0xffffffffu, q0 + b * NBLK * RB, w);
+        nrows = __shfl_sync(0xffffffffu, min(NBLK * RB, q1 - (q0 + b * NBLK * RB)), w);
+      }
+      acc += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) {
+      s_info[0] = found;
+      s_info[1] = first;
+      s_info[2] = nrows;
+      s_dead = 0;
+      s_bad = 0;
+    }
+  }
+  if (tid == 64) {
+    for (int i = 0; i < 2; ++i) {
+      bar_init(bar(s_bars.kready[i]), kDeq / 32);
+      bar_init(bar(s_bars.vready[i]), kDeq / 32);
+      bar_init(bar(s_bars.kfree[i]), 1);
+      bar_init(bar(s_bars.vfree[i]), 1);
+      bar_init(bar(s_bars.sready[i]), 1);
+      bar_init(bar(s_bars.pready[i]), NBLK == 2 ? 4 : 8);
+    }
+    for (int i = 0; i < 4; ++i) bar_init(bar(s_bars.pair[i]), 2);
+    bar_init(bar(s_bars.pvd), 1);
+    bar_init(bar(s_bars.img), 1);
+    bar_init(bar(s_bars.cdone), 1);
+    bar_init(bar(s_bars.aready), 8);
+    bar_init(bar(s_bars.rot), 1);
+    bar_init(bar(s_bars.qready), 8);
+    bar_init(bar(s_bars.odone), 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    fence_async();
+  }
+  __syncthreads();
+  const int seq = s_info[0], row0 = s_info[1], nrows = s_info[2];
+  if (seq < 0) {  // the grid is an upper bound
+    pdl_trigger();
+    pdl_wait();
+    return;
+  }
+  if (warp == kIssueWarp) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&s_tmem)), "r"(512u) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  // byte -> half2 tables: (centroid[hi nibble], centroid[lo nibble]) scaled onto the fp16 grid
+  // byte -> half2 tables: (centroid[hi nibble], centroid[lo nibble]) scaled onto the fp16 grid, one copy per lane
   {
-    uint32_t* lut = reinterpret_cast<uint32_t*>(sm + kOffLut);
-    for (int i = tid; i < 512 * kLutCopies; i += kThreads) {
-      const int e = i / kLutCopies, w = e >> 8, b = e & 255;
+    uint32_t* lut = reinterpret_cast<uint32_t*>(sm + C::kOffLut);
+    for (int i = tid; i < 512 * C::kLutCopies / 4; i += kThreads) {
+      const int e = i / (C::kLutCopies / 4), w = e >> 8, b = e & 255;
       const float* cent = w ? a.v_centroids : a.k_centroids;
       const int nc = w ? a.n_v_centroids : a.n_k_centroids;
       const float sc = w ? a.lut_scale_v : a.lut_scale_k;
-      const float c_hi = (b >> 4) < nc ? __fmul_rn(sc, cent[b >> 4]) : 0.f;
-      const float c_lo = (b & 15) < nc ? __fmul_rn(sc, cent[b & 15]) : 0.f;
-      lut[i] = pack_h2(c_hi, c_lo);
+      const float c_hi = (b >> 4) < nc ? __fmul_rn(sc, __ldg(cent + (b >> 4))) : 0.f;
+      const float c_lo = (b & 15) < nc ? __fmul_rn(sc, __ldg(cent + (b & 15))) : 0.f;
+      const uint32_t v = pack_h2(c_hi, c_lo);
+      reinterpret_cast<uint4*>(lut)[i] = make_uint4(v, v, v, v);
     }
   }
-  // ---- the block's queries: row m = r * G + g = tensor-memory lane m, scaled by 1 / max|q|, split into
-  //      fp16 hi + lo, two dims per 32-bit column.  A warp reaches lanes 32 * (warp % 4) ..., so thread
-  //      (warp, lane) stages dims [32 * (warp / 4), + 32) of row 32 * (warp % 4) + lane ----------------
-  const int row = 32 * (warp & 3) + lane;
-  const int my_r = row / G, my_g = row % G;
-  float* xchg = reinterpret_cast<float*>(sm + kOffXchg);
-  float qv[32];
-  if (tid < 512) {  // (sixteen warps: four per lane quadrant, 32 dims each)
-    const int part = warp >> 2;
-    float qmax = 0.f;
-    if (my_r < nrows) {
-      const float4* src = reinterpret_cast<const float4*>(
-          p.q_rot + ((int64_t)(lr0 + my_r) * sh.Hq + kvh * G + my_g) * kD + 32 * part);
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const float4 x = src[i];
-        qv[4 * i] = x.x; qv[4 * i + 1] = x.y; qv[4 * i + 2] = x.z; qv[4 * i + 3] = x.w;
-      }
-#pragma unroll
-      for (int i = 0; i < 32; ++i) qmax = fmaxf(qmax, fabsf(qv[i]));
-    } else {
-#pragma unroll
-      for (int i = 0; i < 32; ++i) qv[i] = 0.f;
-    }
-    xchg[part * 128 + row] = qmax;
-  }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();  // the tensor-memory address, the table and the partial maxima are in place
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  pdl_trigger();
+  pdl_wait();  // the operand image of Pi; everything else was complete before the kernel in front started
+  fence_before();
+  __syncthreads();  // tensor-memory address and tables in place
+  fence_after();
   const uint32_t tmem = s_tmem;
-  const uint32_t lane_base = tmem + ((uint32_t)(32 * (warp & 3)) << 16);
-  const float qmax = fmaxf(fmaxf(xchg[row], xchg[128 + row]), fmaxf(xchg[256 + row], xchg[384 + row]));
-  // max|q| * sm_scale * log2(e) / alpha_k: the factor between a stored dot product and the score in
-  // the log2 domain (at least the smallest normal number, so that a hidden score, -inf, times it stays -inf)
-  const float qscale = fmaxf(qmax * (a.scale_log2e / a.lut_scale_k), 1.17549435e-38f);
-  if (tid < 512) {
-    const int part = warp >> 2;
-    const float inv = qmax > 0.f ? 1.f / qmax : 0.f;
-#pragma unroll
-    for (int c = 0; c < 2; ++c) {  // 16 dims = 8 columns at a time
-      uint32_t hi[8], lo[8];
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const float x0 = qv[16 * c + 2 * e] * inv, x1 = qv[16 * c + 2 * e + 1] * inv;
-        const float h0 = __half2float(__float2half_rn(x0)), h1 = __half2float(__float2half_rn(x1));
-        hi[e] = pack_h2(h0, h1);
-        lo[e] = pack_h2(x0 - h0, x1 - h1);
-      }
-      tmem_st8_nowait(lane_base + kColQ + 16 * part + 8 * c, hi);
-      if (!FAST) tmem_st8_nowait(lane_base + kColQlo + 16 * part + 8 * c, lo);
+
+  // ---- keys the CTA needs: rows are in query order, their visible ranges move forward with them -----------
+  const int q_end = a.query_start_loc[seq + 1], len = clamp_seq_len(a, max(0, a.seq_lens[seq]));
+  auto row_keys = [&](int row, int& lo, int& hi) {  // visible keys of row `row` of the call
+    const int pos = len - (q_end - row);
+    hi = max(0, min(a.causal ? pos + 1 : len, len));
+    lo = min(a.sliding_window > 0 ? max(0, pos + 1 - a.sliding_window) : 0, hi);
+  };
+  int blk_lo, blk_hi, t_first = 0, n_tiles = 0;
+  {
+    int x;
+    row_keys(row0, blk_lo, x);
+    row_keys(row0 + nrows - 1, x, blk_hi);
+    if (blk_hi > blk_lo) {
+      t_first = blk_lo / kBN * kBN;
+      n_tiles = (blk_hi - t_first + kBN - 1) / kBN;
+      const int per = (n_tiles + pa.splits - 1) / pa.splits;  // this part of the key range
+      t_first += (int)blockIdx.z * per * kBN;
+      n_tiles = max(0, min(per, n_tiles - (int)blockIdx.z * per));
     }
-    tmem_st_wait();
   }
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-  __syncthreads();  // Q is in tensor memory; the exchange area is free again
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-  // ---- softmax threads: row = TMEM lane = 32 * (warp & 3) + lane, column group = warp >> 2 -----------
-  const bool smx = tid < kSmx;
-  const int qt = (warp >> 2) % kTPR;  // which kCols score columns / kOCols output columns of the row
-  const bool row_live = smx && my_r < nrows;
-  // the threads of a row sit in warps w, w + 4, ...: a named barrier per such group of warps
-  auto pair_sync = [&]() { asm volatile("bar.sync %0, %1;" ::"r"(1 + (warp & 3)), "n"(32 * kTPR) : "memory"); };
-  const int kv_lo = row_live ? p.kv_start[lr0 + my_r] : 0;
-  const int kv_hi = row_live ? p.kv_end[lr0 + my_r] : 0;
-  // keys the block needs: rows are in query order, ranges move forward with the row
-  const int blk_lo = p.kv_start[lr0], blk_hi = p.kv_end[lr0 + nrows - 1];
-  const int t_first = blk_hi > blk_lo ? (blk_lo / kBN) * kBN : 0;
-  const int n_tiles = blk_hi > blk_lo ? (blk_hi - t_first + kBN - 1) / kBN : 0;
-  const int32_t* bt = a.block_table + (int64_t)p.row_seq[lr0] * a.bt_stride;
-  const RowLayout lay = row_layout(sh.Hkv, kD);
-  const int x_idx = lay.k_idx + kvh * 64, x_nrm = (lay.k_norm + kvh * 4) & ~15;
-  const int n_sub = (lay.k_norm + kvh * 4) & 15;
-  const int bs_mask = a.block_size - 1, bs_shift = __ffs(a.block_size) - 1;
+  const int n_blk = nrows > RB ? NBLK : 1;  // row blocks in use
 
-  // one lane issues the boxes of tile j into stage j & 1: 4 pages x (indices K+V, norms K+V)
-  // block ids of the four pages of tile j (read ahead of the copy issue: a global round trip)
-  auto load_blks = [&](int j, int (&blk)[4]) {
-    const int t0 = t_first + j * kBN;
+  if (warp == kIssueWarp) {
+    // ================= issuing thread =================
+    if (n_tiles > 0 && elect_one_sync()) {
+      const uint32_t img = base + C::kOffK;
+      uint32_t img_ph = 0, c_ph = 0;
+      bool ok = true;
+      // chunk ch of the image, as rows (rotation) or as column blocks (un-rotation)
+      auto load_chunk = [&](int ch, bool unrot) {
+        expect_tx(bar(s_bars.img), C::kImg);
+        if (C::kChunks == 1) {
+          bulk_load(img, pa.image, C::kImg, bar(s_bars.img));
+        } else if (unrot) {
+          for (int t = 0; t < 2; ++t)
+            bulk_load(img + t * D * 128, pa.image + (size_t)(t * NC + ch) * D * 128, D * 128, bar(s_bars.img));
+        } else {
+          for (int t = 0; t < 2 * NC; ++t)
+            bulk_load(img + t * C::kImgPart, pa.image + (size_t)t * D * 128 + ch * 64 * 128, C::kImgPart, bar(s_bars.img));
+        }
+      };
+      // O = A * B for the blocks in use: A = fp16 hi (and lo) terms at the S and Q columns, B = the image
+      auto rotate = [&](bool unrot, bool a_lo) {
+        for (int ch = 0; ch < C::kChunks && ok; ++ch) {
+          ok = bar_wait(bar(s_bars.img), img_ph & 1, dead);
+          ++img_ph;
+          if (ch == 0) {
+            ok = bar_wait(bar(s_bars.aready), unrot ? 1u : 0u, dead) && ok;
+            fence_after();
+          }
+          if (!ok) return;
+          constexpr uint32_t N = C::kChunks == 1 ? D : 64;
+          const uint32_t idesc = C::idesc(N, unrot);
+          const uint32_t term = unrot ? (C::kChunks == 1 ? NC * C::kImgPart : D * 128) : NC * C::kImgPart;  // bytes of a term
+          for (int b = 0; b < n_blk; ++b) {
+            const uint32_t tb = tmem + b * C::kBlkCols, d = tb + C::kColO + 64 * ch;
+#pragma unroll 1
+            for (int s = 0; s < D / 16; ++s) {
+              const uint32_t off = unrot ? 2048u * s : (s >> 2) * C::kImgPart + 32u * (s & 3);
+              const uint64_t bh = make_desc(img + off, unrot ? C::kImgPart : 0), bl = make_desc(img + term + off, unrot ? C::kImgPart : 0);
+              mma_ta(d, tb + C::kColS + 8 * s, bl, idesc, s > 0);
+              if (a_lo) mma_ta(d, tb + C::kColQ + 8 * s, bh, idesc, true);
+              mma_ta(d, tb + C::kColS + 8 * s, bh, idesc, true);
+            }
+          }
+          if (ch + 1 < C::kChunks) {
+            mma_commit(bar(s_bars.cdone));
+            ok = bar_wait(bar(s_bars.cdone), c_ph & 1, dead);
+            ++c_ph;
+            if (ok) load_chunk(ch + 1, unrot);
+          }
+        }
+        if (ok) mma_commit(bar(s_bars.rot));
+      };
+      load_chunk(0, false);
+      rotate(false, a.q_dtype == TQ4_F32);
+
+      const uint64_t d_k = make_desc(base + C::kOffK, 0), d_v = make_desc(base + C::kOffV, kBN * 128);
+      const uint64_t d_qlo = make_desc(base + C::kOffQlo, 0);
+      constexpr uint32_t idS = C::idesc(kBN, false), idO = C::idesc(D, true);
+      auto issue_s = [&](int b, int j) {  // S = Q K~^T of tile j
+        const uint32_t tb = tmem + b * C::kBlkCols, d = tb + C::kColS + (NBLK == 1 ? 64 * (j & 1) : 0);
+        const uint64_t dk = d_k + (uint64_t)(((j % NKB) * C::kKvBuf) >> 4);
 #pragma unroll
-    for (int pg = 0; pg < 4; ++pg) {
-      const int pos = t0 + 16 * pg;
-      // A volatile load straight into its register, from a clamped address instead of under a
-      // condition: the ids are used an iteration later; an ordinary load gets moved down to its use, and
-      // a select after the load makes the warp wait a global round trip right here, in every iteration.
-      // (Pages past the block's last key are never issued, whatever id is read for them.)
-      const int pos_c = min(pos, max(blk_hi - 1, 0));
-      asm volatile("ld.global.nc.s32 %0, [%1];" : "=r"(blk[pg]) : "l"(bt + (pos_c >> bs_shift)));
-    }
-  };
-  auto issue_tile = [&](int j, const int (&blks)[4]) {
-    const uint32_t st = base + kOffStage + (uint32_t)(j & 1) * kStageBytes, bar = bar_t0 + 8 * (j & 1);
-    const int t0 = t_first + j * kBN;
-    int npages = 0;
+        for (int s = 0; s < D / 16; ++s) {
+          const uint64_t db = dk + (uint64_t)(((s >> 2) * (kBN * 128) + 32 * (s & 3)) >> 4);
+          if (!FAST) {
+            if (C::QLO_SMEM)
+              mma_sa(d, d_qlo + (uint64_t)((b * NC * 16384 + (s >> 2) * 16384 + 32 * (s & 3)) >> 4), db, idS, s > 0);
+            else
+              mma_ta(d, tb + C::kColQlo + 8 * s, db, idS, s > 0);
+          }
+          mma_ta(d, tb + C::kColQ + 8 * s, db, idS, !FAST || s > 0);
+        }
+        mma_commit(bar(s_bars.sready[NBLK == 1 ? j & 1 : b]));
+      };
+      auto issue_pv = [&](int b, int j) {  // O += P V~ of tile j
+        const uint32_t tb = tmem + b * C::kBlkCols, p = tb + C::kColS + (NBLK == 1 ? 64 * (j & 1) : 0);
+        const uint64_t dv0 = d_v + (uint64_t)(((j % NKB) * C::kKvBuf) >> 4);
 #pragma unroll
-    for (int pg = 0; pg < 4; ++pg) npages += (t0 + 16 * pg < blk_hi) ? 1 : 0;
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(npages * 2560) : "memory");
-#pragma unroll
-    for (int pg = 0; pg < 4; ++pg) {
-      const int pos = t0 + 16 * pg;
-      if (pos < blk_hi) {
-        tma_load_4d(st + pg * 2048, &tm_idx, x_idx, pos & bs_mask, 0, blks[pg], bar);
-        tma_load_4d(st + 8192 + pg * 512, &tm_norm, x_nrm, pos & bs_mask, 0, blks[pg], bar);
+        for (int s = 0; s < 4; ++s) {
+          const uint64_t dv = dv0 + (uint64_t)((2048 * s) >> 4);
+          const uint32_t ph = p + 32 * (s >> 1) + 8 * (s & 1);
+          if (!FAST) mma_ta(tb + C::kColO, ph + 16, dv, idO, j > 0 || s > 0);
+          mma_ta(tb + C::kColO, ph, dv, idO, !FAST || j > 0 || s > 0);
+        }
+      };
+      auto wait_k = [&](int j) { ok = ok && bar_wait(bar(s_bars.kready[j % NKB]), (uint32_t)((j / NKB) & 1), dead); };
+      auto wait_v = [&](int j) { ok = ok && bar_wait(bar(s_bars.vready[j % NKB]), (uint32_t)((j / NKB) & 1), dead); };
+      auto wait_p = [&](int i, int n) { ok = ok && bar_wait(bar(s_bars.pready[i]), (uint32_t)(n & 1), dead); };
+
+      ok = ok && bar_wait(bar(s_bars.qready), 0u, dead);
+      wait_k(0);
+      if (ok) {
+        fence_after();
+        for (int b = 0; b < n_blk; ++b) issue_s(b, 0);
+        mma_commit(bar(s_bars.kfree[0]));
+      }
+      for (int j = 0; j < n_tiles && ok; ++j) {
+        if (NBLK == 1) {  // the next tile's scores go into the other S while this tile is in its softmax
+          if (j + 1 < n_tiles) {
+            wait_k(j + 1);
+            if (!ok) break;
+            fence_after();
+            issue_s(0, j + 1);
+            mma_commit(bar(s_bars.kfree[(j + 1) % NKB]));
+          }
+          PF_STAMP(3, j, 0);
+          wait_v(j);
+          PF_STAMP(3, j, 1);
+          wait_p(j & 1, j >> 1);
+          PF_STAMP(3, j, 2);
+          if (!ok) break;
+          fence_after();
+          issue_pv(0, j);
+          mma_commit(bar(s_bars.vfree[j % NKB]));
+          mma_commit(bar(s_bars.pvd));
+        } else {  // the blocks take turns: while one is in its softmax the other has the tensor pipe
+          for (int b = 0; b < n_blk; ++b) {
+            if (b == 0) wait_v(j);
+            wait_p(b, j);
+            PF_STAMP(3, j, 2 * b);
+            if (!ok) break;
+            fence_after();
+            issue_pv(b, j);
+            if (b == n_blk - 1) mma_commit(bar(s_bars.vfree[j % NKB]));
+            if (j + 1 < n_tiles) {
+              if (b == 0) {
+                wait_k(j + 1);
+                if (!ok) break;
+                fence_after();
+              }
+              issue_s(b, j + 1);
+              if (b == n_blk - 1) mma_commit(bar(s_bars.kfree[(j + 1) % NKB]));
+            }
+            PF_STAMP(3, j, 2 * b + 1);
+          }
+        }
+      }
+      if (ok) {
+        mma_commit(bar(s_bars.odone));
+        if (!pa.to_parts && !a.out_rotated) {  // every MMA has read its operands: the image takes the K~ / V~ buffers again
+          ok = bar_wait(bar(s_bars.odone), 0u, dead);
+          if (ok) {
+            load_chunk(0, true);
+            rotate(true, true);
+          }
+        }
       }
     }
-  };
-
-  // ---- dequantise tile j (its packed stage has landed) into buffer j & 1: 512 items
-  //      (K or V, token, 16-byte segment) spread over threads t of nt; norms by the first 64 --------
-  // (item_lo, item_hi): items [0, 256) are the K half of the tile, [256, 512) the V half
-  auto dequant_tile = [&](int j, int t, int nt, int item_lo, int item_hi) {
-    const unsigned char* stg = sm + kOffStage + (j & 1) * kStageBytes;
-    const uint32_t kv_off = (uint32_t)(j & 1) * 16384u;
-    for (int item = item_lo + t; item < item_hi; item += nt) {
-      // 32 consecutive items = 8 tokens x 4 segments; a quarter warp takes 4 tokens x the 2 segments of
-      // one K-block, so that its eight 16-byte stores below (chunk ^ (token & 7)) fall into eight
-      // different bank groups (token-major order made every store a two-way conflict)
-      const int r8 = item & 7, q4 = (item >> 3) & 3;
-      const int u = item >> 8, tok = ((item >> 5) & 7) * 8 + 4 * (q4 & 1) + (r8 & 3), seg = (r8 >> 2) + 2 * (q4 >> 1);
-      const uint4 pk = *reinterpret_cast<const uint4*>(stg + (tok >> 4) * 2048 + u * 1024 + (tok & 15) * 64 + seg * 16);
-      const uint32_t* lut = reinterpret_cast<const uint32_t*>(sm + kOffLut) + u * 256 * kLutCopies + lane;
+    __syncwarp();
+  } else if (warp >= kSmx / 32) {
+    // ================= dequantising warps =================
+    const int t = tid - kSmx;
+    const RowLayout lay = row_layout(sh.Hkv, D);
+    const int32_t* bt = a.block_table + (int64_t)seq * a.bt_stride;
+    const int bs = a.block_size, shift = (bs & (bs - 1)) == 0 ? __ffs(bs) - 1 : -1;
+    const bool al = ((uintptr_t)a.cache | a.cache_block_stride | a.cache_token_stride) % 16 == 0;
+    const bool k_vec = al && (lay.k_idx + kvh * (D / 2)) % 16 == 0, v_vec = al && (lay.v_idx + kvh * (D / 2)) % 16 == 0;
+    // item n of this thread: token and 16-byte segment of the packed row.  Eight lanes take 4 tokens x the 2 segments
+    // of one 64-coordinate block: their operand stores (chunk ^ (token & 7)) fall into eight bank groups.
+    auto item = [&](int n, int& tok, int& seg) -> bool {
+      constexpr int NP = C::NS / 2;
+      const int i = t + kDeq * n;
+      if (i < 2 * kBN * NP) {
+        const int r8 = i & 7, pg = i >> 4, pair = pg % NP, grp = pg / NP;
+        tok = grp * 8 + 4 * ((i >> 3) & 1) + (r8 & 3);
+        seg = 2 * pair + (r8 >> 2);
+        return true;
+      }
+      tok = i - 2 * kBN * NP;
+      seg = C::NS - 1;
+      return (C::NS & 1) && tok < kBN;
+    };
+    struct Item { int page; uint4 k, v; float kn, vn; };
+    Item it[NIT] = {};
+    int next_page[NIT];
+    auto pos_of = [&](int n, int j) {
+      int tok, seg;
+      return item(n, tok, seg) ? t_first + j * kBN + tok : 0x7fffffff;
+    };
+    auto load_page = [&](int n, int j) -> int {
+      const int pos = pos_of(n, j);
+      if (pos >= blk_hi) return -1;
+      return __ldg(bt + (shift >= 0 ? pos >> shift : pos / bs));
+    };
+    auto load16 = [&](const uint8_t* p, bool vec) -> uint4 {
+      if (vec) return __ldg(reinterpret_cast<const uint4*>(p));
+      const uint32_t* w = reinterpret_cast<const uint32_t*>(p);
+      return make_uint4(__ldg(w), __ldg(w + 1), __ldg(w + 2), __ldg(w + 3));
+    };
+    // row of item n's token, or null (past the keys of the CTA, or a page id out of range: reported and hidden)
+    auto row_of = [&](int n, int j, int page) -> const uint8_t* {
+      const int pos = pos_of(n, j);
+      if (pos >= blk_hi) return nullptr;
+      if (page < 0 || page >= a.num_blocks) {
+        if (a.err_flag) atomicOr(a.err_flag, TQ4_DEV_BAD_BLOCK);
+        s_bad = 1;
+        return nullptr;
+      }
+      const int in = shift >= 0 ? pos & (bs - 1) : pos % bs;
+      return a.cache + (int64_t)page * a.cache_block_stride + (int64_t)in * a.cache_token_stride;
+    };
+    const int kn_off = lay.k_norm + 4 * kvh, vn_off = lay.v_norm + 4 * kvh;
+    auto load_k = [&](int n, int j) {
+      int tok, seg;
+      item(n, tok, seg);
+      const uint8_t* row = row_of(n, j, it[n].page);
+      it[n].k = make_uint4(0, 0, 0, 0);
+      it[n].kn = it[n].vn = row ? 0.f : (pos_of(n, j) < blk_hi ? CUDART_NAN_F : 0.f);  // (NaN: hidden token)
+      if (row) {
+        it[n].k = load16(row + lay.k_idx + kvh * (D / 2) + 16 * seg, k_vec);
+        if (seg == 0) {
+          it[n].kn = __ldg(reinterpret_cast<const float*>(row + kn_off));
+          it[n].vn = __ldg(reinterpret_cast<const float*>(row + vn_off));
+        }
+      }
+    };
+    auto load_v = [&](int n, int j) {
+      int tok, seg;
+      item(n, tok, seg);
+      const uint8_t* row = row_of(n, j, it[n].page);
+      it[n].v = row ? load16(row + lay.v_idx + kvh * (D / 2) + 16 * seg, v_vec) : make_uint4(0, 0, 0, 0);
+    };
+    auto expand = [&](const uint4& pk, int which, uint32_t buf, int tok, int seg) {  // 16 bytes -> 32 fp16
+      const uint32_t* lut = reinterpret_cast<const uint32_t*>(sm + C::kOffLut) + which * 256 * C::kLutCopies + (lane & (C::kLutCopies - 1));
       const uint32_t w[4] = {pk.x, pk.y, pk.z, pk.w};
-      unsigned char* dst = sm + (u ? kOffV : kOffK) + kv_off + (seg >> 1) * 8192;
+      unsigned char* dst = sm + buf + (seg >> 1) * (kBN * 128);
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         const uint32_t x = w[c];
-        const uint4 o = make_uint4(lut[(x & 255) * kLutCopies], lut[((x >> 8) & 255) * kLutCopies],
-                                   lut[((x >> 16) & 255) * kLutCopies], lut[(x >> 24) * kLutCopies]);
+        const uint4 o = make_uint4(lut[(x & 255) * C::kLutCopies], lut[((x >> 8) & 255) * C::kLutCopies],
+                                   lut[((x >> 16) & 255) * C::kLutCopies], lut[(x >> 24) * C::kLutCopies]);
         *reinterpret_cast<uint4*>(dst + swz(tok, (seg & 1) * 4 + c)) = o;
       }
-    }
-    if (item_lo == 0 && t < 64) {
-      const unsigned char* nb = stg + 8192 + (t >> 4) * 512 + (t & 15) * 16 + n_sub;
-      const float kn = *reinterpret_cast<const float*>(nb), vn = *reinterpret_cast<const float*>(nb + 256);
-      float* ns = reinterpret_cast<float*>(sm + kOffNorm) + (j & 1) * 192;
-      ns[t] = kn;
-      ns[64 + t] = vn;
-      ns[128 + t] = fmaxf(lg2_approx(vn), -30.f);
-    }
-  };
-  // one page of tile j by the calling thread; the thread with `first` also posts the byte count of
-  // the whole tile (the stage's barrier has one pending arrival, that one: bytes that land before it
-  // cannot complete the phase)
-  auto issue_page = [&](int j, int pg, int blk, bool first) {
-    const uint32_t st = base + kOffStage + (uint32_t)(j & 1) * kStageBytes, bar = bar_t0 + 8 * (j & 1);
-    const int t0 = t_first + j * kBN;
-    if (first) {
-      int npages = 0;
-#pragma unroll
-      for (int q = 0; q < 4; ++q) npages += (t0 + 16 * q < blk_hi) ? 1 : 0;
-      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(npages * 2560) : "memory");
-    }
-    const int pos = t0 + 16 * pg;
-    if (pos < blk_hi) {
-      tma_load_4d(st + pg * 2048, &tm_idx, x_idx, pos & bs_mask, 0, blk, bar);
-      tma_load_4d(st + 8192 + pg * 512, &tm_norm, x_nrm, pos & bs_mask, 0, blk, bar);
-    }
-  };
-  // descriptors of the operand regions; a byte offset inside a region adds offset / 16 to the
-  // address field (all regions lie below 256 KB, the sum never carries into the other fields)
-  const uint64_t d_k = desc_kmajor(base + kOffK), d_v = desc_mnmajor(base + kOffV, 8192);
-  auto issue_s = [&](int j) {  // S = Q K~^T of tile j (one thread)
-    const uint64_t dk = d_k + (uint64_t)((j & 1) * (16384 >> 4));
-#pragma unroll
-    for (int kb = 0; kb < 2; ++kb)
-#pragma unroll
-      for (int s = 0; s < 4; ++s) {
-        const uint64_t db = dk + (uint64_t)((kb * 8192 + 32 * s) >> 4);
-        const uint32_t qo = (uint32_t)(32 * kb + 8 * s);  // dims 64 kb + 16 s ...: two per column
-        if (!FAST) mma_f16_ta(tmem + kColS + 64 * (j & 1), tmem + kColQlo + qo, db, kDescS, (kb | s) ? 1u : 0u);
-        mma_f16_ta(tmem + kColS + 64 * (j & 1), tmem + kColQ + qo, db, kDescS, (FAST && !(kb | s)) ? 0u : 1u);
-      }
-    mma_commit(bar_s0 + 8 * (j & 1));  // one barrier per S buffer: a waiter can never be two phases behind
-  };
-
-  float m_run = -CUDART_INF_F, l_run = 0.f;
-  bool o_zero = true;  // the O accumulator holds nothing yet (first PV overwrites)
-  // ---- pipeline fill: tiles 0 and 1 in flight, tile 0 dequantised by everybody, S_0 issued ---------
-  if (n_tiles > 0) {
-    if (warp == kCopyWarp && elect_one_sync()) {
-      int b0[4], b1[4];
-      load_blks(0, b0);
-      if (n_tiles > 1) load_blks(1, b1);
-      issue_tile(0, b0);
-      if (n_tiles > 1) issue_tile(1, b1);
-    }
-    const bool ok0 = bar_wait_bounded(bar_t0, 0u);
-    dequant_tile(0, tid, kThreads, 0, 512);
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    if (!ok0) s_info[3] = 1;
-    __syncthreads();
-    if (!s_info[3] && warp == kIssueWarp && elect_one_sync()) {
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      issue_s(0);
-    }
-  }
-
-  int blk_next[4] = {0, 0, 0, 0};  // (copy warp) pages of the tile after next
-  if (warp >= kCopyWarp - 3 && n_tiles > 2) load_blks(2, blk_next);
-  // ---- per tile: warps 0-7 turn S_j into P_j while warps 8-15 dequantise tile j+1 and issue S_{j+1};
-  //      then one thread issues O += P_j V~_j --------------------------------------------------------------
-  bool gave_up = n_tiles > 0 && s_info[3] != 0;  // a bounded wait ran out somewhere in the block
-  for (int j = 0; j < n_tiles && !gave_up; ++j) {
-    const int t0 = t_first + j * kBN;
+    };
+    const int role = tid == kSmx ? 2 : -1;  // (time stamps)
+    (void)role;
     bool ok = true;
-    PF_STAMP(j, 0);
-    if (!smx) {
-      if (j + 1 < n_tiles) {
-        // K~ buffer (j+1) & 1, its norms and S buffer (j+1) & 1 were last used for tile j-1, whose
-        // scores the softmax warps consumed before the block barrier that ended the previous iteration
-        ok = bar_wait_bounded(bar_t0 + 8 * ((j + 1) & 1), (uint32_t)(((j + 1) >> 1) & 1));
-        PF_STAMP(j, 1);
-        dequant_tile(j + 1, tid - kSmx, kDeq, 0, 256);  // keys and norms
-        PF_STAMP(j, 2);
-        // S_{j+1} goes into the other S buffer as soon as its K~ is in place: the softmax warps
-        // find it ready when they finish tile j
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        asm volatile("bar.sync 5, %0;" ::"n"(kDeq) : "memory");
-        const bool okw = __all_sync(0xffffffffu, ok);
-        if (okw && warp == kIssueWarp && elect_one_sync()) {
-          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-          issue_s(j + 1);
-        }
-        PF_STAMP(j, 3);
-        // The packed stage of tile j was dequantised during the previous iteration: tile j + 2 goes into
-        // it, most of an iteration before its turn (its page ids were read an iteration ago; those of
-        // tile j + 3 are read after the values).  Issuing the eight copies takes the thread 1 000 - 2 000 cycles: here
-        // they delay only its warp's share of the values; before the keys they would delay S_{j+1}.
-        // Four warps issue one page each: a copy instruction costs its thread ~190 cycles.
-        if (warp >= kCopyWarp - 3) {
-          const int pg = warp - (kCopyWarp - 3);
-          if (j + 2 < n_tiles && elect_one_sync()) issue_page(j + 2, pg, blk_next[pg], pg == 0);
-          __syncwarp();
-        }
-        // the values of tile j + 1 (only O += P V~ of the next iteration reads them): V~ buffer
-        // (j+1) & 1 was read by the MMAs of tile j-1
-        if (j >= 1) ok = bar_wait_bounded(bar_o, (uint32_t)((j - 1) & 1)) && ok;
-        PF_STAMP(j, 4);
-        dequant_tile(j + 1, tid - kSmx, kDeq, 256, 512);
-        PF_STAMP(j, 5);
-        // (page ids of the tile after that: issued here, they cost the warp nothing before the barrier)
-        if (warp >= kCopyWarp - 3 && j + 3 < n_tiles) load_blks(j + 3, blk_next);
+    if (n_tiles > 0) {
+#pragma unroll
+      for (int n = 0; n < NIT; ++n) it[n].page = load_page(n, 0);
+#pragma unroll
+      for (int n = 0; n < NIT; ++n) {
+        load_k(n, 0);
+        load_v(n, 0);
+        next_page[n] = n_tiles > 1 ? load_page(n, 1) : -1;
       }
-    } else {
-      ok = __all_sync(0xffffffffu, bar_wait_bounded(bar_s0 + 8 * (j & 1), (uint32_t)((j >> 1) & 1)));
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      PF_STAMP(j, 1);
-      const float* ns = reinterpret_cast<const float*>(sm + kOffNorm) + (j & 1) * 192 + kCols * qt;
-      // sc[i] = dot product of column i times its key norm (-inf = not visible); the score in the log2
-      // domain is sc[i] * qscale.  Tiles strictly inside the visible range of every row of the warp
-      // take the short path without per-element masks.
-      float sc[kCols];
-      float mt = -CUDART_INF_F;
-      const bool inner = __all_sync(0xffffffffu, ok && row_live && t0 >= kv_lo && t0 + kBN <= kv_hi);
-      // 16 columns at a time (short register lifetimes); the second load is in flight while the first
-      // half is processed
-      constexpr int NH = kCols / 16;
-      uint32_t vbuf[NH][16];
-      if (ok) {
-        tmem_ld16(lane_base + kColS + 64 * (j & 1) + kCols * qt, vbuf[0]);
-        if (NH == 2) tmem_ld16_nowait(lane_base + kColS + 64 * (j & 1) + kCols * qt + 16, vbuf[NH - 1]);
-      }
+      ok = bar_wait(bar(s_bars.rot), 0u, dead);  // the image of Pi has been used
+    }
+    for (int j = 0; j < n_tiles && ok; ++j) {
+      const int b = j % NKB, u = j / NKB;
+      if (u > 0) ok = bar_wait(bar(s_bars.kfree[b]), (uint32_t)((u - 1) & 1), dead);
+      if (!ok) break;
+      PF_STAMP(role, j, 0);
+      float* ns = reinterpret_cast<float*>(sm + C::kOffNorm) + (j % kNormBufs) * 3 * kBN;
 #pragma unroll
-      for (int hh = 0; hh < NH; ++hh) {
-        if (hh == 1) tmem_ld_wait16(vbuf[NH - 1]);
-        uint32_t (&v)[16] = vbuf[hh];
-        const float4* kn4 = reinterpret_cast<const float4*>(ns + 16 * hh);
-        const float4* lg4 = reinterpret_cast<const float4*>(ns + 128 + 16 * hh);
-        if (inner) {
-#pragma unroll
-          for (int i4 = 0; i4 < 4; ++i4) {
-            const float4 kn = kn4[i4], lg = lg4[i4];
-            const float kk[4] = {kn.x, kn.y, kn.z, kn.w}, ll[4] = {lg.x, lg.y, lg.z, lg.w};
-#pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              const float s = __uint_as_float(v[4 * i4 + e]) * kk[e];
-              sc[16 * hh + 4 * i4 + e] = s;
-              mt = fmaxf(mt, fmaf(s, qscale, ll[e]));
-            }
+      for (int n = 0; n < NIT; ++n) {
+        int tok, seg;
+        if (item(n, tok, seg)) {
+          expand(it[n].k, 0, C::kOffK + b * C::kKvBuf, tok, seg);
+          if (seg == 0) {
+            ns[tok] = it[n].kn;
+            ns[kBN + tok] = it[n].vn;
+            ns[2 * kBN + tok] = fmaxf(lg2_approx(it[n].vn), -30.f);
           }
+        }
+      }
+      fence_async();
+      __syncwarp();
+      if (lane == 0) bar_arrive(bar(s_bars.kready[b]));
+      PF_STAMP(role, j, 1);
+      uint4 v_now[NIT];
+#pragma unroll
+      for (int n = 0; n < NIT; ++n) {
+        v_now[n] = it[n].v;
+        it[n].page = next_page[n];
+        if (j + 1 < n_tiles) {
+          load_k(n, j + 1);
+          load_v(n, j + 1);
+          if (j + 2 < n_tiles) next_page[n] = load_page(n, j + 2);
+        }
+      }
+      PF_STAMP(role, j, 2);
+      if (u > 0) ok = bar_wait(bar(s_bars.vfree[b]), (uint32_t)((u - 1) & 1), dead);
+      if (!ok) break;
+      PF_STAMP(role, j, 3);
+#pragma unroll
+      for (int n = 0; n < NIT; ++n) {
+        int tok, seg;
+        if (item(n, tok, seg)) expand(v_now[n], 1, C::kOffV + b * C::kKvBuf, tok, seg);
+      }
+      fence_async();
+      __syncwarp();
+      if (lane == 0) bar_arrive(bar(s_bars.vready[b]));
+      PF_STAMP(role, j, 4);
+    }
+  } else {
+    // ================= softmax warps: a row (half a row at head_dim 256) per thread =================
+    const int blk = NBLK == 2 ? warp >> 2 : 0, part = NBLK == 2 ? 0 : warp >> 2;
+    const int m = 32 * (warp & 3) + lane, my_r = m / G, my_g = m - my_r * G;
+    const int lrow = blk * RB + my_r;                       // row within the CTA
+    const bool live = my_r < RB && lrow < nrows;
+    const int head = kvh * G + my_g, row = row0 + (live ? lrow : 0);
+    const uint32_t tb = tmem + blk * C::kBlkCols + ((uint32_t)(32 * (warp & 3)) << 16);
+    float* xchg = reinterpret_cast<float*>(sm + C::kOffXchg);
+    // maximum (or sum) over the threads of a row
+    // (two buffers in turn: a warp that starts exchange n + 2 has seen its partner arrive at n + 1, past reading n)
+    uint32_t n_xchg = 0;
+    auto row_reduce = [&](float v, auto op) -> float {
+      if (TPR == 1) return v;
+      float* x = xchg + (n_xchg & 1) * 256;
+      x[part * 128 + m] = v;
+      __syncwarp();
+      if (lane == 0) bar_arrive(bar(s_bars.pair[warp & 3]));
+      const bool got = bar_wait(bar(s_bars.pair[warp & 3]), n_xchg & 1, dead);
+      ++n_xchg;
+      return got ? op(v, x[(part ^ 1) * 128 + m]) : v;
+    };
+    auto fmax_op = [](float x, float y) { return fmaxf(x, y); };
+    auto arrive = [&](uint64_t& b) {  // this warp's share of a hand-over to the issuing thread
+      fence_before();
+      __syncwarp();
+      if (lane == 0) bar_arrive(bar(b));
+    };
+    bool ok = true;
+    const bool use = n_tiles > 0 && blk < n_blk;  // (uniform per warp)
+
+    // ---- rotate the queries -----------------------------------------------------------------------
+    float qscale = 0.f;
+    if (use) {
+      const int es = a.q_dtype == TQ4_F32 ? 4 : 2;
+      const bool vec_ok = ((uintptr_t)a.q % 16 == 0) && (a.q_token_stride * es) % 16 == 0 && (a.q_head_stride * es) % 16 == 0;
+      const int64_t qi = (int64_t)row * a.q_token_stride + (int64_t)head * a.q_head_stride + part * DPT;
+      float amax = 0.f;
+#pragma unroll 1
+      for (int c = 0; c < DPT / 32; ++c) {
+        float x[32];
+        if (live) {
+          load32(a.q, a.q_dtype, qi + 32 * c, vec_ok, x);
+#pragma unroll
+          for (int e = 0; e < 32; ++e) amax = fmaxf(amax, fabsf(x[e]));
+        }
+      }
+      float sc, isc;
+      pow2_scale(row_reduce(amax, fmax_op), sc, isc);
+#pragma unroll 1
+      for (int c = 0; c < DPT / 32; ++c) {
+        float x[32];
+        if (live) {
+          load32(a.q, a.q_dtype, qi + 32 * c, vec_ok, x);
         } else {
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
-            const int pos = t0 + kCols * qt + 16 * hh + i;
-            const bool vis = ok && row_live && pos >= kv_lo && pos < kv_hi;
-            const float s = vis ? __uint_as_float(v[i]) * ns[16 * hh + i] : -CUDART_INF_F;
-            sc[16 * hh + i] = s;
-            mt = fmaxf(mt, vis ? fmaf(s, qscale, ns[128 + 16 * hh + i]) : -CUDART_INF_F);
+          for (int e = 0; e < 32; ++e) x[e] = 0.f;
+        }
+        uint32_t h[16], l[16];
+#pragma unroll
+        for (int e = 0; e < 16; ++e) split2(x[2 * e] * sc, x[2 * e + 1] * sc, h[e], l[e]);
+        tmem_st16(tb + C::kColS + (part * DPT) / 2 + 16 * c, h);
+        if (a.q_dtype == TQ4_F32) tmem_st16(tb + C::kColQ + (part * DPT) / 2 + 16 * c, l);
+      }
+      tmem_st_wait();
+      arrive(s_bars.aready);
+      ok = __all_sync(0xffffffffu, bar_wait(bar(s_bars.rot), 0u, dead));
+      fence_after();
+      // largest coordinate of the rotated row, then its terms at that scale
+      float rmax = 0.f;
+      if (ok) {
+#pragma unroll 1
+        for (int c = 0; c < DPT / 32; ++c) {
+          uint32_t v[32];
+          tmem_ld32(tb + C::kColO + part * DPT + 32 * c, v);
+#pragma unroll
+          for (int e = 0; e < 32; ++e) rmax = fmaxf(rmax, fabsf(__uint_as_float(v[e])));
+        }
+      }
+      rmax = row_reduce(rmax, fmax_op);
+      const float inv = rmax > 0.f ? 1.f / rmax : 0.f;
+      // factor between a stored dot product and the score in the log2 domain (at least the smallest normal
+      // number, so that a hidden score, -inf, times it stays -inf)
+      qscale = fmaxf(rmax * isc * (1.f / 256.f) * (a.scale_log2e / a.lut_scale_k), 1.17549435e-38f);
+      if (ok) {
+#pragma unroll 1
+        for (int c = 0; c < DPT / 32; ++c) {
+          uint32_t v[32], h[16], l[16];
+          const int d0 = part * DPT + 32 * c;
+          tmem_ld32(tb + C::kColO + d0, v);
+#pragma unroll
+          for (int e = 0; e < 16; ++e)
+            split2(__uint_as_float(v[2 * e]) * inv, __uint_as_float(v[2 * e + 1]) * inv, h[e], l[e]);
+          tmem_st16(tb + C::kColQ + d0 / 2, h);
+          if (FAST) continue;
+          if (C::QLO_SMEM) {
+            unsigned char* dst = sm + C::kOffQlo + blk * (NC * 16384) + (d0 >> 6) * 16384;
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+              *reinterpret_cast<uint4*>(dst + swz(m, ((d0 & 63) >> 3) + i)) = make_uint4(l[4 * i], l[4 * i + 1], l[4 * i + 2], l[4 * i + 3]);
+          } else {
+            tmem_st16(tb + C::kColQlo + d0 / 2, l);
           }
         }
       }
-      // the row's maximum over both halves (the decisions below must agree in its two threads)
-      PF_STAMP(j, 2);
-      xchg[qt * 128 + row] = mt;
-      pair_sync();
+      tmem_st_wait();
+      fence_async();
+      arrive(s_bars.qready);
+    } else if (n_tiles > 0) {  // a block without rows
+      arrive(s_bars.aready);
+      arrive(s_bars.qready);
+    }
+
+    // ---- the tile loop --------------------------------------------------------------------------------
+    int kv_lo = 0, kv_hi = 0;
+    if (live) row_keys(row, kv_lo, kv_hi);
+    float m_run = -CUDART_INF_F, l_run = 0.f;
+    const int role = tid == 0 ? 0 : tid == 128 ? 1 : -1;  // (time stamps)
+    (void)role;
+    if (use) {
+      for (int j = 0; j < n_tiles && ok; ++j) {
+        PF_STAMP(role, j, 0);
+        const int t0 = t_first + j * kBN + part * CPT;  // first token of this thread's columns
+        const int sb = NBLK == 1 ? j & 1 : blk;
+        ok = __all_sync(0xffffffffu, bar_wait(bar(s_bars.sready[sb]), (uint32_t)((NBLK == 1 ? j >> 1 : j) & 1), dead));
+        if (!ok) break;
+        PF_STAMP(role, j, 1);
+        fence_after();
+        const uint32_t scol = tb + C::kColS + (NBLK == 1 ? 64 * (j & 1) : 0) + part * CPT;
+        const float* ns = reinterpret_cast<const float*>(sm + C::kOffNorm) + (j % kNormBufs) * 3 * kBN + part * CPT;
+        // dot x key norm (x qscale = score in the log2 domain); two columns per instruction.  Tiles inside
+        // the visible range of every row of the warp take the path without per-element masks.
+        const bool inner = __all_sync(0xffffffffu, t0 >= kv_lo && t0 + CPT <= kv_hi) && !*(volatile int*)&s_bad;
+        const f2 qs2 = pack2(qscale, qscale);
+        auto visible = [&](int i) { return t0 + i >= kv_lo && t0 + i < kv_hi && ns[i] == ns[i]; };
+        float mt = -CUDART_INF_F;
 #pragma unroll
-      for (int o = 1; o < kTPR; ++o) mt = fmaxf(mt, xchg[((qt + o) % kTPR) * 128 + row]);
-      PF_STAMP(j, 3);
-      // P and O are still in use by the MMAs of tile j-1
-      if (j >= 1) ok = __all_sync(0xffffffffu, bar_wait_bounded(bar_o, (uint32_t)((j - 1) & 1))) && ok;
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      PF_STAMP(j, 4);
-      // lazily updated reference: moves only when a score (shifted by log2 of its value norm)
-      // exceeds it by more than 2^8; then this row of O is rescaled in tensor memory
-      const bool bump = mt > m_run + 8.f;
-      if (__any_sync(0xffffffffu, bump)) {
-        const float alpha = bump ? (m_run == -CUDART_INF_F ? 0.f : ex2_approx(m_run - mt)) : 1.f;
-        if (bump) { m_run = mt; l_run *= alpha; }
-        if (!o_zero && ok) {
+        for (int h = 0; h < CPT / 32; ++h) {
+          uint32_t v[32];
+          tmem_ld32(scol + 32 * h, v);
+          if (inner) {
 #pragma unroll
-          for (int q = 0; q < kOCols / 16; ++q) {  // this thread's share of the row's 128 columns
-            uint32_t v[16];
-            tmem_ld16(lane_base + kColO + kOCols * qt + 16 * q, v);
+            for (int i4 = 0; i4 < 8; ++i4) {
+              const ulonglong2 kn = reinterpret_cast<const ulonglong2*>(ns + 32 * h)[i4];
+              const ulonglong2 lg = reinterpret_cast<const ulonglong2*>(ns + 2 * kBN + 32 * h)[i4];
+              float u0, u1, u2, u3;
+              unpack2(fma2(mul2(pack2(__uint_as_float(v[4 * i4]), __uint_as_float(v[4 * i4 + 1])), kn.x), qs2, lg.x), u0, u1);
+              unpack2(fma2(mul2(pack2(__uint_as_float(v[4 * i4 + 2]), __uint_as_float(v[4 * i4 + 3])), kn.y), qs2, lg.y), u2, u3);
+              mt = max3(mt, u0, u1);
+              mt = max3(mt, u2, u3);
+            }
+          } else {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
-            tmem_st16(lane_base + kColO + kOCols * qt + 16 * q, v);
+            for (int i = 0; i < 32; ++i)
+              if (visible(32 * h + i)) mt = fmaxf(mt, fmaf(__uint_as_float(v[i]) * ns[32 * h + i], qscale, ns[2 * kBN + 32 * h + i]));
           }
         }
-      }
-      const float m_neg = m_run == -CUDART_INF_F ? 0.f : -m_run;
-      float lsum = 0.f;
-      const float4* vn4 = reinterpret_cast<const float4*>(ns + 64);
-      // (two instances of the loop: inside the visible range of every row of the warp there is nothing
-      //  to select, which saves two instructions per column)
-      auto exp_phase = [&](auto inner_tag) {
-        constexpr bool INNER = decltype(inner_tag)::value;
+        mt = row_reduce(mt, fmax_op);
+        PF_STAMP(role, j, 2);
+        // lazily updated reference: moves only when a score (shifted by log2 of its value norm) exceeds it
+        // by more than 2^8; then this row of O is rescaled in tensor memory (no MMA is working on it)
+        const bool bump = mt > m_run + 8.f;
+        if (__any_sync(0xffffffffu, bump)) {
+          const float alpha = bump ? (m_run == -CUDART_INF_F ? 0.f : ex2_approx(m_run - mt)) : 1.f;
+          if (bump) { m_run = mt; l_run *= alpha; }
+          if (j > 0) {
+            if (NBLK == 1) {
+              ok = __all_sync(0xffffffffu, bar_wait(bar(s_bars.pvd), (uint32_t)((j - 1) & 1), dead));
+              if (!ok) break;
+              fence_after();
+            }
+#pragma unroll 1
+            for (int c = 0; c < DPT / 32; ++c) {
+              uint32_t v[32];
+              tmem_ld32(tb + C::kColO + part * DPT + 32 * c, v);
 #pragma unroll
-        for (int c = 0; c < kCols / 16; ++c) {  // 16 tokens = 8 columns of P at a time
-          uint32_t h[8], lw[8];
+              for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
+              tmem_st32(tb + C::kColO + part * DPT + 32 * c, v);
+            }
+            tmem_st_wait();
+          }
+        }
+        const float m_neg = m_run == -CUDART_INF_F ? 0.f : -m_run;
+        const f2 mn2 = pack2(m_neg, m_neg);
+        f2 ls2 = pack2(0.f, 0.f);
 #pragma unroll
-          for (int e4 = 0; e4 < 4; ++e4) {
-            const float4 va = vn4[4 * c + e4];
-            const float vv[4] = {va.x, va.y, va.z, va.w};
+        for (int h = 0; h < CPT / 32; ++h) {
+          uint32_t v[32], ph[16], pl[16];
+          tmem_ld32(scol + 32 * h, v);
+          if (inner) {
 #pragma unroll
-            for (int e = 0; e < 2; ++e) {
-              const int t = 16 * c + 4 * e4 + 2 * e;
-              const float e0 = ex2_approx(fmaf(sc[t], qscale, m_neg)), e1 = ex2_approx(fmaf(sc[t + 1], qscale, m_neg));
-              lsum += e0 + e1;
-              // (a hidden column has e = 0; its value norm may be anything, so select instead of multiply)
-              const float v0 = (INNER || sc[t] != -CUDART_INF_F) ? e0 * vv[2 * e] : 0.f;
-              const float v1 = (INNER || sc[t + 1] != -CUDART_INF_F) ? e1 * vv[2 * e + 1] : 0.f;
-              const __half2 hp = __floats2half2_rn(v0, v1);
-              const float2 hf2 = __half22float2(hp);
-              h[2 * e4 + e] = *reinterpret_cast<const uint32_t*>(&hp);
-              if (!FAST) lw[2 * e4 + e] = pack_h2(v0 - hf2.x, v1 - hf2.y);  // the fp16 rounding of the weights is recovered by a second term
+            for (int i4 = 0; i4 < 8; ++i4) {
+              const ulonglong2 kn = reinterpret_cast<const ulonglong2*>(ns + 32 * h)[i4];
+              const ulonglong2 vn = reinterpret_cast<const ulonglong2*>(ns + kBN + 32 * h)[i4];
+#pragma unroll
+              for (int p = 0; p < 2; ++p) {
+                float x0, x1;
+                unpack2(fma2(mul2(pack2(__uint_as_float(v[4 * i4 + 2 * p]), __uint_as_float(v[4 * i4 + 2 * p + 1])), p ? kn.y : kn.x), qs2, mn2), x0, x1);
+                const f2 e = pack2(ex2_approx(x0), ex2_approx(x1));
+                ls2 = add2(ls2, e);
+                unpack2(mul2(e, p ? vn.y : vn.x), x0, x1);
+                if (FAST) ph[2 * i4 + p] = pack_h2(x0, x1);
+                else split2(x0, x1, ph[2 * i4 + p], pl[2 * i4 + p]);
+              }
+            }
+          } else {
+#pragma unroll
+            for (int i2 = 0; i2 < 16; ++i2) {
+              float w[2], e[2];
+#pragma unroll
+              for (int q = 0; q < 2; ++q) {
+                const int i = 32 * h + 2 * i2 + q;
+                const bool vis = visible(i);  // (a hidden column's norms may be anything: select, do not multiply)
+                e[q] = vis ? ex2_approx(fmaf(__uint_as_float(v[2 * i2 + q]) * ns[i], qscale, m_neg)) : 0.f;
+                w[q] = vis ? e[q] * ns[kBN + i] : 0.f;
+              }
+              ls2 = add2(ls2, pack2(e[0], e[1]));
+              if (FAST) ph[i2] = pack_h2(w[0], w[1]);
+              else split2(w[0], w[1], ph[i2], pl[i2]);
             }
           }
-          tmem_st8_nowait(lane_base + kColP + (kCols / 2) * qt + 8 * c, h);
-          if (!FAST) tmem_st8_nowait(lane_base + kColPlo + (kCols / 2) * qt + 8 * c, lw);
+          tmem_st16(scol + 32 * h, ph);
+          if (!FAST) tmem_st16(scol + 32 * h + 16, pl);
         }
-      };
-      if (inner) exp_phase(std::true_type{});
-      else exp_phase(std::false_type{});
-      tmem_st_wait();
-      l_run += lsum;  // (this thread's half of the row sum)
-      PF_STAMP(j, 5);
-    }
-    if (!smx) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // (the dequantised values)
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    gave_up = __syncthreads_or(!ok) != 0;  // (the flag travels with the barrier: no shared-memory read)
-    PF_STAMP(j, 7);
-    if (gave_up) break;
-    if (warp == kIssueWarp && elect_one_sync()) {
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint64_t dvb = d_v + (uint64_t)((j & 1) * (16384 >> 4));
-#pragma unroll
-      for (int s = 0; s < 4; ++s) {
-        const uint64_t dv = dvb + (uint64_t)((2048 * s) >> 4);
-        if (!FAST) mma_f16_ta(tmem + kColO, tmem + kColPlo + 8 * s, dv, kDescO, (!o_zero || s) ? 1u : 0u);
-        mma_f16_ta(tmem + kColO, tmem + kColP + 8 * s, dv, kDescO, (FAST && o_zero && !s) ? 0u : 1u);
+        tmem_st_wait();
+        float s0, s1;
+        unpack2(ls2, s0, s1);
+        l_run += s0 + s1;
+        arrive(s_bars.pready[sb]);
+        PF_STAMP(role, j, 3);
       }
-      mma_commit(bar_o);
     }
-    PF_STAMP(j, 8);
-    o_zero = false;
-  }
-  if (gave_up && tid == 0) s_info[3] = 1;
-  if (n_tiles > 0 && !gave_up) {  // the last tile's MMAs
-    if (!bar_wait_bounded(bar_o, (uint32_t)((n_tiles - 1) & 1))) s_info[3] = 1;
-  }
-  __syncthreads();
 
-  // ---- normalised rotated output + log-sum-exp, as one dense partial per (row, head) ------------
-  const bool dead = s_info[3] != 0;
-  if (smx) {
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    xchg[qt * 128 + row] = l_run;  // the row sum = the shares of its threads
-    pair_sync();
-#pragma unroll
-    for (int o = 1; o < kTPR; ++o) l_run += xchg[((qt + o) % kTPR) * 128 + row];
-    const bool have = !dead && !o_zero && l_run > 0.f;
+    // ---- normalise, un-rotate, store ------------------------------------------------------------------
+    l_run = row_reduce(l_run, [](float x, float y) { return x + y; });
+    bool have = use;
+    if (use) {
+      ok = __all_sync(0xffffffffu, ok && bar_wait(bar(s_bars.odone), 0u, dead));
+      fence_after();
+      have = ok && l_run > 0.f;
+    }
     const float inv = have ? 1.f / (a.lut_scale_v * l_run) : 0.f;
-    const int64_t vec = row_live ? (int64_t)(lr0 + my_r) * sh.Hq + kvh * G + my_g : 0;
+    const float lse = have ? (m_run + lg2_approx(l_run)) * 0.6931471805599453f : -CUDART_INF_F;
+    if (pa.to_parts || a.out_rotated) {
+      const int64_t vec = ((int64_t)blockIdx.z * sh.rows + row) * sh.Hq + head;
+      const int64_t oi = pa.to_parts ? vec * D : (int64_t)row * a.out_token_stride + (int64_t)head * a.out_head_stride;
+      void* dst = pa.to_parts ? (void*)pa.part_o : a.out;
+      const int dt = pa.to_parts ? TQ4_F32 : a.out_dtype;
+#pragma unroll 1
+      for (int c = 0; c < DPT / 32; ++c) {
+        uint32_t v[32];
+        if (use && ok) tmem_ld32(tb + C::kColO + part * DPT + 32 * c, v);
+        if (live) {
 #pragma unroll
-    for (int q = 0; q < kOCols / 32; ++q) {  // this thread's columns
-      uint32_t v[32];
-      if (!o_zero && !dead) {
-        tmem_ld32(lane_base + kColO + kOCols * qt + 32 * q, v);
-      } else {
+          for (int i = 0; i < 8; ++i) {
+            float y[4];
 #pragma unroll
-        for (int i = 0; i < 32; ++i) v[i] = 0u;
+            for (int e = 0; e < 4; ++e) y[e] = have ? __uint_as_float(v[4 * i + e]) * inv : 0.f;
+            store4(dst, dt, oi + part * DPT + 32 * c + 4 * i, y);
+          }
+        }
       }
-      if (row_live) {
-        float4* dst = reinterpret_cast<float4*>(p.part_o + vec * kD + kOCols * qt + 32 * q);
+      if (live && part == 0 && pa.to_parts) pa.part_m[vec] = lse;
+      else if (live && part == 0 && a.lse_out) a.lse_out[(int64_t)row * sh.Hq + head] = lse;
+    } else {
+      float isc = 0.f;
+      if (use) {
+        float amax = 0.f, sc = 1.f;
+        if (ok) {
+#pragma unroll 1
+          for (int c = 0; c < DPT / 32; ++c) {
+            uint32_t v[32];
+            tmem_ld32(tb + C::kColO + part * DPT + 32 * c, v);
 #pragma unroll
-        for (int i = 0; i < 8; ++i)
-          dst[i] = make_float4(__uint_as_float(v[4 * i]) * inv, __uint_as_float(v[4 * i + 1]) * inv,
-                               __uint_as_float(v[4 * i + 2]) * inv, __uint_as_float(v[4 * i + 3]) * inv);
+            for (int i = 0; i < 32; ++i) amax = fmaxf(amax, fabsf(__uint_as_float(v[i]) * inv));
+          }
+        }
+        pow2_scale(row_reduce(amax, fmax_op), sc, isc);
+        if (ok) {
+#pragma unroll 1
+          for (int c = 0; c < DPT / 32; ++c) {
+            uint32_t v[32], h[16], l[16];
+            const int d0 = part * DPT + 32 * c;
+            tmem_ld32(tb + C::kColO + d0, v);
+#pragma unroll
+            for (int e = 0; e < 16; ++e)
+              split2(__uint_as_float(v[2 * e]) * inv * sc, __uint_as_float(v[2 * e + 1]) * inv * sc, h[e], l[e]);
+            tmem_st16(tb + C::kColS + d0 / 2, h);
+            tmem_st16(tb + C::kColQ + d0 / 2, l);
+          }
+        }
+        tmem_st_wait();
+        arrive(s_bars.aready);
+        ok = __all_sync(0xffffffffu, bar_wait(bar(s_bars.rot), 1u, dead)) && ok;
+        fence_after();
+      } else if (n_tiles > 0) {  // (not before the first rotation is over: its phase wants one arrival per warp)
+        bar_wait(bar(s_bars.rot), 0u, dead);
+        arrive(s_bars.aready);
       }
+      const float f = have && ok ? isc * (1.f / 256.f) : 0.f;
+      const int64_t oi = (int64_t)row * a.out_token_stride + (int64_t)head * a.out_head_stride + part * DPT;
+#pragma unroll 1
+      for (int c = 0; c < DPT / 32; ++c) {
+        uint32_t v[32];
+        if (use && ok) tmem_ld32(tb + C::kColO + part * DPT + 32 * c, v);
+        if (live) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            float y[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) y[e] = f != 0.f ? __uint_as_float(v[4 * i + e]) * f : 0.f;
+            store4(a.out, a.out_dtype, oi + 32 * c + 4 * i, y);
+          }
+        }
+      }
+      if (live && part == 0 && a.lse_out) a.lse_out[(int64_t)row * sh.Hq + head] = lse;
     }
-    if (row_live && qt == 0)
-      p.part_m[vec] = have ? (m_run + lg2_approx(l_run)) * 0.6931471805599453f : -CUDART_INF_F;
   }
-  if (dead && tid == 0 && a.err_flag) atomicOr(a.err_flag, TQ4_DEV_TIMEOUT);
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  fence_before();
   __syncthreads();
-  if (warp == 0) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
+  if (s_dead && tid == 0 && a.err_flag) atomicOr(a.err_flag, TQ4_DEV_TIMEOUT);
+  if (warp == kIssueWarp) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
   }
 }
 
-// ---- host side -------------------------------------------------------------------------------------
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
-                                  CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
-                                  CUtensorMapFloatOOBfill);
-EncodeTiledFn encode_fn() {
-  static EncodeTiledFn fn = nullptr;
-  static bool tried = false;
-  if (!tried) {
-    tried = true;
-    void* ptr = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(ptr);
-  }
-  return fn;
-}
-// dims (bytes of one half of a token row, tokens in a block, K/V half, blocks); box = 16 tokens x both halves
-bool make_map(CUtensorMap* m, const AttnArgs& a, uint32_t box_bytes) {
-  EncodeTiledFn fn = encode_fn();
-  if (!fn) return false;
-  const cuuint64_t half_bytes = (cuuint64_t)a.sh.Hkv * (a.sh.D / 2 + 4);
-  const cuuint64_t dims[4] = {half_bytes, (cuuint64_t)a.block_size, 2, (cuuint64_t)a.num_blocks};
-  const cuuint64_t strides[3] = {(cuuint64_t)a.cache_token_stride, half_bytes, (cuuint64_t)a.cache_block_stride};
-  const cuuint32_t box[4] = {box_bytes, 16, 2, 1};
-  const cuuint32_t estr[4] = {1, 1, 1, 1};
-  return fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 4, const_cast<uint8_t*>(a.cache), dims, strides, box, estr,
-            CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_NONE,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
-}
-
-template <int G, bool FAST>
-int launch_t(const AttnArgs& a, cudaStream_t st) {
-  const int smem = (int)kSmemBytes + 1024;
-  if (!ensure_dynamic_smem<prefill_tc_kernel<G, FAST>>(smem)) return TQ4_ERR_CUDA;
-  CUtensorMap tm_idx, tm_norm;
-  memset(&tm_idx, 0, sizeof(tm_idx));
-  memset(&tm_norm, 0, sizeof(tm_norm));
-  if (!make_map(&tm_idx, a, 64) || !make_map(&tm_norm, a, 16)) return TQ4_ERR_UNSUPPORTED;
-  constexpr int RB = 128 / G;
-  const unsigned blocks = (unsigned)((a.sh.rows + RB - 1) / RB + a.sh.num_seqs);  // upper bound
-  if (launch_kernel(prefill_tc_kernel<G, FAST>, dim3(blocks, (unsigned)a.sh.Hkv), dim3(kThreads), (size_t)smem, st,
-                    true, a, tm_idx, tm_norm) != cudaSuccess)
+template <int D, bool FAST>
+int launch_t(const AttnArgs& a, const PrefillArgs& pa, cudaStream_t st) {
+  using C = Cfg<D>;
+  constexpr int smem = (int)C::kSmem + 1024;
+  static_assert(smem + 2048 <= 227 * 1024, "shared memory");
+  static_assert(2 * smem > 227 * 1024 || D < 128, "one CTA per SM: it allocates the whole tensor memory");
+  // (head_dim 64 and 96 need less: ask for more than half of the SM so that only one CTA fits)
+  constexpr int ask = smem > 120 * 1024 ? smem : 120 * 1024;
+  if (!ensure_dynamic_smem<prefill_tc_kernel<D, FAST>>(ask)) return TQ4_ERR_CUDA;
+  const int per_cta = C::NBLK * (128 / a.sh.G);
+  const unsigned blocks = (unsigned)((a.sh.rows + per_cta - 1) / per_cta + a.sh.num_seqs);  // upper bound
+  if (launch_kernel(prefill_tc_kernel<D, FAST>, dim3(blocks, (unsigned)a.sh.Hkv, (unsigned)pa.splits), dim3(kThreads),
+                    (size_t)ask, st, true, a, pa) != cudaSuccess)
     return TQ4_ERR_CUDA;
   TQ4_CHECK_LAUNCH();
   return TQ4_OK;
 }
 
-}  // namespace
-
-// Shapes and layouts the tensor-core prefill kernel covers (everything else streams).
-bool prefill_tc_supported(const AttnArgs& a) {
-  static const bool disabled = getenv("TQ4_NO_TC") != nullptr;
-  const int G = a.sh.G;
-  const RowLayout lay = row_layout(a.sh.Hkv, a.sh.D);
-  return !disabled && a.sh.D == kD && (G == 1 || G == 2 || G == 4 || G == 8) && a.query_start_loc != nullptr &&
-         (uintptr_t)a.cache % 16 == 0 && a.cache_block_stride % 16 == 0 && a.cache_token_stride % 16 == 0 &&
-         a.block_size % 16 == 0 && a.block_size <= 256 && (a.block_size & (a.block_size - 1)) == 0 &&
-         lay.v_idx % 16 == 0 && a.num_blocks < (1ll << 31) && encode_fn() != nullptr;
+template <int D>
+int launch_d(const AttnArgs& a, const PrefillArgs& pa, cudaStream_t st, bool fast, uint8_t* image) {
+  constexpr int n = D * ((D + 63) / 64) * 8;
+  // first kernel of the prefill part: a plain launch (what the caller and the streaming part wrote is complete)
+  if (launch_kernel(pi_image_kernel<D>, dim3((n + 255) / 256), dim3(256), 0, st, false, a.rotation, image) != cudaSuccess)
+    return TQ4_ERR_CUDA;
+  TQ4_CHECK_LAUNCH();
+  return fast ? launch_t<D, true>(a, pa, st) : launch_t<D, false>(a, pa, st);
 }
 
-int launch_prefill_tc(const AttnArgs& a, cudaStream_t st, bool fast) {
-  switch (a.sh.G) {
-    case 1: return fast ? launch_t<1, true>(a, st) : launch_t<1, false>(a, st);
-    case 2: return fast ? launch_t<2, true>(a, st) : launch_t<2, false>(a, st);
-    case 4: return fast ? launch_t<4, true>(a, st) : launch_t<4, false>(a, st);
-    case 8: return fast ? launch_t<8, true>(a, st) : launch_t<8, false>(a, st);
+size_t image_bytes(int D) { return (size_t)2 * ((D + 63) / 64) * D * 128; }
+
+}  // namespace
+
+// Every layout of the packed cache is covered (16-byte loads where the rows allow them, 4-byte loads elsewhere).
+bool prefill_tc_supported(const AttnArgs& a) {
+  static const bool disabled = getenv("TQ4_NO_TC") != nullptr;
+  return !disabled && a.query_start_loc != nullptr && a.sh.G <= 128 && a.num_blocks < (1ll << 31) && a.sh.Hkv <= 65535;
+}
+
+// Parts of the key range: as many as fill the SMs when the row blocks do not, at least four tiles each; limited
+// by the room for their partials (`slots` vectors sets of Hq in the scratch).
+int prefill_tc_splits(const AttnArgs& a, int64_t slots) {
+  const int per_cta = (a.sh.D == 256 ? 1 : 2) * (128 / a.sh.G);
+  const int64_t ctas = (int64_t)((a.sh.rows + per_cta - 1) / per_cta) * a.sh.Hkv;
+  int64_t s = sm_count() / (ctas > 0 ? ctas : 1);
+  const int64_t tiles = a.bt_stride * a.block_size / kBN;
+  if (s > tiles / 4) s = tiles / 4;
+  if (s > 8) s = 8;
+  if (a.sh.rows > 0 && s > slots / a.sh.rows) s = slots / a.sh.rows;
+  return s < 1 ? 1 : (int)s;
+}
+size_t prefill_tc_image_bytes(int D) { return image_bytes(D); }
+
+int launch_prefill_tc(const AttnArgs& a, cudaStream_t st, bool fast, int min_rows, int splits, bool to_parts,
+                      uint8_t* image, float* part_o, float* part_m) {
+  const PrefillArgs pa{image, min_rows, splits, to_parts ? 1 : 0, part_o, part_m};
+  switch (a.sh.D) {
+    case 64: return launch_d<64>(a, pa, st, fast, image);
+    case 96: return launch_d<96>(a, pa, st, fast, image);
+    case 128: return launch_d<128>(a, pa, st, fast, image);
+    case 256: return launch_d<256>(a, pa, st, fast, image);
   }
   return TQ4_ERR_UNSUPPORTED;
 }
@@ -785,6 +1151,6 @@ int launch_prefill_tc(const AttnArgs& a, cudaStream_t st, bool fast) {
 
 #ifdef TQ4_TRACE
 extern "C" int tq4_prefill_trace_read(long long* out) {
-  return cudaMemcpyFromSymbol(out, tq4::g_ptrace, sizeof(long long) * 4 * 64 * 16) == cudaSuccess ? 0 : 1;
+  return cudaMemcpyFromSymbol(out, tq4::g_ptrace, sizeof(long long) * 4 * 64 * 8) == cudaSuccess ? 0 : 1;
 }
 #endif

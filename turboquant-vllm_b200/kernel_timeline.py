@@ -114,25 +114,26 @@ def prefill_timeline() -> None:
     r = bench.prefill_case(dev, ops, hq=32, hkv=8, d=128, window=None, modes=(("tcgen05", 3, 2),))
     print("config 4a on the traced build:", r["tcgen05"])
     torch.cuda.synchronize()
-    buf = np.zeros(4 * 64 * 16, dtype=np.int64)
+    print_prefill_trace(nv, reader)
+
+
+def print_prefill_trace(nv, reader: str) -> None:
+    buf = np.zeros(4 * 64 * 8, dtype=np.int64)
     assert getattr(nv.lib(), reader)(buf.ctypes.data) == 0
-    t = buf.reshape(4, 64, 16).astype(np.float64)
-    warps = ["softmax warp 0", "softmax warp 4", "first dequantising warp (issues the MMAs)",
-             "last dequantising warp (issues copies)"]
-    softmax = ["top", "S ready", "scores", "row maximum exchanged", "PV of the previous tile done",
-               "P in tensor memory", None, "block barrier passed", "end of iteration"]
-    dequant = ["top", "packed stage landed", "keys dequantised", "S of the next tile issued",
-               "PV of the previous tile done", "values dequantised", None, "block barrier passed",
-               "PV issued / end of iteration"]
-    for w in range(4):
-        events = softmax if w < 2 else dequant
-        rows = [[t[w, j, e] - t[w, j, 0] for e in range(9)] + [t[w, j + 1, 0] - t[w, j, 0]] for j in range(20, 50)]
+    t = buf.reshape(4, 64, 8).astype(np.float64)
+    roles = {"softmax, first row block": ("top", "scores ready", "row maximum", "P stored"),
+             "softmax, second row block": ("top", "scores ready", "row maximum", "P stored"),
+             "first dequantising warp": ("keys' buffer free", "keys written", "next tile's loads issued",
+                                         "values' buffer free", "values written"),
+             "issuing thread": ("P of block 0 ready", "PV and next S of block 0 issued", "P of block 1 ready",
+                                "PV and next S of block 1 issued")}
+    for w, (name, events) in enumerate(roles.items()):
+        rows = [[t[w, j, e] - t[w, j, 0] for e in range(len(events))] + [t[w, j + 1, 0] - t[w, j, 0]] for j in range(20, 50)]
         m = np.mean(np.array(rows), axis=0)
-        print(f"== {warps[w]}: SM cycles since the top of the iteration (mean of iterations 20..49)")
-        for e in range(9):
-            if events[e] is not None and abs(m[e]) < 1e9:
-                print(f"   {events[e]:32s} {m[e]:8.0f}")
-        print(f"   {'next top':32s} {m[9]:8.0f}")
+        print(f"== {name}: SM cycles since its first event of the tile (mean of tiles 20..49)")
+        for e, what in enumerate(events):
+            print(f"   {what:34s} {m[e]:8.0f}")
+        print(f"   {'next tile':34s} {m[-1]:8.0f}")
 
 
 def compress_timeline() -> None:
