@@ -16,15 +16,19 @@
 //      store the caller's output.  Nothing but queries, cache and outputs touches global memory.
 //
 // Why this shape: a tile costs the tensor pipe 2 x 528 cycles per 128 rows (head_dim 128, two terms), the
-// softmax about 1 500 cycles of latency-bound CUDA-core work and the dequantisation about 600 of
-// shared-memory traffic.  With one row block per CTA these formed one chain of 3 550 cycles a tile; with
-// two blocks the tensor pipe works on one while the other is in its softmax, and a dequantised tile serves
-// 256 rows.  Everything meets at mbarriers only: softmax warps (a thread per row; two at head_dim 256),
-// eight dequantising warps and one issuing thread.
+// softmax about 2 100 cycles of latency-bound CUDA-core work (a thread per row, 64 columns) and the dequantisation
+// about 700 + 700 of shared-memory traffic.  With one row block per CTA these formed one chain of 3 550 cycles a
+// tile; with two blocks the tensor pipe works on one while the other is in its softmax, and a dequantised tile
+// serves 256 rows: 3 600 cycles for twice the rows, 58 % of them tensor work, which at 8 x 2048 rows on 8192 cached
+// tokens (32 / 8 heads) runs into the 1000 W limit.  What bounds it: the chain scores -> softmax -> P -> O and next
+// scores of a block (2 150 + 1 450).  Everything meets at mbarriers only: softmax warps (a thread per row; two at
+// head_dim 256), eight dequantising warps and one issuing thread.
+//   Code that runs once per CTA pays for its instruction fetches (the first version, unrolled, needed 62 000 cycles
+//   before its second tile, this one 30 000): set-up, rotation, masks and the new-reference path are short loops.
 //   Tensor memory, per block: [S | P in place][Q hi][Q lo][O]: 64 + 64 + 128 columns at head_dim 128, where
 //   Q lo does not fit and sits in shared memory; at head_dim 256 there is one block of 448 columns and the 64 left
 //   hold a second S, so that the scores of the next tile are computed during the softmax of this one.
-//   P overwrites S half by half: the columns of tokens 32 h .. + 31 become P hi and P lo of those tokens.
+//   P overwrites S in place: the columns of tokens 16 c .. + 15 become P hi and P lo of those tokens.
 //
 // A block with few CTAs is cut along the keys (gridDim.z): each part leaves its normalised rotated rows and
 // their log-sum-exp in the scratch, and the merge kernel folds and un-rotates them.
@@ -57,6 +61,7 @@ constexpr int kDeq = 256;       // warps 8-15: dequantisation
 constexpr int kThreads = kSmx + kDeq + 32;
 constexpr int kIssueWarp = (kSmx + kDeq) / 32;
 constexpr int kNormBufs = 4;
+constexpr float kHidden = 1e-31f;  // key norm in shared memory of a token whose page id is out of range
 
 template <int D>
 struct Cfg {
@@ -66,7 +71,7 @@ struct Cfg {
   static constexpr int DPT = D / TPR;                      // coordinates per softmax thread
   static constexpr int NC = (D + 63) / 64;                 // 64-coordinate blocks of a row
   static constexpr int NS = D / 32;                        // 16-byte segments of a packed row
-  static constexpr int NKB = D == 256 ? 1 : 2;             // K~ and V~ buffers
+  static constexpr int NKB = 2, NVB = D == 256 ? 1 : 2;    // K~ and V~ buffers
   static constexpr int NIT = (kBN * NS + kDeq - 1) / kDeq;  // segments per dequantising thread
   static constexpr bool QLO_SMEM = D >= 128;               // Q lo in shared memory
   // tensor-memory columns of a block (two S at head_dim 256)
@@ -81,14 +86,19 @@ struct Cfg {
   static constexpr int kChunks = D == 256 ? 4 : 1;         // chunks of 64 (D = 256) or all of the output coordinates
   static constexpr uint32_t kOffK = 0;
   static constexpr uint32_t kOffV = kOffK + NKB * kKvBuf;
-  static constexpr uint32_t kKvEnd = kOffV + NKB * kKvBuf;
+  static constexpr uint32_t kKvEnd = kOffV + NVB * kKvBuf;
   static constexpr uint32_t kImg = 2 * NC * kImgPart;      // the image (chunk) shares the K~ / V~ buffers
   static constexpr uint32_t kOffQlo = kKvEnd > kImg ? kKvEnd : kImg;
-  static constexpr uint32_t kOffLut = kOffQlo + (QLO_SMEM ? NBLK * NC * 128 * 128 : 0);
+  // raw 16-bit query rows on their way in, padded against bank conflicts (the area of Q lo, which is written later)
+  static constexpr uint32_t kQPitch = 2 * D + 16;
+  static constexpr uint32_t kQStage = NBLK * 128 * kQPitch, kQlo = QLO_SMEM ? NBLK * NC * 128 * 128 : 0;
+  static constexpr uint32_t kOffLut = kOffQlo + (((kQStage > kQlo ? kQStage : kQlo) + 1023) & ~1023u);
   static constexpr int kLutCopies = D == 256 ? 16 : 32;    // (16: room; every lookup is then a two-way conflict)
   static constexpr uint32_t kOffNorm = kOffLut + 2 * 256 * kLutCopies * 4;
-  static constexpr uint32_t kOffXchg = kOffNorm + kNormBufs * 3 * kBN * 4;
+  static constexpr uint32_t kOffXchg = kOffNorm + kNormBufs * 2 * kBN * 4;
   static constexpr uint32_t kSmem = kOffXchg + (TPR == 2 ? 2 * 2 * 128 * 4 : 0);
+  // registers a thread: together the 2 x 96 that the two groups of eight warps are launched with
+  static constexpr int kDeqRegs = D == 256 ? 72 : 56, kSmxRegs = 192 - kDeqRegs;
   __host__ __device__ static constexpr uint32_t idesc(uint32_t n, bool b_mn) {  // kind::f16: fp16 operands, fp32 accumulator, M = 128
     return (1u << 4) | (b_mn ? 1u << 16 : 0u) | ((n >> 3) << 17) | ((128u >> 4) << 24);
   }
@@ -187,23 +197,39 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
       : "memory");
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
+// 16 columns, without the wait; tmem_ld16_wait names the registers so that no use of them moves above it.  (No
+// memory clobber on these: the compiler may move shared-memory loads across them.)
+__device__ __forceinline__ void tmem_ld16_async(uint32_t taddr, uint32_t (&v)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
+      "%14, %15}, [%16];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+        "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+      : "r"(taddr));
+}
+__device__ __forceinline__ void tmem_ld16_wait(uint32_t (&v)[16]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]),
+                 "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15]));
+}
+// all 32 or 64 columns of a score tile, with the wait
+template <int N>
+__device__ __forceinline__ void tmem_ld_cols(uint32_t taddr, uint32_t (&v)[N]) {
+#pragma unroll
+  for (int h = 0; h < N / 16; ++h) tmem_ld16_async(taddr + 16 * h, *reinterpret_cast<uint32_t(*)[16]>(v + 16 * h));
+#pragma unroll
+  for (int h = 0; h < N / 16; ++h) tmem_ld16_wait(*reinterpret_cast<uint32_t(*)[16]>(v + 16 * h));
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&v)[8]) {  // (no wait)
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};"
+               ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]));
+}
 __device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {  // (no wait)
   asm volatile(
       "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
       "%15, %16};"
       ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
-        "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
-      : "memory");
-}
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32]) {  // (no wait)
-  asm volatile(
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
-      "%15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"
-      ::"r"(taddr), "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]),
-        "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]),
-        "r"(v[16]), "r"(v[17]), "r"(v[18]), "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]),
-        "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]), "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
-      : "memory");
+        "r"(v[8]), "r"(v[9]), "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]));
 }
 __device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
@@ -266,6 +292,16 @@ __device__ __forceinline__ void pow2_scale(float amax, float& sc, float& isc) {
   }
 }
 
+// two packed 16-bit values
+__device__ __forceinline__ void half_pair(uint32_t w, bool f16, float& x0, float& x1) {
+  if (f16) {
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w));
+    x0 = f.x; x1 = f.y;
+  } else {
+    x0 = __uint_as_float(w << 16); x1 = __uint_as_float(w & 0xFFFF0000u);
+  }
+}
+
 // 32 consecutive elements i .. i + 31 of a typed tensor
 __device__ __forceinline__ void load32(const void* q, int dtype, int64_t i, bool vec_ok, float (&x)[32]) {
   if (!vec_ok) {
@@ -297,6 +333,33 @@ __device__ __forceinline__ void load32(const void* q, int dtype, int64_t i, bool
         x[8 * e + 2 * k + 1] = __uint_as_float(w[k] & 0xFFFF0000u);
       }
     }
+  }
+}
+
+// 32 consecutive outputs
+__device__ __forceinline__ void store32(void* p, int dtype, int64_t i, bool vec_ok, const float (&y)[32]) {
+  if (dtype != TQ4_F32 && vec_ok) {
+    uint4* d = reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(p) + i);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      uint32_t w[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (dtype == TQ4_F16) {
+          w[k] = pack_h2(y[8 * q + 2 * k], y[8 * q + 2 * k + 1]);
+        } else {
+          const __nv_bfloat162 h = __floats2bfloat162_rn(y[8 * q + 2 * k], y[8 * q + 2 * k + 1]);
+          w[k] = *reinterpret_cast<const uint32_t*>(&h);
+        }
+      }
+      d[q] = make_uint4(w[0], w[1], w[2], w[3]);
+    }
+    return;
+  }
+#pragma unroll
+  for (int q = 0; q < 8; ++q) {
+    const float t[4] = {y[4 * q], y[4 * q + 1], y[4 * q + 2], y[4 * q + 3]};
+    store4(p, dtype, i + 4 * q, t);
   }
 }
 
@@ -332,13 +395,14 @@ struct Bars {
   uint64_t img, cdone;            // image chunk landed / used
   uint64_t aready, rot;           // A operand of a rotation staged / rotation complete
   uint64_t pair[4];               // the two warps of a row quadrant (head_dim 256)
+  uint64_t qraw;                  // raw query rows landed
   uint64_t qready, odone;         // queries in place / last MMA of the tile loop complete
 };
 
 template <int D, bool FAST>
 __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs a, const PrefillArgs pa) {
   using C = Cfg<D>;
-  constexpr int NBLK = C::NBLK, TPR = C::TPR, CPT = C::CPT, DPT = C::DPT, NC = C::NC, NKB = C::NKB, NIT = C::NIT;
+  constexpr int NBLK = C::NBLK, TPR = C::TPR, CPT = C::CPT, DPT = C::DPT, NC = C::NC, NKB = C::NKB, NVB = C::NVB, NIT = C::NIT;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   __shared__ __align__(8) Bars s_bars;
   __shared__ uint32_t s_tmem;
@@ -352,6 +416,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
   const uint32_t base = (smem_addr(smem_raw) + 1023u) & ~1023u;
   unsigned char* sm = smem_raw + (base - smem_addr(smem_raw));
 
+  PF_STAMP(tid == 0 ? 0 : -1, 0, 4);
   // ---- which rows are this CTA's?  Sequences in order, a sequence's last rows (the longest) first --------
   if (warp == 0) {
     int acc = 0, found = -1, first = 0, nrows = 0;
@@ -403,6 +468,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
     bar_init(bar(s_bars.cdone), 1);
     bar_init(bar(s_bars.aready), 8);
     bar_init(bar(s_bars.rot), 1);
+    bar_init(bar(s_bars.qraw), kSmx);
     bar_init(bar(s_bars.qready), 8);
     bar_init(bar(s_bars.odone), 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -414,6 +480,25 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
     pdl_trigger();
     pdl_wait();
     return;
+  }
+  // ---- row of a softmax thread (half a row at head_dim 256), and its raw query on the way -------------------
+  const int blk = NBLK == 2 ? (warp >> 2) & 1 : 0, part = NBLK == 2 ? 0 : (warp >> 2) & 1;
+  const int m = 32 * (warp & 3) + lane, my_r = m / G, my_g = m - my_r * G;
+  const int lrow = blk * RB + my_r;                       // row within the CTA
+  const bool live = warp < kSmx / 32 && my_r < RB && lrow < nrows;
+  const int head = kvh * G + my_g, row = row0 + (live ? lrow : 0);
+  const int es = a.q_dtype == TQ4_F32 ? 4 : 2;
+  const bool q_vec = ((uintptr_t)a.q % 16 == 0) && (a.q_token_stride * es) % 16 == 0 && (a.q_head_stride * es) % 16 == 0;
+  const bool q_staged = q_vec && es == 2;
+  const int64_t qi = (int64_t)row * a.q_token_stride + (int64_t)head * a.q_head_stride + part * DPT;
+  const uint32_t q_at = C::kOffQlo + (blk * 128 + m) * C::kQPitch + part * DPT * 2;
+  if (q_staged && warp < kSmx / 32) {
+    if (live) {
+      expect_tx(bar(s_bars.qraw), DPT * 2);
+      bulk_load(base + q_at, reinterpret_cast<const uint16_t*>(a.q) + qi, DPT * 2, bar(s_bars.qraw));
+    } else {
+      bar_arrive(bar(s_bars.qraw));
+    }
   }
   if (warp == kIssueWarp) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&s_tmem)), "r"(512u) : "memory");
@@ -440,6 +525,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
   fence_after();
   const uint32_t tmem = s_tmem;
 
+  PF_STAMP(tid == 0 ? 0 : -1, 0, 5);
   // ---- keys the CTA needs: rows are in query order, their visible ranges move forward with them -----------
   const int q_end = a.query_start_loc[seq + 1], len = clamp_seq_len(a, max(0, a.seq_lens[seq]));
   auto row_keys = [&](int row, int& lo, int& hi) {  // visible keys of row `row` of the call
@@ -465,17 +551,21 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
   if (warp == kIssueWarp) {
     // ================= issuing thread =================
     if (n_tiles > 0 && elect_one_sync()) {
+      // where a chunk's hi and lo terms go: the K~ / V~ buffers before the tile loop; after it the tables (head_dim
+      // 256: the K~ buffer and the tables), which are free before the last values have been multiplied
       const uint32_t img = base + C::kOffK;
+      const uint32_t uhi = base + (D == 256 ? C::kOffK : C::kOffLut), ulo = D == 256 ? base + C::kOffLut : uhi + C::kImg / 2;
       uint32_t img_ph = 0, c_ph = 0;
       bool ok = true;
+      const bool unrotate = !pa.to_parts && !a.out_rotated;
       // chunk ch of the image, as rows (rotation) or as column blocks (un-rotation)
       auto load_chunk = [&](int ch, bool unrot) {
         expect_tx(bar(s_bars.img), C::kImg);
         if (C::kChunks == 1) {
-          bulk_load(img, pa.image, C::kImg, bar(s_bars.img));
+          bulk_load(unrot ? uhi : img, pa.image, C::kImg, bar(s_bars.img));
         } else if (unrot) {
-          for (int t = 0; t < 2; ++t)
-            bulk_load(img + t * D * 128, pa.image + (size_t)(t * NC + ch) * D * 128, D * 128, bar(s_bars.img));
+          bulk_load(uhi, pa.image + (size_t)ch * D * 128, D * 128, bar(s_bars.img));
+          bulk_load(ulo, pa.image + (size_t)(NC + ch) * D * 128, D * 128, bar(s_bars.img));
         } else {
           for (int t = 0; t < 2 * NC; ++t)
             bulk_load(img + t * C::kImgPart, pa.image + (size_t)t * D * 128 + ch * 64 * 128, C::kImgPart, bar(s_bars.img));
@@ -493,13 +583,13 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
           if (!ok) return;
           constexpr uint32_t N = C::kChunks == 1 ? D : 64;
           const uint32_t idesc = C::idesc(N, unrot);
-          const uint32_t term = unrot ? (C::kChunks == 1 ? NC * C::kImgPart : D * 128) : NC * C::kImgPart;  // bytes of a term
+          const uint32_t hi = unrot ? uhi : img, lo = unrot ? ulo : img + C::kImg / 2;
           for (int b = 0; b < n_blk; ++b) {
             const uint32_t tb = tmem + b * C::kBlkCols, d = tb + C::kColO + 64 * ch;
 #pragma unroll 1
             for (int s = 0; s < D / 16; ++s) {
               const uint32_t off = unrot ? 2048u * s : (s >> 2) * C::kImgPart + 32u * (s & 3);
-              const uint64_t bh = make_desc(img + off, unrot ? C::kImgPart : 0), bl = make_desc(img + term + off, unrot ? C::kImgPart : 0);
+              const uint64_t bh = make_desc(hi + off, unrot ? C::kImgPart : 0), bl = make_desc(lo + off, unrot ? C::kImgPart : 0);
               mma_ta(d, tb + C::kColS + 8 * s, bl, idesc, s > 0);
               if (a_lo) mma_ta(d, tb + C::kColQ + 8 * s, bh, idesc, true);
               mma_ta(d, tb + C::kColS + 8 * s, bh, idesc, true);
@@ -538,17 +628,17 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
       };
       auto issue_pv = [&](int b, int j) {  // O += P V~ of tile j
         const uint32_t tb = tmem + b * C::kBlkCols, p = tb + C::kColS + (NBLK == 1 ? 64 * (j & 1) : 0);
-        const uint64_t dv0 = d_v + (uint64_t)(((j % NKB) * C::kKvBuf) >> 4);
+        const uint64_t dv0 = d_v + (uint64_t)(((j % NVB) * C::kKvBuf) >> 4);
 #pragma unroll
         for (int s = 0; s < 4; ++s) {
           const uint64_t dv = dv0 + (uint64_t)((2048 * s) >> 4);
-          const uint32_t ph = p + 32 * (s >> 1) + 8 * (s & 1);
-          if (!FAST) mma_ta(tb + C::kColO, ph + 16, dv, idO, j > 0 || s > 0);
+          const uint32_t ph = p + 16 * s;
+          if (!FAST) mma_ta(tb + C::kColO, ph + 8, dv, idO, j > 0 || s > 0);
           mma_ta(tb + C::kColO, ph, dv, idO, !FAST || j > 0 || s > 0);
         }
       };
       auto wait_k = [&](int j) { ok = ok && bar_wait(bar(s_bars.kready[j % NKB]), (uint32_t)((j / NKB) & 1), dead); };
-      auto wait_v = [&](int j) { ok = ok && bar_wait(bar(s_bars.vready[j % NKB]), (uint32_t)((j / NKB) & 1), dead); };
+      auto wait_v = [&](int j) { ok = ok && bar_wait(bar(s_bars.vready[j % NVB]), (uint32_t)((j / NVB) & 1), dead); };
       auto wait_p = [&](int i, int n) { ok = ok && bar_wait(bar(s_bars.pready[i]), (uint32_t)(n & 1), dead); };
 
       ok = ok && bar_wait(bar(s_bars.qready), 0u, dead);
@@ -572,20 +662,27 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
           PF_STAMP(3, j, 1);
           wait_p(j & 1, j >> 1);
           PF_STAMP(3, j, 2);
+          if (j == n_tiles - 1 && unrotate) {  // (these scores are complete: this returns at once)
+            ok = ok && bar_wait(bar(s_bars.kfree[j % NKB]), (uint32_t)((j / NKB) & 1), dead);
+            if (ok) load_chunk(0, true);
+          }
           if (!ok) break;
           fence_after();
           issue_pv(0, j);
-          mma_commit(bar(s_bars.vfree[j % NKB]));
+          mma_commit(bar(s_bars.vfree[j % NVB]));
           mma_commit(bar(s_bars.pvd));
         } else {  // the blocks take turns: while one is in its softmax the other has the tensor pipe
           for (int b = 0; b < n_blk; ++b) {
-            if (b == 0) wait_v(j);
+            if (b == 0) {
+              wait_v(j);
+              if (j == n_tiles - 1 && unrotate && ok) load_chunk(0, true);
+            }
             wait_p(b, j);
             PF_STAMP(3, j, 2 * b);
             if (!ok) break;
             fence_after();
             issue_pv(b, j);
-            if (b == n_blk - 1) mma_commit(bar(s_bars.vfree[j % NKB]));
+            if (b == n_blk - 1) mma_commit(bar(s_bars.vfree[j % NVB]));
             if (j + 1 < n_tiles) {
               if (b == 0) {
                 wait_k(j + 1);
@@ -601,24 +698,20 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
       }
       if (ok) {
         mma_commit(bar(s_bars.odone));
-        if (!pa.to_parts && !a.out_rotated) {  // every MMA has read its operands: the image takes the K~ / V~ buffers again
-          ok = bar_wait(bar(s_bars.odone), 0u, dead);
-          if (ok) {
-            load_chunk(0, true);
-            rotate(true, true);
-          }
-        }
+        if (unrotate) rotate(true, true);
       }
     }
     __syncwarp();
   } else if (warp >= kSmx / 32) {
     // ================= dequantising warps =================
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(C::kDeqRegs));
     const int t = tid - kSmx;
     const RowLayout lay = row_layout(sh.Hkv, D);
     const int32_t* bt = a.block_table + (int64_t)seq * a.bt_stride;
     const int bs = a.block_size, shift = (bs & (bs - 1)) == 0 ? __ffs(bs) - 1 : -1;
     const bool al = ((uintptr_t)a.cache | a.cache_block_stride | a.cache_token_stride) % 16 == 0;
-    const bool k_vec = al && (lay.k_idx + kvh * (D / 2)) % 16 == 0, v_vec = al && (lay.v_idx + kvh * (D / 2)) % 16 == 0;
+    const bool vec = al && lay.v_idx % 16 == 0;  // (K bytes start at a multiple of 16)
+    const unsigned n_pages = (unsigned)a.num_blocks;
     // item n of this thread: token and 16-byte segment of the packed row.  Eight lanes take 4 tokens x the 2 segments
     // of one 64-coordinate block: their operand stores (chunk ^ (token & 7)) fall into eight bank groups.
     auto item = [&](int n, int& tok, int& seg) -> bool {
@@ -634,55 +727,53 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
       seg = C::NS - 1;
       return (C::NS & 1) && tok < kBN;
     };
-    struct Item { int page; uint4 k, v; float kn, vn; };
+    // What a thread fetches of a tile: its 16 bytes of K and V and (segment 0) the token's norms.  Page ids are
+    // looked up a tile ahead of the rows, the rows a tile ahead of their use.
+    struct Item { uint4 k, v; float kn, vn; };
     Item it[NIT] = {};
-    int next_page[NIT];
-    auto pos_of = [&](int n, int j) {
-      int tok, seg;
-      return item(n, tok, seg) ? t_first + j * kBN + tok : 0x7fffffff;
-    };
-    auto load_page = [&](int n, int j) -> int {
-      const int pos = pos_of(n, j);
-      if (pos >= blk_hi) return -1;
+    int page[NIT] = {}, pos0[NIT];   // page id of the next tile; position in tile 0
+    uint32_t k_off[NIT];        // byte offset of the thread's K bytes in a row; its V bytes are v_delta further
+    constexpr int kPast = (int)0x80000000;
+    const uint32_t v_delta = (uint32_t)(lay.v_idx - lay.k_idx), ts = (uint32_t)a.cache_token_stride;
+    const uint32_t kn_off = (uint32_t)(lay.k_norm + 4 * kvh), vn_delta = (uint32_t)(lay.v_norm - lay.k_norm);
+    bool has_norm[NIT];
+#pragma unroll
+    for (int n = 0; n < NIT; ++n) {
+      int tok, seg = 0;
+      pos0[n] = item(n, tok, seg) ? t_first + tok : 0x3fffffff;
+      k_off[n] = (uint32_t)(lay.k_idx + kvh * (D / 2) + 16 * seg);
+      has_norm[n] = seg == 0;
+    }
+    auto look_up = [&](int n, int j) -> int {
+      const int pos = pos0[n] + j * kBN;
+      if (pos >= blk_hi) return kPast;  // (past the keys of the CTA: masked, whatever is read)
       return __ldg(bt + (shift >= 0 ? pos >> shift : pos / bs));
     };
-    auto load16 = [&](const uint8_t* p, bool vec) -> uint4 {
+    auto load16 = [&](const uint8_t* p) -> uint4 {
       if (vec) return __ldg(reinterpret_cast<const uint4*>(p));
       const uint32_t* w = reinterpret_cast<const uint32_t*>(p);
       return make_uint4(__ldg(w), __ldg(w + 1), __ldg(w + 2), __ldg(w + 3));
     };
-    // row of item n's token, or null (past the keys of the CTA, or a page id out of range: reported and hidden)
-    auto row_of = [&](int n, int j, int page) -> const uint8_t* {
-      const int pos = pos_of(n, j);
-      if (pos >= blk_hi) return nullptr;
-      if (page < 0 || page >= a.num_blocks) {
+    auto fetch = [&](int n, int j) {
+      const int pg = page[n];
+      const bool bad = (unsigned)pg >= n_pages;
+      if (bad && pg != kPast) {  // a page id out of range: reported, its tokens hidden
         if (a.err_flag) atomicOr(a.err_flag, TQ4_DEV_BAD_BLOCK);
         s_bad = 1;
-        return nullptr;
       }
-      const int in = shift >= 0 ? pos & (bs - 1) : pos % bs;
-      return a.cache + (int64_t)page * a.cache_block_stride + (int64_t)in * a.cache_token_stride;
-    };
-    const int kn_off = lay.k_norm + 4 * kvh, vn_off = lay.v_norm + 4 * kvh;
-    auto load_k = [&](int n, int j) {
-      int tok, seg;
-      item(n, tok, seg);
-      const uint8_t* row = row_of(n, j, it[n].page);
-      it[n].k = make_uint4(0, 0, 0, 0);
-      it[n].kn = it[n].vn = row ? 0.f : (pos_of(n, j) < blk_hi ? CUDART_NAN_F : 0.f);  // (NaN: hidden token)
-      if (row) {
-        it[n].k = load16(row + lay.k_idx + kvh * (D / 2) + 16 * seg, k_vec);
-        if (seg == 0) {
-          it[n].kn = __ldg(reinterpret_cast<const float*>(row + kn_off));
-          it[n].vn = __ldg(reinterpret_cast<const float*>(row + vn_off));
-        }
+      const int pos = pos0[n] + j * kBN;
+      const uint32_t in = shift >= 0 ? (uint32_t)(pos & (bs - 1)) : (uint32_t)(pos % bs);
+      // (without a valid page: row 0 of the cache, if there is one)
+      const uint8_t* row = a.cache + (bad ? 0ull : (unsigned long long)(unsigned)pg * (unsigned long long)a.cache_block_stride + in * ts);
+      it[n].kn = pg == kPast ? 1.f : kHidden;
+      it[n].vn = 0.f;
+      if (n_pages == 0) return;
+      it[n].k = load16(row + k_off[n]);
+      it[n].v = load16(row + k_off[n] + v_delta);
+      if (has_norm[n] && !bad) {
+        it[n].kn = __ldg(reinterpret_cast<const float*>(row + kn_off));
+        it[n].vn = __ldg(reinterpret_cast<const float*>(row + kn_off + vn_delta));
       }
-    };
-    auto load_v = [&](int n, int j) {
-      int tok, seg;
-      item(n, tok, seg);
-      const uint8_t* row = row_of(n, j, it[n].page);
-      it[n].v = row ? load16(row + lay.v_idx + kvh * (D / 2) + 16 * seg, v_vec) : make_uint4(0, 0, 0, 0);
     };
     auto expand = [&](const uint4& pk, int which, uint32_t buf, int tok, int seg) {  // 16 bytes -> 32 fp16
       const uint32_t* lut = reinterpret_cast<const uint32_t*>(sm + C::kOffLut) + which * 256 * C::kLutCopies + (lane & (C::kLutCopies - 1));
@@ -699,32 +790,21 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
     const int role = tid == kSmx ? 2 : -1;  // (time stamps)
     (void)role;
     bool ok = true;
-    if (n_tiles > 0) {
-#pragma unroll
-      for (int n = 0; n < NIT; ++n) it[n].page = load_page(n, 0);
-#pragma unroll
-      for (int n = 0; n < NIT; ++n) {
-        load_k(n, 0);
-        load_v(n, 0);
-        next_page[n] = n_tiles > 1 ? load_page(n, 1) : -1;
-      }
-      ok = bar_wait(bar(s_bars.rot), 0u, dead);  // the image of Pi has been used
-    }
-    for (int j = 0; j < n_tiles && ok; ++j) {
+    auto write_k = [&](int j) {  // K~ and norms of tile j from the registers
       const int b = j % NKB, u = j / NKB;
-      if (u > 0) ok = bar_wait(bar(s_bars.kfree[b]), (uint32_t)((u - 1) & 1), dead);
-      if (!ok) break;
+      if (u > 0) ok = bar_wait(bar(s_bars.kfree[b]), (uint32_t)((u - 1) & 1), dead) && ok;
+      if (!ok) return;
       PF_STAMP(role, j, 0);
-      float* ns = reinterpret_cast<float*>(sm + C::kOffNorm) + (j % kNormBufs) * 3 * kBN;
+      float* ns = reinterpret_cast<float*>(sm + C::kOffNorm) + (j % kNormBufs) * 2 * kBN;
 #pragma unroll
       for (int n = 0; n < NIT; ++n) {
         int tok, seg;
         if (item(n, tok, seg)) {
           expand(it[n].k, 0, C::kOffK + b * C::kKvBuf, tok, seg);
           if (seg == 0) {
-            ns[tok] = it[n].kn;
+            // (positive, so that -inf times it stays -inf)
+            ns[tok] = it[n].kn == kHidden ? kHidden : fmaxf(it[n].kn, 1e-30f);
             ns[kBN + tok] = it[n].vn;
-            ns[2 * kBN + tok] = fmaxf(lg2_approx(it[n].vn), -30.f);
           }
         }
       }
@@ -732,20 +812,23 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
       __syncwarp();
       if (lane == 0) bar_arrive(bar(s_bars.kready[b]));
       PF_STAMP(role, j, 1);
-      uint4 v_now[NIT];
+    };
+    uint4 v_now[NIT], v_next[NIT];
+    auto advance = [&](int j) {  // tile j's keys are written: its values step up, tile j + 1 is fetched
 #pragma unroll
       for (int n = 0; n < NIT; ++n) {
-        v_now[n] = it[n].v;
-        it[n].page = next_page[n];
+        v_next[n] = it[n].v;
         if (j + 1 < n_tiles) {
-          load_k(n, j + 1);
-          load_v(n, j + 1);
-          if (j + 2 < n_tiles) next_page[n] = load_page(n, j + 2);
+          fetch(n, j + 1);
+          page[n] = look_up(n, j + 2);
         }
       }
+    };
+    auto write_v = [&](int j) {
+      const int b = j % NVB, u = j / NVB;
       PF_STAMP(role, j, 2);
-      if (u > 0) ok = bar_wait(bar(s_bars.vfree[b]), (uint32_t)((u - 1) & 1), dead);
-      if (!ok) break;
+      if (u > 0) ok = bar_wait(bar(s_bars.vfree[b]), (uint32_t)((u - 1) & 1), dead) && ok;
+      if (!ok) return;
       PF_STAMP(role, j, 3);
 #pragma unroll
       for (int n = 0; n < NIT; ++n) {
@@ -756,14 +839,33 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
       __syncwarp();
       if (lane == 0) bar_arrive(bar(s_bars.vready[b]));
       PF_STAMP(role, j, 4);
+    };
+    if (n_tiles > 0) {
+#pragma unroll
+      for (int n = 0; n < NIT; ++n) page[n] = look_up(n, 0);
+#pragma unroll
+      for (int n = 0; n < NIT; ++n) {
+        fetch(n, 0);
+        page[n] = look_up(n, 1);
+      }
+      ok = bar_wait(bar(s_bars.rot), 0u, dead);  // the image of Pi has been used
+      write_k(0);
+      advance(0);
+    }
+    // The keys run a tile ahead of the values: the scores of tile j + 1 wait for nothing of tile j.  With one V~
+    // buffer (head_dim 256) the next keys come before the values, which have to wait for the MMAs of the tile before
+    // (5 200 -> 4 000 cycles a tile), and the next fetch after both.
+    for (int j = 0; j < n_tiles && ok; ++j) {
+#pragma unroll
+      for (int n = 0; n < NIT; ++n) v_now[n] = v_next[n];
+      if (NVB > 1) write_v(j);
+      if (j + 1 < n_tiles && ok) write_k(j + 1);
+      if (NVB == 1 && ok) write_v(j);
+      if (j + 1 < n_tiles && ok) advance(j + 1);
     }
   } else {
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(C::kSmxRegs));
     // ================= softmax warps: a row (half a row at head_dim 256) per thread =================
-    const int blk = NBLK == 2 ? warp >> 2 : 0, part = NBLK == 2 ? 0 : warp >> 2;
-    const int m = 32 * (warp & 3) + lane, my_r = m / G, my_g = m - my_r * G;
-    const int lrow = blk * RB + my_r;                       // row within the CTA
-    const bool live = my_r < RB && lrow < nrows;
-    const int head = kvh * G + my_g, row = row0 + (live ? lrow : 0);
     const uint32_t tb = tmem + blk * C::kBlkCols + ((uint32_t)(32 * (warp & 3)) << 16);
     float* xchg = reinterpret_cast<float*>(sm + C::kOffXchg);
     // maximum (or sum) over the threads of a row
@@ -791,62 +893,66 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
     // ---- rotate the queries -----------------------------------------------------------------------
     float qscale = 0.f;
     if (use) {
-      const int es = a.q_dtype == TQ4_F32 ? 4 : 2;
-      const bool vec_ok = ((uintptr_t)a.q % 16 == 0) && (a.q_token_stride * es) % 16 == 0 && (a.q_head_stride * es) % 16 == 0;
-      const int64_t qi = (int64_t)row * a.q_token_stride + (int64_t)head * a.q_head_stride + part * DPT;
-      float amax = 0.f;
-#pragma unroll 1
-      for (int c = 0; c < DPT / 32; ++c) {
-        float x[32];
-        if (live) {
-          load32(a.q, a.q_dtype, qi + 32 * c, vec_ok, x);
-#pragma unroll
-          for (int e = 0; e < 32; ++e) amax = fmaxf(amax, fabsf(x[e]));
-        }
-      }
-      float sc, isc;
-      pow2_scale(row_reduce(amax, fmax_op), sc, isc);
-#pragma unroll 1
-      for (int c = 0; c < DPT / 32; ++c) {
-        float x[32];
-        if (live) {
-          load32(a.q, a.q_dtype, qi + 32 * c, vec_ok, x);
-        } else {
+      // (code that runs once per CTA costs its instruction fetches: short rolled loops)
+      if (q_staged) ok = bar_wait(bar(s_bars.qraw), 0u, dead);
+      auto load_q = [&](int c, float (&x)[32]) {
+        if (!live) {
 #pragma unroll
           for (int e = 0; e < 32; ++e) x[e] = 0.f;
-        }
-        uint32_t h[16], l[16];
+        } else if (q_staged) {
+          const uint4* src = reinterpret_cast<const uint4*>(sm + q_at + 64 * c);
+          const bool f16 = a.q_dtype == TQ4_F16;
 #pragma unroll
-        for (int e = 0; e < 16; ++e) split2(x[2 * e] * sc, x[2 * e + 1] * sc, h[e], l[e]);
-        tmem_st16(tb + C::kColS + (part * DPT) / 2 + 16 * c, h);
-        if (a.q_dtype == TQ4_F32) tmem_st16(tb + C::kColQ + (part * DPT) / 2 + 16 * c, l);
+          for (int e = 0; e < 4; ++e) {
+            const uint4 r = src[e];
+            half_pair(r.x, f16, x[8 * e], x[8 * e + 1]);
+            half_pair(r.y, f16, x[8 * e + 2], x[8 * e + 3]);
+            half_pair(r.z, f16, x[8 * e + 4], x[8 * e + 5]);
+            half_pair(r.w, f16, x[8 * e + 6], x[8 * e + 7]);
+          }
+        } else {
+          load32(a.q, a.q_dtype, qi + 32 * c, q_vec, x);
+        }
+      };
+      float amax = 0.f, sc = 1.f, isc = 1.f;
+#pragma unroll 1
+      for (int pass = 0; pass < 2; ++pass) {
+#pragma unroll 1
+        for (int c = 0; c < DPT / 32; ++c) {
+          float x[32];
+          load_q(c, x);
+          if (pass == 0) {
+#pragma unroll
+            for (int e = 0; e < 16; ++e) amax = max3(amax, fabsf(x[2 * e]), fabsf(x[2 * e + 1]));
+          } else {
+            uint32_t h[16], l[16];
+#pragma unroll
+            for (int e = 0; e < 16; ++e) split2(x[2 * e] * sc, x[2 * e + 1] * sc, h[e], l[e]);
+            tmem_st16(tb + C::kColS + (part * DPT) / 2 + 16 * c, h);
+            if (a.q_dtype == TQ4_F32) tmem_st16(tb + C::kColQ + (part * DPT) / 2 + 16 * c, l);
+          }
+        }
+        if (pass == 0) pow2_scale(row_reduce(amax, fmax_op), sc, isc);
       }
       tmem_st_wait();
       arrive(s_bars.aready);
       ok = __all_sync(0xffffffffu, bar_wait(bar(s_bars.rot), 0u, dead));
       fence_after();
       // largest coordinate of the rotated row, then its terms at that scale
-      float rmax = 0.f;
-      if (ok) {
+      float rmax = 0.f, inv = 0.f;
+#pragma unroll 1
+      for (int pass = 0; pass < 2 && ok; ++pass) {
 #pragma unroll 1
         for (int c = 0; c < DPT / 32; ++c) {
           uint32_t v[32];
-          tmem_ld32(tb + C::kColO + part * DPT + 32 * c, v);
-#pragma unroll
-          for (int e = 0; e < 32; ++e) rmax = fmaxf(rmax, fabsf(__uint_as_float(v[e])));
-        }
-      }
-      rmax = row_reduce(rmax, fmax_op);
-      const float inv = rmax > 0.f ? 1.f / rmax : 0.f;
-      // factor between a stored dot product and the score in the log2 domain (at least the smallest normal
-      // number, so that a hidden score, -inf, times it stays -inf)
-      qscale = fmaxf(rmax * isc * (1.f / 256.f) * (a.scale_log2e / a.lut_scale_k), 1.17549435e-38f);
-      if (ok) {
-#pragma unroll 1
-        for (int c = 0; c < DPT / 32; ++c) {
-          uint32_t v[32], h[16], l[16];
           const int d0 = part * DPT + 32 * c;
-          tmem_ld32(tb + C::kColO + d0, v);
+          tmem_ld_cols(tb + C::kColO + d0, v);
+          if (pass == 0) {
+#pragma unroll
+            for (int e = 0; e < 16; ++e) rmax = max3(rmax, fabsf(__uint_as_float(v[2 * e])), fabsf(__uint_as_float(v[2 * e + 1])));
+            continue;
+          }
+          uint32_t h[16], l[16];
 #pragma unroll
           for (int e = 0; e < 16; ++e)
             split2(__uint_as_float(v[2 * e]) * inv, __uint_as_float(v[2 * e + 1]) * inv, h[e], l[e]);
@@ -861,7 +967,13 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
             tmem_st16(tb + C::kColQlo + d0 / 2, l);
           }
         }
+        if (pass == 0) {
+          rmax = row_reduce(rmax, fmax_op);
+          inv = rmax > 0.f ? 1.f / rmax : 0.f;
+        }
       }
+      // factor between a stored dot product and the score in the log2 domain
+      qscale = fmaxf(rmax * isc * (1.f / 256.f) * (a.scale_log2e / a.lut_scale_k), 1.17549435e-38f);
       tmem_st_wait();
       fence_async();
       arrive(s_bars.qready);
@@ -870,6 +982,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
       arrive(s_bars.qready);
     }
 
+    PF_STAMP(tid == 0 ? 0 : -1, 0, 6);
     // ---- the tile loop --------------------------------------------------------------------------------
     int kv_lo = 0, kv_hi = 0;
     if (live) row_keys(row, kv_lo, kv_hi);
@@ -886,100 +999,117 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
         PF_STAMP(role, j, 1);
         fence_after();
         const uint32_t scol = tb + C::kColS + (NBLK == 1 ? 64 * (j & 1) : 0) + part * CPT;
-        const float* ns = reinterpret_cast<const float*>(sm + C::kOffNorm) + (j % kNormBufs) * 3 * kBN + part * CPT;
-        // dot x key norm (x qscale = score in the log2 domain); two columns per instruction.  Tiles inside
-        // the visible range of every row of the warp take the path without per-element masks.
+        const float* ns = reinterpret_cast<const float*>(sm + C::kOffNorm) + (j % kNormBufs) * 2 * kBN + part * CPT;
+        // dot x key norm x qscale - reference, exp2, x value norm, split, store in place; two columns per
+        // instruction.  Tiles inside the visible range of every row of the warp take the path without
+        // per-element masks.  The reference is updated lazily, and looked at only after the fact: when some
+        // weight exceeds 2^8 (or the row has no reference yet) the tile is done again from the scores, which stay in
+        // registers, with a new one.  That saves the pass over the scores that would find the maximum first.
         const bool inner = __all_sync(0xffffffffu, t0 >= kv_lo && t0 + CPT <= kv_hi) && !*(volatile int*)&s_bad;
         const f2 qs2 = pack2(qscale, qscale);
-        auto visible = [&](int i) { return t0 + i >= kv_lo && t0 + i < kv_hi && ns[i] == ns[i]; };
-        float mt = -CUDART_INF_F;
+        uint32_t v[CPT];
+        tmem_ld_cols(scol, v);
+        bool seen = true;  // some key of the tile is visible
+        if (!inner) {      // hidden columns: a score of -inf (key norms are positive in shared memory)
+          int lo = min(max(kv_lo - t0, 0), CPT), hi = min(max(kv_hi - t0, 0), CPT);
+          uint32_t vis[CPT / 32];
+          seen = false;
 #pragma unroll
-        for (int h = 0; h < CPT / 32; ++h) {
-          uint32_t v[32];
-          tmem_ld32(scol + 32 * h, v);
-          if (inner) {
-#pragma unroll
-            for (int i4 = 0; i4 < 8; ++i4) {
-              const ulonglong2 kn = reinterpret_cast<const ulonglong2*>(ns + 32 * h)[i4];
-              const ulonglong2 lg = reinterpret_cast<const ulonglong2*>(ns + 2 * kBN + 32 * h)[i4];
-              float u0, u1, u2, u3;
-              unpack2(fma2(mul2(pack2(__uint_as_float(v[4 * i4]), __uint_as_float(v[4 * i4 + 1])), kn.x), qs2, lg.x), u0, u1);
-              unpack2(fma2(mul2(pack2(__uint_as_float(v[4 * i4 + 2]), __uint_as_float(v[4 * i4 + 3])), kn.y), qs2, lg.y), u2, u3);
-              mt = max3(mt, u0, u1);
-              mt = max3(mt, u2, u3);
-            }
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; ++i)
-              if (visible(32 * h + i)) mt = fmaxf(mt, fmaf(__uint_as_float(v[i]) * ns[32 * h + i], qscale, ns[2 * kBN + 32 * h + i]));
+          for (int w = 0; w < CPT / 32; ++w) {
+            const int l = min(max(lo - 32 * w, 0), 32), h = min(max(hi - 32 * w, 0), 32);
+            vis[w] = h > l ? (0xFFFFFFFFu >> (32 - (h - l))) << l : 0u;
+            if (*(volatile int*)&s_bad)
+              for (int i = 0; i < 32; ++i)
+                if (ns[32 * w + i] == kHidden) vis[w] &= ~(1u << i);
+            seen = seen || vis[w];
           }
+#pragma unroll
+          for (int i = 0; i < CPT; ++i)
+            if (!((vis[i >> 5] >> (i & 31)) & 1u)) v[i] = 0xFF800000u;
         }
-        mt = row_reduce(mt, fmax_op);
-        PF_STAMP(role, j, 2);
-        // lazily updated reference: moves only when a score (shifted by log2 of its value norm) exceeds it
-        // by more than 2^8; then this row of O is rescaled in tensor memory (no MMA is working on it)
-        const bool bump = mt > m_run + 8.f;
-        if (__any_sync(0xffffffffu, bump)) {
+        f2 ls2;
+#pragma unroll 1
+        for (int attempt = 0;; ++attempt) {
+          const float m_neg = m_run == -CUDART_INF_F ? 0.f : -m_run;
+          const f2 mn2 = pack2(m_neg, m_neg);
+          float wmax = 0.f;
+          ls2 = pack2(0.f, 0.f);
+          // norms eight columns ahead of their use: a shared-memory read takes hundreds of cycles under this load
+          ulonglong2 kn[2][2], vn[2][2];
+          auto load_norms = [&](int g) {
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+              kn[g & 1][q] = *reinterpret_cast<const ulonglong2*>(ns + 8 * g + 4 * q);
+              vn[g & 1][q] = *reinterpret_cast<const ulonglong2*>(ns + kBN + 8 * g + 4 * q);
+            }
+          };
+          load_norms(0);
+          uint32_t ph[8], pl[8];
+#pragma unroll
+          for (int g = 0; g < CPT / 8; ++g) {
+            if (g + 1 < CPT / 8) load_norms(g + 1);
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {
+              const int i = 8 * g + 2 * p;
+              const f2 k2 = (p & 1) ? kn[g & 1][p >> 1].y : kn[g & 1][p >> 1].x, v2 = (p & 1) ? vn[g & 1][p >> 1].y : vn[g & 1][p >> 1].x;
+              float x0, x1;
+              unpack2(fma2(mul2(pack2(__uint_as_float(v[i]), __uint_as_float(v[i + 1])), k2), qs2, mn2), x0, x1);
+              const f2 e = pack2(ex2_approx(x0), ex2_approx(x1));
+              ls2 = add2(ls2, e);
+              unpack2(mul2(e, v2), x0, x1);
+              wmax = max3(wmax, x0, x1);
+              const int at = 4 * (g & 1) + p;
+              if (FAST) ph[at] = pack_h2(x0, x1);
+              else {
+                const __half2 h = __floats2half2_rn(x0, x1);
+                const float2 f = __half22float2(h);
+                ph[at] = *reinterpret_cast<const uint32_t*>(&h);
+                float r0, r1;
+                unpack2(fma2(pack2(f.x, f.y), pack2(-1.f, -1.f), pack2(x0, x1)), r0, r1);
+                pl[at] = pack_h2(r0, r1);
+              }
+            }
+            if (g & 1) {
+              tmem_st8(scol + 8 * (g - 1), ph);
+              if (!FAST) tmem_st8(scol + 8 * (g - 1) + 8, pl);
+            }
+          }
+          // (sums past 1e30: a value norm of zero hides an overflow from the weights)
+          float e0, e1;
+          unpack2(ls2, e0, e1);
+          bool need = attempt == 0 && (!(wmax <= 256.f) || !(e0 + e1 < 1e30f) || (seen && m_run == -CUDART_INF_F));
+          if (TPR == 2) need = row_reduce(need ? 1.f : 0.f, fmax_op) > 0.f;
+          if (!__any_sync(0xffffffffu, need)) break;
+          // new reference: largest score of the tile, shifted by log2 of its value norm
+          float mt = -CUDART_INF_F;
+#pragma unroll
+          for (int i = 0; i < CPT; i += 4) {
+            const float4 kn = *reinterpret_cast<const float4*>(ns + i), vn = *reinterpret_cast<const float4*>(ns + kBN + i);
+            mt = max3(mt, fmaf(__uint_as_float(v[i]) * kn.x, qscale, fmaxf(lg2_approx(vn.x), -30.f)),
+                      fmaf(__uint_as_float(v[i + 1]) * kn.y, qscale, fmaxf(lg2_approx(vn.y), -30.f)));
+            mt = max3(mt, fmaf(__uint_as_float(v[i + 2]) * kn.z, qscale, fmaxf(lg2_approx(vn.z), -30.f)),
+                      fmaf(__uint_as_float(v[i + 3]) * kn.w, qscale, fmaxf(lg2_approx(vn.w), -30.f)));
+          }
+          mt = row_reduce(mt, fmax_op);
+          const bool bump = need && mt > m_run;
           const float alpha = bump ? (m_run == -CUDART_INF_F ? 0.f : ex2_approx(m_run - mt)) : 1.f;
-          if (bump) { m_run = mt; l_run *= alpha; }
-          if (j > 0) {
+          if (bump) m_run = mt;
+          l_run *= alpha;
+          if (j > 0) {  // O: no MMA is working on it
             if (NBLK == 1) {
               ok = __all_sync(0xffffffffu, bar_wait(bar(s_bars.pvd), (uint32_t)((j - 1) & 1), dead));
-              if (!ok) break;
               fence_after();
             }
 #pragma unroll 1
-            for (int c = 0; c < DPT / 32; ++c) {
-              uint32_t v[32];
-              tmem_ld32(tb + C::kColO + part * DPT + 32 * c, v);
+            for (int q = 0; q < DPT / 16; ++q) {
+              uint32_t o[16];
+              tmem_ld16_async(tb + C::kColO + part * DPT + 16 * q, o);
+              tmem_ld16_wait(o);
 #pragma unroll
-              for (int i = 0; i < 32; ++i) v[i] = __float_as_uint(__uint_as_float(v[i]) * alpha);
-              tmem_st32(tb + C::kColO + part * DPT + 32 * c, v);
-            }
-            tmem_st_wait();
-          }
-        }
-        const float m_neg = m_run == -CUDART_INF_F ? 0.f : -m_run;
-        const f2 mn2 = pack2(m_neg, m_neg);
-        f2 ls2 = pack2(0.f, 0.f);
-#pragma unroll
-        for (int h = 0; h < CPT / 32; ++h) {
-          uint32_t v[32], ph[16], pl[16];
-          tmem_ld32(scol + 32 * h, v);
-          if (inner) {
-#pragma unroll
-            for (int i4 = 0; i4 < 8; ++i4) {
-              const ulonglong2 kn = reinterpret_cast<const ulonglong2*>(ns + 32 * h)[i4];
-              const ulonglong2 vn = reinterpret_cast<const ulonglong2*>(ns + kBN + 32 * h)[i4];
-#pragma unroll
-              for (int p = 0; p < 2; ++p) {
-                float x0, x1;
-                unpack2(fma2(mul2(pack2(__uint_as_float(v[4 * i4 + 2 * p]), __uint_as_float(v[4 * i4 + 2 * p + 1])), p ? kn.y : kn.x), qs2, mn2), x0, x1);
-                const f2 e = pack2(ex2_approx(x0), ex2_approx(x1));
-                ls2 = add2(ls2, e);
-                unpack2(mul2(e, p ? vn.y : vn.x), x0, x1);
-                if (FAST) ph[2 * i4 + p] = pack_h2(x0, x1);
-                else split2(x0, x1, ph[2 * i4 + p], pl[2 * i4 + p]);
-              }
-            }
-          } else {
-#pragma unroll
-            for (int i2 = 0; i2 < 16; ++i2) {
-              float w[2], e[2];
-#pragma unroll
-              for (int q = 0; q < 2; ++q) {
-                const int i = 32 * h + 2 * i2 + q;
-                const bool vis = visible(i);  // (a hidden column's norms may be anything: select, do not multiply)
-                e[q] = vis ? ex2_approx(fmaf(__uint_as_float(v[2 * i2 + q]) * ns[i], qscale, m_neg)) : 0.f;
-                w[q] = vis ? e[q] * ns[kBN + i] : 0.f;
-              }
-              ls2 = add2(ls2, pack2(e[0], e[1]));
-              if (FAST) ph[i2] = pack_h2(w[0], w[1]);
-              else split2(w[0], w[1], ph[i2], pl[i2]);
+              for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+              tmem_st16(tb + C::kColO + part * DPT + 16 * q, o);
             }
           }
-          tmem_st16(scol + 32 * h, ph);
-          if (!FAST) tmem_st16(scol + 32 * h + 16, pl);
         }
         tmem_st_wait();
         float s0, s1;
@@ -990,6 +1120,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
       }
     }
 
+    PF_STAMP(tid == 0 ? 0 : -1, 0, 7);
     // ---- normalise, un-rotate, store ------------------------------------------------------------------
     l_run = row_reduce(l_run, [](float x, float y) { return x + y; });
     bool have = use;
@@ -1000,6 +1131,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
     }
     const float inv = have ? 1.f / (a.lut_scale_v * l_run) : 0.f;
     const float lse = have ? (m_run + lg2_approx(l_run)) * 0.6931471805599453f : -CUDART_INF_F;
+    const bool out_vec = (uintptr_t)a.out % 16 == 0 && a.out_token_stride % 8 == 0 && a.out_head_stride % 8 == 0;
     if (pa.to_parts || a.out_rotated) {
       const int64_t vec = ((int64_t)blockIdx.z * sh.rows + row) * sh.Hq + head;
       const int64_t oi = pa.to_parts ? vec * D : (int64_t)row * a.out_token_stride + (int64_t)head * a.out_head_stride;
@@ -1010,13 +1142,10 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
         uint32_t v[32];
         if (use && ok) tmem_ld32(tb + C::kColO + part * DPT + 32 * c, v);
         if (live) {
+          float y[32];
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            float y[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) y[e] = have ? __uint_as_float(v[4 * i + e]) * inv : 0.f;
-            store4(dst, dt, oi + part * DPT + 32 * c + 4 * i, y);
-          }
+          for (int e = 0; e < 32; ++e) y[e] = have ? __uint_as_float(v[e]) * inv : 0.f;
+          store32(dst, dt, oi + part * DPT + 32 * c, out_vec, y);
         }
       }
       if (live && part == 0 && pa.to_parts) pa.part_m[vec] = lse;
@@ -1025,28 +1154,26 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
       float isc = 0.f;
       if (use) {
         float amax = 0.f, sc = 1.f;
-        if (ok) {
 #pragma unroll 1
-          for (int c = 0; c < DPT / 32; ++c) {
+        for (int pass = 0; pass < 2; ++pass) {
+#pragma unroll 1
+          for (int c = 0; c < DPT / 32 && ok; ++c) {
             uint32_t v[32];
-            tmem_ld32(tb + C::kColO + part * DPT + 32 * c, v);
-#pragma unroll
-            for (int i = 0; i < 32; ++i) amax = fmaxf(amax, fabsf(__uint_as_float(v[i]) * inv));
-          }
-        }
-        pow2_scale(row_reduce(amax, fmax_op), sc, isc);
-        if (ok) {
-#pragma unroll 1
-          for (int c = 0; c < DPT / 32; ++c) {
-            uint32_t v[32], h[16], l[16];
             const int d0 = part * DPT + 32 * c;
-            tmem_ld32(tb + C::kColO + d0, v);
+            tmem_ld_cols(tb + C::kColO + d0, v);
+            if (pass == 0) {
+#pragma unroll
+              for (int e = 0; e < 16; ++e) amax = max3(amax, fabsf(__uint_as_float(v[2 * e])), fabsf(__uint_as_float(v[2 * e + 1])));
+              continue;
+            }
+            uint32_t h[16], l[16];
 #pragma unroll
             for (int e = 0; e < 16; ++e)
               split2(__uint_as_float(v[2 * e]) * inv * sc, __uint_as_float(v[2 * e + 1]) * inv * sc, h[e], l[e]);
             tmem_st16(tb + C::kColS + d0 / 2, h);
             tmem_st16(tb + C::kColQ + d0 / 2, l);
           }
+          if (pass == 0) pow2_scale(row_reduce(amax * inv, fmax_op), sc, isc);
         }
         tmem_st_wait();
         arrive(s_bars.aready);
@@ -1063,13 +1190,10 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
         uint32_t v[32];
         if (use && ok) tmem_ld32(tb + C::kColO + part * DPT + 32 * c, v);
         if (live) {
+          float y[32];
 #pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            float y[4];
-#pragma unroll
-            for (int e = 0; e < 4; ++e) y[e] = f != 0.f ? __uint_as_float(v[4 * i + e]) * f : 0.f;
-            store4(a.out, a.out_dtype, oi + 32 * c + 4 * i, y);
-          }
+          for (int e = 0; e < 32; ++e) y[e] = f != 0.f ? __uint_as_float(v[e]) * f : 0.f;
+          store32(a.out, a.out_dtype, oi + 32 * c, out_vec, y);
         }
       }
       if (live && part == 0 && a.lse_out) a.lse_out[(int64_t)row * sh.Hq + head] = lse;
@@ -1077,6 +1201,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
   }
   fence_before();
   __syncthreads();
+  PF_STAMP(tid == 0 ? 0 : -1, 1, 4);
   if (s_dead && tid == 0 && a.err_flag) atomicOr(a.err_flag, TQ4_DEV_TIMEOUT);
   if (warp == kIssueWarp) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");

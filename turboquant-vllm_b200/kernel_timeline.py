@@ -121,8 +121,10 @@ def print_prefill_trace(nv, reader: str) -> None:
     buf = np.zeros(4 * 64 * 8, dtype=np.int64)
     assert getattr(nv.lib(), reader)(buf.ctypes.data) == 0
     t = buf.reshape(4, 64, 8).astype(np.float64)
-    roles = {"softmax, first row block": ("top", "scores ready", "row maximum", "P stored"),
-             "softmax, second row block": ("top", "scores ready", "row maximum", "P stored"),
+    e = [t[0, 0, i] - t[0, 0, 4] for i in (5, 6, 7)] + [t[0, 1, 4] - t[0, 0, 4]]
+    print("SM cycles from kernel entry: tables built %.0f, queries rotated %.0f, last tile %.0f, outputs stored %.0f" % tuple(e))
+    roles = {"softmax, first row block": ("top", "scores ready", None, "P stored"),
+             "softmax, second row block": ("top", "scores ready", None, "P stored"),
              "first dequantising warp": ("keys' buffer free", "keys written", "next tile's loads issued",
                                          "values' buffer free", "values written"),
              "issuing thread": ("P of block 0 ready", "PV and next S of block 0 issued", "P of block 1 ready",
@@ -132,7 +134,8 @@ def print_prefill_trace(nv, reader: str) -> None:
         m = np.mean(np.array(rows), axis=0)
         print(f"== {name}: SM cycles since its first event of the tile (mean of tiles 20..49)")
         for e, what in enumerate(events):
-            print(f"   {what:34s} {m[e]:8.0f}")
+            if what:
+                print(f"   {what:34s} {m[e]:8.0f}")
         print(f"   {'next tile':34s} {m[-1]:8.0f}")
 
 
