@@ -1,0 +1,45 @@
+"""The tensor-core write kernel for 16-bit vectors at the edges of its tiles, every head_dim it takes."""
+
+import pytest
+import torch
+
+from oracle import tq4_oracle as O
+from tests.helpers import Prims, index_mismatch, ulp_diff
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("d", [64, 96, 128, 256])
+@pytest.mark.parametrize("n_tok,h,dtype,strided", [
+    (345, 3, torch.bfloat16, False),   # just past the line to this kernel; heads that do not divide a tile
+    (512, 4, torch.float16, True),     # whole tiles; K and V halves of one tensor
+    (1057, 8, torch.bfloat16, True),   # a remainder of one token
+])
+def test_paged_write_tiles(cuda_lib, d, n_tok, h, dtype, strided):
+    from turboquant_vllm.kernels import ops
+
+    pr = Prims(d)
+    p = pr.cuda()
+    k, v = O.synthetic_kv(n_tok, h, d, seed=n_tok + d, dtype=dtype)
+    bs = 16
+    nblk = n_tok // bs + 2
+    width = h * O.padded_slot_bytes(d)
+    slots = torch.randperm(nblk * bs, generator=torch.Generator().manual_seed(d))[:n_tok]
+    slots[3] = slots[-1] = -1
+    keep = slots >= 0
+    ref = torch.zeros(nblk, bs, width, dtype=torch.uint8)
+    O.write_paged(k[keep], v[keep], ref, slots[keep], pr.rot, pr.kb, pr.vb)
+    kc, vc = k.cuda(), v.cuda()
+    if strided:
+        kc, vc = torch.cat([kc, vc], dim=1).split(h, dim=1)
+    cache = torch.zeros(nblk, bs, width, dtype=torch.uint8, device="cuda")
+    ops.tq4_write_paged(kc, vc, cache, slots.cuda(), p["even"], p["odd"], p["kb"], p["vb"])
+    got, want = cache.cpu().view(-1, width), ref.view(-1, width)
+    kn, vi, vn, end = O.row_layout(h, d)
+    for a, b in ((0, kn), (vi, vn)):
+        assert index_mismatch(got[:, a:b].contiguous(), want[:, a:b].contiguous()) <= 1e-4
+    for a in (kn, vn):
+        x, y = (t[:, a:a + 4 * h].contiguous().view(torch.float32) + 1e-30 for t in (got, want))
+        assert ulp_diff(x, y).max() <= 4
+    assert torch.equal(got[:, end:], want[:, end:])
+    assert ops.read_and_clear_errors(torch.device("cuda")) == 0

@@ -9,7 +9,7 @@ from tests.helpers import Prims, build_paged_case, cosine
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("rows", [1, 3, 260])  # 260 rows x 16 vectors: past one wave of 32-column blocks
+@pytest.mark.parametrize("rows", [1, 3, 100, 260])  # a block per vector; 32-column blocks; past one wave of them
 @pytest.mark.parametrize("d", [64, 96, 128, 256])
 def test_step_writes_and_rotates(cuda_lib, d, rows):
     from turboquant_vllm.kernels import ops
@@ -29,7 +29,10 @@ def test_step_writes_and_rotates(cuda_lib, d, rows):
     out = ops.paged_tq4_attention(
         q.cuda(), cache, bt.cuda(), case["seq_lens"].cuda(), p["kc"], p["vc"], p["rot"], hkv, bs,
         out_dtype=torch.float32, write=(k, v, slots.cuda(), p["even"], p["odd"], p["kb"], p["vb"]))
-    assert torch.equal(cache, want)
+    if 2 * hkv * rows <= (512 if d == 256 else 2048):  # above, a stand-alone write rotates on the tensor cores
+        assert torch.equal(cache, want)
+    else:
+        assert (cache != want).float().mean() <= 1e-4
     pick = sorted({0, rows // 2, rows - 1})
     ref = O.paged_decode_fp32(q[pick], want.cpu(), bt[pick], [lens[i] for i in pick], pr.kc, pr.vc, pr.rot, hkv)
     got = out.cpu()[pick]

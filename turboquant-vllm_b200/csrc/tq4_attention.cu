@@ -244,6 +244,59 @@ prologue_kernel(const AttnArgs a, const CompressArgs w, const int has_attn, cons
     if (last > 0) atomicMax(&s_active, min(last, a.sh.rows));
   }
 
+  if (has_attn && a.skip_long > 0) __syncthreads();  // (s_active)
+  // vector counts fit 32 bits (rows <= kMaxRowsPerLaunch, writes <= kSmallRows): no 64-bit divisions
+  const int n_q = has_attn ? (a.skip_long > 0 ? s_active : a.sh.rows) * a.sh.Hq : 0;
+  const int rows_per_src = has_write ? (int)w.n_tokens * w.num_heads : 0;
+  const int n_w = rows_per_src * (has_write ? w.n_sources : 0);
+  const int cq = (n_q + VC - 1) / VC, cw = (n_w + VC - 1) / VC;
+  float4* gx = s_x + warp * D;
+  const bool jact = NJ * lane < JC;                     // this lane owns outputs j0 + NJ * lane .. + NJ - 1
+  const float* pcol = s_pit + (jact ? NJ * lane : 0);   // + d * JC
+  // (source, token, head) of write vector `vec`
+  auto w_coords = [&](int vec, int& src, int& tok, int& h) {
+    src = vec >= rows_per_src ? 1 : 0;
+    const unsigned rem = (unsigned)(vec - src * rows_per_src);
+    tok = (int)(rem / (unsigned)w.num_heads);
+    h = (int)(rem - (unsigned)tok * (unsigned)w.num_heads);
+  };
+
+  // The four vectors of a chunk (lane l: elements l, l + 32, ... of each) and the slots of written ones: fetched before Pi
+  // is staged, the next chunk's while this one is multiplied.
+  float xr[XPL][VC];
+  int64_t slots[VC];
+  auto load_chunk = [&](int c) {
+    if (c >= cq + cw) return;
+    const bool is_w = c >= cq;
+    const int v0 = (is_w ? c - cq : c) * VC;
+    const int nv = is_w ? n_w : n_q;
+    const int dt = is_w ? w.x_dtype : a.q_dtype;
+    const void* base[VC];
+#pragma unroll
+    for (int v = 0; v < VC; ++v) {
+      const int vec = v0 + v;
+      base[v] = nullptr;
+      if (vec < nv) {
+        if (!is_w) {
+          const unsigned rr = (unsigned)vec / (unsigned)a.sh.Hq;
+          const int h = (int)((unsigned)vec - rr * (unsigned)a.sh.Hq);
+          base[v] = byte_offset(a.q, dt, ((int64_t)rr + a.sh.row_offset) * a.q_token_stride +
+                                             h * a.q_head_stride + lane);
+        } else {
+          int src, tok, h;
+          w_coords(vec, src, tok, h);
+          if (w.cache != nullptr) slots[v] = tok < w.n_slots ? write_slot(w, tok) : -1;
+          base[v] = byte_offset(w.x[src], dt, token_offset(w, src, tok) + (int64_t)h * w.head_stride[src] + lane);
+        }
+      }
+    }
+    if (dt == TQ4_F32) load_strip<float, XPL, VC>(base, xr);
+    else if (dt == TQ4_F16) load_strip<__half, XPL, VC>(base, xr);
+    else load_strip<__nv_bfloat16, XPL, VC>(base, xr);
+  };
+  const int first = (bid / P::NSPLIT) * P::WARPS + warp, step = n_blocks * P::WARPS;
+  load_chunk(first);
+
   // ---- stage the slice of Pi^T --------------------------------------------------------------------
   if (has_attn) {
     // thread -> (4 consecutive d of row j), consecutive threads = consecutive j: conflict-free stores
@@ -267,59 +320,23 @@ prologue_kernel(const AttnArgs a, const CompressArgs w, const int has_attn, cons
       }
     }
   } else {  // write only: the caller gave Pi^T split into even / odd output columns
-    for (int i = tid; i < D * JC / 2; i += P::THREADS) {
-      const int k = i / (JC / 2), pp = i - k * (JC / 2);
-      s_pit[k * JC + 2 * pp] = __ldg(w.rot_even + k * HALF + j0 / 2 + pp);
-      s_pit[k * JC + 2 * pp + 1] = __ldg(w.rot_odd + k * HALF + j0 / 2 + pp);
+    constexpr int N = D * JC / 8;  // (row k, four column pairs)
+#pragma unroll 4
+    for (int i = tid; i < N; i += P::THREADS) {
+      const int k = i / (JC / 8), q = i - k * (JC / 8);
+      const float4 e = __ldg(reinterpret_cast<const float4*>(w.rot_even + k * HALF + j0 / 2) + q);
+      const float4 o = __ldg(reinterpret_cast<const float4*>(w.rot_odd + k * HALF + j0 / 2) + q);
+      float4* dst = reinterpret_cast<float4*>(s_pit + k * JC + 8 * q);
+      dst[0] = make_float4(e.x, o.x, e.y, o.y);
+      dst[1] = make_float4(e.z, o.z, e.w, o.w);
     }
   }
   __syncthreads();
 
-  // vector counts fit 32 bits (rows <= kMaxRowsPerLaunch, writes <= kSmallRows): no 64-bit divisions
-  const int n_q = has_attn ? (a.skip_long > 0 ? s_active : a.sh.rows) * a.sh.Hq : 0;
-  const int rows_per_src = has_write ? (int)w.n_tokens * w.num_heads : 0;
-  const int n_w = rows_per_src * (has_write ? w.n_sources : 0);
-  const int cq = (n_q + VC - 1) / VC, cw = (n_w + VC - 1) / VC;
-  float4* gx = s_x + warp * D;
-  const bool jact = NJ * lane < JC;                     // this lane owns outputs j0 + NJ * lane .. + NJ - 1
-  const float* pcol = s_pit + (jact ? NJ * lane : 0);   // + d * JC
-  // (source, token, head) of write vector `vec`
-  auto w_coords = [&](int vec, int& src, int& tok, int& h) {
-    src = vec >= rows_per_src ? 1 : 0;
-    const unsigned rem = (unsigned)(vec - src * rows_per_src);
-    tok = (int)(rem / (unsigned)w.num_heads);
-    h = (int)(rem - (unsigned)tok * (unsigned)w.num_heads);
-  };
-
-  for (int c = (bid / P::NSPLIT) * P::WARPS + warp; c < cq + cw; c += n_blocks * P::WARPS) {
+  for (int c = first; c < cq + cw; c += step) {
     const bool is_w = c >= cq;
     const int v0 = (is_w ? c - cq : c) * VC;
     const int nv = is_w ? n_w : n_q;
-    // ---- load: lane l holds elements l, l+32, ... of each of the four vectors -------------------
-    float xr[XPL][VC];
-    const int dt = is_w ? w.x_dtype : a.q_dtype;
-    const void* base[VC];
-#pragma unroll
-    for (int v = 0; v < VC; ++v) {
-      const int vec = v0 + v;
-      base[v] = nullptr;
-      if (vec < nv) {
-        if (!is_w) {
-          const unsigned rr = (unsigned)vec / (unsigned)a.sh.Hq;
-          const int h = (int)((unsigned)vec - rr * (unsigned)a.sh.Hq);
-          base[v] = byte_offset(a.q, dt, ((int64_t)rr + a.sh.row_offset) * a.q_token_stride +
-                                             h * a.q_head_stride + lane);
-        } else {
-          int src, tok, h;
-          w_coords(vec, src, tok, h);
-          base[v] = byte_offset(w.x[src], dt, (int64_t)tok * w.token_stride[src] +
-                                                  (int64_t)h * w.head_stride[src] + lane);
-        }
-      }
-    }
-    if (dt == TQ4_F32) load_strip<float, XPL, VC>(base, xr);
-    else if (dt == TQ4_F16) load_strip<__half, XPL, VC>(base, xr);
-    else load_strip<__nv_bfloat16, XPL, VC>(base, xr);
     float nrm[VC];
     if (is_w) {
 #pragma unroll
@@ -337,6 +354,10 @@ prologue_kernel(const AttnArgs a, const CompressArgs w, const int has_attn, cons
 #pragma unroll
     for (int i = 0; i < XPL; ++i) gx[lane + 32 * i] = make_float4(xr[i][0], xr[i][1], xr[i][2], xr[i][3]);
     __syncwarp();
+    int64_t slot_of[VC];
+#pragma unroll
+    for (int v = 0; v < VC; ++v) slot_of[v] = slots[v];
+    load_chunk(c + step);
 
     // ---- y[v][jj] = sum_d x[v][d] * Pi[j0 + NJ*lane + jj][d] as (s0 + s1) + (s2 + s3): the two
     // quarter chains of a half advance together (8 NJ independent accumulators); loops stay rolled,
@@ -399,8 +420,7 @@ prologue_kernel(const AttnArgs a, const CompressArgs w, const int has_attn, cons
         uint8_t* dst_idx;
         float* dst_norm;
         if (w.cache != nullptr) {
-          if (tok >= w.n_slots) continue;
-          const int64_t slot = w.slot_mapping[tok];
+          const int64_t slot = slot_of[v];
           if (slot < 0) continue;
           if (slot >= w.num_cache_slots) {
             if (lane == 0 && w.err_flag) atomicOr(w.err_flag, TQ4_DEV_BAD_SLOT);
@@ -983,6 +1003,8 @@ int launch_prologue(const AttnArgs* a, const CompressArgs* w, int head_dim, cuda
   }
   return TQ4_ERR_UNSUPPORTED;
 }
+
+int launch_small_write(const CompressArgs& w, int head_dim, cudaStream_t st) { return launch_prologue(nullptr, &w, head_dim, st); }
 
 }  // namespace tq4
 

@@ -249,21 +249,49 @@ struct CompressArgs {
   // contiguous destination
   uint8_t* packed_out;
   float* norms_out;
-  // paged destination (cache != nullptr selects it)
+  // paged destination (cache != nullptr selects it).  Token t goes to slot_mapping[t], or, with seq > 0, to
+  // row (t / seq) * row_capacity + row_offset + t % seq (token rows of a batch, each appended to); batch_stride is
+  // then the distance of the sequences in x (with token_stride inside them)
   uint8_t* cache;
   const int64_t* slot_mapping;
+  int64_t seq, batch_stride[2], row_capacity, row_offset;
   int64_t n_slots, cache_token_stride, num_cache_slots;
   int* err_flag;
 };
 
-// rows at or below this count are handled by the small-launch kernels
-constexpr int64_t kSmallRows = 8192;
+__device__ __forceinline__ int64_t write_slot(const CompressArgs& a, int64_t tok) {
+  if (a.seq == 0) return a.slot_mapping[tok];
+  const unsigned b = (unsigned)tok / (unsigned)a.seq;
+  return (int64_t)b * a.row_capacity + a.row_offset + ((unsigned)tok - b * (unsigned)a.seq);
+}
+// element offset of token `tok` in source `src`
+__device__ __forceinline__ int64_t token_offset(const CompressArgs& a, int src, int64_t tok) {
+  if (a.seq == 0) return tok * a.token_stride[src];
+  const unsigned b = (unsigned)tok / (unsigned)a.seq;
+  return (int64_t)b * a.batch_stride[src] + (int64_t)((unsigned)tok - b * (unsigned)a.seq) * a.token_stride[src];
+}
+// sequences of every source follow one another like tokens (always so without sequences)
+inline bool tokens_uniform(const CompressArgs& a) {
+  for (int s = 0; s < a.n_sources; ++s)
+    if (a.seq > 0 && a.n_tokens > a.seq && a.batch_stride[s] != a.seq * a.token_stride[s]) return false;
+  return true;
+}
+
+// Which kernel makes a write of so many vectors (B200, graph replays of stand-alone writes, bf16):
+//   head_dim <= 128: a block per vector up to kTinyRows (5.2 us at 32 vectors, 8.4 at 2048; the prologue kernel 8.1 and
+//   10.5, the tensor-core kernel 10.4 and 10.6), above it the tensor-core kernel (10.8 us at 8192 vectors; a block per
+//   vector 24, the prologue kernel 16).  head_dim 256: the prologue kernel up to kTinyRows256 (11 us; a block per
+//   vector 24), above it the tensor-core kernel (10.4 us at 800 vectors, the prologue kernel 15).
+// What the tensor-core kernel cannot address takes the prologue kernel up to kSmallRows; so does the write of a decode step
+// (it shares the launch with the query rotation).
+constexpr int64_t kTinyRows = 2048, kTinyRows256 = 512, kSmallRows = 8192;
+int launch_small_write(const CompressArgs& w, int head_dim, cudaStream_t st);
 int dispatch_compress(const CompressArgs& a, int head_dim, int dtype, cudaStream_t st);
 // tensor-core (tcgen05) compress kernel for large inputs at head_dim 128 (tq4_compress_tc.cu)
 bool compress_tc_eligible(const CompressArgs& a, int head_dim, int dtype);
 int launch_compress_tc(const CompressArgs& a, int dtype, cudaStream_t st);
-// pipelined tcgen05 kernel for dense 16-bit inputs at head_dim 128 (tq4_compress_tc16.cu)
+// pipelined tcgen05 kernel for 16-bit inputs (tq4_compress_tc16.cu)
 bool compress_tc16_eligible(const CompressArgs& a, int head_dim, int dtype);
-int launch_compress_tc16(const CompressArgs& a, int dtype, cudaStream_t st);
+int launch_compress_tc16(const CompressArgs& a, int head_dim, int dtype, cudaStream_t st);
 
 }  // namespace tq4

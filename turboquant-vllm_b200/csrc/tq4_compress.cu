@@ -87,8 +87,7 @@ compress_kernel(const CompressArgs a) {
         int src, h;
         int64_t tok;
         row_coords(row, src, tok, h);
-        const T* xp = reinterpret_cast<const T*>(a.x[src]) + tok * a.token_stride[src] +
-                      (int64_t)h * a.head_stride[src];
+        const T* xp = reinterpret_cast<const T*>(a.x[src]) + token_offset(a, src, tok) + (int64_t)h * a.head_stride[src];
 #pragma unroll
         for (int i = 0; i < XPL; ++i) {
           const int k = lane + 32 * i;
@@ -179,7 +178,7 @@ compress_kernel(const CompressArgs a) {
       float* dst_norm;
       if (a.cache != nullptr) {
         if (tok >= a.n_slots) continue;
-        const int64_t slot = a.slot_mapping[tok];
+        const int64_t slot = write_slot(a, tok);
         if (slot < 0) continue;
         if (slot >= a.num_cache_slots) {
           if (lane == 0 && a.err_flag) atomicOr(a.err_flag, TQ4_DEV_BAD_SLOT);
@@ -208,7 +207,7 @@ compress_kernel(const CompressArgs a) {
   }
 }
 
-// Small launches (decode: a few hundred to a few thousand rows): one CTA of four warps per row,
+// Small launches: one CTA of four warps per row,
 // each warp reduces one quarter of k with Pi^T read straight from L1/L2; the four partial sums
 // are combined as (s0 + s1) + (s2 + s3), the same order the streaming kernel uses, so a row
 // compresses to the same bytes whichever kernel handles it.
@@ -231,8 +230,7 @@ __global__ void __launch_bounds__(128) compress_small_kernel(const CompressArgs 
     const int i = threadIdx.x - 32;
     s_b[i] = i < a.n_bounds[src] ? a.bounds[src][i] : CUDART_INF_F;
   }
-  const T* xp = reinterpret_cast<const T*>(a.x[src]) + tok * a.token_stride[src] +
-                (int64_t)h * a.head_stride[src];
+  const T* xp = reinterpret_cast<const T*>(a.x[src]) + token_offset(a, src, tok) + (int64_t)h * a.head_stride[src];
   float xv[XPL];
   float ss = 0.f;
 #pragma unroll
@@ -295,7 +293,7 @@ __global__ void __launch_bounds__(128) compress_small_kernel(const CompressArgs 
   float* dst_norm;
   if (a.cache != nullptr) {
     if (tok >= a.n_slots) return;
-    const int64_t slot = a.slot_mapping[tok];
+    const int64_t slot = write_slot(a, tok);
     if (slot < 0) return;
     if (slot >= a.num_cache_slots) {
       if (lane == 0 && a.err_flag) atomicOr(a.err_flag, TQ4_DEV_BAD_SLOT);
@@ -326,8 +324,8 @@ int launch_compress(const CompressArgs& a, cudaStream_t st) {
   const int64_t total_rows = a.n_tokens * a.num_heads * a.n_sources;
   if (total_rows == 0) return TQ4_OK;
   if (total_rows > 0x7fffffffll) return TQ4_ERR_INVALID_ARG;  // the kernels index rows with 32 bits
-  if (total_rows <= kSmallRows) {
-    compress_small_kernel<D, T><<<(unsigned)total_rows, 128, 0, st>>>(a);
+  if (D <= 128 && total_rows <= kTinyRows) {
+    compress_small_kernel<D <= 128 ? D : 128, T><<<(unsigned)total_rows, 128, 0, st>>>(a);
     TQ4_CHECK_LAUNCH();
     return TQ4_OK;
   }
@@ -352,10 +350,13 @@ int dispatch_dtype(const CompressArgs& a, int dtype, cudaStream_t st) {
 }
 
 int dispatch_compress(const CompressArgs& a, int head_dim, int dtype, cudaStream_t st) {
-  if (a.n_tokens * a.num_heads * a.n_sources > kSmallRows) {
-    if (compress_tc16_eligible(a, head_dim, dtype)) return launch_compress_tc16(a, dtype, st);
-    if (compress_tc_eligible(a, head_dim, dtype)) return launch_compress_tc(a, dtype, st);
-  }
+  const int64_t vectors = a.n_tokens * a.num_heads * a.n_sources;
+  if (vectors == 0) return TQ4_OK;
+  const bool tiny = head_dim <= 128 && vectors <= kTinyRows;  // (dispatch_dtype: a block per vector)
+  if (vectors > (head_dim == 256 ? kTinyRows256 : kTinyRows) && compress_tc16_eligible(a, head_dim, dtype))
+    return launch_compress_tc16(a, head_dim, dtype, st);
+  if (!tiny && vectors <= kSmallRows) return launch_small_write(a, head_dim, st);
+  if (!tiny && compress_tc_eligible(a, head_dim, dtype)) return launch_compress_tc(a, dtype, st);
   switch (head_dim) {
     case 64: return dispatch_dtype<64>(a, dtype, st);
     case 96: return dispatch_dtype<96>(a, dtype, st);

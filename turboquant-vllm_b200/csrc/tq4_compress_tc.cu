@@ -259,7 +259,7 @@ compress_tc_kernel(const CompressArgs a, const __grid_constant__ CUtensorMap tm_
       const unsigned t = rem / (unsigned)a.num_heads;
       tok = t;
       h = (int)(rem - t * (unsigned)a.num_heads);
-      xp = reinterpret_cast<const T*>(a.x[src]) + tok * a.token_stride[src] + (int64_t)h * a.head_stride[src];
+      xp = reinterpret_cast<const T*>(a.x[src]) + token_offset(a, src, tok) + (int64_t)h * a.head_stride[src];
     }
     // ---- norm, in the summation order of the FMA kernels: p[l] over k = l, l+32, l+64, l+96,
     //      then the butterfly tree 16, 8, 4, 2, 1 -------------------------------------------------
@@ -377,7 +377,7 @@ compress_tc_kernel(const CompressArgs a, const __grid_constant__ CUtensorMap tm_
       uint8_t* dst_idx = nullptr;
       float* dst_norm = nullptr;
       if (a.cache != nullptr) {
-        const int64_t slot = tok < a.n_slots ? a.slot_mapping[tok] : -1;
+        const int64_t slot = tok < a.n_slots ? write_slot(a, tok) : -1;
         if (slot >= a.num_cache_slots) {
           if (half == 0 && a.err_flag) atomicOr(a.err_flag, TQ4_DEV_BAD_SLOT);
         } else if (slot >= 0) {
@@ -413,7 +413,7 @@ bool compress_tc_eligible(const CompressArgs& a, int head_dim, int dtype) {
   if (disabled || head_dim != kD) return false;
   const int es = dtype == TQ4_F32 ? 4 : 2;
   for (int s = 0; s < a.n_sources; ++s) {
-    if (((uintptr_t)a.x[s] & 15) || (a.token_stride[s] * es) % 16 || (a.head_stride[s] * es) % 16) return false;
+    if (((uintptr_t)a.x[s] & 15) || (a.token_stride[s] * es) % 16 || (a.head_stride[s] * es) % 16 || (a.batch_stride[s] * es) % 16) return false;
   }
   return true;
 }
@@ -468,7 +468,7 @@ static int launch_tc(const CompressArgs& a, cudaStream_t st) {
   memset(&m1, 0, sizeof(m1));
   if (sizeof(T) == 2) {
     // staged input tiles need every source to be a dense [rows][128] array
-    bool dense = true;
+    bool dense = tokens_uniform(a);
     for (int s = 0; s < a.n_sources; ++s)
       dense = dense && a.head_stride[s] == kD && a.token_stride[s] == (int64_t)a.num_heads * kD;
     const int64_t rows = a.n_tokens * a.num_heads;

@@ -1,28 +1,37 @@
-// TQ4 compress for prefill-sized 16-bit inputs at head_dim 128, pipelined on the 5th-generation
-// tensor cores.  The rotation of a tile of 128 vectors is a 128 x 128 x 128 GEMM
+// TQ4 compress for prefill-sized 16-bit inputs, pipelined on the 5th-generation tensor cores.  The rotation
+// of a tile of 128 vectors is a 128 x D x D GEMM
 //     Y_raw = X * Pi^T        (tcgen05.mma kind::f16, fp32 accumulator in tensor memory)
 // on the RAW input rows: a 16-bit input is exact as an MMA operand, so the A operand needs no
 // CUDA-core preparation at all and arrives in shared memory by TMA in the swizzled layout the MMA
 // reads.  Pi is the B operand, resident in shared memory as a sum of 16-bit terms (bf16 inputs:
 // three bf16 terms = 24 bits; fp16 inputs: 2^8 * Pi as fp16 hi + lo = 22 bits), one MMA per term.
+// At head_dim 256 the terms do not fit: a CTA owns 64 of the output coordinates (its rows are read by four
+// CTAs, three times from L2).
 // The normalisation commutes with the product: y = Y_raw / (norm + 1e-10) is applied to the fp32
 // accumulator in the epilogue.  A rotated coordinate therefore differs from the fp32 FMA kernels by
 // ~1e-7 absolute, which moves an index only when the coordinate sits that close to a bucket
 // boundary (bound 1e-4 of the indices).  Norms are summed in exactly the order of the FMA kernels
 // (lane-strided FMAs, butterfly tree), so they are bit-identical to them.
 //
-// One persistent CTA per SM, warp-specialised, four input stages and four accumulators in flight:
-//   warp 0      TMA producer: the 128 rows of a tile as two 64-column boxes (128-byte swizzle)
-//   warp 1      MMA issuer: 8 k-steps x terms of tcgen05.mma 128x128x16, then tcgen05.commit onto
-//               the stage's "empty" barrier and the accumulator's "full" barrier
-//   warps 2-17  four epilogue groups of four warps; tile i of the CTA belongs to group i % 4 and uses
-//               input stage i % 4 and accumulator i % 4, so every barrier is waited on by one group
-//               in tile order (a stage shared between groups could show a fast group an older
-//               phase).  The epilogue is CUDA-core work; four warps per scheduler hide its latencies:
-//               thread = row.  Sum of squares from the staged tile -> release the stage -> wait for
-//               the accumulator -> four times: tcgen05.ld of 32 columns, scale, bucketize (binary
-//               search over boundaries held in registers), nibble-pack, one 16-byte store into the
-//               packed output or the paged cache row.
+// One persistent CTA per SM, warp-specialised, four (head_dim 256: two) input stages and accumulators in flight:
+//   warp 0      TMA producer: the 128 rows of a tile as 64-column boxes (128-byte swizzle)
+//   warp 1      MMA issuer: D / 16 k-steps x terms of tcgen05.mma, then tcgen05.commit onto the stage's "empty"
+//               barrier and the accumulator's "full" barrier
+//   warps 2 ..  one epilogue group of four warps per stage; tile i of the CTA belongs to group i % stages and uses
+//               that input stage and accumulator, so every barrier is waited on by one group in tile order (a
+//               stage shared between groups could show a fast group an older phase).  Thread = row: sum
+//               of squares from the staged tile -> release the stage -> wait for the accumulator -> per 32
+//               columns: tcgen05.ld, scale, bucketize, nibble-pack, one 16-byte store into the packed output
+//               or the paged cache row.
+// What bounds it is the epilogue's instruction count, and in it the bucketize.  A search over registers takes 22
+// instructions a coordinate.  Here a coordinate is first mapped to one of 32 uniform cells, each of which holds at
+// most one boundary (checked when the CTA starts, with a margin for the rounding of the map; codebooks whose
+// boundaries are too close for that take the search): two FMAs, two lookups through the warp shuffle
+// (lane c holds cell c's boundary and the index below it), one compare, one add.  The comparison is the
+// search's own, against the same fp32 boundary, so the indices are the same.  Measured (bf16 cache write, K and
+// V): 16384 tokens of 8 heads of 128 48.6 -> 31.1 us (2.7 TB/s), 512 tokens (8192 vectors) 24 -> 10.8 us
+// against a block per vector, 16384 tokens of 4 heads of 256 894 -> 62 us (the 256 columns are split over two CTAs:
+// one cannot hold Pi and two stages of vectors).
 // Every mbarrier wait is bounded; a wait that gives up marks the CTA dead, all roles drain and the
 // kernel reports TQ4_DEV_TIMEOUT.  Tensor memory is released on every path.
 #include <cuda.h>
@@ -49,18 +58,24 @@ __device__ long long g_ctrace[4][32][8];
 
 namespace {
 
-constexpr int kD = 128;
 constexpr int kRows = 128;                       // vectors per tile (MMA M, TMEM lanes)
-constexpr int kStages = 4;                       // input stages = epilogue groups = accumulators
-constexpr int kAccs = kStages;                   // tile i of a CTA uses stage, accumulator and group i % 4
-constexpr int kThreads = 64 + kAccs * 128;       // producer, issuer, kAccs x 4 epilogue warps
-constexpr uint32_t kBlockBytes = kRows * 128;    // one K-block (64 16-bit columns) of an operand: 16 KB
-constexpr uint32_t kTileBytes = 2 * kBlockBytes; // a tile = two K-blocks
+constexpr uint32_t kBlockBytes = kRows * 128;    // one 64-column block of the input tile: 16 KB
 constexpr int kMaxTerms = 3;
-constexpr uint32_t kOffB = 0;                                  // terms x 2 K-blocks of Pi
-constexpr uint32_t kOffA = kMaxTerms * kTileBytes;             // stages x 2 K-blocks of X
-constexpr uint32_t kSmemBytes = kOffA + kStages * kTileBytes;  // 96 KB of Pi terms + 128 KB of input stages
-constexpr uint32_t kTmemCols = kAccs * 128;                    // one accumulator of 128 fp32 columns per group
+
+template <int D>
+struct Cfg {
+  static constexpr int KB = (D + 63) / 64;                 // 64-column blocks of a vector
+  static constexpr int N = D == 256 ? 64 : D;              // output coordinates of a CTA
+  static constexpr int NSPLIT = D / N;
+  static constexpr int STAGES = D == 256 ? 2 : 4;          // input stages = epilogue groups = accumulators
+  static constexpr int THREADS = 64 + STAGES * 128;        // producer, issuer, four warps per group
+  static constexpr uint32_t kBBlock = N * 128;             // a 64-column block of a term of Pi
+  static constexpr uint32_t kTerm = KB * kBBlock;
+  static constexpr uint32_t kTile = KB * kBlockBytes;      // an input stage
+  static constexpr uint32_t kOffA = (kMaxTerms * kTerm + 1023) & ~1023u;
+  static constexpr uint32_t kSmem = kOffA + STAGES * kTile;
+  static constexpr uint32_t kTmemCols = STAGES * N <= 64 ? 64 : STAGES * N <= 128 ? 128 : STAGES * N <= 256 ? 256 : 512;
+};
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 // byte offset of (row, 16-byte chunk c of the row's 128 bytes) inside a K-block (128-byte swizzle)
@@ -70,9 +85,9 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t saddr) {
   return (uint64_t)((saddr & 0x3FFFFu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) |
          ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
-// instruction descriptor: D = F32, A and B of 16-bit format `fmt` (0 = fp16, 1 = bf16), K-major, N = M = 128
-__host__ __device__ constexpr uint32_t instr_desc(uint32_t fmt) {
-  return (1u << 4) | (fmt << 7) | (fmt << 10) | ((128u >> 3) << 17) | ((128u >> 4) << 24);
+// instruction descriptor: D = F32, A and B of 16-bit format `fmt` (0 = fp16, 1 = bf16), K-major, M = 128
+__host__ __device__ constexpr uint32_t instr_desc(uint32_t fmt, uint32_t n) {
+  return (1u << 4) | (fmt << 7) | (fmt << 10) | ((n >> 3) << 17) | ((128u >> 4) << 24);
 }
 __device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t acc) {
   asm volatile(
@@ -114,10 +129,10 @@ __device__ __forceinline__ bool elect_one_sync() {
       : "=r"(pred));
   return pred != 0;
 }
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+__device__ __forceinline__ void tma_load_3d(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint32_t bar) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
-      ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(bar)
+      "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];"
+      ::"r"(dst), "l"(map), "r"(x), "r"(y), "r"(z), "r"(bar)
       : "memory");
 }
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
@@ -158,19 +173,35 @@ struct Fmt<__nv_bfloat16> {
   }
 };
 
-// eight 16-bit elements (one 16-byte chunk) -> fp32
+// pairs of fp32 values in one 64-bit register: one instruction does both
+typedef unsigned long long f2;
+__device__ __forceinline__ f2 pack2(float lo, float hi) {
+  f2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void unpack2(f2 v, float& lo, float& hi) { asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(v)); }
+__device__ __forceinline__ f2 fma2(f2 a, f2 b, f2 c) {
+  f2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ f2 add2(f2 a, f2 b) {
+  f2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+// eight 16-bit elements (one 16-byte chunk) -> fp32 pairs
 template <typename T>
-__device__ __forceinline__ void chunk_to_float(const uint4& v, float (&x)[8]) {
+__device__ __forceinline__ void chunk_to_pairs(const uint4& v, f2 (&x)[4]) {
   const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
   for (int j = 0; j < 4; ++j) {
     if constexpr (std::is_same<T, __nv_bfloat16>::value) {
-      x[2 * j] = __uint_as_float(w[j] << 16);
-      x[2 * j + 1] = __uint_as_float(w[j] & 0xFFFF0000u);
+      x[j] = pack2(__uint_as_float(w[j] << 16), __uint_as_float(w[j] & 0xFFFF0000u));
     } else {
       const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[j]));
-      x[2 * j] = f.x;
-      x[2 * j + 1] = f.y;
+      x[j] = pack2(f.x, f.y);
     }
   }
 }
@@ -190,34 +221,62 @@ __device__ __forceinline__ int bucketize_reg(float y, const float (&b)[15]) {
   return (c1 ? 8 : 0) + (c2 ? 4 : 0) + (c3 ? 2 : 0) + (c4 ? 1 : 0);
 }
 
-// The same search with the two lower levels as table lookups through the warp shuffle: lane l holds
-// boundary l & 15 (`bval`; entry 15 = +inf), and __shfl_sync with a per-thread source lane is a
-// 16-entry lookup in one instruction.  Levels 1 and 2 compare against registers (b[7]; b[3] or b[11]);
-// 11 instructions per coordinate instead of 22, same comparisons, same result.  The shuffle unit
-// cannot take every coordinate (all of them through it: no faster than the register search), so the
-// epilogue sends every second one.
-__device__ __forceinline__ int bucketize_shfl(float y, float b7, float b3, float b11, float bval) {
-  const bool c1 = y > b7;
-  int idx = c1 ? 8 : 0;
-  idx += (y > (c1 ? b11 : b3)) ? 4 : 0;
-  idx += (y > __shfl_sync(0xffffffffu, bval, idx + 1)) ? 2 : 0;
-  idx += (y > __shfl_sync(0xffffffffu, bval, idx)) ? 1 : 0;
-  return idx;
+// The 32-cell map: cell = round(31 * sat(y * s / 31 + 16 / 31)), so y = 0 sits in the middle of cell 16 and
+// everything past the ends in the end cells.  `scale` = s / 31; lane c: the boundary inside cell c (+inf: none) and the
+// number of boundaries in the cells below.
+struct Grid {
+  float scale, bound;
+  int below;
+};
+// Grid of 15 ascending boundaries (padded with +inf); false if no scale puts every boundary into a cell of its own, at
+// least 1e-3 of a cell away from its edges.  One warp; lane i tries the i-th scale.
+__device__ __forceinline__ bool make_grid(const float* b, Grid& g, int lane) {
+  float last = 0.f;
+  for (int i = 0; i < 15; ++i)
+    if (b[i] < CUDART_INF_F) last = fmaxf(last, fabsf(b[i]));
+  const float s = last > 0.f ? 15.3f / last * (1.f - 0.01f * lane) : 1.f;
+  bool ok = last < CUDART_INF_F;
+  float prev = -1.f;
+  for (int i = 0; i < 15; ++i) {
+    if (!(b[i] < CUDART_INF_F)) continue;
+    const float x = fmaf(b[i], s, 16.f), c = rintf(x);
+    ok = ok && c > prev && c >= 0.f && c <= 31.f && fabsf(x - c) < 0.499f;
+    prev = c;
+  }
+  const unsigned m = __ballot_sync(0xffffffffu, ok);
+  if (m == 0) return false;
+  const float best = __shfl_sync(0xffffffffu, s, __ffs(m) - 1);
+  g.scale = best / 31.f;
+  g.bound = CUDART_INF_F;
+  g.below = 0;
+  for (int i = 0; i < 15; ++i) {
+    if (!(b[i] < CUDART_INF_F)) continue;
+    const int c = (int)rintf(fmaf(b[i], best, 16.f));
+    if (c == lane) g.bound = b[i];
+    if (c < lane) ++g.below;
+  }
+  return true;
+}
+__device__ __forceinline__ int bucketize_grid(float y, const Grid& g) {
+  const float u = fmaf(__saturatef(fmaf(y, g.scale, 16.f / 31.f)), 31.f, 8388608.f);  // (2^23: the cell in the low bits)
+  const int c = __float_as_int(u);  // (the shuffle takes the source lane modulo 32)
+  return __shfl_sync(0xffffffffu, g.below, c) + (y > __shfl_sync(0xffffffffu, g.bound, c) ? 1 : 0);
 }
 
 struct Bars {
-  uint64_t full[kStages];    // TMA -> consumers: the stage's tile has landed
-  uint64_t empty[kStages];   // consumers -> TMA: MMAs (1 commit) and the norm readers (4 warps) are done with it
-  uint64_t tfull[kAccs];     // MMA -> epilogue: the accumulator holds the tile's product
-  uint64_t tempty[kAccs];    // epilogue (4 warps) -> MMA: the accumulator has been read
-  uint64_t pi;               // the raw rotation matrix has landed in the staging area
+  uint64_t full[4];    // TMA -> consumers: the stage's tile has landed
+  uint64_t empty[4];   // consumers -> TMA: MMAs (1 commit) and the norm readers (4 warps) are done with it
+  uint64_t tfull[4];   // MMA -> epilogue: the accumulator holds the tile's product
+  uint64_t tempty[4];  // epilogue (4 warps) -> MMA: the accumulator has been read
 };
 
-template <typename T>
-__global__ void __launch_bounds__(kThreads, 1)
-compress_tc16_kernel(const CompressArgs a, const __grid_constant__ CUtensorMap tm_x0,
+template <typename T, int D>
+__global__ void __launch_bounds__(Cfg<D>::THREADS, 1)
+compress_tc16_kernel(const CompressArgs a, const int group_rows, const __grid_constant__ CUtensorMap tm_x0,
                      const __grid_constant__ CUtensorMap tm_x1) {
   using F = Fmt<T>;
+  using C = Cfg<D>;
+  constexpr int N = C::N, STAGES = C::STAGES;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   __shared__ __align__(8) Bars s_bars;
   __shared__ uint32_t s_tmem;
@@ -228,62 +287,54 @@ compress_tc16_kernel(const CompressArgs a, const __grid_constant__ CUtensorMap t
   const uint32_t base = (smem_addr(smem_raw) + 1023u) & ~1023u;  // swizzle atoms need 1024-byte alignment
   unsigned char* sm = smem_raw + (base - smem_addr(smem_raw));
   volatile int* dead = &s_dead;
+  // which output coordinates, and which tiles: CTAs of the same tile stream are neighbours
+  const int split = blockIdx.x % C::NSPLIT, stream = blockIdx.x / C::NSPLIT, n_streams = gridDim.x / C::NSPLIT;
+  const int j0 = split * N;
 
   if (tid < 32) {
     const int src = tid >> 4, i = tid & 15;
     s_bounds[src][i] = (src < a.n_sources && i < a.n_bounds[src]) ? a.bounds[src][i] : CUDART_INF_F;
   }
   if (tid == 0) {
-    for (int s = 0; s < kStages; ++s) {
+    for (int s = 0; s < STAGES; ++s) {
       bar_init(smem_addr(&s_bars.full[s]), 1);
       bar_init(smem_addr(&s_bars.empty[s]), 1 + 4);
+      bar_init(smem_addr(&s_bars.tfull[s]), 1);
+      bar_init(smem_addr(&s_bars.tempty[s]), 4);
     }
-    for (int c = 0; c < kAccs; ++c) {
-      bar_init(smem_addr(&s_bars.tfull[c]), 1);
-      bar_init(smem_addr(&s_bars.tempty[c]), 4);
-    }
-    bar_init(smem_addr(&s_bars.pi), 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     s_dead = 0;
-    // the caller's Pi^T halves (2 x 32 KB fp32) by two bulk copies into the still unused input stages
-    const uint32_t bar = smem_addr(&s_bars.pi);
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(2u * kD * (kD / 2) * 4u) : "memory");
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(base + kOffA), "l"(a.rot_even), "r"((uint32_t)(kD * (kD / 2) * 4)), "r"(bar) : "memory");
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                 ::"r"(base + kOffA + (uint32_t)(kD * (kD / 2) * 4)), "l"(a.rot_odd), "r"((uint32_t)(kD * (kD / 2) * 4)), "r"(bar) : "memory");
   }
   if (warp == 1) {  // the issuing warp owns the tensor-memory allocation
     __syncwarp();
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&s_tmem)),
-                 "r"(kTmemCols) : "memory");
+                 "r"(C::kTmemCols) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
-  // ---- Pi as the B operand: B[n = j][k = d] = Pi[j][d] in 16-bit terms, K-major, swizzled ---------
-  // rot_even[k * 64 + p] = Pi[2p][k], rot_odd[k * 64 + p] = Pi[2p + 1][k], read from the staging area
-  __syncthreads();  // the barrier is initialised, the copies are issued, the boundaries are in shared memory
-  const bool pi_ok = bar_wait_bounded(smem_addr(&s_bars.pi), 0u, &s_dead);
-  const float* raw = reinterpret_cast<const float*>(sm + kOffA);
-  for (int i = tid; i < kD * (kD / 8); i += kThreads) {
-    const int j = i & 127, k8 = i >> 7;  // row j, k = 8 * k8 .. + 7
-    const float* src = raw + (j & 1) * (kD * (kD / 2)) + (j >> 1);
+  // ---- Pi as the B operand: B[n][k] = Pi[j0 + n][k] in 16-bit terms, K-major, swizzled.  rot_even[k * D/2 + p]
+  //      = Pi[2p][k], rot_odd[k * D/2 + p] = Pi[2p + 1][k]; columns past D (D = 96) are zero ---------------------
+#pragma unroll 2
+  for (int i = tid; i < N * C::KB * 8; i += C::THREADS) {
+    const int n = i % N, k8 = i / N, j = j0 + n;  // row n, k = 8 * k8 .. + 7
+    const float* src = ((j & 1) ? a.rot_odd : a.rot_even) + (j >> 1);
+    float x[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) x[e] = 8 * k8 + e < D ? __ldg(src + (8 * k8 + e) * (D / 2)) * F::kScale : 0.f;
     uint16_t t[kMaxTerms][8];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) {
-      float rest = src[(8 * k8 + e) * (kD / 2)] * F::kScale;
+    for (int e = 0; e < 8; ++e)
 #pragma unroll
-      for (int m = 0; m < F::kTerms; ++m) t[m][e] = F::term(rest);
-    }
-    const uint32_t off = (uint32_t)(k8 >> 3) * kBlockBytes + swz(j, k8 & 7);
+      for (int q = 0; q < F::kTerms; ++q) t[q][e] = F::term(x[e]);
+    const uint32_t off = (uint32_t)(k8 >> 3) * C::kBBlock + swz(n, k8 & 7);
 #pragma unroll
-    for (int m = 0; m < F::kTerms; ++m) {
+    for (int q = 0; q < F::kTerms; ++q) {
       uint4 v;
-      v.x = t[m][0] | ((uint32_t)t[m][1] << 16);
-      v.y = t[m][2] | ((uint32_t)t[m][3] << 16);
-      v.z = t[m][4] | ((uint32_t)t[m][5] << 16);
-      v.w = t[m][6] | ((uint32_t)t[m][7] << 16);
-      *reinterpret_cast<uint4*>(sm + kOffB + m * kTileBytes + off) = v;
+      v.x = t[q][0] | ((uint32_t)t[q][1] << 16);
+      v.y = t[q][2] | ((uint32_t)t[q][3] << 16);
+      v.z = t[q][4] | ((uint32_t)t[q][5] << 16);
+      v.w = t[q][6] | ((uint32_t)t[q][7] << 16);
+      *reinterpret_cast<uint4*>(sm + q * C::kTerm + off) = v;
     }
   }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
@@ -296,108 +347,77 @@ compress_tc16_kernel(const CompressArgs a, const __grid_constant__ CUtensorMap t
   const int64_t rows_per_src = a.n_tokens * a.num_heads;
   const int64_t tiles_per_src = (rows_per_src + kRows - 1) / kRows;
   const int64_t n_tiles = tiles_per_src * a.n_sources;
-  const int64_t my_tiles = (int64_t)blockIdx.x < n_tiles ? (n_tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
-  bool ok = pi_ok;
+  const int64_t my_tiles = stream < n_tiles ? (n_tiles - stream + n_streams - 1) / n_streams : 0;
+  bool ok = true;
 
   if (warp == 0) {
     // ================= TMA producer =================
     for (int64_t i = 0; i < my_tiles && ok; ++i) {
-      const int st = (int)(i % kStages);
-      const uint32_t par = (uint32_t)((i / kStages) & 1);
+      const int st = (int)(i % STAGES);
+      const uint32_t par = (uint32_t)((i / STAGES) & 1);
       // (passes at once the first time round; warp-uniform so that the election below is well formed)
       ok = __all_sync(0xffffffffu, bar_wait_bounded(smem_addr(&s_bars.empty[st]), par ^ 1u, dead));
       if (!ok) break;
       CT_STAMP(0, i, 0);
       if (elect_one_sync()) {
-        const int64_t tile = blockIdx.x + i * gridDim.x;
+        const int64_t tile = stream + i * n_streams;
         const int s_ = (int)(tile / tiles_per_src);
         const int y = (int)((tile - (int64_t)s_ * tiles_per_src) * kRows);
         const uint32_t bar = smem_addr(&s_bars.full[st]);
-        const uint32_t dst = base + kOffA + st * kTileBytes;
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(kTileBytes) : "memory");
-        tma_load_2d(dst, s_ ? &tm_x1 : &tm_x0, 0, y, bar);            // rows past the end are zero-filled
-        tma_load_2d(dst + kBlockBytes, s_ ? &tm_x1 : &tm_x0, 64, y, bar);
+        const uint32_t dst = base + C::kOffA + st * C::kTile;
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(C::kTile) : "memory");
+        // rows past the end and columns past D are zero-filled
+#pragma unroll
+        for (int kb = 0; kb < C::KB; ++kb)
+          tma_load_3d(dst + kb * kBlockBytes, s_ ? &tm_x1 : &tm_x0, 64 * kb, 0, y / group_rows, bar);
       }
       __syncwarp();
     }
   } else if (warp == 1) {
     // ================= MMA issuer =================
-    constexpr uint32_t idesc = instr_desc(F::kCode);
+    constexpr uint32_t idesc = instr_desc(F::kCode, N);
     for (int64_t i = 0; i < my_tiles && ok; ++i) {
-      const int st = (int)(i % kStages), acc = (int)(i % kAccs);
-      ok = __all_sync(0xffffffffu,
-                      bar_wait_bounded(smem_addr(&s_bars.full[st]), (uint32_t)((i / kStages) & 1), dead) &&
-                          bar_wait_bounded(smem_addr(&s_bars.tempty[acc]), (uint32_t)((i / kAccs) & 1) ^ 1u, dead));
+      const int st = (int)(i % STAGES);
+      const uint32_t par = (uint32_t)((i / STAGES) & 1);
+      ok = __all_sync(0xffffffffu, bar_wait_bounded(smem_addr(&s_bars.full[st]), par, dead) &&
+                                       bar_wait_bounded(smem_addr(&s_bars.tempty[st]), par ^ 1u, dead));
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       CT_STAMP(1, i, 0);
       if (elect_one_sync()) {
-        const uint32_t tmem_d = tmem_base + (uint32_t)acc * kD;
-        const uint32_t a0 = base + kOffA + st * kTileBytes;
+        const uint32_t tmem_d = tmem_base + (uint32_t)st * N;
+        const uint32_t a0 = base + C::kOffA + st * C::kTile;
 #pragma unroll
-        for (int m = F::kTerms - 1; m >= 0; --m) {  // smallest term first
-          const uint32_t b0 = base + kOffB + m * kTileBytes;
+        for (int q = F::kTerms - 1; q >= 0; --q) {  // smallest term first
 #pragma unroll
-          for (int kb = 0; kb < 2; ++kb)
-#pragma unroll
-            for (int s = 0; s < 4; ++s) {  // four k-steps of 16 columns (32 bytes) per K-block
-              const uint32_t ko = kb * kBlockBytes + 32u * s;
-              mma_f16(tmem_d, make_desc(a0 + ko), make_desc(b0 + ko), idesc, (m != F::kTerms - 1 || kb || s) ? 1u : 0u);
-            }
+          for (int s = 0; s < D / 16; ++s)  // k-steps of 16 columns (32 bytes)
+            mma_f16(tmem_d, make_desc(a0 + (s >> 2) * kBlockBytes + 32u * (s & 3)),
+                    make_desc(base + q * C::kTerm + (s >> 2) * C::kBBlock + 32u * (s & 3)), idesc,
+                    (q != F::kTerms - 1 || s) ? 1u : 0u);
         }
-        mma_commit(smem_addr(&s_bars.empty[st]));   // the tensor core has read the stage
-        mma_commit(smem_addr(&s_bars.tfull[acc]));  // the accumulator is complete
+        mma_commit(smem_addr(&s_bars.empty[st]));  // the tensor core has read the stage
+        mma_commit(smem_addr(&s_bars.tfull[st]));  // the accumulator is complete
       }
       __syncwarp();
       CT_STAMP(1, i, 1);
     }
   } else {
     // ================= epilogue groups =================
-    const int grp = (warp - 2) >> 2;              // tiles i with i % kAccs == grp, accumulator grp
+    const int grp = (warp - 2) >> 2;              // tiles i with i % STAGES == grp, accumulator grp
     const int quarter = warp & 3;                 // the 32 TMEM lanes this warp may read
     const int row_in_tile = 32 * quarter + lane;
-    const RowLayout lay = row_layout(a.num_heads, kD);
-    for (int64_t i = grp; i < my_tiles && ok; i += kAccs) {
-      const int st = (int)(i % kStages), acc = grp;
-      const int64_t tile = blockIdx.x + i * gridDim.x;
+    const RowLayout lay = row_layout(a.num_heads, D);
+    Grid grid[2];
+    bool grid_ok = make_grid(s_bounds[0], grid[0], lane);
+    grid_ok = make_grid(s_bounds[1], grid[1], lane) && grid_ok;
+    for (int64_t i = grp; i < my_tiles && ok; i += STAGES) {
+      const int st = grp;
+      const uint32_t par = (uint32_t)((i / STAGES) & 1);
+      const int64_t tile = stream + i * n_streams;
       const int src = (int)(tile / tiles_per_src);
       const int64_t in_src = (tile - (int64_t)src * tiles_per_src) * kRows + row_in_tile;
       const bool live = in_src < rows_per_src;
-      ok = __all_sync(0xffffffffu, bar_wait_bounded(smem_addr(&s_bars.full[st]), (uint32_t)((i / kStages) & 1), dead));
-      if (!ok) break;
-      if (quarter == 0 && grp < 2) CT_STAMP(2 + grp, i, 0);
-      // ---- norm, in the summation order of the FMA kernels: p[l] over k = l, l+32, l+64, l+96,
-      //      then the butterfly tree 16, 8, 4, 2, 1 --------------------------------------------------
-      float nrm = 0.f;
-      {
-        const unsigned char* xt = sm + kOffA + st * kTileBytes;
-        float p[32];
-#pragma unroll
-        for (int l = 0; l < 32; ++l) p[l] = 0.f;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {  // elements [32 q, 32 q + 32) of the row
-#pragma unroll
-          for (int cc = 0; cc < 4; ++cc) {
-            const int chunk = 4 * q + cc;
-            const uint4 v = *reinterpret_cast<const uint4*>(xt + (chunk >> 3) * kBlockBytes + swz(row_in_tile, chunk & 7));
-            float x[8];
-            chunk_to_float<T>(v, x);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) p[8 * cc + e] = fmaf(x[e], x[e], p[8 * cc + e]);
-          }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-          for (int l = 0; l < o; ++l) p[l] = p[l] + p[l + o];
-        nrm = sqrtf(p[0]);
-      }
-      __syncwarp();
-      if (quarter == 0 && grp < 2) CT_STAMP(2 + grp, i, 1);
-      if (lane == 0) bar_arrive(smem_addr(&s_bars.empty[st]));  // this warp is done with the staged rows
-      // one IEEE division per row; Y_raw * (1 / den) is within an ulp of Y_raw / den
-      const float scale = (1.f / (nrm + 1e-10f)) * (1.f / F::kScale);
-      // where this row goes (resolved before the accumulator is read: the loads overlap the wait)
+      // where this row goes (resolved first: the load of its slot overlaps the waits)
       uint8_t* dst_idx = nullptr;
       float* dst_norm = nullptr;
       if (live) {
@@ -405,45 +425,87 @@ compress_tc16_kernel(const CompressArgs a, const __grid_constant__ CUtensorMap t
         const unsigned tok = rem / (unsigned)a.num_heads;
         const int h = (int)(rem - tok * (unsigned)a.num_heads);
         if (a.cache != nullptr) {
-          const int64_t slot = (int64_t)tok < a.n_slots ? a.slot_mapping[tok] : -1;
+          const int64_t slot = (int64_t)tok < a.n_slots ? write_slot(a, tok) : -1;
           if (slot >= a.num_cache_slots) {
             if (a.err_flag) atomicOr(a.err_flag, TQ4_DEV_BAD_SLOT);
           } else if (slot >= 0) {
             uint8_t* rowp = a.cache + slot * a.cache_token_stride;
-            dst_idx = rowp + (src == 0 ? lay.k_idx : lay.v_idx) + h * (kD / 2);
+            dst_idx = rowp + (src == 0 ? lay.k_idx : lay.v_idx) + h * (D / 2) + j0 / 2;
             dst_norm = reinterpret_cast<float*>(rowp + (src == 0 ? lay.k_norm : lay.v_norm) + h * 4);
           }
         } else {
           const int64_t row = (int64_t)src * rows_per_src + in_src;
-          dst_idx = a.packed_out + row * (kD / 2);
+          dst_idx = a.packed_out + row * (D / 2) + j0 / 2;
           dst_norm = a.norms_out + row;
         }
       }
-      float b[15];
+      ok = __all_sync(0xffffffffu, bar_wait_bounded(smem_addr(&s_bars.full[st]), par, dead));
+      if (!ok) break;
+      if (quarter == 0 && grp < 2) CT_STAMP(2 + grp, i, 0);
+      // ---- norm, in the summation order of the FMA kernels: p[l] over k = l, l + 32, ..., then the butterfly
+      //      tree 16, 8, 4, 2, 1 (pairs l, l + 1 in one instruction: each lane of it is an ordinary FMA) ------------
+      float nrm = 0.f;
+      {
+        const unsigned char* xt = sm + C::kOffA + st * C::kTile;
+        f2 p[16];
 #pragma unroll
-      for (int bi = 0; bi < 15; ++bi) b[bi] = s_bounds[src][bi];
-      const float bval = s_bounds[src][lane & 15];  // (entry 15 is +inf)
+        for (int l = 0; l < 16; ++l) p[l] = 0ull;
+#pragma unroll 1
+        for (int q = 0; q < D / 32; ++q) {  // elements [32 q, 32 q + 32) of the row
+#pragma unroll
+          for (int cc = 0; cc < 4; ++cc) {
+            const int chunk = 4 * q + cc;
+            const uint4 v = *reinterpret_cast<const uint4*>(xt + (chunk >> 3) * kBlockBytes + swz(row_in_tile, chunk & 7));
+            f2 x[4];
+            chunk_to_pairs<T>(v, x);
+#pragma unroll
+            for (int e = 0; e < 4; ++e) p[4 * cc + e] = fma2(x[e], x[e], p[4 * cc + e]);
+          }
+        }
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+          for (int l = 0; l < o; ++l) p[l] = add2(p[l], p[l + o]);
+        float p0, p1;
+        unpack2(p[0], p0, p1);
+        nrm = sqrtf(p0 + p1);
+      }
+      __syncwarp();
+      if (quarter == 0 && grp < 2) CT_STAMP(2 + grp, i, 1);
+      if (lane == 0) bar_arrive(smem_addr(&s_bars.empty[st]));  // this warp is done with the staged rows
+      // one IEEE division per row; Y_raw * (1 / den) is within an ulp of Y_raw / den
+      const float scale = (1.f / (nrm + 1e-10f)) * (1.f / F::kScale);
       const bool wide = dst_idx != nullptr && ((uintptr_t)dst_idx & 15) == 0;  // else rows are 4-byte aligned
+      const Grid g = src ? grid[1] : grid[0];
 
-      ok = __all_sync(0xffffffffu, bar_wait_bounded(smem_addr(&s_bars.tfull[acc]), (uint32_t)((i / kAccs) & 1), dead));
+      ok = __all_sync(0xffffffffu, bar_wait_bounded(smem_addr(&s_bars.tfull[st]), par, dead));
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (quarter == 0 && grp < 2) CT_STAMP(2 + grp, i, 2);
-      // four chunks of 32 coordinates -> 16 bytes each; the loop stays rolled so that its body (32
-      // register searches) fits the instruction cache
+      // chunks of 32 coordinates -> 16 bytes each; the loop stays rolled so that its body fits the instruction cache
 #pragma unroll 1
-      for (int q = 0; q < 4; ++q) {
+      for (int q = 0; q < N / 32; ++q) {
         uint32_t v[32];
-        tmem_ld32(tmem_base + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(acc * kD + 32 * q), v);
+        tmem_ld32(tmem_base + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(st * N + 32 * q), v);
         uint32_t word[4];
+        if (grid_ok) {
 #pragma unroll
-        for (int w = 0; w < 4; ++w) {  // 8 coordinates -> 4 bytes -> one word
-          word[w] = 0;
+          for (int w = 0; w < 4; ++w) {  // 8 coordinates -> 4 bytes -> one word
+            word[w] = 0;
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const int ie = bucketize_reg(__uint_as_float(v[8 * w + 2 * e]) * scale, b);
-            const int io = bucketize_shfl(__uint_as_float(v[8 * w + 2 * e + 1]) * scale, b[7], b[3], b[11], bval);
-            word[w] |= (uint32_t)((ie << 4) | io) << (8 * e);
+            for (int e = 0; e < 8; ++e)
+              word[w] += (uint32_t)bucketize_grid(__uint_as_float(v[8 * w + e]) * scale, g) << (8 * (e >> 1) + ((e & 1) ? 0 : 4));
+          }
+        } else {
+          float b[15];
+#pragma unroll
+          for (int bi = 0; bi < 15; ++bi) b[bi] = s_bounds[src][bi];
+#pragma unroll
+          for (int w = 0; w < 4; ++w) {
+            word[w] = 0;
+#pragma unroll
+            for (int e = 0; e < 8; ++e)
+              word[w] += (uint32_t)bucketize_reg(__uint_as_float(v[8 * w + e]) * scale, b) << (8 * (e >> 1) + ((e & 1) ? 0 : 4));
           }
         }
         if (wide) {
@@ -455,8 +517,8 @@ compress_tc16_kernel(const CompressArgs a, const __grid_constant__ CUtensorMap t
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) bar_arrive(smem_addr(&s_bars.tempty[acc]));  // the accumulator may be overwritten
-      if (dst_norm) *dst_norm = nrm;
+      if (lane == 0) bar_arrive(smem_addr(&s_bars.tempty[st]));  // the accumulator may be overwritten
+      if (dst_norm && split == 0) *dst_norm = nrm;
       if (quarter == 0 && grp < 2) CT_STAMP(2 + grp, i, 3);
     }
   }
@@ -467,7 +529,7 @@ compress_tc16_kernel(const CompressArgs a, const __grid_constant__ CUtensorMap t
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 1) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kTmemCols) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(C::kTmemCols) : "memory");
   }
 }
 
@@ -488,54 +550,76 @@ EncodeTiledFn encode_fn() {
   }
   return fn;
 }
-// rows of one source as a 2-D tensor [rows][128] of 16-bit elements; box = 128 rows x 64 columns
-bool make_x_map(CUtensorMap* m, const void* x, int64_t rows) {
+// One source as a 3-D tensor [groups][rows of a group][D] of 16-bit elements: a group is a token and its rows the heads
+// when the heads divide a tile (any token and head stride), else one row of a dense array.  Box: 128 rows x 64 columns.
+bool make_x_map(CUtensorMap* m, const CompressArgs& a, int src, int D, int group_rows) {
   EncodeTiledFn fn = encode_fn();
+  const int64_t rows = a.n_tokens * a.num_heads;
   if (!fn || rows <= 0) return false;
-  const cuuint64_t dims[2] = {(cuuint64_t)kD, (cuuint64_t)rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)kD * 2};
-  const cuuint32_t box[2] = {64, (cuuint32_t)kRows};
-  const cuuint32_t estr[2] = {1, 1};
-  return fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT16, 2, const_cast<void*>(x), dims, strides, box, estr,
+  const cuuint64_t dims[3] = {(cuuint64_t)D, (cuuint64_t)group_rows, (cuuint64_t)(rows / group_rows)};
+  const cuuint64_t strides[2] = {(cuuint64_t)(group_rows > 1 ? a.head_stride[src] : D) * 2,
+                                 (cuuint64_t)(group_rows > 1 ? a.token_stride[src] : D) * 2};
+  const cuuint32_t box[3] = {64, (cuuint32_t)group_rows, (cuuint32_t)(kRows / group_rows)};
+  const cuuint32_t estr[3] = {1, 1, 1};
+  return fn(m, CU_TENSOR_MAP_DATA_TYPE_UINT16, 3, const_cast<void*>(a.x[src]), dims, strides, box, estr,
             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <typename T>
+// rows that a group of the input map has: the heads of a token, or 1 for a dense array of rows; 0: not covered
+int group_of(const CompressArgs& a, int D) {
+  bool dense = true;
+  for (int s = 0; s < a.n_sources; ++s)
+    dense = dense && a.head_stride[s] == D && a.token_stride[s] == (int64_t)a.num_heads * D;
+  if (dense) return 1;
+  if (a.num_heads > 1 && kRows % a.num_heads == 0) return a.num_heads;
+  return 0;
+}
+
+template <typename T, int D>
 int launch_t(const CompressArgs& a, cudaStream_t st) {
+  using C = Cfg<D>;
   CUtensorMap m0, m1;
   memset(&m0, 0, sizeof(m0));
   memset(&m1, 0, sizeof(m1));
-  const int64_t rows = a.n_tokens * a.num_heads;
-  if (!make_x_map(&m0, a.x[0], rows) || !make_x_map(&m1, a.x[a.n_sources > 1 ? 1 : 0], rows))
-    return TQ4_ERR_CUDA;
-  const int smem = (int)kSmemBytes + 1024;
-  if (!ensure_dynamic_smem<compress_tc16_kernel<T>>(smem)) return TQ4_ERR_CUDA;
-  int64_t blocks = ((rows + kRows - 1) / kRows) * a.n_sources;
-  if (blocks > sm_count()) blocks = sm_count();
-  compress_tc16_kernel<T><<<(unsigned)blocks, kThreads, smem, st>>>(a, m0, m1);
+  const int group = group_of(a, D);
+  if (!make_x_map(&m0, a, 0, D, group) || !make_x_map(&m1, a, a.n_sources > 1 ? 1 : 0, D, group)) return TQ4_ERR_CUDA;
+  const int smem = (int)C::kSmem + 1024;
+  if (!ensure_dynamic_smem<compress_tc16_kernel<T, D>>(smem)) return TQ4_ERR_CUDA;
+  int64_t streams = ((a.n_tokens * a.num_heads + kRows - 1) / kRows) * a.n_sources;
+  if (streams > sm_count() / C::NSPLIT) streams = sm_count() / C::NSPLIT;
+  compress_tc16_kernel<T, D><<<(unsigned)(streams * C::NSPLIT), C::THREADS, smem, st>>>(a, group, m0, m1);
   TQ4_CHECK_LAUNCH();
   return TQ4_OK;
 }
 
-}  // namespace
-
-// 16-bit inputs whose rows are dense [tokens * heads][128] arrays (the layout vLLM hands to the cache
-// write): the pipelined kernel.  Everything else stays on the kernels in tq4_compress_tc.cu / tq4_compress.cu.
-bool compress_tc16_eligible(const CompressArgs& a, int head_dim, int dtype) {
-  static const bool disabled = getenv("TQ4_NO_TC") != nullptr || getenv("TQ4_NO_TC16") != nullptr;
-  if (disabled || head_dim != kD || (dtype != TQ4_F16 && dtype != TQ4_BF16)) return false;
-  if (a.n_tokens * a.num_heads >= (1ll << 31) || encode_fn() == nullptr) return false;
-  for (int s = 0; s < a.n_sources; ++s) {
-    if (((uintptr_t)a.x[s] & 15) || a.head_stride[s] != kD || a.token_stride[s] != (int64_t)a.num_heads * kD)
-      return false;
+template <typename T>
+int launch_d(const CompressArgs& a, int head_dim, cudaStream_t st) {
+  switch (head_dim) {
+    case 64: return launch_t<T, 64>(a, st);
+    case 96: return launch_t<T, 96>(a, st);
+    case 128: return launch_t<T, 128>(a, st);
+    case 256: return launch_t<T, 256>(a, st);
   }
-  if (((uintptr_t)a.rot_even | (uintptr_t)a.rot_odd) & 15) return false;  // bulk copies of the rotation halves
-  return true;
+  return TQ4_ERR_UNSUPPORTED;
 }
 
-int launch_compress_tc16(const CompressArgs& a, int dtype, cudaStream_t st) {
-  return dtype == TQ4_F16 ? launch_t<__half>(a, st) : launch_t<__nv_bfloat16>(a, st);
+}  // namespace
+
+// 16-bit inputs whose rows TMA can address: dense arrays, or strided tokens and heads (K and V as views of one
+// projection) when the heads divide a tile.  Everything else stays on the kernels in tq4_compress_tc.cu / tq4_compress.cu.
+bool compress_tc16_eligible(const CompressArgs& a, int head_dim, int dtype) {
+  static const bool disabled = getenv("TQ4_NO_TC") != nullptr || getenv("TQ4_NO_TC16") != nullptr;
+  if (disabled || !supported_head_dim(head_dim) || (dtype != TQ4_F16 && dtype != TQ4_BF16)) return false;
+  if (a.n_tokens * a.num_heads >= (1ll << 31) || encode_fn() == nullptr || !tokens_uniform(a)) return false;
+  for (int s = 0; s < a.n_sources; ++s)
+    if (((uintptr_t)a.x[s] & 15) || a.head_stride[s] <= 0 || a.token_stride[s] <= 0 || a.head_stride[s] % 8 || a.token_stride[s] % 8)
+      return false;
+  return group_of(a, head_dim) != 0;
+}
+
+int launch_compress_tc16(const CompressArgs& a, int head_dim, int dtype, cudaStream_t st) {
+  return dtype == TQ4_F16 ? launch_d<__half>(a, head_dim, st) : launch_d<__nv_bfloat16>(a, head_dim, st);
 }
 
 }  // namespace tq4
