@@ -441,6 +441,133 @@ prologue_kernel(const AttnArgs a, const CompressArgs w, const int has_attn, cons
   }
 }
 
+// The same for a step of a few vectors: a block of four warps per vector, each warp one quarter of the
+// reduction with Pi^T read straight from L1 / L2 (the caller's even / odd halves), as the write kernel for few vectors does.
+// No staging, half the code: latency is all that counts here.
+template <int D>
+__global__ void __launch_bounds__(128) tiny_prologue_kernel(const AttnArgs a, const CompressArgs w) {
+  constexpr int HALF = D / 2, NBL = (HALF + 31) / 32, XPL = D / 32, KQ = D / 4;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ float s_x[D];
+  __shared__ float s_part[3][2 * NBL][32];
+  __shared__ float s_b[16];
+  pdl_trigger();
+  if (blockIdx.x == 0) {  // the planning block
+    build_plan(a, reinterpret_cast<int*>(smem_raw));
+    return;
+  }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int n_q = a.sh.rows * a.sh.Hq, vec = (int)blockIdx.x - 1;
+  const bool is_w = vec >= n_q;
+  int src = 0, tok = 0, h = 0;
+  int64_t slot = -1, at;
+  const void* x;
+  int dt;
+  if (is_w) {
+    const int rows_per_src = (int)w.n_tokens * w.num_heads, r = vec - n_q;
+    src = r >= rows_per_src ? 1 : 0;
+    const unsigned rem = (unsigned)(r - src * rows_per_src);
+    tok = (int)(rem / (unsigned)w.num_heads);
+    h = (int)(rem - (unsigned)tok * (unsigned)w.num_heads);
+    x = w.x[src];
+    dt = w.x_dtype;
+    at = token_offset(w, src, tok) + (int64_t)h * w.head_stride[src];
+    slot = tok < w.n_slots ? write_slot(w, tok) : -1;
+    if (threadIdx.x >= 32 && threadIdx.x < 48) {
+      const int i = threadIdx.x - 32;
+      s_b[i] = i < w.n_bounds[src] ? w.bounds[src][i] : CUDART_INF_F;
+    }
+  } else {
+    const int row = vec / a.sh.Hq;
+    x = a.q;
+    dt = a.q_dtype;
+    at = ((int64_t)row + a.sh.row_offset) * a.q_token_stride + (int64_t)(vec - row * a.sh.Hq) * a.q_head_stride;
+  }
+  float xv[XPL], norm = 0.f;
+#pragma unroll
+  for (int i = 0; i < XPL; ++i) xv[i] = load_as_float(x, dt, at + lane + 32 * i);
+  float den = 1.f;
+  if (is_w) {
+    float ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < XPL; ++i) ss = fmaf(xv[i], xv[i], ss);
+    norm = sqrtf(warp_sum(ss));
+    den = norm + 1e-10f;
+  }
+  if (warp == 0) {
+#pragma unroll
+    for (int i = 0; i < XPL; ++i) s_x[lane + 32 * i] = is_w ? xv[i] / den : xv[i];
+  }
+  __syncthreads();
+  float acc[2 * NBL];
+#pragma unroll
+  for (int i = 0; i < 2 * NBL; ++i) acc[i] = 0.f;
+  for (int kb = 0; kb < KQ; kb += 8) {  // eight k-steps of Pi^T in flight before the first FMA of the batch
+    float pe[8][NBL], po[8][NBL];
+#pragma unroll
+    for (int u = 0; u < 8; ++u)
+#pragma unroll
+      for (int i = 0; i < NBL; ++i) {
+        const int p = lane + 32 * i, k = warp * KQ + kb + u;
+        pe[u][i] = p < HALF ? __ldg(w.rot_even + k * HALF + p) : 0.f;
+        po[u][i] = p < HALF ? __ldg(w.rot_odd + k * HALF + p) : 0.f;
+      }
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+      const float xk = s_x[warp * KQ + kb + u];
+#pragma unroll
+      for (int i = 0; i < NBL; ++i) {
+        acc[2 * i] = fmaf(xk, pe[u][i], acc[2 * i]);
+        acc[2 * i + 1] = fmaf(xk, po[u][i], acc[2 * i + 1]);
+      }
+    }
+  }
+  if (warp > 0) {
+#pragma unroll
+    for (int i = 0; i < 2 * NBL; ++i) s_part[warp - 1][i][lane] = acc[i];
+  }
+  __syncthreads();
+  if (warp != 0) return;
+#pragma unroll
+  for (int i = 0; i < 2 * NBL; ++i) acc[i] = (acc[i] + s_part[0][i][lane]) + (s_part[1][i][lane] + s_part[2][i][lane]);
+  if (!is_w) {
+#pragma unroll
+    for (int i = 0; i < NBL; ++i)
+      if (lane + 32 * i < HALF)
+        *reinterpret_cast<float2*>(a.plan.q_rot + (int64_t)vec * D + 2 * (lane + 32 * i)) = make_float2(acc[2 * i], acc[2 * i + 1]);
+    return;
+  }
+  if (slot < 0) return;
+  if (slot >= w.num_cache_slots) {
+    if (lane == 0 && w.err_flag) atomicOr(w.err_flag, TQ4_DEV_BAD_SLOT);
+    return;
+  }
+  const RowLayout lay = row_layout(w.num_heads, D);
+  uint8_t* rowp = w.cache + slot * w.cache_token_stride;
+  uint8_t* dst = rowp + (src == 0 ? lay.k_idx : lay.v_idx) + h * HALF;
+#pragma unroll
+  for (int i = 0; i < NBL; ++i)
+    if (lane + 32 * i < HALF)
+      dst[lane + 32 * i] = (uint8_t)((bucketize_sorted16(acc[2 * i], s_b) << 4) | bucketize_sorted16(acc[2 * i + 1], s_b));
+  if (lane == 0) *reinterpret_cast<float*>(rowp + (src == 0 ? lay.k_norm : lay.v_norm) + h * 4) = norm;
+}
+
+// Vectors up to which a step takes a block per vector.  One decode call, graph replay, without -> with it:
+// 36 vectors (batch 1, 28 + 4 + 4) 19.4 -> 16.3 us, 192 (batch 4) 20.9 -> 17.7, 576 (batch 32, 14 + 2 + 2, head_dim 64)
+// 23.7 -> 23.3, 768 (batch 16) 42.1 -> 40.7: every vector reads all of Pi^T, so the
+// gain shrinks as they grow in number.
+constexpr int64_t kTinyStep = 1024;
+
+template <int D>
+int launch_tiny_prologue(const AttnArgs& a, const CompressArgs& w, int64_t vectors, cudaStream_t st) {
+  const size_t smem = 2 * (size_t)a.sh.rows * sizeof(int);
+  // (first kernel of an entry point: plain stream-ordered launch, see launch_prologue_jc)
+  if (launch_kernel(tiny_prologue_kernel<D>, dim3((unsigned)vectors + 1), dim3(128), smem, st, false, a, w) != cudaSuccess)
+    return TQ4_ERR_CUDA;
+  TQ4_CHECK_LAUNCH();
+  return TQ4_OK;
+}
+
 template <int D, int JC>
 int launch_prologue_jc(const AttnArgs* a, const CompressArgs* w, cudaStream_t st, int64_t blocks) {
   using P = PrologueCfg<D, JC>;
@@ -471,6 +598,9 @@ int launch_prologue_t(const AttnArgs* a, const CompressArgs* w, cudaStream_t st)
   const int64_t n_w = w ? w->n_tokens * w->num_heads * w->n_sources : 0;
   const int64_t chunks = (n_q + VC - 1) / VC + (n_w + VC - 1) / VC;
   const int64_t blocks = (chunks + WARPS - 1) / WARPS;
+  if constexpr (D <= 128)
+    if (a && w && w->cache && a->skip_long == 0 && n_q + n_w <= kTinyStep)
+      return launch_tiny_prologue<D>(*a, *w, n_q + n_w, st);
   const int64_t wave = 3 * (int64_t)sm_count() / (D / 32);
   if (blocks <= wave) return launch_prologue_jc<D, 32>(a, w, st, blocks);
   // a mixed call streams few of its rows (the kernel finds out how many)
