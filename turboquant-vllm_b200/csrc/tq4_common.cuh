@@ -278,13 +278,15 @@ inline bool tokens_uniform(const CompressArgs& a) {
 }
 
 // Which kernel makes a write of so many vectors (B200, graph replays of stand-alone writes, bf16):
-//   head_dim <= 128: a block per vector up to kTinyRows (5.2 us at 32 vectors, 8.4 at 2048; the prologue kernel 8.1 and
-//   10.5, the tensor-core kernel 10.4 and 10.6), above it the tensor-core kernel (10.8 us at 8192 vectors; a block per
-//   vector 24, the prologue kernel 16).  head_dim 256: the prologue kernel up to kTinyRows256 (11 us; a block per
-//   vector 24), above it the tensor-core kernel (10.4 us at 800 vectors, the prologue kernel 15).
-// What the tensor-core kernel cannot address takes the prologue kernel up to kSmallRows; so does the write of a decode step
-// (it shares the launch with the query rotation).
-constexpr int64_t kTinyRows = 2048, kTinyRows256 = 512, kSmallRows = 8192;
+//   a block per vector (head_dim <= 128) up to kTinyRows: 5.2 us at 32 vectors, 8.4 at 2048; the prologue kernel 8.1
+//     and 10.5, the tensor-core kernel 10.4 and 10.6
+//   the tensor-core kernel above tc_rows().  At head_dim 64 and 96 that is kTinyRows; at 256 512 vectors (10.4 us at 800, the
+//     prologue kernel 15).  At head_dim 128 it would pay from there on too (8192 vectors: 10.8 us, the prologue kernel 16,
+//     a block per vector 24), but up to kSmallRows a vector is promised the same bytes however the calls are cut, and
+//     only the FMA kernels agree with one another bit for bit
+//   the prologue kernel in between, and up to kSmallRows for what the tensor-core kernel cannot address
+constexpr int64_t kTinyRows = 2048, kSmallRows = 8192;
+constexpr int64_t tc_rows(int head_dim) { return head_dim == 128 ? kSmallRows : head_dim == 256 ? 512 : kTinyRows; }
 int launch_small_write(const CompressArgs& w, int head_dim, cudaStream_t st);
 int dispatch_compress(const CompressArgs& a, int head_dim, int dtype, cudaStream_t st);
 // tensor-core (tcgen05) compress kernel for large inputs at head_dim 128 (tq4_compress_tc.cu)

@@ -353,7 +353,7 @@ int dispatch_compress(const CompressArgs& a, int head_dim, int dtype, cudaStream
   const int64_t vectors = a.n_tokens * a.num_heads * a.n_sources;
   if (vectors == 0) return TQ4_OK;
   const bool tiny = head_dim <= 128 && vectors <= kTinyRows;  // (dispatch_dtype: a block per vector)
-  if (vectors > (head_dim == 256 ? kTinyRows256 : kTinyRows) && compress_tc16_eligible(a, head_dim, dtype))
+  if (vectors > tc_rows(head_dim) && compress_tc16_eligible(a, head_dim, dtype))
     return launch_compress_tc16(a, head_dim, dtype, st);
   if (!tiny && vectors <= kSmallRows) return launch_small_write(a, head_dim, st);
   if (!tiny && compress_tc_eligible(a, head_dim, dtype)) return launch_compress_tc(a, dtype, st);
