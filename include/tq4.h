@@ -110,6 +110,39 @@ int tq4_write_paged(const void* key, const void* value, int kv_dtype,
                     int* err_flag, void* stream);
 
 /*
+ * The same for token rows of a batch that are appended to: key / value [batch, heads, n_new, D] with the
+ * element strides {batch, head, token} (innermost stride 1); token s of sequence b goes to row
+ * b * capacity + offset + s of `rows` (row_bytes apart, the layout of a cache token row).
+ * Replaces: the per-step torch.cat of the contiguous HuggingFace-side cache,
+ *           src/turboquant_vllm/kv_cache.py:640-672.
+ */
+int tq4_append_rows(const void* key, const void* value, int kv_dtype, int batch, int n_new,
+                    int num_kv_heads, int head_dim, const int64_t* k_strides, const int64_t* v_strides,
+                    const float* rot_t_even, const float* rot_t_odd,
+                    const float* k_boundaries, int n_k_boundaries,
+                    const float* v_boundaries, int n_v_boundaries,
+                    uint8_t* rows, int64_t row_bytes, int64_t capacity, int64_t offset, void* stream);
+
+/*
+ * One update of a HuggingFace-style cache layer in one launch: key / value [batch, heads, n_new, D] (element
+ * strides {batch, head, token}) are compressed into the index and norm buffers [batch, heads, capacity, D/2 or
+ * D] / [batch, heads, capacity] behind `offset` tokens (k_nibble / v_nibble: two indices a byte, else one), and
+ * the reconstructed vectors centroids[idx] * norm * Pi are stored in key's type into k_dec / v_dec
+ * [batch, heads, dec_capacity, D] behind dec_offset tokens (both null: left out).
+ * Replaces: CompressedDynamicCache._compressed_update's chain of quantize, pack, cat, unpack and dequantize,
+ *           src/turboquant_vllm/kv_cache.py:602-760.
+ */
+int tq4_cache_update(const void* key, const void* value, int dtype, int batch, int num_heads, int n_new,
+                     int head_dim, const int64_t* k_strides, const int64_t* v_strides, const float* rotation,
+                     const float* k_boundaries, int n_k_boundaries,
+                     const float* v_boundaries, int n_v_boundaries,
+                     const float* k_centroids, int n_k_centroids,
+                     const float* v_centroids, int n_v_centroids, int k_nibble, int v_nibble,
+                     uint8_t* k_idx, float* k_norms, uint8_t* v_idx, float* v_norms,
+                     int64_t capacity, int64_t offset, void* k_dec, void* v_dec,
+                     int64_t dec_capacity, int64_t dec_offset, void* stream);
+
+/*
  * Decompress rows (rotated space): out[(n,h), 0:D] = centroids[idx] * norm, cast to out_dtype.
  * Replaces: tq4_decompress() + _tq4_decompress_kernel, src/turboquant_vllm/triton/tq4_decompress.py:43-101,126-184.
  */

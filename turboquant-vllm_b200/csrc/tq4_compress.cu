@@ -475,3 +475,53 @@ extern "C" int tq4_write_paged(const void* key, const void* value, int kv_dtype,
   tq4::prof_end(TQ4_PROF_WRITE, (cudaStream_t)stream);
   return rc;
 }
+
+extern "C" int tq4_append_rows(const void* key, const void* value, int kv_dtype, int batch, int n_new, int num_kv_heads,
+                               int head_dim, const int64_t* k_strides, const int64_t* v_strides,
+                               const float* rot_t_even, const float* rot_t_odd, const float* k_boundaries,
+                               int n_k_boundaries, const float* v_boundaries, int n_v_boundaries, uint8_t* rows,
+                               int64_t row_bytes, int64_t capacity, int64_t offset, void* stream) {
+  if (batch < 0 || n_new < 0 || num_kv_heads <= 0 || offset < 0 || offset + n_new > capacity) return TQ4_ERR_INVALID_ARG;
+  if (!tq4::supported_head_dim(head_dim)) return TQ4_ERR_UNSUPPORTED;
+  if (n_k_boundaries < 0 || n_k_boundaries > TQ4_MAX_BOUNDARIES || n_v_boundaries < 0 || n_v_boundaries > TQ4_MAX_BOUNDARIES)
+    return TQ4_ERR_UNSUPPORTED;
+  if (batch == 0 || n_new == 0) return TQ4_OK;
+  if (!key || !value || !k_strides || !v_strides || !rot_t_even || !rot_t_odd || !k_boundaries || !v_boundaries || !rows)
+    return TQ4_ERR_INVALID_ARG;
+  if (((uintptr_t)rot_t_even | (uintptr_t)rot_t_odd) & 15) return TQ4_ERR_INVALID_ARG;
+  if (((uintptr_t)rows & 3) || (row_bytes & 3) || row_bytes < tq4::row_data_bytes(num_kv_heads, head_dim) ||
+      (int64_t)batch * n_new > 0x7fffffffll)
+    return TQ4_ERR_INVALID_ARG;
+  tq4::CompressArgs a{};
+  const void* x[2] = {key, value};
+  const int64_t* strides[2] = {k_strides, v_strides};
+  for (int s = 0; s < 2; ++s) {
+    a.x[s] = x[s];
+    a.batch_stride[s] = strides[s][0];
+    a.head_stride[s] = strides[s][1];
+    a.token_stride[s] = strides[s][2];
+  }
+  a.bounds[0] = k_boundaries;
+  a.n_bounds[0] = n_k_boundaries;
+  a.bounds[1] = v_boundaries;
+  a.n_bounds[1] = n_v_boundaries;
+  a.n_tokens = (int64_t)batch * n_new;
+  a.num_heads = num_kv_heads;
+  a.n_sources = 2;
+  a.x_dtype = kv_dtype;
+  a.rot_even = rot_t_even;
+  a.rot_odd = rot_t_odd;
+  a.cache = rows;
+  a.seq = n_new;
+  a.row_capacity = capacity;
+  a.row_offset = offset;
+  a.n_slots = a.n_tokens;
+  a.cache_token_stride = row_bytes;
+  a.num_cache_slots = (int64_t)batch * capacity;
+  // one new token per sequence: the sequences are the tokens
+  for (int s = 0; n_new == 1 && s < 2; ++s) a.token_stride[s] = a.batch_stride[s];
+  tq4::prof_begin(TQ4_PROF_WRITE, (cudaStream_t)stream);
+  const int rc = tq4::dispatch_compress(a, head_dim, kv_dtype, (cudaStream_t)stream);
+  tq4::prof_end(TQ4_PROF_WRITE, (cudaStream_t)stream);
+  return rc;
+}

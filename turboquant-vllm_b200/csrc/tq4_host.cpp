@@ -9,7 +9,6 @@
 
 #include <ATen/core/Tensor.h>
 #include <ATen/ops/empty.h>
-#include <ATen/ops/empty_strided.h>
 #include <ATen/ops/zeros.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -288,6 +287,91 @@ PyObject* write_paged(PyObject*, PyObject* const* p, Py_ssize_t n) {
   });
 }
 
+// [batch, heads, tokens, head_dim] K or V of an update, innermost stride 1
+struct States {
+  at::Tensor t;
+  int64_t strides[3];
+  States(PyObject* o, const char* name) : t(cuda_tensor(o, name)) {
+    TQ4_ASSERT(t.dim() == 4, "key and value must be [batch, heads, tokens, head_dim]");
+    t = inner_contiguous(t);
+    for (int i = 0; i < 3; ++i) strides[i] = t.stride(i);
+  }
+};
+
+// append_rows(key, value, rows, offset, rotation_T_even, rotation_T_odd, k_boundaries, v_boundaries)
+PyObject* append_rows(PyObject*, PyObject* const* p, Py_ssize_t n) {
+  if (!expect("append_rows", n, 8)) return nullptr;
+  return guarded([&]() -> PyObject* {
+    const States k(p[0], "key"), v(p[1], "value");
+    const at::Tensor& rows = cuda_tensor(p[2], "rows");
+    const int64_t offset = as_int(p[3]);
+    const at::Tensor &even = cuda_tensor(p[4], "rotation_T_even"), &odd = cuda_tensor(p[5], "rotation_T_odd");
+    const at::Tensor &kb = cuda_tensor(p[6], "k_boundaries"), &vb = cuda_tensor(p[7], "v_boundaries");
+    TQ4_ASSERT(k.t.sizes() == v.t.sizes() && k.t.scalar_type() == v.t.scalar_type(), "key and value must be alike");
+    TQ4_ASSERT(rows.scalar_type() == at::kByte && rows.dim() == 3 && rows.is_contiguous() && rows.size(0) == k.t.size(0),
+               "rows must be contiguous uint8 [batch, capacity, bytes]");
+    const int dt = dtype_code(k.t.scalar_type());
+    Launch launch(device_index(k.t));
+    int st;
+    Py_BEGIN_ALLOW_THREADS
+    st = tq4_append_rows(k.t.data_ptr(), v.t.data_ptr(), dt, (int)k.t.size(0), (int)k.t.size(2), (int)k.t.size(1), (int)k.t.size(3),
+                         k.strides, v.strides, (const float*)even.data_ptr(), (const float*)odd.data_ptr(),
+                         (const float*)kb.data_ptr(), (int)kb.numel(), (const float*)vb.data_ptr(), (int)vb.numel(),
+                         (uint8_t*)rows.data_ptr(), rows.size(2), rows.size(1), offset, launch.stream);
+    Py_END_ALLOW_THREADS
+    check(st, "tq4_append_rows");
+    Py_RETURN_NONE;
+  });
+}
+
+// cache_update(key, value, rotation, k_boundaries, v_boundaries, k_centroids, v_centroids, k_nibble, v_nibble,
+//              k_idx, k_norms, v_idx, v_norms, offset, k_dec, v_dec, dec_offset)
+PyObject* cache_update(PyObject*, PyObject* const* p, Py_ssize_t n) {
+  if (!expect("cache_update", n, 17)) return nullptr;
+  return guarded([&]() -> PyObject* {
+    const States k(p[0], "key"), v(p[1], "value");
+    const at::Tensor& rot = cuda_tensor(p[2], "rotation");
+    const at::Tensor &kb = cuda_tensor(p[3], "k_boundaries"), &vb = cuda_tensor(p[4], "v_boundaries");
+    const at::Tensor &kc = cuda_tensor(p[5], "k_centroids"), &vc = cuda_tensor(p[6], "v_centroids");
+    const int k_nib = truth(p[7]), v_nib = truth(p[8]);
+    const at::Tensor &ki = cuda_tensor(p[9], "k_idx"), &kn = cuda_tensor(p[10], "k_norms");
+    const at::Tensor &vi = cuda_tensor(p[11], "v_idx"), &vn = cuda_tensor(p[12], "v_norms");
+    const int64_t offset = as_int(p[13]), dec_offset = as_int(p[16]);
+    TQ4_ASSERT(k.t.sizes() == v.t.sizes() && k.t.scalar_type() == v.t.scalar_type(), "key and value must be alike");
+    const int64_t b = k.t.size(0), h = k.t.size(1), d = k.t.size(3);
+    auto buffer = [&](const at::Tensor& t, int64_t width, at::ScalarType type) {
+      TQ4_ASSERT(t.dim() == 4 && t.size(0) == b && t.size(1) == h && t.size(3) == width && t.is_contiguous() && t.scalar_type() == type,
+                 "buffers must be contiguous [batch, heads, capacity, width]");
+      return t.size(2);
+    };
+    const int64_t cap = buffer(ki, k_nib ? d / 2 : d, at::kByte);
+    TQ4_ASSERT(buffer(vi, v_nib ? d / 2 : d, at::kByte) == cap && buffer(kn, 1, at::kFloat) == cap && buffer(vn, 1, at::kFloat) == cap,
+               "index and norm buffers must have one capacity");
+    void *kd = nullptr, *vd = nullptr;
+    int64_t dec_cap = 0;
+    if (p[14] != Py_None) {
+      const at::Tensor &a = cuda_tensor(p[14], "k_dec"), &c = cuda_tensor(p[15], "v_dec");
+      dec_cap = buffer(a, d, k.t.scalar_type());
+      TQ4_ASSERT(buffer(c, d, k.t.scalar_type()) == dec_cap, "the two dequantised buffers must have one capacity");
+      kd = a.data_ptr();
+      vd = c.data_ptr();
+    }
+    const int dt = dtype_code(k.t.scalar_type());
+    Launch launch(device_index(k.t));
+    int st;
+    Py_BEGIN_ALLOW_THREADS
+    st = tq4_cache_update(k.t.data_ptr(), v.t.data_ptr(), dt, (int)b, (int)h, (int)k.t.size(2), (int)d, k.strides, v.strides,
+                          (const float*)rot.data_ptr(), (const float*)kb.data_ptr(), (int)kb.numel(),
+                          (const float*)vb.data_ptr(), (int)vb.numel(), (const float*)kc.data_ptr(), (int)kc.numel(),
+                          (const float*)vc.data_ptr(), (int)vc.numel(), k_nib, v_nib, (uint8_t*)ki.data_ptr(),
+                          (float*)kn.data_ptr(), (uint8_t*)vi.data_ptr(), (float*)vn.data_ptr(), cap, offset, kd, vd, dec_cap,
+                          dec_offset, launch.stream);
+    Py_END_ALLOW_THREADS
+    check(st, "tq4_cache_update");
+    Py_RETURN_NONE;
+  });
+}
+
 // error_flag(device_index) -> the device's int32 flag tensor
 PyObject* error_flag(PyObject*, PyObject* const* p, Py_ssize_t n) {
   if (!expect("error_flag", n, 1)) return nullptr;
@@ -301,6 +385,8 @@ PyObject* error_flag(PyObject*, PyObject* const* p, Py_ssize_t n) {
 PyMethodDef kMethods[] = {
     {"attention", (PyCFunction)(void (*)(void))attention, METH_FASTCALL, "Paged TQ4 attention, optionally with a cache write."},
     {"write_paged", (PyCFunction)(void (*)(void))write_paged, METH_FASTCALL, "Compress K and V into the paged cache."},
+    {"append_rows", (PyCFunction)(void (*)(void))append_rows, METH_FASTCALL, "Compress K and V into token rows of a batch."},
+    {"cache_update", (PyCFunction)(void (*)(void))cache_update, METH_FASTCALL, "Compress, store and reconstruct an update."},
     {"error_flag", (PyCFunction)(void (*)(void))error_flag, METH_FASTCALL, "Device error flag."},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_tq4_host", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};

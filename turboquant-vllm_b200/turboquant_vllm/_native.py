@@ -40,6 +40,13 @@ _SIGNATURES = {
                                 c_int64, c_int64, c_int64, c_int64, c_void_p, c_int64,
                                 c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int,
                                 c_void_p, c_int64, c_int64, c_void_p, c_void_p]),
+    "tq4_append_rows": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p,
+                                c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p,
+                                c_int64, c_int64, c_int64, c_void_p]),
+    "tq4_cache_update": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p,
+                                 c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int,
+                                 c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_void_p, c_void_p,
+                                 c_int64, c_int64, c_void_p]),
     "tq4_decompress_rows": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int64, c_int,
                                     c_void_p, c_int, c_void_p]),
     "tq4_decompress_cache": (c_int, [c_void_p, c_int64, c_int64, c_int, c_int, c_void_p, c_int,

@@ -6,8 +6,8 @@ wrapped cache, keeps uint8 centroid indices (nibble-packed at 4 bits) plus fp32 
 hands the fused attention path the packed tensors through ``get_compressed``, and otherwise
 returns incrementally dequantised K/V.  Differences under the surface:
 
-* compress and dequantise are single launches of the sm_100a kernels (norm + rotate + bucketize
-  + pack; unpack + LUT + scale), not chains of PyTorch ops;
+* an update is one launch (norm + rotate + bucketize + pack into the layer's buffers, and in the default
+  mode the reconstructed K/V behind the ones held), not a chain of PyTorch ops;
 * storage grows by capacity doubling, so appending a token does not re-copy the whole layer
   (the reference ``torch.cat``s every step);
 * in fused mode a 4-bit layer is kept as token rows in the paged kernels' own format
@@ -19,12 +19,16 @@ returns incrementally dequantised K/V.  Differences under the surface:
 
 from __future__ import annotations
 
+import sys
+import threading
 import warnings
+import weakref
 from dataclasses import dataclass
 from typing import Any
 
 import torch
 
+from turboquant_vllm import _native as nv
 from turboquant_vllm.compressors import CompressedValues, TurboQuantCompressorMSE
 from turboquant_vllm.quantizer import nibble_pack, nibble_unpack
 from turboquant_vllm.token_rows import TokenRowStore
@@ -33,6 +37,10 @@ from turboquant_vllm.token_rows import TokenRowStore
 def _packed_size(bits: int, head_dim: int) -> int:
     """Index bytes per token per head: nibble-packed at 4 bits, one byte per index otherwise."""
     return head_dim // 2 if bits == 4 else head_dim
+
+
+_UPDATE_DIMS, _UPDATE_DTYPES = (64, 96, 128, 256), (torch.float16, torch.bfloat16, torch.float32)
+_STORE_DTYPES = (torch.uint8, torch.float32, torch.uint8, torch.float32)
 
 
 @dataclass
@@ -51,18 +59,24 @@ class _GrowBuffer:
         self.buf: torch.Tensor | None = None
         self.len = 0
 
+    def reserve(self, b: int, h: int, n: int, w: int, dtype: torch.dtype, device: torch.device) -> torch.Tensor:
+        """The buffer with room for ``n`` more tokens of ``[b, h, ., w]``; a new one if it held another shape."""
+        buf = self.buf
+        if buf is None or buf.shape[:2] != (b, h) or buf.shape[3] != w:
+            cap = max(64, 1 << (max(n, 1) - 1).bit_length())
+            self.buf = torch.empty(b, h, cap, w, dtype=dtype, device=device)
+            self.len = 0
+        elif self.len + n > buf.shape[2]:
+            cap = max(2 * buf.shape[2], 1 << (self.len + n - 1).bit_length())
+            grown = torch.empty(b, h, cap, w, dtype=dtype, device=device)
+            grown[:, :, : self.len] = buf[:, :, : self.len]
+            self.buf = grown
+        return self.buf
+
     def append(self, x: torch.Tensor) -> torch.Tensor:
         n = x.shape[2]
-        if self.buf is None or self.buf.shape[:2] != x.shape[:2] or self.buf.shape[3] != x.shape[3]:
-            cap = max(64, 1 << (max(n, 1) - 1).bit_length())
-            self.buf = torch.empty(*x.shape[:2], cap, x.shape[3], dtype=x.dtype, device=x.device)
-            self.len = 0
-        elif self.len + n > self.buf.shape[2]:
-            cap = max(2 * self.buf.shape[2], 1 << (self.len + n - 1).bit_length())
-            grown = torch.empty(*x.shape[:2], cap, x.shape[3], dtype=x.dtype, device=x.device)
-            grown[:, :, : self.len] = self.buf[:, :, : self.len]
-            self.buf = grown
-        self.buf[:, :, self.len : self.len + n] = x
+        buf = self.reserve(x.shape[0], x.shape[1], n, x.shape[3], x.dtype, x.device)
+        buf[:, :, self.len : self.len + n] = x
         self.len += n
         return self.view()
 
@@ -84,6 +98,49 @@ class _RowsField:
 
     def view(self) -> torch.Tensor:
         return self.store.views()[self.which]
+
+
+# Wrappers alive.  A wrapped cache and its wrapper hold one another (either alone has to keep both), so dropping both
+# leaves their device memory to Python's cycle collector, which counts objects, not bytes: a program that makes a cache
+# per generation piled up dead ones and spent half of a short generation in cudaMalloc.  Each new wrapper
+# therefore cuts those pairs that only their own cycle holds.
+_wrappers: set = set()
+_wrappers_lock = threading.RLock()
+
+
+def _only_cycle_holds(w: "CompressedDynamicCache") -> bool:
+    """Whether every reference to the wrapper ``w``, its cache and the four methods between them is one of theirs."""
+    probe = object()
+    base = sys.getrefcount(probe)  # what this frame adds to an object that it names
+    c = w.cache
+    held = getattr(c, "__dict__", {})
+    own = [held.get("update"), held.get("get_seq_length")]
+    if any(getattr(m, "__self__", None) is not w for m in own):
+        return False
+    originals = [w._original_update, w._original_get_seq_length]
+    for methods in (own, originals):
+        while methods:
+            m = methods.pop()
+            if sys.getrefcount(m) != base + 1:
+                return False
+    m = None
+    bound = sum(getattr(x, "__self__", None) is c for x in (w._original_update, w._original_get_seq_length))
+    # w: its two methods in the cache, the caller's name for it; c: w.cache and the original methods bound to it
+    return sys.getrefcount(w) == base + 3 and sys.getrefcount(c) == base + 1 + bound
+
+
+def _release_unreachable() -> None:
+    if not getattr(sys, "_is_gil_enabled", lambda: True)():
+        return  # reference counts are not exact
+    with _wrappers_lock:
+        for ref in list(_wrappers):
+            w = ref()
+            if w is None:
+                _wrappers.discard(ref)
+            elif _only_cycle_holds(w):
+                _wrappers.discard(ref)
+                del w.cache.update, w.cache.get_seq_length
+            w = None
 
 
 class CompressedDynamicCache:
@@ -165,10 +222,13 @@ class CompressedDynamicCache:
                 "`DynamicCache(config=model.config)` for correct Gemma support.",
                 UserWarning, stacklevel=2,
             )
+        _release_unreachable()
         self._original_update = cache.update
         self._original_get_seq_length = cache.get_seq_length
         cache.update = self._compressed_update
         cache.get_seq_length = self._compressed_get_seq_length
+        with _wrappers_lock:
+            _wrappers.add(weakref.ref(self))
 
     # ----- compressors ------------------------------------------------------------------------
     def _get_compressors(self, dim: int):
@@ -269,29 +329,68 @@ class CompressedDynamicCache:
             return key_states, value_states
         if self._rows[layer_idx] is not None:
             self._rows_to_buffers(layer_idx, k_comp, v_comp)
-        new_k = self._compress_tensor(k_comp, key_states, nibble_packed=self._k_nibble_packed)
-        new_v = self._compress_tensor(v_comp, value_states, nibble_packed=self._v_nibble_packed)
-        self._pad_to(layer_idx)
-        if self._k_store[layer_idx] is None:
-            self._k_store[layer_idx] = (_GrowBuffer(), _GrowBuffer())
-            self._v_store[layer_idx] = (_GrowBuffer(), _GrowBuffer())
-        ks, vs = self._k_store[layer_idx], self._v_store[layer_idx]
-        ks[0].append(new_k.indices)
-        ks[1].append(new_k.norms)
-        vs[0].append(new_v.indices)
-        vs[1].append(new_v.norms)
+        ks = self._k_store[layer_idx] or (_GrowBuffer(), _GrowBuffer())
+        vs = self._v_store[layer_idx] or (_GrowBuffer(), _GrowBuffer())
+        dec = ()
+        if not self.fused_mode:  # (in fused mode the kernel reads get_compressed(); no K/V is reconstructed)
+            dec = (self._dec_k[layer_idx] or _GrowBuffer(), self._dec_v[layer_idx] or _GrowBuffer())
+        if not self._update_in_place(key_states, value_states, ks + vs, dec, k_comp.quantizer, v_comp.quantizer):
+            new_k = self._compress_tensor(k_comp, key_states, nibble_packed=self._k_nibble_packed)
+            new_v = self._compress_tensor(v_comp, value_states, nibble_packed=self._v_nibble_packed)
+            ks[0].append(new_k.indices)
+            ks[1].append(new_k.norms)
+            vs[0].append(new_v.indices)
+            vs[1].append(new_v.norms)
+            if dec:
+                dec[0].append(self._dequantize_layer(k_comp, new_k))
+                dec[1].append(self._dequantize_layer(v_comp, new_v))
+        self._k_store[layer_idx], self._v_store[layer_idx] = ks, vs
+        if dec:
+            self._dec_k[layer_idx], self._dec_v[layer_idx] = dec
 
         layer = self.cache.layers[layer_idx]
         self._ensure_layer_initialized(layer, key_states, value_states)
-        if self.fused_mode:  # the fused kernel reads get_compressed(); K/V here are placeholders
+        if self.fused_mode:  # placeholders
             layer.keys, layer.values = key_states, value_states
             return key_states, value_states
-        if self._dec_k[layer_idx] is None:
-            self._dec_k[layer_idx], self._dec_v[layer_idx] = _GrowBuffer(), _GrowBuffer()
-        dk = self._dec_k[layer_idx].append(self._dequantize_layer(k_comp, new_k))
-        dv = self._dec_v[layer_idx].append(self._dequantize_layer(v_comp, new_v))
-        layer.keys, layer.values = dk, dv
-        return dk, dv
+        layer.keys, layer.values = dec[0].view(), dec[1].view()
+        return layer.keys, layer.values
+
+    def _update_in_place(self, key_states, value_states, store, dec, k_quant, v_quant) -> bool:
+        """Compress, store and (``dec``) reconstruct the new tokens in one launch behind the tokens held.
+
+        False, with nothing changed, for shapes and types the kernel does not take, K and V that are not
+        alike, or buffers that hold something else: the caller then goes tensor by tensor.
+        """
+        dev, dtype = key_states.device, key_states.dtype
+        if (key_states.dim() != 4 or key_states.shape != value_states.shape or dtype != value_states.dtype
+                or dev != value_states.device or not key_states.is_cuda or dtype not in _UPDATE_DTYPES):
+            return False
+        b, h, n, d = key_states.shape
+        if n == 0 or d not in _UPDATE_DIMS or k_quant.bits > 4 or v_quant.bits > 4:
+            return False
+        rot, _, _, k_cents, k_bounds = k_quant.device_primitives(dev)
+        v_rot, _, _, v_cents, v_bounds = v_quant.device_primitives(dev)
+        if rot is not v_rot:
+            return False
+        bufs = []
+        for group, widths, types in (
+            (store, (_packed_size(self.k_bits, d), 1, _packed_size(self.v_bits, d), 1), _STORE_DTYPES),
+            (dec, (d, d), (dtype, dtype)),
+        ):
+            for g, w, t in zip(group, widths, types):
+                first, buf = group[0], g.buf
+                if g.len != first.len or (buf is None) != (first.buf is None) or buf is not None and (
+                        buf.shape != (b, h, first.buf.shape[2], w) or buf.dtype != t or buf.device != dev):
+                    return False
+                bufs.append((g, w, t))
+        out = [g.reserve(b, h, n, w, t, dev) for g, w, t in bufs]
+        nv.host().cache_update(
+            key_states, value_states, rot, k_bounds, v_bounds, k_cents, v_cents, self._k_nibble_packed,
+            self._v_nibble_packed, *out[:4], store[0].len, *(out[4:] or (None, None)), dec[0].len if dec else 0)
+        for g, _, _ in bufs:
+            g.len += n
+        return True
 
     # ----- token-row storage (fused mode) -------------------------------------------------------------
     def _append_rows(self, layer_idx: int, key_states, value_states, k_comp, v_comp) -> None:

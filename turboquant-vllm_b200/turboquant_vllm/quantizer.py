@@ -9,6 +9,9 @@ this package has no CPU compute path.
 
 from __future__ import annotations
 
+import threading
+from collections import OrderedDict
+
 import torch
 
 from turboquant_vllm.lloyd_max import LloydMaxCodebook, solve_lloyd_max
@@ -29,6 +32,36 @@ def _generate_rotation_matrix(dim: int, seed: int = 42) -> torch.Tensor:
     signs = torch.sign(torch.diagonal(r))
     signs = torch.where(signs == 0, torch.ones_like(signs), signs)
     return q * signs.unsqueeze(0)
+
+
+class _Recent:
+    """The last ``size`` results of pure functions of their key: safe with several threads, older ones dropped.
+
+    A cache object is made per generation, and its rotation (a QR on the host, about a millisecond at
+    head_dim 128) and device tensors (ten small copies) depend only on ``(dim, bits, seed)``: a
+    generation of some tokens spent half its time on them."""
+
+    def __init__(self, size: int) -> None:
+        self._size, self._lock, self._held = size, threading.Lock(), OrderedDict()
+
+    def get(self, key, make):
+        with self._lock:
+            hit = self._held.get(key)
+            if hit is not None:
+                self._held.move_to_end(key)
+                return hit
+        made = make()
+        with self._lock:
+            made = self._held.setdefault(key, made)
+            self._held.move_to_end(key)
+            while len(self._held) > self._size:
+                self._held.popitem(last=False)
+        return made
+
+
+_rotations = _Recent(8)
+_device_rotations = _Recent(8)   # at most 8 x 768 KB (head_dim 256)
+_device_codebooks = _Recent(16)
 
 
 def nibble_unpack(packed: torch.Tensor) -> torch.Tensor:
@@ -58,7 +91,10 @@ class TurboQuantMSE:
         self.bits = bits
         cents, bounds = solve_lloyd_max(dim, bits)
         self.codebook = LloydMaxCodebook(centroids=cents, boundaries=bounds, bits=bits, dim=dim)
-        self.rotation = _generate_rotation_matrix(dim, seed=seed)
+        self.rotation = _rotations.get((dim, seed), lambda: _generate_rotation_matrix(dim, seed=seed)).clone()
+        self._seed = seed
+        # the tensors as made here, to tell whether a caller has changed or replaced one since
+        self._made = [(x, x._version) for x in (self.rotation, cents, bounds)]
         self._dev: dict[torch.device, tuple[torch.Tensor, ...]] = {}
 
     def device_primitives(self, device: torch.device):
@@ -66,14 +102,22 @@ class TurboQuantMSE:
         device = torch.device(device)
         prim = self._dev.get(device)
         if prim is None:
-            rot_t = self.rotation.T.contiguous()
-            prim = (
-                self.rotation.to(device).contiguous(),
-                rot_t[:, 0::2].contiguous().to(device),
-                rot_t[:, 1::2].contiguous().to(device),
-                self.codebook.centroids.to(device),
-                self.codebook.boundaries.to(device),
-            )
+            def rotation():
+                rot_t = self.rotation.T.contiguous()
+                return (self.rotation.to(device).contiguous(), rot_t[:, 0::2].contiguous().to(device),
+                        rot_t[:, 1::2].contiguous().to(device))
+
+            def codebook():
+                return self.codebook.centroids.to(device), self.codebook.boundaries.to(device)
+
+            now = (self.rotation, self.codebook.centroids, self.codebook.boundaries)
+            if device.type == "cuda" and all(x is y and x._version == n for x, (y, n) in zip(now, self._made)):
+                # shared by the quantisers first used on one stream (the allocator's unit of reuse)
+                where = (device, torch.cuda.current_stream(device).cuda_stream)
+                prim = (_device_rotations.get((self.dim, self._seed, *where), rotation)
+                        + _device_codebooks.get((self.dim, self.bits, *(n for _, n in self._made[1:]), *where), codebook))
+            else:
+                prim = rotation() + codebook()
             self._dev[device] = prim
         return prim
 

@@ -6,7 +6,7 @@ The reference keeps a layer's compressed K/V as four tensors ``[B, H, S, D/2]`` 
 token rows ``[B, capacity, H*(D+8)]`` -- ``[K_idx | K_norm | V_idx | V_norm]`` per token, exactly the
 row the paged cache holds -- so that
 
-* an update is a single launch of the paged write kernel (norm, rotate, bucketize, pack, scatter),
+* an update is a single launch of the cache write kernel (norm, rotate, bucketize, pack, scatter),
 * attention is the paged kernel itself over 256-token pages with an identity block table
   (batch ``b`` owns pages ``b*P .. b*P+P-1``), with no re-packing and no second kernel family,
 * the four reference tensors are zero-copy strided views of the buffer.
@@ -21,27 +21,25 @@ import math
 
 import torch
 
+from turboquant_vllm import _native as nv
+
 PAGE_TOKENS = 256  # tokens per page of the identity-mapped row buffer (the kernels' largest page)
-_TABLE_ENTRIES = 1 << 22  # largest batch * capacity for which the per-step index rows are kept (48 MB)
+_TABLE_ENTRIES = 1 << 22  # largest batch * capacity for which the length rows are kept (16 MB)
 
 
-_index_row_cache: dict = {}  # (device, batch, capacity) -> (len_rows, slot_rows); shared by all layers
+_index_row_cache: dict = {}  # (device, batch, capacity) -> len_rows; shared by all layers
 
 
-def _index_rows(device: torch.device, batch: int, cap: int):
-    """``len_rows [cap+1, B]`` int32 (row n = n repeated) and ``slot_rows [cap, B]`` int64
-    (row n = b*cap + n), or ``(None, None)`` when they would be too large."""
+def _len_rows(device: torch.device, batch: int, cap: int):
+    """``[cap+1, B]`` int32 (row n = n repeated), or ``None`` when it would be too large."""
     if batch * (cap + 1) > _TABLE_ENTRIES:
-        return None, None
+        return None
     key = (device, batch, cap)
     hit = _index_row_cache.get(key)
     if hit is None:
         if len(_index_row_cache) >= 4:  # layers of a model share one entry; keep the dict small
             _index_row_cache.pop(next(iter(_index_row_cache)))
-        steps = torch.arange(cap + 1, device=device)
-        base = torch.arange(batch, dtype=torch.int64, device=device) * cap
-        hit = (steps.to(torch.int32)[:, None].expand(cap + 1, batch).contiguous(),
-               (steps[:cap, None] + base[None, :]).contiguous())
+        hit = torch.arange(cap + 1, dtype=torch.int32, device=device)[:, None].expand(cap + 1, batch).contiguous()
         _index_row_cache[key] = hit
     return hit
 
@@ -85,10 +83,8 @@ class TokenRowStore:
         pages = cap // PAGE_TOKENS
         self._block_table = torch.arange(self.batch * pages, dtype=torch.int32, device=self.device).view(
             self.batch, pages)
-        self._slot_base = torch.arange(self.batch, dtype=torch.int64, device=self.device) * cap
-        # decode steps index ready-made rows instead of launching small kernels: row n of
-        # _len_rows is [n]*B (sequence lengths), row n of _slot_rows the slots of token n
-        self._len_rows, self._slot_rows = _index_rows(self.device, self.batch, cap)
+        # a decode step takes its sequence lengths from a ready row instead of launching a fill
+        self._len_rows = _len_rows(self.device, self.batch, cap)
 
     def matches(self, batch: int, heads: int, dim: int, device: torch.device) -> bool:
         return (batch, heads, dim) == (self.batch, self.heads, self.dim) and torch.device(device) == self.device
@@ -97,11 +93,9 @@ class TokenRowStore:
     def append(self, key_states: torch.Tensor, value_states: torch.Tensor, k_quantizer, v_quantizer) -> None:
         """Compress ``[B, H, S_new, D]`` K and V and store them behind the tokens already held.
 
-        One launch: the paged write kernel scatters the packed rows to slots
+        One launch: the cache write kernel, told that token ``s`` of sequence ``b`` goes to row
         ``b*capacity + len + s``.
         """
-        from turboquant_vllm.kernels.ops import tq4_write_paged
-
         b, h, s, d = key_states.shape
         assert (b, h, d) == (self.batch, self.heads, self.dim) and value_states.shape == key_states.shape
         if s == 0:
@@ -109,13 +103,7 @@ class TokenRowStore:
         self._reserve(self.len + s)
         _, even, odd, _, k_bounds = k_quantizer.device_primitives(self.device)
         v_bounds = v_quantizer.device_primitives(self.device)[4]  # K and V share the rotation (one seed)
-        key = key_states.transpose(1, 2).reshape(b * s, h, d)
-        value = value_states.transpose(1, 2).reshape(b * s, h, d)
-        if s == 1:
-            slots = self._slot_rows[self.len] if self._slot_rows is not None else self._slot_base + self.len
-        else:
-            slots = (self._slot_base[:, None] + torch.arange(self.len, self.len + s, device=self.device)).reshape(-1)
-        tq4_write_paged(key, value, self.paged_cache(), slots, even, odd, k_bounds, v_bounds)
+        nv.host().append_rows(key_states, value_states, self.rows, self.len, even, odd, k_bounds, v_bounds)
         self.len += s
 
     @classmethod
