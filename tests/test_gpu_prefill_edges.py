@@ -13,14 +13,16 @@ CASES = [  # head_dim, q heads, KV heads, lengths, new rows, mode, window, causa
     (128, 4, 4, [64], [16], 3, None, True, True),            # one row block, one full tile
     (128, 8, 2, [300, 90], [120, 90], 3, None, True, True),  # a last CTA with one of its two blocks in use
     (128, 28, 4, [150], [150], 3, None, True, True),         # groups of 7: 126 of 128 lanes
-    (128, 8, 4, [65], [65], 0, None, True, True),            # one key in the second tile
-    (128, 32, 8, [3000], [40], 0, None, True, True),         # cut along the keys
+    (128, 8, 4, [65], [65], 3, None, True, True),            # one key in the second tile
+    (128, 32, 8, [3000], [40], 3, None, True, True),         # cut along the keys
     (128, 4, 1, [700], [333], 3, None, False, False),        # 136-byte rows: 4-byte loads; not causal
     (64, 14, 2, [333], [200], 3, None, True, True),
     (96, 4, 4, [300, 41], [100, 9], 3, None, True, False),
     (256, 8, 4, [300, 90], [120, 90], 3, 64, True, True),
     (256, 2, 2, [700], [9], 3, None, True, True),
-    (128, 8, 2, [300, 90, 50, 77], [120, 1, 7, 77], 0, None, True, True),   # long and short sequences
+    (128, 32, 8, [300, 90, 50, 77], [120, 1, 7, 77], 0, None, True, True),  # long and short sequences
+    (256, 8, 4, [900, 90, 8], [300, 1, 8], 0, None, True, True),
+    (128, 8, 2, [300, 90, 50, 77], [120, 1, 7, 77], 0, None, True, True),   # few rows: the streaming kernel alone
     (256, 8, 4, [900, 90, 8], [12, 1, 8], 0, None, True, True),
 ]
 

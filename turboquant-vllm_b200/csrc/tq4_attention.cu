@@ -1267,7 +1267,15 @@ static int attention_impl(
   const bool prefill_ok = prefill_tc_supported(a);
   if ((mode == 3 || mode == 4) && !prefill_ok) return TQ4_ERR_UNSUPPORTED;
   const bool all_long = mode == 3 || mode == 4 || (num_seqs == 1 && num_rows >= kPrefillMinRows) || num_rows >= 256 * (int64_t)num_seqs;
-  const bool use_prefill = prefill_ok && (mode == 3 || mode == 4 || (mode == 0 && num_rows >= kPrefillMinRows && (num_seqs > 1 || all_long)));
+  // A call of few rows is the streaming kernel's alone: one pass of launches instead of two, and none of the fixed costs
+  // of a prefill tile (Pi's image, rotating and un-rotating 128 rows: 20 us).  45 drawn steps: up to 4096 rows times
+  // query heads streaming took 0.43 - 1.0 of the time (34 rows beside 21 running sequences, 28 / 4 heads: 25.9
+  // against 49.9 us), above 5000 1.3 - 2.5 times it; head_dim 256, where it reads each row twice: the line is at 2048.
+  // And not where long contexts, by the width of the block table, make it re-read more than some 50 us of bytes.
+  const int64_t keys = bt_stride * block_size;
+  const bool few = use_mma && num_rows * num_q_heads <= (head_dim == 256 ? 2048 : 4096) &&
+                   num_rows * keys * row_data_bytes(num_kv_heads, head_dim) <= (1ll << 28);
+  const bool use_prefill = prefill_ok && (mode == 3 || mode == 4 || (mode == 0 && !few && num_rows >= kPrefillMinRows && (num_seqs > 1 || all_long)));
   const bool use_stream = !use_prefill || !all_long;
   a.skip_long = use_prefill && use_stream ? kPrefillMinRows : 0;
 
