@@ -4,13 +4,13 @@
 //   norm = |x|, y = x / (norm + 1e-10) * Pi^T, idx = #{boundary < y}          as the compress kernels, bit for bit
 //   z = (centroid[idx] * norm) * Pi, rounded to the type of x
 //
-// (measured: generation of 8 tokens behind 4 prompts of 1100, 2 layers of 8 heads of 128, 7800 -> 730 us)
 // Takes the place of a chain of some fifty launches per update (compress, unpack, repack, decompress, a GEMM, casts,
 // copies into the buffers), which bounded a step by its host time.  A warp takes four vectors, a lane D / 32
 // consecutive coordinates of each; both products read Pi from shared memory (once transposed, once as
 // it is; at head_dim 256, where that does not fit, in chunks of 64 rows) and the vectors from a strip per warp.
 // A step of a few tokens is latency bound (staging Pi: 128 KB per block), so its vectors are spread over the blocks
 // first; a prompt is bound by FMA issue.
+// Measured: a generation of 8 tokens behind 4 prompts of 1100, 2 layers of 8 heads of 128, 7800 -> 730 us.
 #include <math_constants.h>
 
 #include "tq4_common.cuh"
@@ -32,9 +32,28 @@ struct UpdateArgs {
   const float* rotation;
 };
 
-template <int D>
+// two fp32 operations an instruction, each rounded as alone
+struct F2 { unsigned long long v; };
+__device__ __forceinline__ F2 pack2(float a, float b) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ void unpack2(F2 x, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x.v)); }
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+
+template <int D, int VC_>
 struct Cfg {
-  static constexpr int WARPS = 8, VC = 4, NJ = D / 32;
+  static constexpr int WARPS = 8, VC = VC_, NJ = D / 32;
   static constexpr int NCH = D == 256 ? 4 : 1, KC = D / NCH;  // chunks of the reduction, rows of Pi in each
   static constexpr size_t kPi = (size_t)KC * D * 4;
   static constexpr size_t kStrip = (size_t)WARPS * D * VC * 4, kIdx = (size_t)WARPS * VC * D;
@@ -57,15 +76,33 @@ __device__ __forceinline__ void load_row(const float* p, float (&v)[NJ]) {
   }
 }
 
-template <int D>
+// acc[i][j] += (vectors 2 i, 2 i + 1 of the strip's entry) * ps[j]
+template <int D, int NJ, int VC>
+__device__ __forceinline__ void rank1(const float4* x, const float (&ps)[NJ], F2 (&acc)[VC / 2][NJ]) {
+  F2 p2[NJ];
+#pragma unroll
+  for (int j = 0; j < NJ; ++j) p2[j] = pack2(ps[j], ps[j]);
+#pragma unroll
+  for (int g = 0; g < VC / 4; ++g) {
+    const float4 x4 = x[g * D];
+    const F2 lo = pack2(x4.x, x4.y), hi = pack2(x4.z, x4.w);
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+      acc[2 * g][j] = fma2(lo, p2[j], acc[2 * g][j]);
+      acc[2 * g + 1][j] = fma2(hi, p2[j], acc[2 * g + 1][j]);
+    }
+  }
+}
+
+template <int D, int VC>
 __global__ void __launch_bounds__(256) cache_update_kernel(const UpdateArgs a) {
-  using C = Cfg<D>;
-  constexpr int NJ = C::NJ, VC = C::VC, KC = C::KC, NCH = C::NCH, KQ = D / 4, XPL = D / 32;
+  using C = Cfg<D, VC>;
+  constexpr int NJ = C::NJ, G = VC / 4, KC = C::KC, NCH = C::NCH, KQ = D / 4, XPL = D / 32;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   float* s_pit = reinterpret_cast<float*>(smem_raw);           // [KC][D]: Pi[j][k0 + k] at [k][j]
   float* s_pi = s_pit + KC * D;                                // [KC][D]: Pi[k0 + k][j] at [k][j]
-  float4* s_x = reinterpret_cast<float4*>(s_pi + KC * D);      // [WARPS][D], four vectors per entry
-  uint8_t* s_i = reinterpret_cast<uint8_t*>(s_x + C::WARPS * D);  // [WARPS][VC][D] indices
+  float4* s_x = reinterpret_cast<float4*>(s_pi + KC * D);      // [WARPS][G][D], four vectors per entry
+  uint8_t* s_i = reinterpret_cast<uint8_t*>(s_x + C::WARPS * D * G);  // [WARPS][VC][D] indices
   __shared__ float s_b[2][16], s_c[2][16];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (tid < 32) {
@@ -85,14 +122,14 @@ __global__ void __launch_bounds__(256) cache_update_kernel(const UpdateArgs a) {
     for (int i = tid; i < KC * D / 4; i += 256)
       reinterpret_cast<float4*>(s_pi)[i] = __ldg(reinterpret_cast<const float4*>(a.rotation + (size_t)ch * KC * D) + i);
   };
-  const int per_src = a.batch * a.heads * a.n_new, n_vec = 2 * per_src;
+  const int per_src = a.batch * a.heads * a.n_new;
   const int chunks_src = (per_src + VC - 1) / VC, n_chunks = 2 * chunks_src;  // (a chunk holds vectors of one source)
   if (NCH == 1) {
     stage_t(0);
     stage(0);
   }
   __syncthreads();
-  float4* gx = s_x + warp * D;
+  float4* gx = s_x + warp * D * G;
   uint8_t* gi = s_i + warp * VC * D;
   const float* pt = s_pit + NJ * lane;
   const float* pp = s_pi + NJ * lane;
@@ -137,11 +174,14 @@ __global__ void __launch_bounds__(256) cache_update_kernel(const UpdateArgs a) {
       }
       __syncwarp();
 #pragma unroll
-      for (int i = 0; i < XPL; ++i) gx[lane + 32 * i] = make_float4(xr[i][0], xr[i][1], xr[i][2], xr[i][3]);
+      for (int i = 0; i < XPL; ++i)
+#pragma unroll
+        for (int g = 0; g < G; ++g)
+          gx[g * D + lane + 32 * i] = make_float4(xr[i][4 * g], xr[i][4 * g + 1], xr[i][4 * g + 2], xr[i][4 * g + 3]);
       __syncwarp();
     }
     // ---- rotate: four quarter chains, (s0 + s1) + (s2 + s3) -------------------------------------------
-    float t[VC][NJ], u[VC][NJ], acc[VC][NJ];
+    F2 t[VC / 2][NJ], u[VC / 2][NJ], acc[VC / 2][NJ];
 #pragma unroll 1
     for (int q = 0; q < 4; ++q) {
       if (NCH > 1) {
@@ -150,42 +190,40 @@ __global__ void __launch_bounds__(256) cache_update_kernel(const UpdateArgs a) {
         __syncthreads();
       }
 #pragma unroll
-      for (int v = 0; v < VC; ++v)
+      for (int v = 0; v < VC / 2; ++v)
 #pragma unroll
-        for (int j = 0; j < NJ; ++j) acc[v][j] = 0.f;
+        for (int j = 0; j < NJ; ++j) acc[v][j].v = 0;
       const float* pq = pt + (NCH > 1 ? 0 : q * KQ * D);
 #pragma unroll 4
       for (int k = 0; k < KQ; ++k) {
         float ps[NJ];
         load_row<NJ>(pq + k * D, ps);
-        const float4 x4 = gx[q * KQ + k];
-        const float xs[VC] = {x4.x, x4.y, x4.z, x4.w};
-#pragma unroll
-        for (int v = 0; v < VC; ++v)
-#pragma unroll
-          for (int j = 0; j < NJ; ++j) acc[v][j] = fmaf(xs[v], ps[j], acc[v][j]);
+        rank1<D, NJ, VC>(gx + q * KQ + k, ps, acc);
       }
 #pragma unroll
-      for (int v = 0; v < VC; ++v)
+      for (int v = 0; v < VC / 2; ++v)
 #pragma unroll
         for (int j = 0; j < NJ; ++j) {
           if (q == 0 || q == 2) u[v][j] = acc[v][j];
-          else if (q == 1) t[v][j] = u[v][j] + acc[v][j];
-          else t[v][j] = t[v][j] + (u[v][j] + acc[v][j]);
+          else if (q == 1) t[v][j] = add2(u[v][j], acc[v][j]);
+          else t[v][j] = add2(t[v][j], add2(u[v][j], acc[v][j]));
         }
     }
     // ---- indices, norms, and what they stand for --------------------------------------------------------
     __syncwarp();
 #pragma unroll
     for (int j = 0; j < NJ; ++j) {
-      float r[VC];
+      float r[VC], y[VC];
+#pragma unroll
+      for (int v = 0; v < VC / 2; ++v) unpack2(t[v][j], y[2 * v], y[2 * v + 1]);
 #pragma unroll
       for (int v = 0; v < VC; ++v) {
-        const int i = bucketize_sorted16(t[v][j], s_b[src]);
+        const int i = bucketize_sorted16(y[v], s_b[src]);
         gi[v * D + NJ * lane + j] = (uint8_t)i;
         r[v] = s_c[src][i] * nrm[v];
       }
-      gx[NJ * lane + j] = make_float4(r[0], r[1], r[2], r[3]);
+#pragma unroll
+      for (int g = 0; g < G; ++g) gx[g * D + 32 * j + lane] = make_float4(r[4 * g], r[4 * g + 1], r[4 * g + 2], r[4 * g + 3]);
     }
     __syncwarp();
 #pragma unroll
@@ -204,12 +242,12 @@ __global__ void __launch_bounds__(256) cache_update_kernel(const UpdateArgs a) {
       }
       if (lane == 0) a.norms[src][row] = nrm[v];
     }
-    // ---- un-rotate ------------------------------------------------------------------------------------------
+    // ---- un-rotate (entry 32 j + l of the strip is coordinate NJ l + j: stored without bank conflicts) ------------------------------------------------------------------------------------------
     if (a.dec[0] == nullptr) continue;
 #pragma unroll
-    for (int v = 0; v < VC; ++v)
+    for (int v = 0; v < VC / 2; ++v)
 #pragma unroll
-      for (int j = 0; j < NJ; ++j) acc[v][j] = 0.f;
+      for (int j = 0; j < NJ; ++j) acc[v][j].v = 0;
 #pragma unroll 1
     for (int ch = 0; ch < NCH; ++ch) {
       if (NCH > 1) {
@@ -217,18 +255,20 @@ __global__ void __launch_bounds__(256) cache_update_kernel(const UpdateArgs a) {
         stage(ch);
         __syncthreads();
       }
+#pragma unroll 1
+      for (int j = 0; j < NJ; ++j)
 #pragma unroll 4
-      for (int k = 0; k < KC; ++k) {
-        float ps[NJ];
-        load_row<NJ>(pp + k * D, ps);
-        const float4 x4 = gx[ch * KC + k];
-        const float xs[VC] = {x4.x, x4.y, x4.z, x4.w};
-#pragma unroll
-        for (int v = 0; v < VC; ++v)
-#pragma unroll
-          for (int j = 0; j < NJ; ++j) acc[v][j] = fmaf(xs[v], ps[j], acc[v][j]);
-      }
+        for (int l = 0; l < 32 / NCH; ++l) {
+          float ps[NJ];
+          load_row<NJ>(pp + (NJ * l + j) * D, ps);
+          rank1<D, NJ, VC>(gx + 32 * j + ch * (32 / NCH) + l, ps, acc);
+        }
     }
+    float z[VC][NJ];
+#pragma unroll
+    for (int v = 0; v < VC / 2; ++v)
+#pragma unroll
+      for (int j = 0; j < NJ; ++j) unpack2(acc[v][j], z[2 * v][j], z[2 * v + 1][j]);
 #pragma unroll
     for (int v = 0; v < VC; ++v) {
       if (at[v] < 0) continue;
@@ -236,27 +276,34 @@ __global__ void __launch_bounds__(256) cache_update_kernel(const UpdateArgs a) {
       if constexpr (NJ % 4 == 0) {
 #pragma unroll
         for (int j = 0; j < NJ; j += 4) {
-          const float y[4] = {acc[v][j], acc[v][j + 1], acc[v][j + 2], acc[v][j + 3]};
+          const float y[4] = {z[v][j], z[v][j + 1], z[v][j + 2], z[v][j + 3]};
           store4(a.dec[src], a.dtype, o + j, y);
         }
       } else {
 #pragma unroll
-        for (int j = 0; j < NJ; ++j) store_from_float(a.dec[src], a.dtype, o + j, acc[v][j]);
+        for (int j = 0; j < NJ; ++j) store_from_float(a.dec[src], a.dtype, o + j, z[v][j]);
       }
     }
   }
-  (void)n_vec;
 }
 
-template <int D>
+template <int D, int VC>
 int launch_update(const UpdateArgs& a, cudaStream_t st) {
-  using C = Cfg<D>;
-  if (!ensure_dynamic_smem<cache_update_kernel<D>>((int)C::kSmem)) return TQ4_ERR_CUDA;
+  using C = Cfg<D, VC>;
+  if (!ensure_dynamic_smem<cache_update_kernel<D, VC>>((int)C::kSmem)) return TQ4_ERR_CUDA;
   const int64_t chunks = 2 * (((int64_t)a.batch * a.heads * a.n_new + C::VC - 1) / C::VC);
   const int64_t most = sm_count();
-  cache_update_kernel<D><<<(unsigned)(chunks < most ? chunks : most), 256, C::kSmem, st>>>(a);
+  cache_update_kernel<D, VC><<<(unsigned)(chunks < most ? chunks : most), 256, C::kSmem, st>>>(a);
   TQ4_CHECK_LAUNCH();
   return TQ4_OK;
+}
+
+// Eight vectors a warp (half the reads of Pi per FMA) once every warp of the GPU has that many
+template <int D>
+int launch_update(const UpdateArgs& a, cudaStream_t st) {
+  if constexpr (D <= 128)
+    if (2 * (int64_t)a.batch * a.heads * a.n_new >= 64 * (int64_t)sm_count()) return launch_update<D, 8>(a, st);
+  return launch_update<D, 4>(a, st);
 }
 
 }  // namespace

@@ -298,6 +298,55 @@ struct States {
   }
 };
 
+// attend_rows(q, rows, block_table, len_rows, len, k_centroids, v_centroids, rotation, num_kv_heads, page_tokens,
+//             sm_scale, out_dtype): one query row per sequence, q [B, Hq, 1, D], over `len` token rows each
+// -> [B, 1, Hq, D].  Everything a generation step needs of `attention`, with no tensor made but the result.
+PyObject* attend_rows(PyObject*, PyObject* const* p, Py_ssize_t n) {
+  if (!expect("attend_rows", n, 12)) return nullptr;
+  return guarded([&]() -> PyObject* {
+    const at::Tensor q = inner_contiguous(cuda_tensor(p[0], "q"));
+    const at::Tensor &rows = cuda_tensor(p[1], "rows"), &bt = cuda_tensor(p[2], "block_table"), &lens = cuda_tensor(p[3], "len_rows");
+    const int64_t len = as_int(p[4]), hkv = as_int(p[8]), page = as_int(p[9]);
+    const at::Tensor &kc = cuda_tensor(p[5], "k_centroids"), &vc = cuda_tensor(p[6], "v_centroids");
+    at::Tensor rot = cuda_tensor(p[7], "rotation");
+    TQ4_ASSERT(q.dim() == 4 && q.size(2) == 1, "q must be [batch, heads, 1, head_dim]");
+    const int64_t b = q.size(0), hq = q.size(1), d = q.size(3);
+    TQ4_ASSERT(hkv > 0 && hq % hkv == 0, "query heads must be a multiple of the KV heads");
+    TQ4_ASSERT(rows.scalar_type() == at::kByte && rows.dim() == 3 && rows.is_contiguous() && rows.size(0) == b && page > 0 &&
+                   rows.size(1) % page == 0,
+               "rows must be contiguous uint8 [batch, capacity, bytes], whole pages");
+    TQ4_ASSERT(bt.scalar_type() == at::kInt && bt.dim() == 2 && bt.size(0) == b && bt.is_contiguous(), "block_table must be contiguous int32");
+    TQ4_ASSERT(lens.scalar_type() == at::kInt && lens.dim() == 2 && lens.size(1) == b && lens.is_contiguous() && len >= 0 &&
+                   len < lens.size(0),
+               "len_rows must be contiguous int32 [capacity + 1, batch]");
+    TQ4_ASSERT(rot.scalar_type() == at::kFloat, "rotation must be float32");
+    if (!rot.is_contiguous()) rot = rot.contiguous();
+    const float scale = p[10] == Py_None ? (float)(1.0 / std::sqrt((double)d)) : (float)as_double(p[10]);
+    const int dev = device_index(q);
+    Launch launch(dev);
+    const at::ScalarType dt = p[11] == Py_None ? q.scalar_type() : as_dtype(p[11]);
+    at::Tensor out = at::empty({b, 1, hq, d}, q.options().dtype(dt).requires_grad(false));
+    const size_t need = tq4_attention_workspace_bytes(b > 1 ? b : 1, (int)hq, (int)hkv, (int)d);
+    if (need == 0)
+      fail(PyExc_ValueError, "unsupported attention shape: Hq=" + std::to_string(hq) + ", Hkv=" + std::to_string(hkv) +
+                                 ", D=" + std::to_string(d));
+    const at::Tensor& ws = workspace_of(dev, (int64_t)need);
+    int* flag = (int*)flag_of(dev).data_ptr();
+    const int q_dt = dtype_code(q.scalar_type()), out_dt = dtype_code(dt);
+    int st;
+    Py_BEGIN_ALLOW_THREADS
+    st = tq4_paged_attention(
+        q.data_ptr(), q_dt, b, (int)b, (int)hq, (int)hkv, (int)d, q.stride(0), q.stride(1), (const uint8_t*)rows.data_ptr(),
+        page * rows.size(2), rows.size(2), b * (rows.size(1) / page), (int)page, (const int32_t*)bt.data_ptr(), bt.size(1),
+        (const int32_t*)lens.data_ptr() + len * b, nullptr, (const float*)kc.data_ptr(), (int)kc.numel(),
+        (const float*)vc.data_ptr(), (int)vc.numel(), (const float*)rot.data_ptr(), scale, 0, 0, out.data_ptr(), out_dt,
+        out.stride(0), out.stride(2), nullptr, 0, ws.data_ptr(), (size_t)ws.numel() * ws.element_size(), 0, flag, launch.stream);
+    Py_END_ALLOW_THREADS
+    check(st, "attend_rows");
+    return THPVariable_Wrap(std::move(out));
+  });
+}
+
 // append_rows(key, value, rows, offset, rotation_T_even, rotation_T_odd, k_boundaries, v_boundaries)
 PyObject* append_rows(PyObject*, PyObject* const* p, Py_ssize_t n) {
   if (!expect("append_rows", n, 8)) return nullptr;
@@ -385,6 +434,7 @@ PyObject* error_flag(PyObject*, PyObject* const* p, Py_ssize_t n) {
 PyMethodDef kMethods[] = {
     {"attention", (PyCFunction)(void (*)(void))attention, METH_FASTCALL, "Paged TQ4 attention, optionally with a cache write."},
     {"write_paged", (PyCFunction)(void (*)(void))write_paged, METH_FASTCALL, "Compress K and V into the paged cache."},
+    {"attend_rows", (PyCFunction)(void (*)(void))attend_rows, METH_FASTCALL, "Attention of one query row per sequence over token rows."},
     {"append_rows", (PyCFunction)(void (*)(void))append_rows, METH_FASTCALL, "Compress K and V into token rows of a batch."},
     {"cache_update", (PyCFunction)(void (*)(void))cache_update, METH_FASTCALL, "Compress, store and reconstruct an update."},
     {"error_flag", (PyCFunction)(void (*)(void))error_flag, METH_FASTCALL, "Device error flag."},

@@ -152,10 +152,13 @@ class TokenRowStore:
         (src/turboquant_vllm/triton/flash_attention_tq4_kv.py:163-199, 301-302): ``is_causal`` lets
         query ``i`` see keys ``0..i``; a single query row is never masked.
         """
-        from turboquant_vllm.kernels.ops import paged_tq4_attention
-
         b, hq, sq, d = q.shape
         assert b == self.batch and d == self.dim and hq % self.heads == 0
+        if sq == 1 and self._len_rows is not None:
+            return nv.host().attend_rows(q, self.rows, self._block_table, self._len_rows, self.len, k_centroids, v_centroids,
+                                         rotation, self.heads, PAGE_TOKENS, sm_scale, out_dtype)
+        from turboquant_vllm.kernels.ops import paged_tq4_attention
+
         dev = self.device
         q_rows = q.transpose(1, 2).reshape(b * sq, hq, d)
         table = self._block_table
