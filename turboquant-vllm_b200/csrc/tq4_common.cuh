@@ -278,15 +278,15 @@ inline bool tokens_uniform(const CompressArgs& a) {
 }
 
 // Which kernel makes a write of so many vectors (B200, graph replays of stand-alone writes, bf16):
-//   a block per vector (head_dim <= 128) up to kTinyRows: 5.2 us at 32 vectors, 8.4 at 2048; the prologue kernel 8.1
-//     and 10.5, the tensor-core kernel 10.4 and 10.6
-//   the tensor-core kernel above tc_rows().  At head_dim 64 and 96 that is kTinyRows; at 256 512 vectors (10.4 us at 800, the
-//     prologue kernel 15).  At head_dim 128 it would pay from there on too (8192 vectors: 10.8 us, the prologue kernel 16,
-//     a block per vector 24), but up to kSmallRows a vector is promised the same bytes however the calls are cut, and
-//     only the FMA kernels agree with one another bit for bit
+//   a block per vector up to tiny_rows(): a few us plus 1.1 / 1.7 / 2.5 us per 1000 vectors of 64 / 96 / 128, against 8 - 10 us
+//     of the tensor-core kernel and 16 us of the prologue kernel at 4800 vectors of 128; at 256 it never pays
+//   the tensor-core kernel above tc_rows().  At head_dim 128 it would pay earlier (8192 vectors: 10.8 us, the prologue
+//     kernel 16, a block per vector 24), but up to kSmallRows a vector is promised the same bytes however the calls are cut,
+//     and only the FMA kernels agree with one another bit for bit.  At 256 the prologue kernel takes 15 us at 800
 //   the prologue kernel in between, and up to kSmallRows for what the tensor-core kernel cannot address
-constexpr int64_t kTinyRows = 2048, kSmallRows = 8192;
-constexpr int64_t tc_rows(int head_dim) { return head_dim == 128 ? kSmallRows : head_dim == 256 ? 512 : kTinyRows; }
+constexpr int64_t kSmallRows = 8192;
+constexpr int64_t tiny_rows(int head_dim) { return head_dim == 64 ? 5500 : head_dim == 96 ? 2400 : head_dim == 128 ? 4096 : 0; }
+constexpr int64_t tc_rows(int head_dim) { return head_dim == 128 ? kSmallRows : head_dim == 256 ? 512 : tiny_rows(head_dim); }
 int launch_small_write(const CompressArgs& w, int head_dim, cudaStream_t st);
 int dispatch_compress(const CompressArgs& a, int head_dim, int dtype, cudaStream_t st);
 // tensor-core (tcgen05) compress kernel for large inputs at head_dim 128 (tq4_compress_tc.cu)

@@ -210,9 +210,12 @@ compress_kernel(const CompressArgs a) {
 // Small launches: one CTA of four warps per row,
 // each warp reduces one quarter of k with Pi^T read straight from L1/L2; the four partial sums
 // are combined as (s0 + s1) + (s2 + s3), the same order the streaming kernel uses, so a row
-// compresses to the same bytes whichever kernel handles it.
-template <int D, typename T>
-__global__ void __launch_bounds__(128) compress_small_kernel(const CompressArgs a) {
+// compresses to the same bytes whichever kernel handles it.  Bound by latency (one vector is 64 KB of loads and a
+// chain of sums), so what does not depend on the vector -- its slot, the first batch of Pi^T -- is
+// loaded before it (512 vectors of 128 5.7 -> 4.7 us, 624 5.9 -> 5.0), within the 32 registers that let 16 blocks share an
+// SM: with more in flight few vectors gain another 0.5 us, but at 1500 - 2400 a second wave costs 1 us.  SEQ: slots computed from sequence and position instead of read.
+template <int D, typename T, bool SEQ>
+__global__ void __launch_bounds__(128, 16) compress_small_kernel(const CompressArgs a) {
   using Cfg = CompressCfg<D>;
   constexpr int HALF = Cfg::HALF, NBL = Cfg::NBL, XPL = Cfg::XPL, KQ = D / 4;
   __shared__ float s_x[D];
@@ -230,7 +233,27 @@ __global__ void __launch_bounds__(128) compress_small_kernel(const CompressArgs 
     const int i = threadIdx.x - 32;
     s_b[i] = i < a.n_bounds[src] ? a.bounds[src][i] : CUDART_INF_F;
   }
-  const T* xp = reinterpret_cast<const T*>(a.x[src]) + token_offset(a, src, tok) + (int64_t)h * a.head_stride[src];
+  const int64_t at = SEQ ? token_offset(a, src, tok) : tok * a.token_stride[src];
+  const T* xp = reinterpret_cast<const T*>(a.x[src]) + at + (int64_t)h * a.head_stride[src];
+  int64_t slot = -1;
+  if (a.cache != nullptr && tok < a.n_slots && warp == 0) slot = SEQ ? write_slot(a, tok) : a.slot_mapping[tok];
+  // explicit load batches: 4 k-steps of Pi^T (up to 16 independent loads; more cost blocks per SM) are in flight before
+  // the first FMA of the batch consumes them
+  constexpr int B = 4;
+  const int k0 = warp * KQ;
+  float pe[B][NBL], po[B][NBL];
+  auto load_batch = [&](int kb) {
+#pragma unroll
+    for (int u = 0; u < B; ++u)
+#pragma unroll
+      for (int i = 0; i < NBL; ++i) {
+        const int p = lane + 32 * i;
+        const int k = k0 + kb + u;
+        pe[u][i] = (p < HALF) ? __ldg(a.rot_even + k * HALF + p) : 0.f;
+        po[u][i] = (p < HALF) ? __ldg(a.rot_odd + k * HALF + p) : 0.f;
+      }
+  };
+  load_batch(0);
   float xv[XPL];
   float ss = 0.f;
 #pragma unroll
@@ -253,23 +276,11 @@ __global__ void __launch_bounds__(128) compress_small_kernel(const CompressArgs 
   float acc[2 * NBL];
 #pragma unroll
   for (int i = 0; i < 2 * NBL; ++i) acc[i] = 0.f;
-  const int k0 = warp * KQ;
-  // explicit load batches: 8 k-steps of Pi^T (up to 32 independent loads) are in flight before
-  // the first FMA of the batch consumes them
-  static_assert(KQ % 8 == 0, "quarter of head_dim must be a multiple of 8");
-  for (int kb = 0; kb < KQ; kb += 8) {
-    float pe[8][NBL], po[8][NBL];
 #pragma unroll
-    for (int u = 0; u < 8; ++u)
+  for (int kb = 0; kb < KQ; kb += B) {
+    if (kb > 0) load_batch(kb);
 #pragma unroll
-      for (int i = 0; i < NBL; ++i) {
-        const int p = lane + 32 * i;
-        const int k = k0 + kb + u;
-        pe[u][i] = (p < HALF) ? __ldg(a.rot_even + k * HALF + p) : 0.f;
-        po[u][i] = (p < HALF) ? __ldg(a.rot_odd + k * HALF + p) : 0.f;
-      }
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
+    for (int u = 0; u < B; ++u) {
       const float xk = s_x[k0 + kb + u];
 #pragma unroll
       for (int i = 0; i < NBL; ++i) {
@@ -292,9 +303,7 @@ __global__ void __launch_bounds__(128) compress_small_kernel(const CompressArgs 
   uint8_t* dst_idx;
   float* dst_norm;
   if (a.cache != nullptr) {
-    if (tok >= a.n_slots) return;
-    const int64_t slot = write_slot(a, tok);
-    if (slot < 0) return;
+    if (slot < 0) return;  // (a padding token, or one without a slot)
     if (slot >= a.num_cache_slots) {
       if (lane == 0 && a.err_flag) atomicOr(a.err_flag, TQ4_DEV_BAD_SLOT);
       return;
@@ -324,8 +333,9 @@ int launch_compress(const CompressArgs& a, cudaStream_t st) {
   const int64_t total_rows = a.n_tokens * a.num_heads * a.n_sources;
   if (total_rows == 0) return TQ4_OK;
   if (total_rows > 0x7fffffffll) return TQ4_ERR_INVALID_ARG;  // the kernels index rows with 32 bits
-  if (D <= 128 && total_rows <= kTinyRows) {
-    compress_small_kernel<D <= 128 ? D : 128, T><<<(unsigned)total_rows, 128, 0, st>>>(a);
+  if (total_rows <= tiny_rows(D)) {
+    if (a.seq) compress_small_kernel<D <= 128 ? D : 128, T, true><<<(unsigned)total_rows, 128, 0, st>>>(a);
+    else compress_small_kernel<D <= 128 ? D : 128, T, false><<<(unsigned)total_rows, 128, 0, st>>>(a);
     TQ4_CHECK_LAUNCH();
     return TQ4_OK;
   }
@@ -352,7 +362,7 @@ int dispatch_dtype(const CompressArgs& a, int dtype, cudaStream_t st) {
 int dispatch_compress(const CompressArgs& a, int head_dim, int dtype, cudaStream_t st) {
   const int64_t vectors = a.n_tokens * a.num_heads * a.n_sources;
   if (vectors == 0) return TQ4_OK;
-  const bool tiny = head_dim <= 128 && vectors <= kTinyRows;  // (dispatch_dtype: a block per vector)
+  const bool tiny = vectors <= tiny_rows(head_dim);  // (dispatch_dtype: a block per vector)
   if (vectors > tc_rows(head_dim) && compress_tc16_eligible(a, head_dim, dtype))
     return launch_compress_tc16(a, head_dim, dtype, st);
   if (!tiny && vectors <= kSmallRows) return launch_small_write(a, head_dim, st);
