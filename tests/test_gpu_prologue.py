@@ -29,10 +29,7 @@ def test_step_writes_and_rotates(cuda_lib, d, rows):
     out = ops.paged_tq4_attention(
         q.cuda(), cache, bt.cuda(), case["seq_lens"].cuda(), p["kc"], p["vc"], p["rot"], hkv, bs,
         out_dtype=torch.float32, write=(k, v, slots.cuda(), p["even"], p["odd"], p["kb"], p["vb"]))
-    if 2 * hkv * rows <= {64: 5500, 96: 2400, 128: 8192, 256: 512}[d]:  # above, a stand-alone write rotates on the tensor cores
-        assert torch.equal(cache, want)
-    else:
-        assert (cache != want).float().mean() <= 1e-4
+    assert torch.equal(cache, want)
     pick = sorted({0, rows // 2, rows - 1})
     ref = O.paged_decode_fp32(q[pick], want.cpu(), bt[pick], [lens[i] for i in pick], pr.kc, pr.vc, pr.rot, hkv)
     got = out.cpu()[pick]

@@ -282,14 +282,14 @@ inline bool tokens_uniform(const CompressArgs& a) {
 //     of the tensor-core kernel and 16 us of the prologue kernel at 4800 vectors of 128; at 256 it never pays
 //   the tensor-core kernel above tc_rows().  At head_dim 128 it would pay earlier (8192 vectors: 10.8 us, the prologue
 //     kernel 16, a block per vector 24), but up to kSmallRows a vector is promised the same bytes however the calls are cut,
-//     and only the FMA kernels agree with one another bit for bit.  At 256 the prologue kernel takes 15 us at 800
+//     and there only the FMA kernels agree with one another bit for bit.  At 256 the prologue kernel takes 15 us at 800
 //   the prologue kernel in between, and up to kSmallRows for what the tensor-core kernel cannot address
 constexpr int64_t kSmallRows = 8192;
-constexpr int64_t tiny_rows(int head_dim) { return head_dim == 64 ? 5500 : head_dim == 96 ? 2400 : head_dim == 128 ? 4096 : 0; }
-constexpr int64_t tc_rows(int head_dim) { return head_dim == 128 ? kSmallRows : head_dim == 256 ? 512 : tiny_rows(head_dim); }
+constexpr int64_t tiny_rows(int head_dim) { return head_dim == 64 ? 6500 : head_dim == 96 ? 3000 : head_dim == 128 ? 4096 : 0; }
+constexpr int64_t tc_rows(int head_dim) { return head_dim == 128 ? kSmallRows : head_dim == 256 ? 1000 : tiny_rows(head_dim); }
 int launch_small_write(const CompressArgs& w, int head_dim, cudaStream_t st);
 int dispatch_compress(const CompressArgs& a, int head_dim, int dtype, cudaStream_t st);
-// tensor-core (tcgen05) compress kernel for large inputs at head_dim 128 (tq4_compress_tc.cu)
+// tensor-core (tcgen05) compress kernel for large fp32 or oddly strided inputs at head_dim 128 (tq4_compress_tc.cu)
 bool compress_tc_eligible(const CompressArgs& a, int head_dim, int dtype);
 int launch_compress_tc(const CompressArgs& a, int dtype, cudaStream_t st);
 // pipelined tcgen05 kernel for 16-bit inputs (tq4_compress_tc16.cu)

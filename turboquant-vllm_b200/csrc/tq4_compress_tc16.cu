@@ -29,8 +29,9 @@
 // boundaries are too close for that take the search): two FMAs, two lookups through the warp shuffle
 // (lane c holds cell c's boundary and the index below it), one compare, one add.  The comparison is the
 // search's own, against the same fp32 boundary, so the indices are the same.  Measured (bf16 cache write, K and
-// V): 16384 tokens of 8 heads of 128 48.6 -> 31.1 us (2.7 TB/s), 512 tokens (8192 vectors) 24 -> 10.8 us
-// against a block per vector, 16384 tokens of 4 heads of 256 894 -> 62 us (the 256 columns are split over two CTAs:
+// V): 16384 tokens of 8 heads of 128 48.6 -> 31.1 us (2.7 TB/s), 8208 vectors 24 -> 11.1 us
+// against a block per vector, 16384 tokens of 4 heads of 256 894 -> 79 us (62 without the
+// second sums below; the 256 columns are split over CTAs:
 // one cannot hold Pi and two stages of vectors).
 // Every mbarrier wait is bounded; a wait that gives up marks the CTA dead, all roles drain and the
 // kernel reports TQ4_DEV_TIMEOUT.  Tensor memory is released on every path.
@@ -221,6 +222,11 @@ __device__ __forceinline__ int bucketize_reg(float y, const float (&b)[15]) {
   return (c1 ? 8 : 0) + (c2 ? 4 : 0) + (c3 ? 2 : 0) + (c4 ? 1 : 0);
 }
 
+// The two roundings of a coordinate (this kernel's product, the FMA kernels' chains) lie 2e-8 apart on average; a coordinate
+// nearer than this to a boundary (about 1e-5 of them) is summed again the FMA kernels' way, so that the bytes are theirs.
+// (Not at head_dim 128, whose large writes have been the tensor cores' own for longer than there was a choice.)
+constexpr float kNear = 1.5e-7f;
+
 // The 32-cell map: cell = round(31 * sat(y * s / 31 + 16 / 31)), so y = 0 sits in the middle of cell 16 and
 // everything past the ends in the end cells.  `scale` = s / 31; lane c: the boundary inside cell c (+inf: none) and the
 // number of boundaries in the cells below.
@@ -263,6 +269,67 @@ __device__ __forceinline__ int bucketize_grid(float y, const Grid& g) {
   return __shfl_sync(0xffffffffu, g.below, c) + (y > __shfl_sync(0xffffffffu, g.bound, c) ? 1 : 0);
 }
 
+// The same, with the distance to the boundary (its sign decides: y - bound is zero only where they are equal)
+__device__ __forceinline__ int bucketize_grid(float y, const Grid& g, float& d) {
+  const float u = fmaf(__saturatef(fmaf(y, g.scale, 16.f / 31.f)), 31.f, 8388608.f);
+  const int c = __float_as_int(u);
+  d = y - __shfl_sync(0xffffffffu, g.bound, c);
+  return __shfl_sync(0xffffffffu, g.below, c) + (d > 0.f ? 1 : 0);
+}
+
+// 32 coordinates of a row that are summed again, later: where they go, the row, 2 * chunk + source
+struct Again {
+  uint8_t* dst;
+  unsigned row, where;
+};
+constexpr int kAgainMax = 8;  // a warp's list
+
+// The chunks on a warp's list by the sums of the FMA kernels: the norm, then lane = coordinate, four quarter chains in
+// ascending k, combined as (s0 + s1) + (s2 + s3).  Kept out of the tile loop, whose code has to stay short.
+template <typename T, int D>
+__device__ __noinline__ void sum_again(const T* x0, const T* x1, const float* even, const float* odd, const CompressArgs* a,
+                                       const float (*bounds)[16], const Again* list, int n, int j0, int lane) {
+  constexpr int XPL = D / 32, KQ = D / 4, B = 8, STEP = D == 256 ? 32 : B;  // (STEP: from one register of the row)
+  static_assert(KQ % STEP == 0, "whole batches");
+  for (int m = 0; m < n; ++m) {
+    const Again e = list[m];
+    const int src = e.where & 1, j = j0 + 32 * (int)(e.where >> 1) + lane;
+    const unsigned tok = e.row / (unsigned)a->num_heads, h = e.row - tok * (unsigned)a->num_heads;
+    const T* x = (src ? x1 : x0) + token_offset(*a, src, tok) + (int64_t)h * a->head_stride[src];
+    const float* pi = ((j & 1) ? odd : even) + (j >> 1);
+    float xs[XPL], ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < XPL; ++i) xs[i] = to_float<T>(x[lane + 32 * i]);
+#pragma unroll
+    for (int i = 0; i < XPL; ++i) ss = fmaf(xs[i], xs[i], ss);
+    const float den = sqrtf(warp_sum(ss)) + 1e-10f;
+#pragma unroll
+    for (int i = 0; i < XPL; ++i) xs[i] = xs[i] / den;
+    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+    for (int o = 0; o < KQ; o += STEP) {  // the four quarters side by side: 32 loads in flight
+#pragma unroll 1
+      for (int l = 0; l < STEP; l += B) {
+        float p[4][B];
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+#pragma unroll
+          for (int c = 0; c < B; ++c) p[q][c] = __ldg(pi + (q * KQ + o + l + c) * (D / 2));
+#pragma unroll
+        for (int c = 0; c < B; ++c)
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            acc[q] = fmaf(__shfl_sync(0xffffffffu, xs[(q * KQ + o) / 32], (q * KQ + o) % 32 + l + c), p[q][c], acc[q]);
+      }
+    }
+    const float t = (acc[0] + acc[1]) + (acc[2] + acc[3]);
+    uint32_t w = (uint32_t)bucketize_sorted16(t, bounds[src]) << (8 * ((lane & 7) >> 1) + ((lane & 1) ? 0 : 4));
+#pragma unroll
+    for (int o = 1; o < 8; o <<= 1) w |= __shfl_xor_sync(0xffffffffu, w, o);
+    if ((lane & 7) == 0) reinterpret_cast<uint32_t*>(e.dst)[lane >> 3] = w;
+  }
+}
+
 struct Bars {
   uint64_t full[4];    // TMA -> consumers: the stage's tile has landed
   uint64_t empty[4];   // consumers -> TMA: MMAs (1 commit) and the norm readers (4 warps) are done with it
@@ -272,16 +339,18 @@ struct Bars {
 
 template <typename T, int D>
 __global__ void __launch_bounds__(Cfg<D>::THREADS, 1)
-compress_tc16_kernel(const CompressArgs a, const int group_rows, const __grid_constant__ CUtensorMap tm_x0,
+compress_tc16_kernel(const __grid_constant__ CompressArgs a, const int group_rows, const __grid_constant__ CUtensorMap tm_x0,
                      const __grid_constant__ CUtensorMap tm_x1) {
   using F = Fmt<T>;
   using C = Cfg<D>;
   constexpr int N = C::N, STAGES = C::STAGES;
+  constexpr bool kAgain = D != 128;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   __shared__ __align__(8) Bars s_bars;
   __shared__ uint32_t s_tmem;
   __shared__ int s_dead;
   __shared__ float s_bounds[2][16];
+  __shared__ Again s_again[kAgain ? kAgainMax * (C::THREADS / 32 - 2) : 1];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   if (warp == 0) CT_STAMP(0, 31, 6);  // kernel entry
   const uint32_t base = (smem_addr(smem_raw) + 1023u) & ~1023u;  // swizzle atoms need 1024-byte alignment
@@ -410,6 +479,8 @@ compress_tc16_kernel(const CompressArgs a, const int group_rows, const __grid_co
     Grid grid[2];
     bool grid_ok = make_grid(s_bounds[0], grid[0], lane);
     grid_ok = make_grid(s_bounds[1], grid[1], lane) && grid_ok;
+    [[maybe_unused]] Again* my_again = s_again + (kAgain ? kAgainMax * (warp - 2) : 0);
+    [[maybe_unused]] int n_again = 0;
     for (int64_t i = grp; i < my_tiles && ok; i += STAGES) {
       const int st = grp;
       const uint32_t par = (uint32_t)((i / STAGES) & 1);
@@ -488,13 +559,26 @@ compress_tc16_kernel(const CompressArgs a, const int group_rows, const __grid_co
         uint32_t v[32];
         tmem_ld32(tmem_base + ((uint32_t)(32 * quarter) << 16) + (uint32_t)(st * N + 32 * q), v);
         uint32_t word[4];
+        [[maybe_unused]] float closest = CUDART_INF_F;  // of the chunk's coordinates to their boundaries
         if (grid_ok) {
 #pragma unroll
           for (int w = 0; w < 4; ++w) {  // 8 coordinates -> 4 bytes -> one word
             word[w] = 0;
 #pragma unroll
-            for (int e = 0; e < 8; ++e)
-              word[w] += (uint32_t)bucketize_grid(__uint_as_float(v[8 * w + e]) * scale, g) << (8 * (e >> 1) + ((e & 1) ? 0 : 4));
+            for (int e = 0; e < 8; e += 2) {
+              const float y0 = __uint_as_float(v[8 * w + e]) * scale, y1 = __uint_as_float(v[8 * w + e + 1]) * scale;
+              int i0, i1;
+              if constexpr (kAgain) {
+                float d0, d1;
+                i0 = bucketize_grid(y0, g, d0);
+                i1 = bucketize_grid(y1, g, d1);
+                closest = fminf(closest, fminf(fabsf(d0), fabsf(d1)));
+              } else {
+                i0 = bucketize_grid(y0, g);
+                i1 = bucketize_grid(y1, g);
+              }
+              word[w] += ((uint32_t)i0 << (4 * e + 4)) + ((uint32_t)i1 << (4 * e));
+            }
           }
         } else {
           float b[15];
@@ -504,8 +588,12 @@ compress_tc16_kernel(const CompressArgs a, const int group_rows, const __grid_co
           for (int w = 0; w < 4; ++w) {
             word[w] = 0;
 #pragma unroll
-            for (int e = 0; e < 8; ++e)
-              word[w] += (uint32_t)bucketize_reg(__uint_as_float(v[8 * w + e]) * scale, b) << (8 * (e >> 1) + ((e & 1) ? 0 : 4));
+            for (int e = 0; e < 8; ++e) {
+              const float y = __uint_as_float(v[8 * w + e]) * scale;
+              const int idx = bucketize_reg(y, b);
+              if (kAgain && bucketize_reg(y - kNear, b) != bucketize_reg(y + kNear, b)) closest = 0.f;
+              word[w] += (uint32_t)idx << (8 * (e >> 1) + ((e & 1) ? 0 : 4));
+            }
           }
         }
         if (wide) {
@@ -514,12 +602,33 @@ compress_tc16_kernel(const CompressArgs a, const int group_rows, const __grid_co
 #pragma unroll
           for (int w = 0; w < 4; ++w) reinterpret_cast<uint32_t*>(dst_idx)[4 * q + w] = word[w];
         }
+        if constexpr (kAgain) {
+          // (a zero vector is zero either way)
+          uint32_t who = __ballot_sync(0xffffffffu, closest < kNear && dst_idx != nullptr && nrm != 0.f);
+#pragma unroll 1
+          for (; who != 0; who &= who - 1) {
+            if (n_again == kAgainMax) {
+              __syncwarp();
+              sum_again<T, D>(reinterpret_cast<const T*>(a.x[0]), reinterpret_cast<const T*>(a.x[1]), a.rot_even, a.rot_odd, &a,
+                              s_bounds, my_again, n_again, j0, lane);
+              __syncwarp();
+              n_again = 0;
+            }
+            if (lane == __ffs(who) - 1) my_again[n_again] = Again{dst_idx + 16 * q, (unsigned)in_src, 2u * q + src};
+            ++n_again;
+          }
+        }
       }
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) bar_arrive(smem_addr(&s_bars.tempty[st]));  // the accumulator may be overwritten
       if (dst_norm && split == 0) *dst_norm = nrm;
       if (quarter == 0 && grp < 2) CT_STAMP(2 + grp, i, 3);
+    }
+    if constexpr (kAgain) {
+      __syncwarp();
+      sum_again<T, D>(reinterpret_cast<const T*>(a.x[0]), reinterpret_cast<const T*>(a.x[1]), a.rot_even, a.rot_odd, &a, s_bounds,
+                      my_again, n_again, j0, lane);
     }
   }
   if (!ok) {
