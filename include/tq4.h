@@ -64,9 +64,9 @@ const char* tq4_status_string(int status);
  * Exactness: given the same rotated coordinates y the bytes are bit-exact (tq4_pack_rotated_rows);
  * end to end a coordinate within ~1e-7 of a boundary may land in the neighbouring bucket, because
  * the rotation's summation order differs from the reference's matmul: at most 1e-4 of the indices
- * (measured 6e-7 on the FFMA kernels, 5e-7 on the tensor-core kernels that take inputs of more
- * than 8192 vectors at head_dim 128; setting TQ4_NO_TC in the environment keeps every input on the
- * FFMA kernels).  Norms are within 3 ulp of a CPU torch.norm and identical across all kernels here.
+ * (measured 6e-7 on the FFMA kernels, 5e-7 on the tensor-core kernels that take 16-bit inputs of more
+ * than 6500 / 3000 / 8192 / 1000 vectors at head_dim 64 / 96 / 128 / 256 and fp32 ones above 8192 at 128; setting
+ * TQ4_NO_TC in the environment keeps every input on the FFMA kernels).  Norms are within 3 ulp of a CPU torch.norm and identical across all kernels here.
  * Replaces: tq4_compress() + _tq4_compress_kernel, src/turboquant_vllm/triton/tq4_compress.py:46-148,173-245
  *           (arithmetic contract = its PyTorch path, :248-295 / quantizer.py:112-151).
  * rot_t_even / rot_t_odd: [D, D/2] fp32, the even / odd columns of Pi^T (same split as the
@@ -134,13 +134,17 @@ int tq4_append_rows(const void* key, const void* value, int kv_dtype, int batch,
  */
 int tq4_cache_update(const void* key, const void* value, int dtype, int batch, int num_heads, int n_new,
                      int head_dim, const int64_t* k_strides, const int64_t* v_strides, const float* rotation,
+                     const float* rot_t_even, const float* rot_t_odd,
                      const float* k_boundaries, int n_k_boundaries,
                      const float* v_boundaries, int n_v_boundaries,
                      const float* k_centroids, int n_k_centroids,
                      const float* v_centroids, int n_v_centroids, int k_nibble, int v_nibble,
                      uint8_t* k_idx, float* k_norms, uint8_t* v_idx, float* v_norms,
                      int64_t capacity, int64_t offset, void* k_dec, void* v_dec,
-                     int64_t dec_capacity, int64_t dec_offset, void* stream);
+                     int64_t dec_capacity, int64_t dec_offset, void* scratch, size_t scratch_bytes,
+                     void* stream);
+/* Bytes of 16-byte aligned scratch that such an update needs (0: none, scratch may be null). */
+size_t tq4_cache_update_scratch_bytes(int batch, int num_heads, int n_new, int head_dim);
 
 /*
  * Decompress rows (rotated space): out[(n,h), 0:D] = centroids[idx] * norm, cast to out_dtype.
@@ -196,8 +200,9 @@ size_t tq4_attention_workspace_bytes(int64_t max_query_rows, int num_q_heads, in
  *              rotated space (normalised) for a later cross-GPU combine.
  * workspace    >= tq4_attention_workspace_bytes(num_rows, Hq, Hkv, D), 16-byte aligned
  * mode         0 = auto, 1 = fp32 CUDA-core kernel, 2 = streaming tensor-core LUT kernel (mma.sync),
- *              3 = chunked-prefill tcgen05 kernel (needs query_start_loc, head_dim 128, 16-byte
- *              aligned K/V regions; TQ4_ERR_UNSUPPORTED otherwise),
+ *              3 = chunked-prefill tcgen05 kernel for every sequence (needs query_start_loc and at most 128
+ *              query heads per KV head; TQ4_ERR_UNSUPPORTED otherwise).  Mode 0 gives it the sequences of 8
+ *              and more new rows of calls large enough to pay for it, the streaming kernel the others,
  *              4 = the same kernel in its fast form: queries and probabilities enter the tensor
  *              cores as single fp16 terms (mode 3 splits both into hi + lo), which halves the
  *              tensor work and lets their 2^-11 rounding reach the output (about 1e-3 absolute:

@@ -10,7 +10,7 @@
 // it is; at head_dim 256, where that does not fit, in chunks of 64 rows) and the vectors from a strip per warp.
 // A step of a few tokens is latency bound (staging Pi: 128 KB per block), so its vectors are spread over the blocks
 // first; a prompt is bound by FMA issue.
-// Measured: a generation of 8 tokens behind 4 prompts of 1100, 2 layers of 8 heads of 128, 7800 -> 730 us.
+// Measured: a generation of 8 tokens behind 4 prompts of 1100, 2 layers of 8 heads of 128, 7800 -> 452 us.
 #include <math_constants.h>
 
 #include "tq4_common.cuh"
@@ -30,6 +30,9 @@ struct UpdateArgs {
   int64_t cap, dec_cap, offset, dec_offset;
   int batch, heads, n_new, dtype;
   const float* rotation;
+  const float *rot_even, *rot_odd;  // even / odd columns of Pi^T
+  const uint8_t* packed;               // DONE: the compressed vectors, K then V, [B, S, H, D / 2] and [B, S, H]
+  const float* packed_norms;
 };
 
 // two fp32 operations an instruction, each rounded as alone
@@ -76,6 +79,119 @@ __device__ __forceinline__ void load_row(const float* p, float (&v)[NJ]) {
   }
 }
 
+// The same for a step of a few tokens: a block per vector, each warp one quarter of both reductions (head_dim 256: for half
+// of the columns) with Pi read through L1 / L2 -- along rows of Pi^T (the even / odd halves) to rotate, along rows of Pi to
+// rotate back -- in batches of four rows a lane.  Bound by latency; staging Pi for four vectors a warp, as below,
+// cost 18 us for
+// a token of four sequences at head_dim 128 and 63 at 256, against 5.5 and 9.
+template <int D>
+struct TinyCfg {
+  static constexpr int CS = D == 256 ? 2 : 1, WARPS = 4 * CS, THREADS = 32 * WARPS;
+  static constexpr int HALF = D / 2, NBL = (HALF / CS + 31) / 32, NJ = D / 32 / CS, B = 4;
+};
+template <int D>
+__global__ void __launch_bounds__(TinyCfg<D>::THREADS) cache_update_tiny_kernel(const UpdateArgs a) {
+  using C = TinyCfg<D>;
+  constexpr int HALF = C::HALF, NBL = C::NBL, NJ = C::NJ, B = C::B, XPL = D / 32, KQ = D / 4;
+  static_assert(KQ % B == 0, "whole batches");
+  __shared__ __align__(16) float s_part[4][D];
+  __shared__ float s_x[D], s_b[16], s_c[16];
+  __shared__ uint8_t s_i[D];
+  const int tid = threadIdx.x, lane = tid & 31, q = (tid >> 5) & 3, half = tid >> 7;  // quarter, column half
+  const int per_src = a.batch * a.heads * a.n_new;
+  const int src = (int)blockIdx.x >= per_src ? 1 : 0, vec = (int)blockIdx.x - src * per_src;
+  const int bh = vec / a.n_new, s = vec - bh * a.n_new, b = bh / a.heads, h = bh - b * a.heads;
+  const int64_t at = (int64_t)b * a.batch_stride[src] + (int64_t)h * a.head_stride[src] + (int64_t)s * a.token_stride[src];
+  const int k0 = q * KQ, p0 = half * (HALF / C::CS) + lane;
+  float pe[B][NBL], po[B][NBL];
+  auto load_t = [&](int kb) {
+#pragma unroll
+    for (int u = 0; u < B; ++u)
+#pragma unroll
+      for (int i = 0; i < NBL; ++i) {
+        const int p = p0 + 32 * i, k = k0 + kb + u;
+        pe[u][i] = p < HALF ? __ldg(a.rot_even + k * HALF + p) : 0.f;
+        po[u][i] = p < HALF ? __ldg(a.rot_odd + k * HALF + p) : 0.f;
+      }
+  };
+  load_t(0);
+  if (tid < 16) s_b[tid] = tid < a.n_bounds[src] ? a.bounds[src][tid] : CUDART_INF_F;
+  else if (tid < 32) s_c[tid - 16] = tid - 16 < a.n_cents[src] ? a.cents[src][tid - 16] : 0.f;
+  float xv[XPL], ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < XPL; ++i) xv[i] = load_as_float(a.x[src], a.dtype, at + lane + 32 * i);
+#pragma unroll
+  for (int i = 0; i < XPL; ++i) ss = fmaf(xv[i], xv[i], ss);
+  const float norm = sqrtf(warp_sum(ss)), den = norm + 1e-10f;
+  if (tid < 32) {
+#pragma unroll
+    for (int i = 0; i < XPL; ++i) s_x[lane + 32 * i] = xv[i] / den;
+  }
+  __syncthreads();
+  {
+    float acc[2 * NBL] = {};
+#pragma unroll
+    for (int kb = 0; kb < KQ; kb += B) {
+      if (kb > 0) load_t(kb);
+#pragma unroll
+      for (int u = 0; u < B; ++u) {
+        const float xk = s_x[k0 + kb + u];
+#pragma unroll
+        for (int i = 0; i < NBL; ++i) {
+          acc[2 * i] = fmaf(xk, pe[u][i], acc[2 * i]);
+          acc[2 * i + 1] = fmaf(xk, po[u][i], acc[2 * i + 1]);
+        }
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < NBL; ++i)
+      if (p0 + 32 * i < HALF) *reinterpret_cast<float2*>(&s_part[q][2 * (p0 + 32 * i)]) = make_float2(acc[2 * i], acc[2 * i + 1]);
+  }
+  // the first rows of Pi are on their way while the indices are found
+  float pr[B][NJ];
+  const int j0 = half * (D / C::CS) + lane;
+  auto load_r = [&](int kb) {
+#pragma unroll
+    for (int u = 0; u < B; ++u)
+#pragma unroll
+      for (int i = 0; i < NJ; ++i) pr[u][i] = __ldg(a.rotation + (k0 + kb + u) * D + j0 + 32 * i);
+  };
+  if (a.dec[0] != nullptr) load_r(0);
+  __syncthreads();
+  for (int j = tid; j < D; j += C::THREADS) {
+    const float y = (s_part[0][j] + s_part[1][j]) + (s_part[2][j] + s_part[3][j]);
+    const int i = bucketize_sorted16(y, s_b);
+    s_i[j] = (uint8_t)i;
+    s_x[j] = s_c[i] * norm;
+  }
+  __syncthreads();
+  const int64_t row = (int64_t)bh * a.cap + a.offset + s;
+  if (a.nibble[src]) {
+    for (int i = tid; i < HALF; i += C::THREADS) a.idx[src][row * HALF + i] = (uint8_t)((s_i[2 * i] << 4) | s_i[2 * i + 1]);
+  } else {
+    for (int i = tid; i < D; i += C::THREADS) a.idx[src][row * D + i] = s_i[i];
+  }
+  if (tid == 0) a.norms[src][row] = norm;
+  if (a.dec[0] == nullptr) return;
+  float acc[NJ] = {};
+#pragma unroll
+  for (int kb = 0; kb < KQ; kb += B) {
+    if (kb > 0) load_r(kb);
+#pragma unroll
+    for (int u = 0; u < B; ++u) {
+      const float xk = s_x[k0 + kb + u];
+#pragma unroll
+      for (int i = 0; i < NJ; ++i) acc[i] = fmaf(xk, pr[u][i], acc[i]);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < NJ; ++i) s_part[q][j0 + 32 * i] = acc[i];
+  __syncthreads();
+  const int64_t o = ((int64_t)bh * a.dec_cap + a.dec_offset + s) * D;
+  for (int j = tid; j < D; j += C::THREADS)
+    store_from_float(a.dec[src], a.dtype, o + j, (s_part[0][j] + s_part[1][j]) + (s_part[2][j] + s_part[3][j]));
+}
+
 // acc[i][j] += (vectors 2 i, 2 i + 1 of the strip's entry) * ps[j]
 template <int D, int NJ, int VC>
 __device__ __forceinline__ void rank1(const float4* x, const float (&ps)[NJ], F2 (&acc)[VC / 2][NJ]) {
@@ -94,7 +210,8 @@ __device__ __forceinline__ void rank1(const float4* x, const float (&ps)[NJ], F2
   }
 }
 
-template <int D, int VC>
+// DONE: the vectors come compressed
+template <int D, int VC, bool DONE>
 __global__ void __launch_bounds__(256) cache_update_kernel(const UpdateArgs a) {
   using C = Cfg<D, VC>;
   constexpr int NJ = C::NJ, G = VC / 4, KC = C::KC, NCH = C::NCH, KQ = D / 4, XPL = D / 32;
@@ -125,7 +242,7 @@ __global__ void __launch_bounds__(256) cache_update_kernel(const UpdateArgs a) {
   const int per_src = a.batch * a.heads * a.n_new;
   const int chunks_src = (per_src + VC - 1) / VC, n_chunks = 2 * chunks_src;  // (a chunk holds vectors of one source)
   if (NCH == 1) {
-    stage_t(0);
+    if (!DONE) stage_t(0);
     stage(0);
   }
   __syncthreads();
@@ -142,6 +259,38 @@ __global__ void __launch_bounds__(256) cache_update_kernel(const UpdateArgs a) {
     float nrm[VC];
     int64_t at[VC];  // (b * heads + h) and token of the vector
     int tok[VC];
+    F2 acc[VC / 2][NJ];
+    if constexpr (DONE) {
+      static_assert(NJ == 4, "a lane's coordinates are two bytes");
+      __syncwarp();
+      float r[NJ][VC];
+#pragma unroll
+      for (int v = 0; v < VC; ++v) {
+        const int vec = v0 + v;
+        at[v] = -1;
+        tok[v] = 0;
+        uint32_t w = 0;
+        nrm[v] = 0.f;
+        if (act && vec < per_src) {
+          const int bh = vec / a.n_new, s = vec - bh * a.n_new, b = bh / a.heads, h = bh - b * a.heads;
+          at[v] = bh;
+          tok[v] = s;
+          const int64_t from = src * (int64_t)per_src + ((int64_t)b * a.n_new + s) * a.heads + h;
+          w = __ldg(reinterpret_cast<const uint16_t*>(a.packed + from * (D / 2)) + lane);
+          nrm[v] = __ldg(a.packed_norms + from);
+        }
+        // byte p = index 2 p << 4 | index 2 p + 1
+        *reinterpret_cast<uint32_t*>(gi + v * D + NJ * lane) = ((w >> 4) & 15u) | (w & 15u) << 8 | ((w >> 12) & 15u) << 16 | ((w >> 8) & 15u) << 24;
+        r[0][v] = s_c[src][(w >> 4) & 15] * nrm[v];
+        r[1][v] = s_c[src][w & 15] * nrm[v];
+        r[2][v] = s_c[src][(w >> 12) & 15] * nrm[v];
+        r[3][v] = s_c[src][(w >> 8) & 15] * nrm[v];
+      }
+#pragma unroll
+      for (int j = 0; j < NJ; ++j)
+#pragma unroll
+        for (int g = 0; g < G; ++g) gx[g * D + 32 * j + lane] = make_float4(r[j][4 * g], r[j][4 * g + 1], r[j][4 * g + 2], r[j][4 * g + 3]);
+    } else {
     {
       const void* p[VC];
 #pragma unroll
@@ -181,7 +330,7 @@ __global__ void __launch_bounds__(256) cache_update_kernel(const UpdateArgs a) {
       __syncwarp();
     }
     // ---- rotate: four quarter chains, (s0 + s1) + (s2 + s3) -------------------------------------------
-    F2 t[VC / 2][NJ], u[VC / 2][NJ], acc[VC / 2][NJ];
+    F2 t[VC / 2][NJ], u[VC / 2][NJ];
 #pragma unroll 1
     for (int q = 0; q < 4; ++q) {
       if (NCH > 1) {
@@ -224,6 +373,7 @@ __global__ void __launch_bounds__(256) cache_update_kernel(const UpdateArgs a) {
       }
 #pragma unroll
       for (int g = 0; g < G; ++g) gx[g * D + 32 * j + lane] = make_float4(r[4 * g], r[4 * g + 1], r[4 * g + 2], r[4 * g + 3]);
+    }
     }
     __syncwarp();
 #pragma unroll
@@ -287,36 +437,60 @@ __global__ void __launch_bounds__(256) cache_update_kernel(const UpdateArgs a) {
   }
 }
 
-template <int D, int VC>
+template <int D, int VC, bool DONE = false>
 int launch_update(const UpdateArgs& a, cudaStream_t st) {
   using C = Cfg<D, VC>;
-  if (!ensure_dynamic_smem<cache_update_kernel<D, VC>>((int)C::kSmem)) return TQ4_ERR_CUDA;
+  if (!ensure_dynamic_smem<cache_update_kernel<D, VC, DONE>>((int)C::kSmem)) return TQ4_ERR_CUDA;
   const int64_t chunks = 2 * (((int64_t)a.batch * a.heads * a.n_new + C::VC - 1) / C::VC);
   const int64_t most = sm_count();
-  cache_update_kernel<D, VC><<<(unsigned)(chunks < most ? chunks : most), 256, C::kSmem, st>>>(a);
+  cache_update_kernel<D, VC, DONE><<<(unsigned)(chunks < most ? chunks : most), 256, C::kSmem, st>>>(a);
   TQ4_CHECK_LAUNCH();
   return TQ4_OK;
 }
 
-// Eight vectors a warp (half the reads of Pi per FMA) once every warp of the GPU has that many
+// A block per vector up to kTinyUpdate vectors (B200, bf16; 16 vectors / 1024 / 3000, against four a warp: head_dim 64 3.5 / 4.4 /
+// 8.8 and 10.1 us, 96 4.4 / 6.6 / 14.7 and 14.0, 128 5.4 / 8.5 / 19 and 19, 256 8.7 / 27 / 68 and 65).  Eight vectors a warp
+// (half the reads of Pi per FMA) once every warp of the GPU has that many.
+constexpr int64_t kTinyUpdate = 2800;
 template <int D>
 int launch_update(const UpdateArgs& a, cudaStream_t st) {
+  const int64_t vectors = 2 * (int64_t)a.batch * a.heads * a.n_new;
+  if (vectors <= kTinyUpdate) {
+    cache_update_tiny_kernel<D><<<(unsigned)vectors, TinyCfg<D>::THREADS, 0, st>>>(a);
+    TQ4_CHECK_LAUNCH();
+    return TQ4_OK;
+  }
+  if constexpr (D == 128)
+    if (a.packed) return launch_update<D, 8, true>(a, st);
   if constexpr (D <= 128)
-    if (2 * (int64_t)a.batch * a.heads * a.n_new >= 64 * (int64_t)sm_count()) return launch_update<D, 8>(a, st);
+    if (vectors >= 64 * (int64_t)sm_count()) return launch_update<D, 8>(a, st);
   return launch_update<D, 4>(a, st);
+}
+
+// The writes that the tensor cores make (dispatch_compress, head_dim 128 above kSmallRows vectors a tensor) are made by them
+// here too: the indices are the same whichever call a vector arrives in, and half of the FMAs go away
+// (the generation named above: 486 -> 452 us, host time).
+bool compress_first(int batch, int heads, int n_new, int head_dim) {
+  return head_dim == 128 && (int64_t)batch * heads * n_new > kSmallRows;
 }
 
 }  // namespace
 }  // namespace tq4
 
+extern "C" size_t tq4_cache_update_scratch_bytes(int batch, int num_heads, int n_new, int head_dim) {
+  if (batch <= 0 || num_heads <= 0 || n_new <= 0 || !tq4::compress_first(batch, num_heads, n_new, head_dim)) return 0;
+  return (size_t)2 * batch * num_heads * n_new * (head_dim / 2 + sizeof(float));
+}
+
 extern "C" int tq4_cache_update(const void* key, const void* value, int dtype, int batch, int num_heads, int n_new,
                                 int head_dim, const int64_t* k_strides, const int64_t* v_strides,
-                                const float* rotation, const float* k_boundaries, int n_k_boundaries,
+                                const float* rotation, const float* rot_t_even, const float* rot_t_odd,
+                                const float* k_boundaries, int n_k_boundaries,
                                 const float* v_boundaries, int n_v_boundaries, const float* k_centroids,
                                 int n_k_centroids, const float* v_centroids, int n_v_centroids, int k_nibble,
                                 int v_nibble, uint8_t* k_idx, float* k_norms, uint8_t* v_idx, float* v_norms,
                                 int64_t capacity, int64_t offset, void* k_dec, void* v_dec, int64_t dec_capacity,
-                                int64_t dec_offset, void* stream) {
+                                int64_t dec_offset, void* scratch, size_t scratch_bytes, void* stream) {
   using namespace tq4;
   if (batch < 0 || num_heads <= 0 || n_new < 0 || offset < 0 || dec_offset < 0) return TQ4_ERR_INVALID_ARG;
   if (!supported_head_dim(head_dim) || dtype < 0 || dtype > 2) return TQ4_ERR_UNSUPPORTED;
@@ -324,10 +498,10 @@ extern "C" int tq4_cache_update(const void* key, const void* value, int dtype, i
       n_k_centroids <= 0 || n_k_centroids > TQ4_MAX_CENTROIDS || n_v_centroids <= 0 || n_v_centroids > TQ4_MAX_CENTROIDS)
     return TQ4_ERR_UNSUPPORTED;
   if (batch == 0 || n_new == 0) return TQ4_OK;
-  if (!key || !value || !k_strides || !v_strides || !rotation || !k_boundaries || !v_boundaries || !k_centroids || !v_centroids ||
+  if (!key || !value || !k_strides || !v_strides || !rotation || !rot_t_even || !rot_t_odd || !k_boundaries || !v_boundaries || !k_centroids || !v_centroids ||
       !k_idx || !k_norms || !v_idx || !v_norms || (k_dec == nullptr) != (v_dec == nullptr))
     return TQ4_ERR_INVALID_ARG;
-  if (((uintptr_t)rotation & 15) || ((uintptr_t)k_idx & 3) || ((uintptr_t)v_idx & 3) || offset + n_new > capacity ||
+  if ((((uintptr_t)rotation | (uintptr_t)rot_t_even | (uintptr_t)rot_t_odd) & 15) || ((uintptr_t)k_idx & 3) || ((uintptr_t)v_idx & 3) || offset + n_new > capacity ||
       (k_dec && dec_offset + n_new > dec_capacity) || (int64_t)batch * num_heads * n_new > 0x3fffffffll)
     return TQ4_ERR_INVALID_ARG;
   UpdateArgs a{};
@@ -351,6 +525,36 @@ extern "C" int tq4_cache_update(const void* key, const void* value, int dtype, i
   a.dec_cap = dec_capacity; a.dec_offset = dec_offset;
   a.batch = batch; a.heads = num_heads; a.n_new = n_new; a.dtype = dtype;
   a.rotation = rotation;
+  a.rot_even = rot_t_even;
+  a.rot_odd = rot_t_odd;
+  if (compress_first(batch, num_heads, n_new, head_dim)) {
+    if (!scratch || ((uintptr_t)scratch & 15) || scratch_bytes < tq4_cache_update_scratch_bytes(batch, num_heads, n_new, head_dim))
+      return TQ4_ERR_WORKSPACE;
+    const int64_t vectors = 2 * (int64_t)batch * num_heads * n_new;
+    CompressArgs c{};
+    for (int i = 0; i < 2; ++i) {
+      c.x[i] = a.x[i];
+      c.batch_stride[i] = a.batch_stride[i];
+      c.head_stride[i] = a.head_stride[i];
+      c.token_stride[i] = a.token_stride[i];
+      c.bounds[i] = a.bounds[i];
+      c.n_bounds[i] = a.n_bounds[i];
+    }
+    c.n_tokens = (int64_t)batch * n_new;
+    c.num_heads = num_heads;
+    c.n_sources = 2;
+    c.x_dtype = dtype;
+    c.rot_even = rot_t_even;
+    c.rot_odd = rot_t_odd;
+    c.seq = n_new;
+    for (int i = 0; n_new == 1 && i < 2; ++i) c.token_stride[i] = c.batch_stride[i];  // the sequences are the tokens
+    c.norms_out = (float*)scratch;  // (the norms first: a multiple of four bytes each)
+    c.packed_out = (uint8_t*)scratch + vectors * sizeof(float);
+    const int rc = dispatch_compress(c, head_dim, dtype, (cudaStream_t)stream);
+    if (rc != TQ4_OK) return rc;
+    a.packed = c.packed_out;
+    a.packed_norms = c.norms_out;
+  }
   switch (head_dim) {
     case 64: return launch_update<64>(a, (cudaStream_t)stream);
     case 96: return launch_update<96>(a, (cudaStream_t)stream);

@@ -373,19 +373,20 @@ PyObject* append_rows(PyObject*, PyObject* const* p, Py_ssize_t n) {
   });
 }
 
-// cache_update(key, value, rotation, k_boundaries, v_boundaries, k_centroids, v_centroids, k_nibble, v_nibble,
+// cache_update(key, value, rotation, rotation_T_even, rotation_T_odd, k_boundaries, v_boundaries, k_centroids, v_centroids, k_nibble, v_nibble,
 //              k_idx, k_norms, v_idx, v_norms, offset, k_dec, v_dec, dec_offset)
 PyObject* cache_update(PyObject*, PyObject* const* p, Py_ssize_t n) {
-  if (!expect("cache_update", n, 17)) return nullptr;
+  if (!expect("cache_update", n, 19)) return nullptr;
   return guarded([&]() -> PyObject* {
     const States k(p[0], "key"), v(p[1], "value");
     const at::Tensor& rot = cuda_tensor(p[2], "rotation");
-    const at::Tensor &kb = cuda_tensor(p[3], "k_boundaries"), &vb = cuda_tensor(p[4], "v_boundaries");
-    const at::Tensor &kc = cuda_tensor(p[5], "k_centroids"), &vc = cuda_tensor(p[6], "v_centroids");
-    const int k_nib = truth(p[7]), v_nib = truth(p[8]);
-    const at::Tensor &ki = cuda_tensor(p[9], "k_idx"), &kn = cuda_tensor(p[10], "k_norms");
-    const at::Tensor &vi = cuda_tensor(p[11], "v_idx"), &vn = cuda_tensor(p[12], "v_norms");
-    const int64_t offset = as_int(p[13]), dec_offset = as_int(p[16]);
+    const at::Tensor &even = cuda_tensor(p[3], "rotation_T_even"), &odd = cuda_tensor(p[4], "rotation_T_odd");
+    const at::Tensor &kb = cuda_tensor(p[5], "k_boundaries"), &vb = cuda_tensor(p[6], "v_boundaries");
+    const at::Tensor &kc = cuda_tensor(p[7], "k_centroids"), &vc = cuda_tensor(p[8], "v_centroids");
+    const int k_nib = truth(p[9]), v_nib = truth(p[10]);
+    const at::Tensor &ki = cuda_tensor(p[11], "k_idx"), &kn = cuda_tensor(p[12], "k_norms");
+    const at::Tensor &vi = cuda_tensor(p[13], "v_idx"), &vn = cuda_tensor(p[14], "v_norms");
+    const int64_t offset = as_int(p[15]), dec_offset = as_int(p[18]);
     TQ4_ASSERT(k.t.sizes() == v.t.sizes() && k.t.scalar_type() == v.t.scalar_type(), "key and value must be alike");
     const int64_t b = k.t.size(0), h = k.t.size(1), d = k.t.size(3);
     auto buffer = [&](const at::Tensor& t, int64_t width, at::ScalarType type) {
@@ -398,8 +399,8 @@ PyObject* cache_update(PyObject*, PyObject* const* p, Py_ssize_t n) {
                "index and norm buffers must have one capacity");
     void *kd = nullptr, *vd = nullptr;
     int64_t dec_cap = 0;
-    if (p[14] != Py_None) {
-      const at::Tensor &a = cuda_tensor(p[14], "k_dec"), &c = cuda_tensor(p[15], "v_dec");
+    if (p[16] != Py_None) {
+      const at::Tensor &a = cuda_tensor(p[16], "k_dec"), &c = cuda_tensor(p[17], "v_dec");
       dec_cap = buffer(a, d, k.t.scalar_type());
       TQ4_ASSERT(buffer(c, d, k.t.scalar_type()) == dec_cap, "the two dequantised buffers must have one capacity");
       kd = a.data_ptr();
@@ -407,14 +408,18 @@ PyObject* cache_update(PyObject*, PyObject* const* p, Py_ssize_t n) {
     }
     const int dt = dtype_code(k.t.scalar_type());
     Launch launch(device_index(k.t));
+    const size_t need = tq4_cache_update_scratch_bytes((int)b, (int)h, (int)k.t.size(2), (int)d);
+    at::Tensor scratch;
+    if (need) scratch = at::empty({(int64_t)need}, k.t.options().dtype(at::kByte).requires_grad(false));
     int st;
     Py_BEGIN_ALLOW_THREADS
     st = tq4_cache_update(k.t.data_ptr(), v.t.data_ptr(), dt, (int)b, (int)h, (int)k.t.size(2), (int)d, k.strides, v.strides,
-                          (const float*)rot.data_ptr(), (const float*)kb.data_ptr(), (int)kb.numel(),
+                          (const float*)rot.data_ptr(), (const float*)even.data_ptr(), (const float*)odd.data_ptr(),
+                          (const float*)kb.data_ptr(), (int)kb.numel(),
                           (const float*)vb.data_ptr(), (int)vb.numel(), (const float*)kc.data_ptr(), (int)kc.numel(),
                           (const float*)vc.data_ptr(), (int)vc.numel(), k_nib, v_nib, (uint8_t*)ki.data_ptr(),
                           (float*)kn.data_ptr(), (uint8_t*)vi.data_ptr(), (float*)vn.data_ptr(), cap, offset, kd, vd, dec_cap,
-                          dec_offset, launch.stream);
+                          dec_offset, need ? scratch.data_ptr() : nullptr, need, launch.stream);
     Py_END_ALLOW_THREADS
     check(st, "tq4_cache_update");
     Py_RETURN_NONE;

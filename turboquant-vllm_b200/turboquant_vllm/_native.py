@@ -44,9 +44,10 @@ _SIGNATURES = {
                                 c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p,
                                 c_int64, c_int64, c_int64, c_void_p]),
     "tq4_cache_update": (c_int, [c_void_p, c_void_p, c_int, c_int, c_int, c_int, c_int, c_void_p, c_void_p, c_void_p,
-                                 c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int,
+                                 c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_void_p, c_int, c_int, c_int,
                                  c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_void_p, c_void_p,
-                                 c_int64, c_int64, c_void_p]),
+                                 c_int64, c_int64, c_void_p, c_size_t, c_void_p]),
+    "tq4_cache_update_scratch_bytes": (c_size_t, [c_int, c_int, c_int, c_int]),
     "tq4_decompress_rows": (c_int, [c_void_p, c_void_p, c_void_p, c_int, c_int64, c_int,
                                     c_void_p, c_int, c_void_p]),
     "tq4_decompress_cache": (c_int, [c_void_p, c_int64, c_int64, c_int, c_int, c_void_p, c_int,

@@ -245,7 +245,7 @@ def paged_tq4_attention(
     ``query_start_loc=None``: decode, row i is the one new token of sequence i.  Otherwise
     int32 ``[num_seqs + 1]`` offsets of each sequence's query chunk (bottom-right aligned
     causal mask).  ``mode``: 0 auto, 1 fp32 CUDA-core kernel, 2 streaming tensor-core LUT kernel,
-    3 chunked-prefill tcgen05 kernel (head_dim 128 only), 4 the same with single fp16 terms for
+    3 chunked-prefill tcgen05 kernel, 4 the same with single fp16 terms for
     queries and probabilities (faster, about 1e-3 absolute error; never picked automatically).
     """
     return nv.host().attention(
@@ -275,7 +275,9 @@ def tq4_write_and_attention(
 ) -> torch.Tensor:
     """One decode step of a layer: :func:`tq4_write_paged` of the new tokens, then
     :func:`paged_tq4_attention`, in three launches: the cache write rides in the kernel that rotates
-    the queries and plans the tiles.  The results equal the two calls in sequence bit for bit.  (With
+    the queries and plans the tiles.  The results equal the two calls in sequence bit for bit while the
+    write is small enough for the FMA kernels (6500 / 3000 / 8192 / 1000 vectors at head_dim 64 / 96 / 128 / 256;
+    above that a stand-alone write rotates on the tensor cores, within the write path's bound).  (With
     ``TQ4_FUSED_PROLOGUE=1`` that work happens inside the attention kernel: two launches, token i must be
     the newest token of sequence i, the norms are equal and the indices agree within the write path's
     1e-4 bound.)"""

@@ -369,7 +369,7 @@ class CompressedDynamicCache:
         b, h, n, d = key_states.shape
         if n == 0 or d not in _UPDATE_DIMS or k_quant.bits > 4 or v_quant.bits > 4:
             return False
-        rot, _, _, k_cents, k_bounds = k_quant.device_primitives(dev)
+        rot, even, odd, k_cents, k_bounds = k_quant.device_primitives(dev)
         v_rot, _, _, v_cents, v_bounds = v_quant.device_primitives(dev)
         if rot is not v_rot:
             return False
@@ -386,7 +386,7 @@ class CompressedDynamicCache:
                 bufs.append((g, w, t))
         out = [g.reserve(b, h, n, w, t, dev) for g, w, t in bufs]
         nv.host().cache_update(
-            key_states, value_states, rot, k_bounds, v_bounds, k_cents, v_cents, self._k_nibble_packed,
+            key_states, value_states, rot, even, odd, k_bounds, v_bounds, k_cents, v_cents, self._k_nibble_packed,
             self._v_nibble_packed, *out[:4], store[0].len, *(out[4:] or (None, None)), dec[0].len if dec else 0)
         for g, _, _ in bufs:
             g.len += n
