@@ -47,9 +47,8 @@ FALLBACK_HBM_GBS = 6650.0
 # the N = 1 workload.  A STORED figure from an ncu capture (the timed run cannot measure DRAM
 # traffic): it is reported together with the name of the capture it comes from and only while the
 # kernel build named there is the one that runs; otherwise `traffic` is null.
-NCU_TRAFFIC = {"bytes": 308781824,  # dram__bytes_read.sum 304 016 384 + dram__bytes_write.sum 4 765 440
-               "capture": "profiles/attention_mma_kernel_b64_ctx4096_ncu_full.md (form A: attention kernel "
-                          "behind the prologue kernel, one launch, ncu --set full)"}
+NCU_TRAFFIC = {"bytes": 310690560,  # dram__bytes_read.sum 304 323 328 + dram__bytes_write.sum 6 367 232
+               "capture": "profiles/kernels_ncu.md (attention kernel behind the prologue kernel, one launch)"}
 
 
 def measured_peak_gbs():
