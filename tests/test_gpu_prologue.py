@@ -30,6 +30,9 @@ def test_step_writes_and_rotates(cuda_lib, d, rows):
         q.cuda(), cache, bt.cuda(), case["seq_lens"].cuda(), p["kc"], p["vc"], p["rot"], hkv, bs,
         out_dtype=torch.float32, write=(k, v, slots.cuda(), p["even"], p["odd"], p["kb"], p["vb"]))
     assert torch.equal(cache, want)
+    alone = ops.paged_tq4_attention(  # without a write: the queries of few rows are rotated from Pi itself
+        q.cuda(), want, bt.cuda(), case["seq_lens"].cuda(), p["kc"], p["vc"], p["rot"], hkv, bs, out_dtype=torch.float32)
+    assert torch.equal(alone, out)
     pick = sorted({0, rows // 2, rows - 1})
     ref = O.paged_decode_fp32(q[pick], want.cpu(), bt[pick], [lens[i] for i in pick], pr.kc, pr.vc, pr.rot, hkv)
     got = out.cpu()[pick]

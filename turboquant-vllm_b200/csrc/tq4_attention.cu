@@ -444,7 +444,9 @@ prologue_kernel(const AttnArgs a, const CompressArgs w, const int has_attn, cons
 // The same for a step of a few vectors: a block of four warps per vector, each warp one quarter of the
 // reduction with Pi^T read straight from L1 / L2 (the caller's even / odd halves), as the write kernel for few vectors does.
 // No staging, half the code: latency is all that counts here.
-template <int D>
+// Q_ONLY: no write, so no Pi^T from the caller: a lane reads the rows of Pi of its two coordinates, a 128-byte line of each at a
+// time (the same bytes, four k a load; the sums are the same).
+template <int D, bool Q_ONLY>
 __global__ void __launch_bounds__(128) tiny_prologue_kernel(const AttnArgs a, const CompressArgs w) {
   constexpr int HALF = D / 2, NBL = (HALF + 31) / 32, XPL = D / 32, KQ = D / 4;
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -458,7 +460,7 @@ __global__ void __launch_bounds__(128) tiny_prologue_kernel(const AttnArgs a, co
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int n_q = a.sh.rows * a.sh.Hq, vec = (int)blockIdx.x - 1;
-  const bool is_w = vec >= n_q;
+  const bool is_w = !Q_ONLY && vec >= n_q;
   int src = 0, tok = 0, h = 0;
   int64_t slot = -1, at;
   const void* x;
@@ -504,14 +506,30 @@ __global__ void __launch_bounds__(128) tiny_prologue_kernel(const AttnArgs a, co
   for (int i = 0; i < 2 * NBL; ++i) acc[i] = 0.f;
   for (int kb = 0; kb < KQ; kb += 8) {  // eight k-steps of Pi^T in flight before the first FMA of the batch
     float pe[8][NBL], po[8][NBL];
-#pragma unroll
-    for (int u = 0; u < 8; ++u)
+    if constexpr (Q_ONLY) {
 #pragma unroll
       for (int i = 0; i < NBL; ++i) {
-        const int p = lane + 32 * i, k = warp * KQ + kb + u;
-        pe[u][i] = p < HALF ? __ldg(w.rot_even + k * HALF + p) : 0.f;
-        po[u][i] = p < HALF ? __ldg(w.rot_odd + k * HALF + p) : 0.f;
+        const int p = lane + 32 * i;
+#pragma unroll
+        for (int u = 0; u < 8; u += 4) {
+          const float* row = a.rotation + 2 * p * D + warp * KQ + kb + u;
+          const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
+          const float4 e = p < HALF ? __ldg(reinterpret_cast<const float4*>(row)) : z;
+          const float4 o = p < HALF ? __ldg(reinterpret_cast<const float4*>(row + D)) : z;
+          pe[u][i] = e.x; pe[u + 1][i] = e.y; pe[u + 2][i] = e.z; pe[u + 3][i] = e.w;
+          po[u][i] = o.x; po[u + 1][i] = o.y; po[u + 2][i] = o.z; po[u + 3][i] = o.w;
+        }
       }
+    } else {
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+#pragma unroll
+        for (int i = 0; i < NBL; ++i) {
+          const int p = lane + 32 * i, k = warp * KQ + kb + u;
+          pe[u][i] = p < HALF ? __ldg(w.rot_even + k * HALF + p) : 0.f;
+          po[u][i] = p < HALF ? __ldg(w.rot_odd + k * HALF + p) : 0.f;
+        }
+    }
 #pragma unroll
     for (int u = 0; u < 8; ++u) {
       const float xk = s_x[warp * KQ + kb + u];
@@ -558,11 +576,11 @@ __global__ void __launch_bounds__(128) tiny_prologue_kernel(const AttnArgs a, co
 // gain shrinks as they grow in number.
 constexpr int64_t kTinyStep = 1024;
 
-template <int D>
+template <int D, bool Q_ONLY>
 int launch_tiny_prologue(const AttnArgs& a, const CompressArgs& w, int64_t vectors, cudaStream_t st) {
   const size_t smem = 2 * (size_t)a.sh.rows * sizeof(int);
   // (first kernel of an entry point: plain stream-ordered launch, see launch_prologue_jc)
-  if (launch_kernel(tiny_prologue_kernel<D>, dim3((unsigned)vectors + 1), dim3(128), smem, st, false, a, w) != cudaSuccess)
+  if (launch_kernel(tiny_prologue_kernel<D, Q_ONLY>, dim3((unsigned)vectors + 1), dim3(128), smem, st, false, a, w) != cudaSuccess)
     return TQ4_ERR_CUDA;
   TQ4_CHECK_LAUNCH();
   return TQ4_OK;
@@ -599,8 +617,12 @@ int launch_prologue_t(const AttnArgs* a, const CompressArgs* w, cudaStream_t st)
   const int64_t chunks = (n_q + VC - 1) / VC + (n_w + VC - 1) / VC;
   const int64_t blocks = (chunks + WARPS - 1) / WARPS;
   if constexpr (D <= 128)
-    if (a && w && w->cache && a->skip_long == 0 && n_q + n_w <= kTinyStep)
-      return launch_tiny_prologue<D>(*a, *w, n_q + n_w, st);
+    if (a && a->skip_long == 0) {
+      if (w && w->cache && n_w > 0 && n_q + n_w <= kTinyStep) return launch_tiny_prologue<D, false>(*a, *w, n_q + n_w, st);
+      // without Pi^T a block occupies its SM's load pipe for 2 us (rows of Pi across the lanes): one block an SM
+      // (32 vectors: a call 1.3 us shorter; 580: 13 us longer)
+      if (n_w == 0 && n_q <= sm_count()) return launch_tiny_prologue<D, true>(*a, CompressArgs{}, n_q, st);
+    }
   const int64_t wave = 3 * (int64_t)sm_count() / (D / 32);
   if (blocks <= wave) return launch_prologue_jc<D, 32>(a, w, st, blocks);
   // a mixed call streams few of its rows (the kernel finds out how many)
