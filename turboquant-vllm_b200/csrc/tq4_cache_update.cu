@@ -10,7 +10,7 @@
 // it is; at head_dim 256, where that does not fit, in chunks of 64 rows) and the vectors from a strip per warp.
 // A step of a few tokens is latency bound (staging Pi: 128 KB per block), so its vectors are spread over the blocks
 // first; a prompt is bound by FMA issue.
-// Measured: a generation of 8 tokens behind 4 prompts of 1100, 2 layers of 8 heads of 128, 7800 -> 452 us.
+// Measured: a generation of 8 tokens behind 4 prompts of 1100, 2 layers of 8 heads of 128, 7800 -> 357 us.
 #include <math_constants.h>
 
 #include "tq4_common.cuh"
@@ -469,7 +469,7 @@ int launch_update(const UpdateArgs& a, cudaStream_t st) {
 
 // The writes that the tensor cores make (dispatch_compress, head_dim 128 above kSmallRows vectors a tensor) are made by them
 // here too: the indices are the same whichever call a vector arrives in, and half of the FMAs go away
-// (the generation named above: 486 -> 452 us, host time).
+// (the generation named above: 486 -> 452 us, then host time).
 bool compress_first(int batch, int heads, int n_new, int head_dim) {
   return head_dim == 128 && (int64_t)batch * heads * n_new > kSmallRows;
 }

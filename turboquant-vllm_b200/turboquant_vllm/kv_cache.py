@@ -58,6 +58,7 @@ class _GrowBuffer:
     def __init__(self) -> None:
         self.buf: torch.Tensor | None = None
         self.len = 0
+        self.fit = None  # (first buffer of a layer) what the last in-place update found to fit together
 
     def reserve(self, b: int, h: int, n: int, w: int, dtype: torch.dtype, device: torch.device) -> torch.Tensor:
         """The buffer with room for ``n`` more tokens of ``[b, h, ., w]``; a new one if it held another shape."""
@@ -82,7 +83,7 @@ class _GrowBuffer:
 
     def view(self) -> torch.Tensor:
         assert self.buf is not None
-        return self.buf[:, :, : self.len]
+        return self.buf.narrow(2, 0, self.len)
 
 
 class _RowsField:
@@ -367,6 +368,22 @@ class CompressedDynamicCache:
                 or dev != value_states.device or not key_states.is_cuda or dtype not in _UPDATE_DTYPES):
             return False
         b, h, n, d = key_states.shape
+        groups, first = store + dec, store[0]
+        fit = first.fit
+        if fit is not None and n and fit[0] == (b, h, d, dtype, dev, k_quant, v_quant, len(dec)):
+            # the buffers of the update before, with room for this one
+            _, prims, out = fit
+            held, at = first.len, dec[0].len if dec else 0
+            if held + n <= out[0].shape[2] and (not dec or at + n <= out[4].shape[2]):
+                for g, t, want in zip(groups, out, (held, held, held, held, at, at)):
+                    if g.buf is not t or g.len != want:
+                        break
+                else:
+                    nv.host().cache_update(key_states, value_states, *prims, self._k_nibble_packed, self._v_nibble_packed,
+                                           *out[:4], held, *(out[4:] or (None, None)), at)
+                    for g in groups:
+                        g.len += n
+                    return True
         if n == 0 or d not in _UPDATE_DIMS or k_quant.bits > 4 or v_quant.bits > 4:
             return False
         rot, even, odd, k_cents, k_bounds = k_quant.device_primitives(dev)
@@ -385,9 +402,11 @@ class CompressedDynamicCache:
                     return False
                 bufs.append((g, w, t))
         out = [g.reserve(b, h, n, w, t, dev) for g, w, t in bufs]
+        prims = (rot, even, odd, k_bounds, v_bounds, k_cents, v_cents)
         nv.host().cache_update(
-            key_states, value_states, rot, even, odd, k_bounds, v_bounds, k_cents, v_cents, self._k_nibble_packed,
-            self._v_nibble_packed, *out[:4], store[0].len, *(out[4:] or (None, None)), dec[0].len if dec else 0)
+            key_states, value_states, *prims, self._k_nibble_packed, self._v_nibble_packed, *out[:4], store[0].len,
+            *(out[4:] or (None, None)), dec[0].len if dec else 0)
+        store[0].fit = ((b, h, d, dtype, dev, k_quant, v_quant, len(dec)), prims, out)
         for g, _, _ in bufs:
             g.len += n
         return True
