@@ -15,6 +15,8 @@ CASES = [  # head_dim, q heads, KV heads, lengths, new rows, mode, window, causa
     (128, 28, 4, [150], [150], 3, None, True, True),         # groups of 7: 126 of 128 lanes
     (128, 8, 4, [65], [65], 3, None, True, True),            # one key in the second tile
     (128, 32, 8, [3000], [40], 3, None, True, True),         # cut along the keys
+    (128, 32, 8, [3000, 0, 20], [8, 8, 8], 3, None, True, True),  # ... parts without keys, a sequence without any
+    (256, 8, 4, [2000, 0, 20], [8, 8, 8], 3, None, True, True),
     (128, 4, 1, [700], [333], 3, None, False, False),        # 136-byte rows: 4-byte loads; not causal
     (64, 14, 2, [333], [200], 3, None, True, True),
     (96, 4, 4, [300, 41], [100, 9], 3, None, True, False),

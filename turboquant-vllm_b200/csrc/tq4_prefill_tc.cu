@@ -32,7 +32,9 @@
 //
 // A block with few CTAs is cut along the keys (gridDim.z): each part leaves its normalised rotated rows and
 // their log-sum-exp in the scratch, and the merge kernel folds and un-rotates them.
-// Every wait is bounded; a wait that gives up marks the CTA dead, all roles drain, TQ4_DEV_TIMEOUT is raised.
+// Every wait is bounded; a wait that gives up marks the CTA dead, all roles drain, TQ4_DEV_TIMEOUT is raised.  On
+// every way out, the empty key parts' and the dead CTA's among them, a CTA first waits for the copies and MMAs it
+// issued: they work on its shared and tensor memory, which the next CTA of the SM is given.
 #include <math_constants.h>
 
 #include <cstdlib>
@@ -149,18 +151,28 @@ __device__ __forceinline__ void bar_init(uint32_t bar, uint32_t count) {
 __device__ __forceinline__ void bar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// Bounded wait that also gives up as soon as another role has marked the CTA dead; marks it itself otherwise.
+__device__ __forceinline__ bool bar_try(uint32_t bar, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(done) : "r"(bar), "r"(parity) : "memory");
+  return done != 0;
+}
+// Bounded wait for another role: also gives up as soon as the CTA is marked dead; marks it itself otherwise.
 __device__ __forceinline__ bool bar_wait(uint32_t bar, uint32_t parity, volatile int* dead) {
   for (int it = 0; it < (1 << 22); ++it) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done) : "r"(bar), "r"(parity) : "memory");
-    if (done) return true;
+    if (bar_try(bar, parity)) return true;
     if ((it & 1023) == 1023 && *dead) return false;
   }
+  *dead = 1;
+  return false;
+}
+// Bounded wait for copies or MMAs in flight, which no other role can hold up: a dead CTA sees them home, too.
+__device__ __forceinline__ bool bar_wait_own(uint32_t bar, uint32_t parity, volatile int* dead) {
+  for (int it = 0; it < (1 << 22); ++it)
+    if (bar_try(bar, parity)) return true;
   *dead = 1;
   return false;
 }
@@ -397,6 +409,7 @@ struct Bars {
   uint64_t pair[4];               // the two warps of a row quadrant (head_dim 256)
   uint64_t qraw;                  // raw query rows landed
   uint64_t qready, odone;         // queries in place / last MMA of the tile loop complete
+  uint64_t drain;                 // a dead CTA's last MMA complete
 };
 
 template <int D, bool FAST>
@@ -471,6 +484,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
     bar_init(bar(s_bars.qraw), kSmx);
     bar_init(bar(s_bars.qready), 8);
     bar_init(bar(s_bars.odone), 1);
+    bar_init(bar(s_bars.drain), 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     fence_async();
   }
@@ -555,11 +569,12 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
       // 256: the K~ buffer and the tables), which are free before the last values have been multiplied
       const uint32_t img = base + C::kOffK;
       const uint32_t uhi = base + (D == 256 ? C::kOffK : C::kOffLut), ulo = D == 256 ? base + C::kOffLut : uhi + C::kImg / 2;
-      uint32_t img_ph = 0, c_ph = 0;
+      uint32_t img_ph = 0, img_n = 0, c_ph = 0;  // image chunks waited for / asked for
       bool ok = true;
       const bool unrotate = !pa.to_parts && !a.out_rotated;
       // chunk ch of the image, as rows (rotation) or as column blocks (un-rotation)
       auto load_chunk = [&](int ch, bool unrot) {
+        ++img_n;
         expect_tx(bar(s_bars.img), C::kImg);
         if (C::kChunks == 1) {
           bulk_load(unrot ? uhi : img, pa.image, C::kImg, bar(s_bars.img));
@@ -574,7 +589,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
       // O = A * B for the blocks in use: A = fp16 hi (and lo) terms at the S and Q columns, B = the image
       auto rotate = [&](bool unrot, bool a_lo) {
         for (int ch = 0; ch < C::kChunks && ok; ++ch) {
-          ok = bar_wait(bar(s_bars.img), img_ph & 1, dead);
+          ok = bar_wait_own(bar(s_bars.img), img_ph & 1, dead);
           ++img_ph;
           if (ch == 0) {
             ok = bar_wait(bar(s_bars.aready), unrot ? 1u : 0u, dead) && ok;
@@ -699,6 +714,11 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
       if (ok) {
         mma_commit(bar(s_bars.odone));
         if (unrotate) rotate(true, true);
+      }
+      if (!ok) {  // (the CTA is dead)
+        if (img_n != img_ph) bar_wait_own(bar(s_bars.img), img_ph & 1, dead);
+        mma_commit(bar(s_bars.drain));
+        bar_wait_own(bar(s_bars.drain), 0u, dead);
       }
     }
     __syncwarp();
@@ -889,12 +909,13 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
     };
     bool ok = true;
     const bool use = n_tiles > 0 && blk < n_blk;  // (uniform per warp)
+    // the raw queries, for every live row of the CTA: waited for whether this part has keys or not
+    if (q_staged && (use || n_tiles == 0)) ok = bar_wait_own(bar(s_bars.qraw), 0u, dead);
 
     // ---- rotate the queries -----------------------------------------------------------------------
     float qscale = 0.f;
     if (use) {
       // (code that runs once per CTA costs its instruction fetches: short rolled loops)
-      if (q_staged) ok = bar_wait(bar(s_bars.qraw), 0u, dead);
       auto load_q = [&](int c, float (&x)[32]) {
         if (!live) {
 #pragma unroll
