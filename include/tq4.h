@@ -207,7 +207,8 @@ size_t tq4_attention_workspace_bytes(int64_t max_query_rows, int num_q_heads, in
  *              cores as single fp16 terms (mode 3 splits both into hi + lo), which halves the
  *              tensor work and lets their 2^-11 rounding reach the output (about 1e-3 absolute:
  *              at the edge of the 2e-3 parity bound, hence never chosen by mode 0)
- * A row that sees no key (seq_len 0) gets zeros.
+ * A row that sees no key (seq_len 0) gets zeros, and so does a row past the last offset of
+ * query_start_loc, which belongs to no sequence.
  */
 int tq4_paged_attention(const void* q, int q_dtype, int64_t num_rows, int num_seqs,
                         int num_q_heads, int num_kv_heads, int head_dim,

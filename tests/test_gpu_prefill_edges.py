@@ -50,6 +50,34 @@ def test_prefill_edges(cuda_lib, d, hq, hkv, lens, new, mode, window, causal, pa
     assert ops.read_and_clear_errors(torch.device("cuda")) == 0
 
 
+@pytest.mark.parametrize("d,hq,hkv,lens,new,rows,mode", [
+    (128, 8, 2, [300, 90], [120, 90], 211, 3),     # one row past the last offset
+    (128, 32, 8, [3000, 50], [40, 9], 300, 3),     # many, the call cut along the keys
+    (256, 8, 4, [300], [20], 300, 3),
+    (64, 14, 2, [400], [400], 600, 0),             # one long sequence: the prefill kernel alone
+    (128, 32, 8, [300, 90], [120, 1], 300, 0),     # both kernels
+    (128, 32, 8, [300, 90], [120, 1], 300, 2),
+])
+def test_rows_of_no_sequence_are_zero(cuda_lib, d, hq, hkv, lens, new, rows, mode):
+    """Rows past the last offset of query_start_loc: zeros and an LSE of -inf, whichever kernel the call takes."""
+    from turboquant_vllm.kernels import ops
+
+    pr = Prims(d)
+    p = pr.cuda()
+    case = build_paged_case(lens, hkv, d, 16, pr, seed=5, padded=True)
+    q = torch.randn(rows, hq, d, generator=torch.Generator().manual_seed(1)).bfloat16().cuda()
+    qsl = torch.tensor(np.concatenate([[0], np.cumsum(new)]), dtype=torch.int32).cuda()
+    n = sum(new)
+    args = (case["cache"].cuda(), case["block_table"].cuda(), case["seq_lens"].cuda(), p["kc"], p["vc"], p["rot"], hkv, 16)
+    ws = torch.full((ops.attention_workspace_bytes(rows, hq, hkv, d),), 0x7f, dtype=torch.uint8, device="cuda")
+    for rotated in (False, True):
+        out, lse = torch.full((rows, hq, d), 7.0, device="cuda"), torch.full((rows, hq), 7.0, device="cuda")
+        ops.paged_tq4_attention(q, *args, query_start_loc=qsl, mode=mode, out=out, lse_out=lse, out_rotated=rotated, workspace=ws)
+        assert (out[n:] == 0).all() and (lse[n:] == float("-inf")).all()
+        want = ops.paged_tq4_attention(q[:n], *args, query_start_loc=qsl, mode=2, out_dtype=torch.float32, out_rotated=rotated)
+        assert (out[:n] - want).abs().max() <= 2e-3 and torch.isfinite(lse[:n]).all()
+
+
 def test_prefill_hides_and_reports_bad_pages(cuda_lib):
     from turboquant_vllm import _native as nv
     from turboquant_vllm.kernels import ops

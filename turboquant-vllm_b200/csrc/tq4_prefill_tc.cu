@@ -419,7 +419,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   __shared__ __align__(8) Bars s_bars;
   __shared__ uint32_t s_tmem;
-  __shared__ int s_info[4];      // sequence, first row, rows, - of the CTA
+  __shared__ int s_info[3];      // sequence, first row and rows of the CTA
   __shared__ int s_dead, s_bad;  // a wait gave up / some page id is out of range
   const AttnShape& sh = a.sh;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -460,8 +460,8 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
     }
     if (lane == 0) {
       s_info[0] = found;
-      s_info[1] = first;
-      s_info[2] = nrows;
+      s_info[1] = found < 0 ? (int)blockIdx.x - acc : first;  // (without rows: which of the spare CTAs, and how many)
+      s_info[2] = found < 0 ? (int)gridDim.x - acc : nrows;
       s_dead = 0;
       s_bad = 0;
     }
@@ -490,9 +490,25 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
   }
   __syncthreads();
   const int seq = s_info[0], row0 = s_info[1], nrows = s_info[2];
-  if (seq < 0) {  // the grid is an upper bound
+  if (seq < 0) {  // the grid is an upper bound: ceil(rows / per CTA) + sequences, so at least one CTA is spare
     pdl_trigger();
     pdl_wait();
+    // Rows past the last offset belong to no sequence and see no key: zeros, as the streaming kernel writes.  (In a
+    // call of both kernels they are the streaming kernel's.)
+    const int tail = min(max(a.query_start_loc[sh.num_seqs], 0), sh.rows);
+    if (pa.min_rows <= 1) {
+      const float zero[4] = {0.f, 0.f, 0.f, 0.f};
+      for (int r = tail + row0; r < sh.rows; r += nrows) {
+        for (int i = tid; i < G * (D / 4); i += kThreads) {
+          const int h = kvh * G + i / (D / 4), d = 4 * (i % (D / 4));
+          if (!pa.to_parts)
+            store4(a.out, a.out_dtype, (int64_t)r * a.out_token_stride + (int64_t)h * a.out_head_stride + d, zero);
+          if (d > 0) continue;
+          if (pa.to_parts) pa.part_m[((int64_t)blockIdx.z * sh.rows + r) * sh.Hq + h] = -CUDART_INF_F;
+          else if (a.lse_out) a.lse_out[(int64_t)r * sh.Hq + h] = -CUDART_INF_F;
+        }
+      }
+    }
     return;
   }
   // ---- row of a softmax thread (half a row at head_dim 256), and its raw query on the way -------------------
