@@ -504,3 +504,30 @@ def test_prefill_head_dim_256_sliding_window(ops, mode):
                num_kv_heads=hkv, block_size=bs, query_start_loc=qsl.cuda(), causal=True, sliding_window=64,
                out_dtype=torch.float32)
     _check(out, ref)
+
+
+@pytest.mark.parametrize("window", [None, False, 0, 40, 40.0, 40.9, np.float32(40), torch.tensor(40)])
+def test_sliding_window_is_what_int_takes(ops, window):
+    """None, False and 0 are no window; a float or a scalar of a library counts as its integer part."""
+    pr = Prims(128)
+    p = pr.cuda()
+    case = build_paged_case([90, 33], 2, 128, 16, pr, seed=2)
+    q = torch.randn(2, 8, 128, generator=torch.Generator().manual_seed(3)).cuda()
+    args = (q, case["cache"].cuda(), case["block_table"].cuda(), case["seq_lens"].cuda(), p["kc"], p["vc"], p["rot"], 2, 16)
+    want = ops.paged_tq4_attention(*args, sliding_window=int(window or 0))
+    assert torch.equal(ops.paged_tq4_attention(*args, sliding_window=window), want)
+
+
+def test_write_takes_any_iterable_of_seven(ops):
+    pr = Prims(128)
+    p = pr.cuda()
+    case = build_paged_case([90, 33], 2, 128, 16, pr, seed=2)
+    q = torch.randn(2, 8, 128, generator=torch.Generator().manual_seed(3)).cuda()
+    kv = torch.randn(2, 2, 128, generator=torch.Generator().manual_seed(4)).cuda()
+    slots = case["slot_mapping"][[89, 122]].cuda()
+    write = (kv, kv + 1, slots, p["even"], p["odd"], p["kb"], p["vb"])
+    args = (case["block_table"].cuda(), case["seq_lens"].cuda(), p["kc"], p["vc"], p["rot"], 2, 16)
+    outs = [ops.paged_tq4_attention(q, case["cache"].cuda(), *args, write=w) for w in (write, list(write), iter(write))]
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+    with pytest.raises(ValueError):
+        ops.paged_tq4_attention(q, case["cache"].cuda(), *args, write=write[:6])

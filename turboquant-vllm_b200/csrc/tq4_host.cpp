@@ -62,6 +62,18 @@ int64_t as_int(PyObject* o) {
   if (v == -1 && PyErr_Occurred()) throw PyError{};
   return v;
 }
+// int(o or 0): None, False and 0 are "none", and whatever int() takes is taken (a float, a NumPy or tensor scalar)
+int64_t int_or_zero(PyObject* o) {
+  const int truthy = PyObject_IsTrue(o);
+  if (truthy < 0) throw PyError{};
+  if (!truthy) return 0;
+  PyObject* i = PyNumber_Long(o);
+  if (!i) throw PyError{};
+  const long long v = PyLong_AsLongLong(i);
+  Py_DECREF(i);
+  if (v == -1 && PyErr_Occurred()) throw PyError{};
+  return v;
+}
 double as_double(PyObject* o) {
   const double v = PyFloat_AsDouble(o);
   if (v == -1.0 && PyErr_Occurred()) throw PyError{};
@@ -201,7 +213,7 @@ PyObject* attention(PyObject*, PyObject* const* p, Py_ssize_t n) {
     const size_t have = (size_t)ws.numel() * ws.element_size();
     if (have < need)
       fail(PyExc_ValueError, "workspace has " + std::to_string(have) + " bytes, " + std::to_string(need) + " needed");
-    const int causal = truth(p[11]) ? 1 : 0, window = p[12] == Py_None ? 0 : (int)as_int(p[12]);
+    const int causal = truth(p[11]) ? 1 : 0, window = (int)int_or_zero(p[12]);
     const int rotated = truth(p[16]) ? 1 : 0, mode = (int)as_int(p[18]);
     int* flag = (int*)flag_of(dev).data_ptr();
     const int q_dt = dtype_code(q.scalar_type()), out_dt = dtype_code(out.scalar_type());
@@ -218,8 +230,14 @@ PyObject* attention(PyObject*, PyObject* const* p, Py_ssize_t n) {
           mode, flag, launch.stream);
       Py_END_ALLOW_THREADS
     } else {
-      TQ4_ASSERT(PyTuple_Check(p[19]) && PyTuple_GET_SIZE(p[19]) == 7, "write must be a tuple of seven tensors");
-      auto item = [&](int i, const char* name) -> const at::Tensor& { return cuda_tensor(PyTuple_GET_ITEM(p[19], i), name); };
+      // any iterable of seven, held until the call returns
+      struct Held {
+        PyObject* o;
+        ~Held() { Py_XDECREF(o); }
+      } seq{PySequence_Tuple(p[19])};
+      if (!seq.o) throw PyError{};
+      if (PyTuple_GET_SIZE(seq.o) != 7) fail(PyExc_ValueError, "write must hold seven tensors");
+      auto item = [&](int i, const char* name) -> const at::Tensor& { return cuda_tensor(PyTuple_GET_ITEM(seq.o, i), name); };
       at::Tensor key = item(0, "key"), value = item(1, "value");
       const at::Tensor slots = slots64(item(2, "slot_mapping"));
       const at::Tensor &even = item(3, "rotation_T_even"), &odd = item(4, "rotation_T_odd");
