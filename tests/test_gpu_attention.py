@@ -531,3 +531,67 @@ def test_write_takes_any_iterable_of_seven(ops):
     assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
     with pytest.raises(ValueError):
         ops.paged_tq4_attention(q, case["cache"].cuda(), *args, write=write[:6])
+
+
+def _scratch_case(seed, rows, lo, hi):
+    """A decode call without a workspace of its own, as a closure that returns its output."""
+    from turboquant_vllm.kernels import ops
+
+    pr = Prims(128)
+    p = pr.cuda()
+    lens = [lo + (hi - lo) * i // max(rows - 1, 1) for i in range(rows)]
+    nblk = -(-hi // 16)
+    gen = torch.Generator(device="cuda").manual_seed(seed)
+    cache = torch.randint(0, 256, (rows * nblk, 16, 8 * 136), dtype=torch.uint8, device="cuda", generator=gen)
+    for lo_b in (8 * 64, 8 * 132):  # norms
+        cache[..., lo_b : lo_b + 32] = torch.ones(8, device="cuda").view(torch.uint8)
+    bt = torch.randperm(rows * nblk, device="cuda", generator=gen).to(torch.int32).view(rows, nblk)
+    sl = torch.tensor(lens, dtype=torch.int32, device="cuda")
+    q = torch.randn(rows, 32, 128, device="cuda", generator=gen)
+    torch.cuda.synchronize()
+    return lambda: ops.paged_tq4_attention(q, cache, bt, sl, p["kc"], p["vc"], p["rot"], 8, 16)
+
+
+def test_scratch_is_not_shared_between_threads_or_streams(ops):
+    """Calls without a workspace from several threads and streams at a time, each growing its scratch."""
+    import threading
+
+    sizes = [(1, 40, 40), (3, 1, 900), (40, 5, 700), (7, 30, 3000), (150, 1, 300)]
+    calls = [[_scratch_case(10 * i + j, *s) for j, s in enumerate(sizes)] for i in range(6)]
+    want = [[c() for c in mine] for mine in calls]
+    torch.cuda.synchronize()
+    shared, bad = torch.cuda.Stream(), []
+
+    def work(i):
+        # six threads: two share a stream, and there are more of them than the scratch that is held
+        with torch.cuda.stream(shared if i < 2 else torch.cuda.Stream()):
+            for _ in range(15):
+                got = [c() for c in calls[i]]
+                torch.cuda.current_stream().synchronize()
+                if not all(torch.equal(a, b) for a, b in zip(got, want[i])):
+                    bad.append(i)
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(6)]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    assert not bad
+
+
+def test_captured_call_owns_its_scratch(ops):
+    """A captured call without a workspace: later calls, larger ones among them, leave its scratch alone."""
+    small, large = _scratch_case(1, 5, 10, 900), _scratch_case(2, 300, 1, 200)
+    want = small()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = small()
+    for _ in range(3):
+        out.zero_()
+        with torch.cuda.stream(torch.cuda.Stream()):
+            large()
+            junk = torch.full((64 << 20,), 0xFF, dtype=torch.uint8, device="cuda")
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
+        del junk

@@ -10,14 +10,19 @@
 #include <ATen/core/Tensor.h>
 #include <ATen/ops/empty.h>
 #include <ATen/ops/zeros.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/Dtype.h>
 #include <torch/csrc/autograd/python_variable.h>
 
+#include <algorithm>
 #include <cmath>
+#include <cstdint>
 #include <stdexcept>
 #include <string>
+#include <thread>
+#include <vector>
 
 #include "tq4.h"
 
@@ -98,10 +103,23 @@ void check(int status, const char* what) {
   fail(PyExc_RuntimeError, msg + " (tq4 status " + std::to_string(status) + ")");
 }
 
-// Per-device error flag and attention scratch (grown on demand).  Never destroyed: the CUDA context may
-// be gone by the time static objects are.  Reached with the GIL held only.
+// Attention scratch of the callers that bring none, grown on demand.  A call is several launches that hand data
+// on through it, made without the GIL, so no two calls that can run at a time may share one: it belongs to a
+// stream (kernels of two streams overlap) and a thread (launches of two threads interleave).  The last
+// kMaxScratch of a device are held.  One that is dropped or outgrown returns to its own stream's pool, so its
+// memory is reused behind the kernels that still work on it; a call keeps its tensor until it has launched.
+struct Scratch {
+  void* stream;
+  std::thread::id thread;
+  at::Tensor t;
+  uint64_t used;
+};
+constexpr size_t kMaxScratch = 4;
+// Per-device error flag and scratch.  Never destroyed: the CUDA context may be gone by the time static objects
+// are.  Reached with the GIL held only.
 at::Tensor* g_flag[kMaxDevices];
-at::Tensor* g_workspace[kMaxDevices];
+std::vector<Scratch>* g_scratch[kMaxDevices];
+uint64_t g_scratch_clock = 0;
 
 int device_index(const at::Tensor& t) {
   const int i = t.get_device();
@@ -113,14 +131,6 @@ at::Tensor& flag_of(int dev) {
     g_flag[dev] = new at::Tensor(at::zeros({1}, at::TensorOptions().dtype(at::kInt).device(at::kCUDA, dev)));
   return *g_flag[dev];
 }
-at::Tensor& workspace_of(int dev, int64_t bytes) {
-  if (!g_workspace[dev]) g_workspace[dev] = new at::Tensor();
-  at::Tensor& w = *g_workspace[dev];
-  if (!w.defined() || w.numel() < bytes)
-    w = at::empty({bytes}, at::TensorOptions().dtype(at::kByte).device(at::kCUDA, dev));
-  return w;
-}
-
 // The device's stream, with the device current for the duration of a call: the C entry points launch on
 // the current device.
 struct Launch {
@@ -130,6 +140,33 @@ struct Launch {
     guard.set_index((c10::DeviceIndex)dev);
     stream = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev).stream();
   }
+};
+
+at::Tensor workspace_of(int dev, void* stream, int64_t bytes) {
+  const auto opts = at::TensorOptions().dtype(at::kByte).device(at::kCUDA, dev);
+  // a captured call gets memory of its graph's pool: it is replayed, on any stream, for as long as the graph lives
+  if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) return at::empty({bytes}, opts);
+  if (!g_scratch[dev]) g_scratch[dev] = new std::vector<Scratch>();
+  std::vector<Scratch>& all = *g_scratch[dev];
+  const std::thread::id me = std::this_thread::get_id();
+  auto it = std::find_if(all.begin(), all.end(), [&](const Scratch& s) { return s.stream == stream && s.thread == me; });
+  if (it == all.end()) {
+    if (all.size() == kMaxScratch)
+      all.erase(std::min_element(all.begin(), all.end(), [](const Scratch& a, const Scratch& b) { return a.used < b.used; }));
+    it = all.insert(all.end(), Scratch{stream, me, at::Tensor(), 0});
+  }
+  it->used = ++g_scratch_clock;
+  if (!it->t.defined() || it->t.numel() < bytes) {
+    it->t.reset();
+    it->t = at::empty({bytes}, opts);
+  }
+  return it->t;
+}
+
+// The GIL given up for the launches of a call; taken back on the way out of an exception, too.
+struct NoGil {
+  PyThreadState* state = PyEval_SaveThread();
+  ~NoGil() { PyEval_RestoreThread(state); }
 };
 
 template <typename F>
@@ -209,7 +246,7 @@ PyObject* attention(PyObject*, PyObject* const* p, Py_ssize_t n) {
     if (need == 0)
       fail(PyExc_ValueError, "unsupported attention shape: Hq=" + std::to_string(hq) + ", Hkv=" + std::to_string(hkv) +
                                  ", D=" + std::to_string(d));
-    const at::Tensor& ws = p[17] == Py_None ? workspace_of(dev, (int64_t)need) : cuda_tensor(p[17], "workspace");
+    const at::Tensor ws = p[17] == Py_None ? workspace_of(dev, launch.stream, (int64_t)need) : cuda_tensor(p[17], "workspace");
     const size_t have = (size_t)ws.numel() * ws.element_size();
     if (have < need)
       fail(PyExc_ValueError, "workspace has " + std::to_string(have) + " bytes, " + std::to_string(need) + " needed");
@@ -219,16 +256,17 @@ PyObject* attention(PyObject*, PyObject* const* p, Py_ssize_t n) {
     const int q_dt = dtype_code(q.scalar_type()), out_dt = dtype_code(out.scalar_type());
     int st;
     if (p[19] == Py_None) {
-      Py_BEGIN_ALLOW_THREADS
-      st = tq4_paged_attention(
-          q.data_ptr(), q_dt, t, (int)lens.numel(), (int)hq, (int)hkv, (int)d, q.stride(0),
-          q.stride(1), (const uint8_t*)cache.data_ptr(), cache.stride(0), cache.stride(1), cache.size(0), (int)block,
-          (const int32_t*)bt.data_ptr(), bt.stride(0), (const int32_t*)lens.data_ptr(),
-          qsl ? (const int32_t*)qsl->data_ptr() : nullptr, (const float*)kc.data_ptr(), (int)kc.numel(),
-          (const float*)vc.data_ptr(), (int)vc.numel(), (const float*)rot.data_ptr(), scale, causal, window,
-          out.data_ptr(), out_dt, out.stride(0), out.stride(1), lse, rotated, ws.data_ptr(), have,
-          mode, flag, launch.stream);
-      Py_END_ALLOW_THREADS
+      {
+        const NoGil no_gil;
+        st = tq4_paged_attention(
+            q.data_ptr(), q_dt, t, (int)lens.numel(), (int)hq, (int)hkv, (int)d, q.stride(0),
+            q.stride(1), (const uint8_t*)cache.data_ptr(), cache.stride(0), cache.stride(1), cache.size(0), (int)block,
+            (const int32_t*)bt.data_ptr(), bt.stride(0), (const int32_t*)lens.data_ptr(),
+            qsl ? (const int32_t*)qsl->data_ptr() : nullptr, (const float*)kc.data_ptr(), (int)kc.numel(),
+            (const float*)vc.data_ptr(), (int)vc.numel(), (const float*)rot.data_ptr(), scale, causal, window,
+            out.data_ptr(), out_dt, out.stride(0), out.stride(1), lse, rotated, ws.data_ptr(), have,
+            mode, flag, launch.stream);
+      }
     } else {
       // any iterable of seven, held until the call returns
       struct Held {
@@ -249,19 +287,20 @@ PyObject* attention(PyObject*, PyObject* const* p, Py_ssize_t n) {
       key = inner_contiguous(key);
       value = inner_contiguous(value);
       const int kv_dt = dtype_code(key.scalar_type());
-      Py_BEGIN_ALLOW_THREADS
-      st = tq4_write_and_attention(
-          key.data_ptr(), value.data_ptr(), kv_dt, key.size(0), key.stride(0), key.stride(1),
-          value.stride(0), value.stride(1), (const int64_t*)slots.data_ptr(), slots.numel(), (const float*)even.data_ptr(),
-          (const float*)odd.data_ptr(), (const float*)kb.data_ptr(), (int)kb.numel(), (const float*)vb.data_ptr(),
-          (int)vb.numel(), q.data_ptr(), q_dt, t, (int)lens.numel(), (int)hq, (int)hkv, (int)d,
-          q.stride(0), q.stride(1), (uint8_t*)cache.data_ptr(), cache.stride(0), cache.stride(1), cache.size(0), (int)block,
-          (const int32_t*)bt.data_ptr(), bt.stride(0), (const int32_t*)lens.data_ptr(),
-          qsl ? (const int32_t*)qsl->data_ptr() : nullptr, (const float*)kc.data_ptr(), (int)kc.numel(),
-          (const float*)vc.data_ptr(), (int)vc.numel(), (const float*)rot.data_ptr(), scale, causal, window,
-          out.data_ptr(), out_dt, out.stride(0), out.stride(1), lse, rotated, ws.data_ptr(), have,
-          mode, flag, launch.stream);
-      Py_END_ALLOW_THREADS
+      {
+        const NoGil no_gil;
+        st = tq4_write_and_attention(
+            key.data_ptr(), value.data_ptr(), kv_dt, key.size(0), key.stride(0), key.stride(1),
+            value.stride(0), value.stride(1), (const int64_t*)slots.data_ptr(), slots.numel(), (const float*)even.data_ptr(),
+            (const float*)odd.data_ptr(), (const float*)kb.data_ptr(), (int)kb.numel(), (const float*)vb.data_ptr(),
+            (int)vb.numel(), q.data_ptr(), q_dt, t, (int)lens.numel(), (int)hq, (int)hkv, (int)d,
+            q.stride(0), q.stride(1), (uint8_t*)cache.data_ptr(), cache.stride(0), cache.stride(1), cache.size(0), (int)block,
+            (const int32_t*)bt.data_ptr(), bt.stride(0), (const int32_t*)lens.data_ptr(),
+            qsl ? (const int32_t*)qsl->data_ptr() : nullptr, (const float*)kc.data_ptr(), (int)kc.numel(),
+            (const float*)vc.data_ptr(), (int)vc.numel(), (const float*)rot.data_ptr(), scale, causal, window,
+            out.data_ptr(), out_dt, out.stride(0), out.stride(1), lse, rotated, ws.data_ptr(), have,
+            mode, flag, launch.stream);
+      }
     }
     check(st, "paged_tq4_attention");
     if (!own_out) {
@@ -292,14 +331,15 @@ PyObject* write_paged(PyObject*, PyObject* const* p, Py_ssize_t n) {
     int* flag = (int*)flag_of(dev).data_ptr();
     const int kv_dt = dtype_code(key.scalar_type());
     int st;
-    Py_BEGIN_ALLOW_THREADS
-    st = tq4_write_paged(key.data_ptr(), value.data_ptr(), kv_dt, key.size(0), (int)key.size(1),
-                         (int)key.size(2), key.stride(0), key.stride(1), value.stride(0), value.stride(1),
-                         (const int64_t*)slots.data_ptr(), slots.numel(), (const float*)even.data_ptr(),
-                         (const float*)odd.data_ptr(), (const float*)kb.data_ptr(), (int)kb.numel(),
-                         (const float*)vb.data_ptr(), (int)vb.numel(), (uint8_t*)cache.data_ptr(), cache.size(2),
-                         cache.size(0) * cache.size(1), flag, launch.stream);
-    Py_END_ALLOW_THREADS
+    {
+      const NoGil no_gil;
+      st = tq4_write_paged(key.data_ptr(), value.data_ptr(), kv_dt, key.size(0), (int)key.size(1),
+                           (int)key.size(2), key.stride(0), key.stride(1), value.stride(0), value.stride(1),
+                           (const int64_t*)slots.data_ptr(), slots.numel(), (const float*)even.data_ptr(),
+                           (const float*)odd.data_ptr(), (const float*)kb.data_ptr(), (int)kb.numel(),
+                           (const float*)vb.data_ptr(), (int)vb.numel(), (uint8_t*)cache.data_ptr(), cache.size(2),
+                           cache.size(0) * cache.size(1), flag, launch.stream);
+    }
     check(st, "tq4_write_paged");
     Py_RETURN_NONE;
   });
@@ -348,18 +388,19 @@ PyObject* attend_rows(PyObject*, PyObject* const* p, Py_ssize_t n) {
     if (need == 0)
       fail(PyExc_ValueError, "unsupported attention shape: Hq=" + std::to_string(hq) + ", Hkv=" + std::to_string(hkv) +
                                  ", D=" + std::to_string(d));
-    const at::Tensor& ws = workspace_of(dev, (int64_t)need);
+    const at::Tensor ws = workspace_of(dev, launch.stream, (int64_t)need);
     int* flag = (int*)flag_of(dev).data_ptr();
     const int q_dt = dtype_code(q.scalar_type()), out_dt = dtype_code(dt);
     int st;
-    Py_BEGIN_ALLOW_THREADS
-    st = tq4_paged_attention(
-        q.data_ptr(), q_dt, b, (int)b, (int)hq, (int)hkv, (int)d, q.stride(0), q.stride(1), (const uint8_t*)rows.data_ptr(),
-        page * rows.size(2), rows.size(2), b * (rows.size(1) / page), (int)page, (const int32_t*)bt.data_ptr(), bt.size(1),
-        (const int32_t*)lens.data_ptr() + len * b, nullptr, (const float*)kc.data_ptr(), (int)kc.numel(),
-        (const float*)vc.data_ptr(), (int)vc.numel(), (const float*)rot.data_ptr(), scale, 0, 0, out.data_ptr(), out_dt,
-        out.stride(0), out.stride(2), nullptr, 0, ws.data_ptr(), (size_t)ws.numel() * ws.element_size(), 0, flag, launch.stream);
-    Py_END_ALLOW_THREADS
+    {
+      const NoGil no_gil;
+      st = tq4_paged_attention(
+          q.data_ptr(), q_dt, b, (int)b, (int)hq, (int)hkv, (int)d, q.stride(0), q.stride(1), (const uint8_t*)rows.data_ptr(),
+          page * rows.size(2), rows.size(2), b * (rows.size(1) / page), (int)page, (const int32_t*)bt.data_ptr(), bt.size(1),
+          (const int32_t*)lens.data_ptr() + len * b, nullptr, (const float*)kc.data_ptr(), (int)kc.numel(),
+          (const float*)vc.data_ptr(), (int)vc.numel(), (const float*)rot.data_ptr(), scale, 0, 0, out.data_ptr(), out_dt,
+          out.stride(0), out.stride(2), nullptr, 0, ws.data_ptr(), (size_t)ws.numel() * ws.element_size(), 0, flag, launch.stream);
+    }
     check(st, "attend_rows");
     return THPVariable_Wrap(std::move(out));
   });
@@ -380,12 +421,13 @@ PyObject* append_rows(PyObject*, PyObject* const* p, Py_ssize_t n) {
     const int dt = dtype_code(k.t.scalar_type());
     Launch launch(device_index(k.t));
     int st;
-    Py_BEGIN_ALLOW_THREADS
-    st = tq4_append_rows(k.t.data_ptr(), v.t.data_ptr(), dt, (int)k.t.size(0), (int)k.t.size(2), (int)k.t.size(1), (int)k.t.size(3),
-                         k.strides, v.strides, (const float*)even.data_ptr(), (const float*)odd.data_ptr(),
-                         (const float*)kb.data_ptr(), (int)kb.numel(), (const float*)vb.data_ptr(), (int)vb.numel(),
-                         (uint8_t*)rows.data_ptr(), rows.size(2), rows.size(1), offset, launch.stream);
-    Py_END_ALLOW_THREADS
+    {
+      const NoGil no_gil;
+      st = tq4_append_rows(k.t.data_ptr(), v.t.data_ptr(), dt, (int)k.t.size(0), (int)k.t.size(2), (int)k.t.size(1), (int)k.t.size(3),
+                           k.strides, v.strides, (const float*)even.data_ptr(), (const float*)odd.data_ptr(),
+                           (const float*)kb.data_ptr(), (int)kb.numel(), (const float*)vb.data_ptr(), (int)vb.numel(),
+                           (uint8_t*)rows.data_ptr(), rows.size(2), rows.size(1), offset, launch.stream);
+    }
     check(st, "tq4_append_rows");
     Py_RETURN_NONE;
   });
@@ -430,15 +472,16 @@ PyObject* cache_update(PyObject*, PyObject* const* p, Py_ssize_t n) {
     at::Tensor scratch;
     if (need) scratch = at::empty({(int64_t)need}, k.t.options().dtype(at::kByte).requires_grad(false));
     int st;
-    Py_BEGIN_ALLOW_THREADS
-    st = tq4_cache_update(k.t.data_ptr(), v.t.data_ptr(), dt, (int)b, (int)h, (int)k.t.size(2), (int)d, k.strides, v.strides,
-                          (const float*)rot.data_ptr(), (const float*)even.data_ptr(), (const float*)odd.data_ptr(),
-                          (const float*)kb.data_ptr(), (int)kb.numel(),
-                          (const float*)vb.data_ptr(), (int)vb.numel(), (const float*)kc.data_ptr(), (int)kc.numel(),
-                          (const float*)vc.data_ptr(), (int)vc.numel(), k_nib, v_nib, (uint8_t*)ki.data_ptr(),
-                          (float*)kn.data_ptr(), (uint8_t*)vi.data_ptr(), (float*)vn.data_ptr(), cap, offset, kd, vd, dec_cap,
-                          dec_offset, need ? scratch.data_ptr() : nullptr, need, launch.stream);
-    Py_END_ALLOW_THREADS
+    {
+      const NoGil no_gil;
+      st = tq4_cache_update(k.t.data_ptr(), v.t.data_ptr(), dt, (int)b, (int)h, (int)k.t.size(2), (int)d, k.strides, v.strides,
+                            (const float*)rot.data_ptr(), (const float*)even.data_ptr(), (const float*)odd.data_ptr(),
+                            (const float*)kb.data_ptr(), (int)kb.numel(),
+                            (const float*)vb.data_ptr(), (int)vb.numel(), (const float*)kc.data_ptr(), (int)kc.numel(),
+                            (const float*)vc.data_ptr(), (int)vc.numel(), k_nib, v_nib, (uint8_t*)ki.data_ptr(),
+                            (float*)kn.data_ptr(), (uint8_t*)vi.data_ptr(), (float*)vn.data_ptr(), cap, offset, kd, vd, dec_cap,
+                            dec_offset, need ? scratch.data_ptr() : nullptr, need, launch.stream);
+    }
     check(st, "tq4_cache_update");
     Py_RETURN_NONE;
   });
