@@ -95,3 +95,34 @@ def test_prefill_hides_and_reports_bad_pages(cuda_lib):
     torch.cuda.synchronize()
     assert ops.read_and_clear_errors(torch.device("cuda")) == nv.DEV_BAD_BLOCK
     assert (out[0] - out[1]).abs().max() <= 2e-3
+
+
+@pytest.mark.parametrize("d,hq,hkv,lens,new,cut", [
+    (128, 32, 8, [3000], [40], True),
+    (128, 32, 8, [1200, 1200, 900], [200, 40, 1], True),   # behind the plan of the streaming part
+    (64, 14, 2, [1200], [200], True),
+    (256, 8, 4, [1200], [100], True),
+    (128, 28, 4, [1200], [1200], False),                   # the row blocks fill the GPU
+])
+def test_announced_scratch_is_room_for_the_key_parts(cuda_lib, d, hq, hkv, lens, new, cut):
+    """A workspace of exactly the announced bytes: calls of few row blocks are cut along the keys (a merge follows
+    the prefill kernel), and nothing is written past its end."""
+    from turboquant_vllm import _native as nv
+    from turboquant_vllm.kernels import ops
+
+    pr = Prims(d)
+    p = pr.cuda()
+    case = build_paged_case(lens, hkv, d, 16, pr, seed=5, padded=True)
+    rows = sum(new)
+    q = torch.randn(rows, hq, d, generator=torch.Generator().manual_seed(1)).bfloat16().cuda()
+    qsl = torch.tensor(np.concatenate([[0], np.cumsum(new)]), dtype=torch.int32).cuda()
+    args = (q, case["cache"].cuda(), case["block_table"].cuda(), case["seq_lens"].cuda(), p["kc"], p["vc"], p["rot"], hkv, 16)
+    need = ops.attention_workspace_bytes(rows, hq, hkv, d)
+    ws = torch.full((need + 4096,), 0x55, dtype=torch.uint8, device="cuda")
+    nv.profile_start(8)
+    out = ops.paged_tq4_attention(*args, query_start_loc=qsl, out_dtype=torch.float32, workspace=ws[:need])
+    merges, passes = (len(nv.profile_read(k, 8)) for k in (nv.PROF_COMBINE, nv.PROF_ATTENTION))
+    nv.profile_stop()
+    assert merges == passes - 1 + cut and (ws[need:] == 0x55).all()
+    want = ops.paged_tq4_attention(*args, query_start_loc=qsl, out_dtype=torch.float32, mode=2)
+    assert (out - want).abs().max() <= 2e-3

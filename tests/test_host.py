@@ -272,3 +272,16 @@ def test_error_check_switch(monkeypatch):
     for val, want in (("1", True), ("true", True), ("0", False), ("", False)):
         monkeypatch.setenv("TQ4_CHECK_ERRORS", val)
         assert ops.error_checks_enabled() is want
+
+
+@pytest.mark.parametrize("rows,hq,hkv,d,mb", [
+    (2048, 32, 8, 128, 78), (8192, 8, 4, 256, 112), (2048, 28, 4, 128, 107), (2048, 14, 2, 64, 47), (64, 32, 8, 128, 12.1),
+    # (partials of 256 rows in three parts are more than the streaming kernel leaves: 18.3 MB without them)
+    (256, 32, 8, 128, 26),
+])
+def test_attention_scratch_holds_the_key_parts_in_the_streaming_partials_room(cuda_lib, rows, hq, hkv, d, mb):
+    """Scratch is allocated per layer.  A prefill call cut along the keys starts when the streaming part is done, so
+    its partials need no room of their own next to that part's."""
+    from turboquant_vllm.kernels import ops
+
+    assert ops.attention_workspace_bytes(rows, hq, hkv, d) <= mb * 1e6

@@ -2,6 +2,7 @@
 // the split merge + un-rotation kernel, and the C entry points.
 #include <math_constants.h>
 
+#include <algorithm>
 #include <cstdlib>
 
 #include "tq4_attention.cuh"
@@ -1191,15 +1192,24 @@ static size_t workspace_min(int64_t max_query_rows, int num_q_heads, int num_kv_
   return a > b ? a : b;
 }
 
-// ... plus room for the partials of prefill calls that are cut along the keys: up to eight parts of the
-// rows, as long as the row blocks alone do not fill the GPU.
+// ... and room for a prefill call that is cut along the keys: Pi's image and the partials of up to eight parts of the rows,
+// as long as these do not fill the GPU.  They lie where the streaming part's partials were (attention_impl), behind
+// the plan in a call of both kernels; only calls of few heads or rows need more than the plan has anyway.
 extern "C" size_t tq4_attention_workspace_bytes(int64_t max_query_rows, int num_q_heads,
                                                 int num_kv_heads, int head_dim) {
   const size_t least = workspace_min(max_query_rows, num_q_heads, num_kv_heads, head_dim);
   if (least == 0) return 0;
+  if (max_query_rows < tq4::kPrefillMinRows) return least;
   int64_t vectors = 8 * max_query_rows * num_q_heads;
   if (vectors > tq4::kPrefillSplitVectors) vectors = tq4::kPrefillSplitVectors;
-  return max_query_rows < tq4::kPrefillMinRows ? least : least + (size_t)vectors * (head_dim + 1) * 4;
+  const int64_t rows = max_query_rows < tq4::kMaxRowsPerLaunch ? max_query_rows : tq4::kMaxRowsPerLaunch;
+  tq4::AttnPlan p;
+  size_t front = 0;  // (for whichever kernel has more spans)
+  constexpr int64_t spans = std::max(tq4::kMaxCtasPerSlice, tq4::kMaxSms * tq4::kMmaWarpsPerCta);
+  tq4::carve_plan(p, nullptr, rows, num_q_heads, head_dim, 1, spans, &front);
+  // (a vector set of Hq and the alignment of the image on top: prefill_tc_splits counts whole sets)
+  const size_t cut = front + 128 + tq4::prefill_tc_image_bytes(head_dim) + (size_t)(vectors + num_q_heads) * (head_dim + 1) * 4;
+  return cut > least ? cut : least;
 }
 
 // Shared body of tq4_paged_attention and tq4_write_and_attention: `wr` (optional) is a cache write

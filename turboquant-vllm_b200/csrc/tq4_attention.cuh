@@ -24,7 +24,7 @@ constexpr int kMmaWarpsPerCta = 16;    // tensor-core LUT kernel (one CTA per SM
 constexpr int kMaxCtasPerSlice = 148 * 4;  // upper bound used for workspace sizing (fp32 kernel)
 constexpr int kMaxSms = 160;               // tensor-core kernel: one CTA per SM, one span per warp phase
 constexpr int kMaxRowsPerLaunch = 4096;    // larger query batches are processed in pieces
-constexpr int kPrefillSplitVectors = 2 * 148 * 256;  // (row, head) partials of a prefill call cut along the keys
+constexpr int kPrefillSplitVectors = kMaxSms * 256;  // (row, head) partials of a prefill call cut along the keys: at most one CTA per SM
 constexpr int kFusedMaxRows = 512;         // decode calls up to this size can plan and rotate inside the attention kernel
 // A row is cut into at most this many spans (= partials the merge kernel has to fold for it): a call of
 // a few long rows would otherwise hand the merge kernel hundreds of partials per row on a handful of
@@ -131,9 +131,9 @@ inline bool make_shape(AttnShape& s, int Hq, int Hkv, int D, int max_warps = kMa
   return true;
 }
 
-// Carve the workspace.  Returns the number of bytes used.
+// Carve the workspace.  Returns the number of bytes used; `front`: how many lie in front of the partials.
 inline size_t carve_plan(AttnPlan& p, void* ws, int64_t rows, int Hq, int D, int TPC,
-                         int64_t max_spans = kMaxCtasPerSlice) {
+                         int64_t max_spans = kMaxCtasPerSlice, size_t* front = nullptr) {
   const int64_t slots = rows + max_spans;
   unsigned char* b = reinterpret_cast<unsigned char*>(ws);
   size_t off = 0;
@@ -152,6 +152,7 @@ inline size_t carve_plan(AttnPlan& p, void* ws, int64_t rows, int Hq, int D, int
   p.row_rec = reinterpret_cast<int*>(take((size_t)rows * 32));
   p.span_rec = reinterpret_cast<int*>(take((size_t)max_spans * 48));
   p.scalars = reinterpret_cast<int*>(take(64));
+  if (front) *front = off;
   p.part_o = reinterpret_cast<float*>(take((size_t)slots * TPC * Hq * D * 4));
   p.part_m = reinterpret_cast<float*>(take((size_t)slots * TPC * Hq * 4));
   p.part_l = reinterpret_cast<float*>(take((size_t)slots * TPC * Hq * 4));
