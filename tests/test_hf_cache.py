@@ -73,6 +73,41 @@ def test_mixed_attention_config_and_disabled_passthrough_cpu():
         cache.update(k, k, 2)  # compression needs a CUDA tensor
 
 
+class _AsIfCuda(torch.Tensor):
+    is_cuda = True
+
+
+def test_growth_lets_each_old_buffer_go_cpu(monkeypatch):
+    """When a layer outgrows its buffers, the old one of each is gone before the next one is grown (the two
+    dequantised ones are what the layer hands out as keys and values: they stay until the update returns)."""
+    import weakref
+
+    from turboquant_vllm import _native as nv
+    from turboquant_vllm import kv_cache as K
+
+    calls, prims = [], tuple(torch.zeros(1) for _ in range(5))
+    monkeypatch.setattr(K.TurboQuantCompressorMSE, "__init__", lambda self, d, bits, seed: setattr(
+        self, "quantizer", types.SimpleNamespace(bits=bits, device_primitives=lambda dev: prims)))
+    monkeypatch.setattr(nv, "host", lambda: types.SimpleNamespace(cache_update=lambda *a: calls.append(len(a))))
+    alive = []
+    reserve = K._GrowBuffer.reserve
+
+    def watched(self, *args):
+        old = None if self.buf is None else weakref.ref(self.buf)
+        new = reserve(self, *args)
+        if old is not None and self.buf is not old():
+            alive.append(old() is not None)
+        return new
+
+    monkeypatch.setattr(K._GrowBuffer, "reserve", watched)
+    cache = DynamicCache()
+    _cls()(cache, head_dim=64, k_bits=4, v_bits=3)
+    for n in (60, 1, 1, 1, 1, 1):  # the capacity is 64: the last update grows
+        kv = torch.randn(1, 2, n, 64).as_subclass(_AsIfCuda)
+        cache.update(kv, kv + 1, 0)
+    assert len(calls) == 6 and alive == [False] * 4 + [True] * 2
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("tag,kb,vb", [("b4", 4, 4), ("k4v3", 4, 3)])
 def test_update_matches_reference_trace(cuda_lib, golden, tag, kb, vb):

@@ -401,6 +401,8 @@ class CompressedDynamicCache:
                         buf.shape != (b, h, first.buf.shape[2], w) or buf.dtype != t or buf.device != dev):
                     return False
                 bufs.append((g, w, t))
+        # nothing here may hold the old buffers: each goes when its copy is made, not when all six have grown
+        store[0].fit = fit = out = buf = t = None
         out = [g.reserve(b, h, n, w, t, dev) for g, w, t in bufs]
         prims = (rot, even, odd, k_bounds, v_bounds, k_cents, v_cents)
         nv.host().cache_update(
