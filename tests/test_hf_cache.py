@@ -73,6 +73,71 @@ def test_mixed_attention_config_and_disabled_passthrough_cpu():
         cache.update(k, k, 2)  # compression needs a CUDA tensor
 
 
+def test_only_unreachable_wrappers_are_unwound_cpu():
+    """A new wrapper cuts the pairs of cache and wrapper that nobody holds any more, and no other."""
+    import gc
+    import weakref
+
+    from turboquant_vllm import kv_cache as K
+
+    C = _cls()
+    assert K._counts_are_exact  # (CPython up to 3.13; where it is off, nothing is ever cut)
+
+    def make():
+        cache = DynamicCache()
+        return C(cache, head_dim=64, k_bits=4, v_bits=3), cache
+
+    def hold_in_generator(w):
+        yield
+        yield w
+
+    gc.collect()
+    gc.disable()
+    try:
+        live = [make()[0], make()[1], make()[1].update, make()[1].get_seq_length, make()[0]._original_update, make()[0].restore]
+        live.append(hold_in_generator(make()[0]))
+        next(live[-1])
+        live.append(lambda w=make()[0]: w)
+        cycle = [make()[1]]  # held by a cycle of the user's: the collector's business
+        cycle.append(cycle)
+        live.append(weakref.ref(cycle[0]))
+        wrapped = [x for x in (r() for r in K._wrappers) if x is not None]
+        assert len(wrapped) >= 9
+        held = [weakref.ref(w.cache) for w in wrapped]
+        del wrapped, cycle
+        dead = [weakref.ref(x) for x in make()]
+        assert all(r() is not None for r in dead)  # (their own cycle keeps both)
+
+        def use(cache):  # a live cache whose only name is this argument
+            C(DynamicCache(), head_dim=64, bits=4)
+            return hasattr(cache.update, "__self__") and isinstance(cache.update.__self__, C)
+
+        assert use(make()[1])
+        assert all(r() is None for r in dead)
+        assert all(r() is not None and isinstance(r().update.__self__, C) for r in held)
+    finally:
+        gc.enable()
+
+
+@pytest.mark.parametrize("which,off", [("wrapper", -1), ("wrapper", 1), ("cache", -1), ("cache", 1), ("method", -1), ("method", 1)])
+def test_reference_counts_of_another_interpreter_switch_the_release_off_cpu(monkeypatch, which, off):
+    """Where names or arguments are counted otherwise, the check at import notices and nothing is released."""
+    import sys
+
+    from turboquant_vllm import kv_cache as K
+
+    real = sys.getrefcount
+
+    def count(o):
+        kind = "wrapper" if isinstance(o, K.CompressedDynamicCache) else "method" if isinstance(o, types.MethodType) else "cache"
+        return real(o) - 1 + (off if kind == which and type(o) is not object else 0)  # (- 1: this frame's name)
+
+    monkeypatch.setattr(K.sys, "getrefcount", lambda o: real(o) - 1)
+    assert K._counts_tell()
+    monkeypatch.setattr(K.sys, "getrefcount", count)
+    assert not K._counts_tell()
+
+
 class _AsIfCuda(torch.Tensor):
     is_cuda = True
 

@@ -21,6 +21,7 @@ from __future__ import annotations
 
 import sys
 import threading
+import types
 import warnings
 import weakref
 from dataclasses import dataclass
@@ -130,9 +131,59 @@ def _only_cycle_holds(w: "CompressedDynamicCache") -> bool:
     return sys.getrefcount(w) == base + 3 and sys.getrefcount(c) == base + 1 + bound
 
 
-def _release_unreachable() -> None:
+def _counts_tell() -> bool:
+    """Whether this interpreter's reference counts tell a dead pair from a live one, tried on stand-ins.
+
+    The arithmetic of :func:`_only_cycle_holds` rests on how names and arguments are counted, which is the
+    interpreter's own affair; where any of these pairs is judged wrongly, nothing is released by it."""
     if not getattr(sys, "_is_gil_enabled", lambda: True)():
-        return  # reference counts are not exact
+        return False  # (free threading: the counts are not exact)
+
+    class Cache:
+        def update(self): ...
+        def get_seq_length(self): ...
+
+    def pair():
+        c, w = Cache(), object.__new__(CompressedDynamicCache)
+        w.cache, w._original_update, w._original_get_seq_length = c, c.update, c.get_seq_length
+        c.update, c.get_seq_length = w._compressed_update, w._compressed_get_seq_length
+        return w
+
+    def judged_dead(ref):
+        w = ref()
+        return _only_cycle_holds(w)
+
+    def with_held(part):
+        w = pair()
+        ref, held = weakref.ref(w), part(w)
+        w = None
+        return judged_dead(ref), held
+
+    def as_argument(w):
+        return judged_dead(weakref.ref(w))
+
+    def suspended(w):
+        yield
+        yield w
+
+    def held_by_generator(w):
+        g = suspended(w)
+        next(g)
+        return g
+
+    live = (lambda w: w, lambda w: w.cache, lambda w: w.cache.update, lambda w: w.cache.get_seq_length,
+            lambda w: w._original_update, lambda w: w._original_get_seq_length, lambda w: w.restore,
+            lambda w: types.MethodType(Cache.update, w.cache), lambda w: [w], lambda w: lambda: w, held_by_generator)
+    try:
+        return (with_held(lambda w: None)[0] and not as_argument(pair()) and not as_argument(w=pair())
+                and not any(with_held(part)[0] for part in live))
+    except Exception:  # noqa: BLE001  (an interpreter without getrefcount, say)
+        return False
+
+
+def _release_unreachable() -> None:
+    if not _counts_are_exact:
+        return
     with _wrappers_lock:
         for ref in list(_wrappers):
             w = ref()
@@ -547,5 +598,7 @@ class CompressedDynamicCache:
             "vram_estimate": {n: round(per_token * n / 2**20, 2) for n in (4096, 16384, 32768)},
         }
 
+
+_counts_are_exact = _counts_tell()
 
 __all__ = ["CompressedDynamicCache", "CompressedValues"]
