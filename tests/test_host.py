@@ -274,6 +274,35 @@ def test_error_check_switch(monkeypatch):
         assert ops.error_checks_enabled() is want
 
 
+def test_host_binding_is_bound_to_python_and_torch(cuda_lib, monkeypatch, tmp_path):
+    """The binding links to the C++ of one torch and one Python: built for another, it is stale and not loaded."""
+    import importlib.metadata
+    import importlib.util
+
+    from turboquant_vllm import _native as nv
+
+    path = os.path.join(os.path.dirname(os.path.dirname(nv.library_path())), "..", "build.py")
+
+    def build_module():
+        spec = importlib.util.spec_from_file_location("tq4_build_again", path)
+        mod = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(mod)
+        return mod
+
+    now = build_module()
+    assert os.path.samefile(now.HOST_OUT, nv._HOST_PATH) and not now.host_needs_build() and not now.needs_build()
+    with monkeypatch.context() as m:
+        m.setattr(importlib.metadata, "version", lambda name: "99.0")
+        assert build_module().host_needs_build()
+    with monkeypatch.context() as m:
+        m.setattr(now.sysconfig, "get_config_var", lambda name: "cpython-399")
+        assert build_module().host_needs_build()
+    monkeypatch.setattr(nv, "_host", None)
+    monkeypatch.setattr(nv, "_HOST_PATH", str(tmp_path / "_tq4_host.other.so"))
+    with pytest.raises(RuntimeError, match="for this Python and torch"):
+        nv.host()
+
+
 @pytest.mark.parametrize("rows,hq,hkv,d,mb", [
     (2048, 32, 8, 128, 78), (8192, 8, 4, 256, 112), (2048, 28, 4, 128, 107), (2048, 14, 2, 64, 47), (64, 32, 8, 128, 12.1),
     # (partials of 256 rows in three parts are more than the streaming kernel leaves: 18.3 MB without them)

@@ -1,14 +1,17 @@
-"""Build libtq4_sm100a.so (the C-ABI CUDA library) and _tq4_host.so (its CPython binding) in-tree.
+"""Build libtq4_sm100a.so (the C-ABI CUDA library) and _tq4_host.*.so (its CPython binding) in-tree.
 
 Usage:  python turboquant-vllm_b200/build.py [--force] [--verbose]
 Both land in turboquant-vllm_b200/turboquant_vllm/lib/.  The CUDA library is compiled with nvcc for
 sm_100a and has a plain C ABI (include/tq4.h, no torch headers); the binding (csrc/tq4_host.cpp) is
-compiled with g++ against the headers of the installed torch and links to it.
+compiled with g++ against the headers of the installed torch and links to it.  Its name carries the
+Python ABI and the torch version it was built for, as the package looks for it: after a change of
+either, the old binary is neither loaded nor taken for up to date.
 """
 from __future__ import annotations
 
 import argparse
 import glob
+import importlib.metadata
 import importlib.util
 import os
 import subprocess
@@ -21,7 +24,15 @@ CSRC = os.path.join(HERE, "csrc")
 OUT_DIR = os.path.join(HERE, "turboquant_vllm", "lib")
 OUT = os.path.join(OUT_DIR, "libtq4_sm100a.so")
 HOST_SRC = os.path.join(CSRC, "tq4_host.cpp")
-HOST_OUT = os.path.join(OUT_DIR, "_tq4_host.so")
+
+
+
+def host_name() -> str:
+    """File name of the CPython binding for this interpreter and the installed torch."""
+    return f"_tq4_host.{sysconfig.get_config_var('SOABI')}.torch{importlib.metadata.version('torch')}.so"
+
+
+HOST_OUT = os.path.join(OUT_DIR, host_name())
 
 
 def sources() -> list[str]:

@@ -49,7 +49,6 @@ def build_trace_library() -> str:
             raise SystemExit(f"nvcc failed on {src}")
     if jobs or not os.path.exists(TRACE_LIB):
         subprocess.check_call([nvcc, "-shared", "-gencode", "arch=compute_100a,code=sm_100a", "-o", TRACE_LIB, *objs])
-    shutil.copy(os.path.join(LIB_DIR, "_tq4_host.so"), os.path.dirname(TRACE_LIB))
     return TRACE_LIB
 
 
@@ -61,7 +60,7 @@ def _load(kind: str):
     from turboquant_vllm import _native as nv
 
     nv._LIB_PATH = build_trace_library()
-    nv._HOST_PATH = os.path.join(os.path.dirname(TRACE_LIB), "_tq4_host.so")
+    nv._HOST_PATH = shutil.copy(nv._HOST_PATH, os.path.dirname(TRACE_LIB))  # (finds its library beside it)
     reader = {"decode": "tq4_trace_read", "prefill": "tq4_prefill_trace_read", "compress": "tq4_compress_trace_read"}[kind]
     nv._SIGNATURES[reader] = (ctypes.c_int, [ctypes.c_void_p])
     return nv, reader

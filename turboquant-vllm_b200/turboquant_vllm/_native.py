@@ -12,14 +12,18 @@ from __future__ import annotations
 import contextlib
 import ctypes
 import importlib.machinery
+import importlib.metadata
 import importlib.util
 import os
+import sysconfig
 from ctypes import c_char_p, c_float, c_int, c_int64, c_size_t, c_void_p
 
 import torch
 
 _LIB_PATH = os.path.join(os.path.dirname(os.path.abspath(__file__)), "lib", "libtq4_sm100a.so")
-_HOST_PATH = os.path.join(os.path.dirname(_LIB_PATH), "_tq4_host.so")
+# (as turboquant-vllm_b200/build.py names it: a binding built for another Python or torch is not picked up)
+_HOST_PATH = os.path.join(os.path.dirname(_LIB_PATH),
+                          f"_tq4_host.{sysconfig.get_config_var('SOABI')}.torch{importlib.metadata.version('torch')}.so")
 _lib = None
 _host = None
 
@@ -131,8 +135,8 @@ def host():
     if _host is None:
         lib()
         if not os.path.exists(_HOST_PATH):
-            raise RuntimeError(f"TQ4 host extension not found at {_HOST_PATH}. Build it with "
-                               "`python turboquant-vllm_b200/build.py`.")
+            raise RuntimeError(f"TQ4 host extension not found at {_HOST_PATH}. Build it, for this Python and "
+                               "torch, with `python turboquant-vllm_b200/build.py`.")
         loader = importlib.machinery.ExtensionFileLoader("_tq4_host", _HOST_PATH)
         mod = importlib.util.module_from_spec(importlib.util.spec_from_file_location("_tq4_host", _HOST_PATH, loader=loader))
         loader.exec_module(mod)
