@@ -268,6 +268,34 @@ int tq4_write_and_attention(const void* key, const void* value, int kv_dtype, in
                             int* err_flag, void* stream);
 
 /*
+ * tq4_write_and_attention for a caller that knows on the host how long the longest sequence of the call is:
+ * max_seq_len (> 0; 0 = not known).  Only the choice of kernels and of their grids reads it, never a result:
+ * the block table of a serving engine is as wide as its model allows whatever the contexts are, and without
+ * max_seq_len that width (bt_stride * block_size) has to stand for them.  n_tokens == 0: no write.
+ */
+int tq4_attention_step(const void* key, const void* value, int kv_dtype, int64_t n_tokens,
+                       int64_t k_token_stride, int64_t k_head_stride,
+                       int64_t v_token_stride, int64_t v_head_stride,
+                       const int64_t* slot_mapping, int64_t n_slots,
+                       const float* rot_t_even, const float* rot_t_odd,
+                       const float* k_boundaries, int n_k_boundaries,
+                       const float* v_boundaries, int n_v_boundaries,
+                       const void* q, int q_dtype, int64_t num_rows, int num_seqs,
+                       int num_q_heads, int num_kv_heads, int head_dim,
+                       int64_t q_token_stride, int64_t q_head_stride,
+                       uint8_t* cache, int64_t cache_block_stride, int64_t cache_token_stride,
+                       int64_t num_blocks, int block_size,
+                       const int32_t* block_table, int64_t bt_stride,
+                       const int32_t* seq_lens, const int32_t* query_start_loc, int64_t max_seq_len,
+                       const float* k_centroids, int n_k_centroids,
+                       const float* v_centroids, int n_v_centroids,
+                       const float* rotation, float sm_scale, int causal, int sliding_window,
+                       void* out, int out_dtype, int64_t out_token_stride, int64_t out_head_stride,
+                       float* lse_out, int out_rotated,
+                       void* workspace, size_t workspace_bytes, int mode,
+                       int* err_flag, void* stream);
+
+/*
  * Merge `world` per-shard partial results of a sequence-split (split-KV) attention and
  * un-rotate: parts_o fp32 [world, num_rows, Hq, D] (each normalised, rotated space),
  * parts_lse fp32 [world, num_rows, Hq] (natural log; -inf = shard saw no key).

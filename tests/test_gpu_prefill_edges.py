@@ -126,3 +126,35 @@ def test_announced_scratch_is_room_for_the_key_parts(cuda_lib, d, hq, hkv, lens,
     assert merges == passes - 1 + cut and (ws[need:] == 0x55).all()
     want = ops.paged_tq4_attention(*args, query_start_loc=qsl, out_dtype=torch.float32, mode=2)
     assert (out - want).abs().max() <= 2e-3
+
+
+@pytest.mark.parametrize("hq,hkv,lens,new,bound,launches", [
+    # 19 rows whose table would let every one read 65 536 keys: one streaming pass (attention, merge), or two passes
+    (32, 8, [60, 40, 90], [17, 1, 1], 90, (1, 1)),
+    (32, 8, [60, 40, 90], [17, 1, 1], None, (2, 2)),
+    (32, 8, [60, 40, 90], [17, 1, 1], 10**9, (2, 2)),
+    (32, 8, [300], [300], 300, (1, 0)),    # five tiles: not cut (36 us against 52 in three parts, B200)
+    (32, 8, [300], [300], None, (1, 1)),
+])
+def test_known_length_decides_instead_of_the_table_width(cuda_lib, hq, hkv, lens, new, bound, launches):
+    """max_seq_len: the kernels chosen on a table as wide as the model allows, and no other results."""
+    from turboquant_vllm import _native as nv
+    from turboquant_vllm.kernels import ops
+
+    pr = Prims(128)
+    p = pr.cuda()
+    case = build_paged_case(lens, hkv, 128, 16, pr, seed=5, padded=True)
+    rows = sum(new)
+    q = torch.randn(rows, hq, 128, generator=torch.Generator().manual_seed(1)).bfloat16().cuda()
+    qsl = torch.tensor(np.concatenate([[0], np.cumsum(new)]), dtype=torch.int32).cuda()
+    table = torch.zeros(len(lens), 4096, dtype=torch.int32)
+    table[:, : case["block_table"].shape[1]] = case["block_table"]
+    args = (q, case["cache"].cuda(), table.cuda(), case["seq_lens"].cuda(), p["kc"], p["vc"], p["rot"], hkv, 16)
+    nv.profile_start(8)
+    out = ops.paged_tq4_attention(*args, query_start_loc=qsl, out_dtype=torch.float32, max_seq_len=bound)
+    assert tuple(len(nv.profile_read(k, 8)) for k in (nv.PROF_ATTENTION, nv.PROF_COMBINE)) == launches
+    nv.profile_stop()
+    # (too small a value is only a worse choice)
+    wrong = ops.paged_tq4_attention(*args, query_start_loc=qsl, out_dtype=torch.float32, max_seq_len=1)
+    want = ops.paged_tq4_attention(*args, query_start_loc=qsl, out_dtype=torch.float32, mode=2)
+    assert (out - want).abs().max() <= 2e-3 and (wrong - want).abs().max() <= 2e-3

@@ -1212,15 +1212,15 @@ extern "C" size_t tq4_attention_workspace_bytes(int64_t max_query_rows, int num_
   return cut > least ? cut : least;
 }
 
-// Shared body of tq4_paged_attention and tq4_write_and_attention: `wr` (optional) is a cache write
-// of new tokens that must land before the attention reads the cache.
+// Shared body of the attention entry points: `wr` (optional) is a cache write of new tokens that must land
+// before the attention reads the cache.
 static int attention_impl(
     const tq4::CompressArgs* wr,
     const void* q, int q_dtype, int64_t num_rows, int num_seqs, int num_q_heads, int num_kv_heads,
     int head_dim, int64_t q_token_stride, int64_t q_head_stride, const uint8_t* cache,
     int64_t cache_block_stride, int64_t cache_token_stride, int64_t num_blocks, int block_size,
     const int32_t* block_table, int64_t bt_stride, const int32_t* seq_lens,
-    const int32_t* query_start_loc, const float* k_centroids, int n_k_centroids,
+    const int32_t* query_start_loc, int64_t max_seq_len, const float* k_centroids, int n_k_centroids,
     const float* v_centroids, int n_v_centroids, const float* rotation, float sm_scale, int causal,
     int sliding_window, void* out, int out_dtype, int64_t out_token_stride, int64_t out_head_stride,
     float* lse_out, int out_rotated, void* workspace, size_t workspace_bytes, int mode,
@@ -1272,6 +1272,8 @@ static int attention_impl(
   a.bt_stride = bt_stride;
   a.seq_lens = seq_lens;
   a.query_start_loc = query_start_loc;
+  a.max_keys = bt_stride * block_size;
+  if (max_seq_len > 0 && max_seq_len < a.max_keys) a.max_keys = max_seq_len;
   a.k_centroids = k_centroids;
   a.v_centroids = v_centroids;
   a.n_k_centroids = n_k_centroids;
@@ -1303,8 +1305,10 @@ static int attention_impl(
   // of a prefill tile (Pi's image, rotating and un-rotating 128 rows: 20 us).  45 drawn steps: up to 4096 rows times
   // query heads streaming took 0.43 - 1.0 of the time (34 rows beside 21 running sequences, 28 / 4 heads: 25.9
   // against 49.9 us), above 5000 1.3 - 2.5 times it; head_dim 256, where it reads each row twice: the line is at 2048.
-  // And not where long contexts, by the width of the block table, make it re-read more than some 50 us of bytes.
-  const int64_t keys = bt_stride * block_size;
+  // And not where long contexts make it re-read more than some 50 us of bytes.  Their length is the caller's
+  // max_seq_len: by the width of a server's table (32 768 tokens) 34 rows of at most 26 keys took 66.6 us instead of 25.6,
+  // 80 of at most 985 took 87.1 instead of 50.2 (32 / 8 heads of 128).
+  const int64_t keys = a.max_keys;
   const bool few = use_mma && num_rows * num_q_heads <= (head_dim == 256 ? 2048 : 4096) &&
                    num_rows * keys * row_data_bytes(num_kv_heads, head_dim) <= (1ll << 28);
   const bool use_prefill = prefill_ok && (mode == 3 || mode == 4 || (mode == 0 && !few && num_rows >= kPrefillMinRows && (num_seqs > 1 || all_long)));
@@ -1436,13 +1440,13 @@ extern "C" int tq4_paged_attention(
     int* err_flag, void* stream) {
   return attention_impl(nullptr, q, q_dtype, num_rows, num_seqs, num_q_heads, num_kv_heads, head_dim,
                         q_token_stride, q_head_stride, cache, cache_block_stride, cache_token_stride,
-                        num_blocks, block_size, block_table, bt_stride, seq_lens, query_start_loc,
+                        num_blocks, block_size, block_table, bt_stride, seq_lens, query_start_loc, 0,
                         k_centroids, n_k_centroids, v_centroids, n_v_centroids, rotation, sm_scale,
                         causal, sliding_window, out, out_dtype, out_token_stride, out_head_stride,
                         lse_out, out_rotated, workspace, workspace_bytes, mode, err_flag, stream);
 }
 
-extern "C" int tq4_write_and_attention(
+extern "C" int tq4_attention_step(
     const void* key, const void* value, int kv_dtype, int64_t n_tokens, int64_t k_token_stride,
     int64_t k_head_stride, int64_t v_token_stride, int64_t v_head_stride,
     const int64_t* slot_mapping, int64_t n_slots, const float* rot_t_even, const float* rot_t_odd,
@@ -1451,7 +1455,7 @@ extern "C" int tq4_write_and_attention(
     int head_dim, int64_t q_token_stride, int64_t q_head_stride, uint8_t* cache,
     int64_t cache_block_stride, int64_t cache_token_stride, int64_t num_blocks, int block_size,
     const int32_t* block_table, int64_t bt_stride, const int32_t* seq_lens,
-    const int32_t* query_start_loc, const float* k_centroids, int n_k_centroids,
+    const int32_t* query_start_loc, int64_t max_seq_len, const float* k_centroids, int n_k_centroids,
     const float* v_centroids, int n_v_centroids, const float* rotation, float sm_scale, int causal,
     int sliding_window, void* out, int out_dtype, int64_t out_token_stride, int64_t out_head_stride,
     float* lse_out, int out_rotated, void* workspace, size_t workspace_bytes, int mode,
@@ -1500,10 +1504,34 @@ extern "C" int tq4_write_and_attention(
   }
   return attention_impl(wr, q, q_dtype, num_rows, num_seqs, num_q_heads, num_kv_heads, head_dim,
                         q_token_stride, q_head_stride, cache, cache_block_stride, cache_token_stride,
-                        num_blocks, block_size, block_table, bt_stride, seq_lens, query_start_loc,
+                        num_blocks, block_size, block_table, bt_stride, seq_lens, query_start_loc, max_seq_len,
                         k_centroids, n_k_centroids, v_centroids, n_v_centroids, rotation, sm_scale,
                         causal, sliding_window, out, out_dtype, out_token_stride, out_head_stride,
                         lse_out, out_rotated, workspace, workspace_bytes, mode, err_flag, stream);
+}
+
+extern "C" int tq4_write_and_attention(
+    const void* key, const void* value, int kv_dtype, int64_t n_tokens, int64_t k_token_stride,
+    int64_t k_head_stride, int64_t v_token_stride, int64_t v_head_stride,
+    const int64_t* slot_mapping, int64_t n_slots, const float* rot_t_even, const float* rot_t_odd,
+    const float* k_boundaries, int n_k_boundaries, const float* v_boundaries, int n_v_boundaries,
+    const void* q, int q_dtype, int64_t num_rows, int num_seqs, int num_q_heads, int num_kv_heads,
+    int head_dim, int64_t q_token_stride, int64_t q_head_stride, uint8_t* cache,
+    int64_t cache_block_stride, int64_t cache_token_stride, int64_t num_blocks, int block_size,
+    const int32_t* block_table, int64_t bt_stride, const int32_t* seq_lens,
+    const int32_t* query_start_loc, const float* k_centroids, int n_k_centroids,
+    const float* v_centroids, int n_v_centroids, const float* rotation, float sm_scale, int causal,
+    int sliding_window, void* out, int out_dtype, int64_t out_token_stride, int64_t out_head_stride,
+    float* lse_out, int out_rotated, void* workspace, size_t workspace_bytes, int mode,
+    int* err_flag, void* stream) {
+  return tq4_attention_step(key, value, kv_dtype, n_tokens, k_token_stride, k_head_stride, v_token_stride, v_head_stride,
+                            slot_mapping, n_slots, rot_t_even, rot_t_odd, k_boundaries, n_k_boundaries, v_boundaries,
+                            n_v_boundaries, q, q_dtype, num_rows, num_seqs, num_q_heads, num_kv_heads, head_dim,
+                            q_token_stride, q_head_stride, cache, cache_block_stride, cache_token_stride, num_blocks,
+                            block_size, block_table, bt_stride, seq_lens, query_start_loc, 0, k_centroids, n_k_centroids,
+                            v_centroids, n_v_centroids, rotation, sm_scale, causal, sliding_window, out, out_dtype,
+                            out_token_stride, out_head_stride, lse_out, out_rotated, workspace, workspace_bytes, mode,
+                            err_flag, stream);
 }
 
 extern "C" int tq4_combine_partials(const float* parts_o, const float* parts_lse, int world,

@@ -82,6 +82,7 @@ struct AttnArgs {
   int64_t bt_stride;
   const int32_t* seq_lens;
   const int32_t* query_start_loc;  // nullptr = decode
+  int64_t max_keys;  // host side only: no sequence is longer (as far as the caller says, and the block table's width)
   const float* k_centroids;
   const float* v_centroids;
   int n_k_centroids, n_v_centroids;

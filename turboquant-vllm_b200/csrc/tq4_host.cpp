@@ -195,9 +195,9 @@ at::Tensor slots64(const at::Tensor& s) {
 
 // attention(q, kv_cache, block_table, seq_lens, k_centroids, v_centroids, rotation, num_kv_heads, block_size,
 //           sm_scale, query_start_loc, causal, sliding_window, out, out_dtype, lse_out, out_rotated, workspace,
-//           mode, write)
+//           mode, write, max_seq_len)
 PyObject* attention(PyObject*, PyObject* const* p, Py_ssize_t n) {
-  if (!expect("attention", n, 20)) return nullptr;
+  if (!expect("attention", n, 21)) return nullptr;
   return guarded([&]() -> PyObject* {
     at::Tensor q = cuda_tensor(p[0], "q");
     const at::Tensor& cache = cuda_tensor(p[1], "kv_cache");
@@ -251,56 +251,52 @@ PyObject* attention(PyObject*, PyObject* const* p, Py_ssize_t n) {
     if (have < need)
       fail(PyExc_ValueError, "workspace has " + std::to_string(have) + " bytes, " + std::to_string(need) + " needed");
     const int causal = truth(p[11]) ? 1 : 0, window = (int)int_or_zero(p[12]);
+    const int64_t max_seq_len = p[20] == Py_None ? 0 : as_int(p[20]);
     const int rotated = truth(p[16]) ? 1 : 0, mode = (int)as_int(p[18]);
     int* flag = (int*)flag_of(dev).data_ptr();
     const int q_dt = dtype_code(q.scalar_type()), out_dt = dtype_code(out.scalar_type());
-    int st;
-    if (p[19] == Py_None) {
-      {
-        const NoGil no_gil;
-        st = tq4_paged_attention(
-            q.data_ptr(), q_dt, t, (int)lens.numel(), (int)hq, (int)hkv, (int)d, q.stride(0),
-            q.stride(1), (const uint8_t*)cache.data_ptr(), cache.stride(0), cache.stride(1), cache.size(0), (int)block,
-            (const int32_t*)bt.data_ptr(), bt.stride(0), (const int32_t*)lens.data_ptr(),
-            qsl ? (const int32_t*)qsl->data_ptr() : nullptr, (const float*)kc.data_ptr(), (int)kc.numel(),
-            (const float*)vc.data_ptr(), (int)vc.numel(), (const float*)rot.data_ptr(), scale, causal, window,
-            out.data_ptr(), out_dt, out.stride(0), out.stride(1), lse, rotated, ws.data_ptr(), have,
-            mode, flag, launch.stream);
-      }
-    } else {
-      // any iterable of seven, held until the call returns
-      struct Held {
+    // the new tokens to be written first, if any
+    at::Tensor key, value, slots, even, odd, kb, vb;
+    int kv_dt = TQ4_F32;
+    if (p[19] != Py_None) {
+      struct Held {  // any iterable of seven
         PyObject* o;
         ~Held() { Py_XDECREF(o); }
       } seq{PySequence_Tuple(p[19])};
       if (!seq.o) throw PyError{};
       if (PyTuple_GET_SIZE(seq.o) != 7) fail(PyExc_ValueError, "write must hold seven tensors");
       auto item = [&](int i, const char* name) -> const at::Tensor& { return cuda_tensor(PyTuple_GET_ITEM(seq.o, i), name); };
-      at::Tensor key = item(0, "key"), value = item(1, "value");
-      const at::Tensor slots = slots64(item(2, "slot_mapping"));
-      const at::Tensor &even = item(3, "rotation_T_even"), &odd = item(4, "rotation_T_odd");
-      const at::Tensor &kb = item(5, "k_boundaries"), &vb = item(6, "v_boundaries");
+      key = item(0, "key");
+      value = item(1, "value");
+      slots = slots64(item(2, "slot_mapping"));
+      even = item(3, "rotation_T_even");
+      odd = item(4, "rotation_T_odd");
+      kb = item(5, "k_boundaries");
+      vb = item(6, "v_boundaries");
       TQ4_ASSERT(cache.is_contiguous(), "the fused write addresses flat slots: block-major contiguous cache");
       TQ4_ASSERT(key.sizes() == value.sizes() && key.scalar_type() == value.scalar_type() && key.dim() == 3 &&
                      key.size(1) == hkv && key.size(2) == d,
                  "key and value must be [tokens, KV heads, head_dim] of one type");
       key = inner_contiguous(key);
       value = inner_contiguous(value);
-      const int kv_dt = dtype_code(key.scalar_type());
-      {
-        const NoGil no_gil;
-        st = tq4_write_and_attention(
-            key.data_ptr(), value.data_ptr(), kv_dt, key.size(0), key.stride(0), key.stride(1),
-            value.stride(0), value.stride(1), (const int64_t*)slots.data_ptr(), slots.numel(), (const float*)even.data_ptr(),
-            (const float*)odd.data_ptr(), (const float*)kb.data_ptr(), (int)kb.numel(), (const float*)vb.data_ptr(),
-            (int)vb.numel(), q.data_ptr(), q_dt, t, (int)lens.numel(), (int)hq, (int)hkv, (int)d,
-            q.stride(0), q.stride(1), (uint8_t*)cache.data_ptr(), cache.stride(0), cache.stride(1), cache.size(0), (int)block,
-            (const int32_t*)bt.data_ptr(), bt.stride(0), (const int32_t*)lens.data_ptr(),
-            qsl ? (const int32_t*)qsl->data_ptr() : nullptr, (const float*)kc.data_ptr(), (int)kc.numel(),
-            (const float*)vc.data_ptr(), (int)vc.numel(), (const float*)rot.data_ptr(), scale, causal, window,
-            out.data_ptr(), out_dt, out.stride(0), out.stride(1), lse, rotated, ws.data_ptr(), have,
-            mode, flag, launch.stream);
-      }
+      kv_dt = dtype_code(key.scalar_type());
+    }
+    auto floats = [](const at::Tensor& t) { return t.defined() ? (const float*)t.data_ptr() : nullptr; };
+    const bool wr = key.defined();
+    int st;
+    {
+      const NoGil no_gil;
+      st = tq4_attention_step(
+          wr ? key.data_ptr() : nullptr, wr ? value.data_ptr() : nullptr, kv_dt, wr ? key.size(0) : 0, wr ? key.stride(0) : 0,
+          wr ? key.stride(1) : 0, wr ? value.stride(0) : 0, wr ? value.stride(1) : 0,
+          wr ? (const int64_t*)slots.data_ptr() : nullptr, wr ? slots.numel() : 0, floats(even), floats(odd), floats(kb),
+          wr ? (int)kb.numel() : 0, floats(vb), wr ? (int)vb.numel() : 0, q.data_ptr(), q_dt, t, (int)lens.numel(), (int)hq,
+          (int)hkv, (int)d, q.stride(0), q.stride(1), (uint8_t*)cache.data_ptr(), cache.stride(0), cache.stride(1),
+          cache.size(0), (int)block, (const int32_t*)bt.data_ptr(), bt.stride(0), (const int32_t*)lens.data_ptr(),
+          qsl ? (const int32_t*)qsl->data_ptr() : nullptr, max_seq_len, (const float*)kc.data_ptr(), (int)kc.numel(),
+          (const float*)vc.data_ptr(), (int)vc.numel(), (const float*)rot.data_ptr(), scale, causal, window,
+          out.data_ptr(), out_dt, out.stride(0), out.stride(1), lse, rotated, ws.data_ptr(), have,
+          mode, flag, launch.stream);
     }
     check(st, "paged_tq4_attention");
     if (!own_out) {

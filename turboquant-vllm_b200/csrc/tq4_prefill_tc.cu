@@ -1284,12 +1284,14 @@ bool prefill_tc_supported(const AttnArgs& a) {
 }
 
 // Parts of the key range: as many as fill the SMs when the row blocks do not, at least four tiles each; limited
-// by the room for their partials (`slots` vectors sets of Hq in the scratch).
+// by the room for their partials (`slots` vectors sets of Hq in the scratch).  The tiles are those of the caller's
+// max_seq_len: by the width of a server's table a prompt of 300 tokens (32 / 8 heads of 128) was cut into parts of at
+// most two tiles, 52.3 instead of 35.9 us.
 int prefill_tc_splits(const AttnArgs& a, int64_t slots) {
   const int per_cta = (a.sh.D == 256 ? 1 : 2) * (128 / a.sh.G);
   const int64_t ctas = (int64_t)((a.sh.rows + per_cta - 1) / per_cta) * a.sh.Hkv;
   int64_t s = sm_count() / (ctas > 0 ? ctas : 1);
-  const int64_t tiles = a.bt_stride * a.block_size / kBN;
+  const int64_t tiles = a.max_keys / kBN;
   if (s > tiles / 4) s = tiles / 4;
   if (s > 8) s = 8;
   if (a.sh.rows > 0 && s > slots / a.sh.rows) s = slots / a.sh.rows;

@@ -235,6 +235,7 @@ def paged_tq4_attention(
     workspace: torch.Tensor | None = None,
     mode: int = 0,
     write: tuple | None = None,
+    max_seq_len: int | None = None,
 ) -> torch.Tensor:
     """Attention of ``q [T, Hq, D]`` over the packed paged cache.
 
@@ -247,10 +248,14 @@ def paged_tq4_attention(
     causal mask).  ``mode``: 0 auto, 1 fp32 CUDA-core kernel, 2 streaming tensor-core LUT kernel,
     3 chunked-prefill tcgen05 kernel, 4 the same with single fp16 terms for
     queries and probabilities (faster, about 1e-3 absolute error; never picked automatically).
+    ``max_seq_len``: length of the longest sequence, if the caller has it on the host.  Only the choice of
+    kernels reads it, for which the width of ``block_table`` stands in otherwise (a serving engine's
+    is as wide as its model allows).
     """
     return nv.host().attention(
         q, kv_cache, block_table, seq_lens, k_centroids, v_centroids, rotation, num_kv_heads, block_size, sm_scale,
-        query_start_loc, causal, sliding_window, out, out_dtype, lse_out, out_rotated, workspace, mode, write)
+        query_start_loc, causal, sliding_window, out, out_dtype, lse_out, out_rotated, workspace, mode, write,
+        max_seq_len)
 
 
 def tq4_write_and_attention(
@@ -343,6 +348,7 @@ def fused_paged_tq4_prefill(
     sliding_window: int | None = None,
     workspace: torch.Tensor | None = None,
     mode: int = 0,
+    max_seq_len: int | None = None,
 ) -> torch.Tensor:
     """Multi-sequence, prefix-aware chunked prefill over the packed cache."""
     assert q.shape[2] == head_dim
@@ -350,7 +356,7 @@ def fused_paged_tq4_prefill(
         q, kv_cache, block_table, seq_lens, centroids,
         centroids if v_centroids is None else v_centroids, rotation, num_kv_heads, block_size,
         sm_scale, query_start_loc=query_start_loc, causal=causal, sliding_window=sliding_window,
-        out=out, workspace=workspace, mode=mode,
+        out=out, workspace=workspace, mode=mode, max_seq_len=max_seq_len,
     )
 
 

@@ -470,6 +470,7 @@ class TQ4AttentionImpl(FlashAttentionImpl):
             key, value, slot_mapping = write
             write = (key, value, slot_mapping, self._tq4_rot_T_even, self._tq4_rot_T_odd,
                      self._k_boundaries, self._v_boundaries)
+        longest = getattr(attn_metadata, "max_seq_len", None)  # (the block table is max_model_len wide)
         ops.paged_tq4_attention(
             query[:n], kv_cache, attn_metadata.block_table, attn_metadata.seq_lens,
             self._k_centroids, self._v_centroids, self._tq4_rotation, self.num_kv_heads,
@@ -477,7 +478,7 @@ class TQ4AttentionImpl(FlashAttentionImpl):
             query_start_loc=None if decode else attn_metadata.query_start_loc,
             causal=bool(getattr(attn_metadata, "causal", True)),
             sliding_window=self._sliding_window_tokens(),
-            out=output[:n], workspace=ws, write=write,
+            out=output[:n], workspace=ws, write=write, max_seq_len=longest if isinstance(longest, int) else None,
         )
         # opt-in (TQ4_CHECK_ERRORS=1): surface out-of-range slots / block ids and timed-out device
         # waits as an exception instead of silently skipped rows; never during graph capture
