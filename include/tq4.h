@@ -207,6 +207,13 @@ size_t tq4_attention_workspace_bytes(int64_t max_query_rows, int num_q_heads, in
  *              cores as single fp16 terms (mode 3 splits both into hi + lo), which halves the
  *              tensor work and lets their 2^-11 rounding reach the output (about 1e-3 absolute:
  *              at the edge of the 2e-3 parity bound, hence never chosen by mode 0)
+ * Precision of modes 0, 2 and 3: 4e-5 to 1.1e-4 of relative 2-norm against 64 bits on N(0, 1) data with outlier
+ * channels, fp32 outputs, nearly all of it the centroids on the fp16 grid of the tensor cores; a 16-bit output's own
+ * rounding is 2e-4 (fp16) or 1.7e-3 (bf16).  The streaming kernel adds little to that (fp32 rotations, short sums).  The
+ * prefill kernel rotates and un-rotates with two-term fp16 products (22 bits) and sums its output in tensor memory,
+ * whose additions truncate: at most 8 * 2^-23 per 64 keys of a part.  Measured distance of the two kernels, keys not
+ * cut: 1.4e-6 at 400 keys, 6e-6 at 4096, 1.3e-5 at 10 000, 3.6e-5 at 32 000 (in all 8.76e-5 against 8.53e-5 at 10 000
+ * keys, 1.06e-4 against 9.05e-5 at 32 000).
  * A row that sees no key (seq_len 0) gets zeros, and so does a row past the last offset of
  * query_start_loc, which belongs to no sequence.
  */

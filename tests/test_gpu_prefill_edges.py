@@ -158,3 +158,35 @@ def test_known_length_decides_instead_of_the_table_width(cuda_lib, hq, hkv, lens
     wrong = ops.paged_tq4_attention(*args, query_start_loc=qsl, out_dtype=torch.float32, max_seq_len=1)
     want = ops.paged_tq4_attention(*args, query_start_loc=qsl, out_dtype=torch.float32, mode=2)
     assert (out - want).abs().max() <= 2e-3 and (wrong - want).abs().max() <= 2e-3
+
+
+@pytest.mark.parametrize("d,hq,hkv,lens,new", [
+    (128, 32, 8, [2900, 1500, 700], [400, 300, 700]),
+    (128, 28, 4, [700], [333]),                # cut along the keys
+    (64, 14, 2, [2900, 300], [500, 300]),
+    (96, 8, 8, [2900, 300], [300, 300]),
+    (256, 8, 4, [2900, 300], [300, 300]),
+])
+@pytest.mark.parametrize("q_dtype", [torch.bfloat16, torch.float32])
+def test_prefill_kernel_next_to_the_streaming_kernel(cuda_lib, d, hq, hkv, lens, new, q_dtype):
+    """Both read keys and values through the same fp16 tables, so what separates them is the prefill kernel's own:
+    the sum O in tensor memory, truncated by every MMA (eight a tile of 64 keys, at most 2^-23 of the sum each), and
+    two-term fp16 operands (2^-22 of a row's largest coordinate: with scores of about ten, 2^-18 of a weight)."""
+    from turboquant_vllm.kernels import ops
+
+    p, gen = Prims(d).cuda(), torch.Generator(device="cuda").manual_seed(1)
+    rand = lambda *shape: torch.randn(*shape, device="cuda", generator=gen)  # noqa: E731
+    pages = [-(-n // 16) for n in lens]
+    cache = torch.zeros(sum(pages), 16, hkv * O.padded_slot_bytes(d), dtype=torch.uint8, device="cuda")
+    k, v = rand(2, cache.shape[0] * 16, hkv, d)
+    k[..., 5] *= 8
+    ops.tq4_write_paged(k, v, cache, torch.arange(k.shape[0], device="cuda"), p["even"], p["odd"], p["kb"], p["vb"])
+    table = torch.zeros(len(lens), max(pages), dtype=torch.int32, device="cuda")
+    for i, n in enumerate(pages):
+        table[i, :n] = torch.arange(n) + sum(pages[:i])
+    q = rand(sum(new), hq, d).to(q_dtype)
+    qsl = torch.tensor(np.concatenate([[0], np.cumsum(new)]), dtype=torch.int32).cuda()
+    args = (q, cache, table, torch.tensor(lens, dtype=torch.int32).cuda(), p["kc"], p["vc"], p["rot"], hkv, 16)
+    a, b = (ops.paged_tq4_attention(*args, query_start_loc=qsl, out_dtype=torch.float32, mode=m).double() for m in (3, 2))
+    tiles = -(-max(lens) // 64)
+    assert (a - b).norm() / b.norm() <= 8 * tiles * 2.0**-23 + 2.0**-18
