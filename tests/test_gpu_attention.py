@@ -595,3 +595,55 @@ def test_captured_call_owns_its_scratch(ops):
         torch.cuda.synchronize()
         assert torch.equal(out, want)
         del junk
+
+
+def test_first_calls_of_several_threads(cuda_lib):
+    """A fresh process whose first calls come from eight threads at a time: every shape, and every set-up step."""
+    import os
+    import subprocess
+    import sys
+
+    prog = """
+import sys, threading, torch
+sys.path.insert(0, {pkg!r})
+from turboquant_vllm import TurboQuantMSE
+from turboquant_vllm.kernels import ops
+torch.zeros(1, device="cuda")
+work, bad, go = [], [], threading.Barrier(8)
+for i in range(8):
+    hkv, d = ((8, 128), (4, 128), (8, 128), (1, 128), (8, 64), (8, 96), (4, 256), (2, 128))[i]
+    p = TurboQuantMSE(d, 4)
+    r = p.rotation.cuda().contiguous()
+    rt = r.T.contiguous()
+    even, odd = rt[:, 0::2].contiguous(), rt[:, 1::2].contiguous()
+    c, b = p.codebook.centroids.cuda(), p.codebook.boundaries.cuda()
+    width = hkv * (1 << (d + 7).bit_length())
+    cache = torch.zeros(64, 16, width, dtype=torch.uint8, device="cuda")
+    table = torch.arange(64, dtype=torch.int32, device="cuda").view(4, 16)
+    lens = torch.full((4,), 256, dtype=torch.int32, device="cuda")
+    kv = torch.randn(1024, hkv, d, device="cuda").bfloat16()
+    q = torch.randn(4, 4 * hkv, d, device="cuda").bfloat16()
+    work.append((kv, cache, even, odd, b, q, table, lens, c, r, hkv))
+torch.cuda.synchronize()
+def run(kv, cache, even, odd, b, q, table, lens, c, r, hkv):
+    try:
+        with torch.cuda.stream(torch.cuda.Stream()):
+            go.wait()
+            ops.tq4_write_paged(kv, kv, cache, torch.arange(1024, device="cuda"), even, odd, b, b)
+            out = ops.paged_tq4_attention(q, cache, table, lens, c, c, r, hkv, 16)
+            torch.cuda.current_stream().synchronize()
+            assert torch.isfinite(out).all() and out.abs().max() > 0
+    except BaseException as e:
+        bad.append(repr(e))
+threads = [threading.Thread(target=run, args=w) for w in work]
+for t in threads: t.start()
+for t in threads: t.join()
+print(bad)
+sys.exit(bool(bad))
+"""
+    import turboquant_vllm
+
+    pkg = os.path.dirname(os.path.dirname(turboquant_vllm.__file__))
+    for _ in range(3):
+        done = subprocess.run([sys.executable, "-c", prog.format(pkg=pkg)], capture_output=True, text=True, timeout=300)
+        assert done.returncode == 0, done.stdout + done.stderr

@@ -1,10 +1,14 @@
 // Shared device/host helpers for the TQ4 sm_100a kernels.
 #pragma once
 
+#include <cuda.h>
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <atomic>
+#include <mutex>
 
 #include "tq4.h"
 
@@ -217,12 +221,16 @@ inline int sm_count() {
 }
 
 // Opt `Kernel` in to `bytes` of dynamic shared memory on the current device (once per device and
-// kernel; again if a later call asks for more).
+// kernel; again if a later call asks for more).  Entry points run without the GIL, so several threads may come
+// here for the first time together: the attribute and the record of it change under one lock.
 template <auto Kernel>
 inline bool ensure_dynamic_smem(int bytes, bool max_carveout = false) {
-  static int set_bytes[kMaxDevices];
+  static std::atomic<int> set_bytes[kMaxDevices];
+  static std::mutex lock;
   const int dev = device_ordinal();
   if (dev < 0) return false;
+  if (set_bytes[dev] >= bytes && set_bytes[dev] > 0) return true;
+  const std::lock_guard<std::mutex> held(lock);
   if (set_bytes[dev] >= bytes && set_bytes[dev] > 0) return true;
   if (cudaFuncSetAttribute(Kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess)
     return false;
@@ -230,6 +238,22 @@ inline bool ensure_dynamic_smem(int bytes, bool max_carveout = false) {
     cudaFuncSetAttribute(Kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
   set_bytes[dev] = bytes;
   return true;
+}
+
+// The driver's tensor-map encoder (the library does not link to libcuda), looked up once; null if it has none.
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
+                                  CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
+                                  CUtensorMapFloatOOBfill);
+inline EncodeTiledFn encode_tiled_fn() {
+  static const EncodeTiledFn fn = []() -> EncodeTiledFn {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    const bool found = cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
+                       q == cudaDriverEntryPointSuccess;
+    return found ? reinterpret_cast<EncodeTiledFn>(p) : nullptr;
+  }();
+  return fn;
 }
 
 // Arguments of the compress / cache-write kernels (tq4_compress.cu) and of the write part of the

@@ -16,7 +16,6 @@
 //   48 x tcgen05.mma 128x128x8 over two K-steps of 64, D in 128 TMEM columns   tensor cores
 //   tcgen05.ld of the thread's 64 columns, bucketize, pack, store              CUDA cores
 // Pi (hi and lo) stays resident in shared memory: 2 x 64 KB.  Every wait is bounded.
-#include <cuda.h>
 #include <math_constants.h>
 
 #include <cstdlib>
@@ -418,26 +417,9 @@ bool compress_tc_eligible(const CompressArgs& a, int head_dim, int dtype) {
   return true;
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
-                                  CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
-                                  CUtensorMapFloatOOBfill);
-static EncodeTiledFn encode_fn() {
-  static EncodeTiledFn fn = nullptr;
-  static bool tried = false;
-  if (!tried) {
-    tried = true;
-    void* ptr = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(ptr);
-  }
-  return fn;
-}
 // rows of one source as a 2-D tensor [rows][128] of 16-bit elements; box = 128 rows x 64 columns
 static bool make_x_map(CUtensorMap* m, const void* x, int64_t rows) {
-  EncodeTiledFn fn = encode_fn();
+  EncodeTiledFn fn = encode_tiled_fn();
   if (!fn || rows <= 0) return false;
   const cuuint64_t dims[2] = {(cuuint64_t)kD, (cuuint64_t)rows};
   const cuuint64_t strides[1] = {(cuuint64_t)kD * 2};

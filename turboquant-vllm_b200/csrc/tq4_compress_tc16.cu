@@ -35,7 +35,6 @@
 // one cannot hold Pi and two stages of vectors).
 // Every mbarrier wait is bounded; a wait that gives up marks the CTA dead, all roles drain and the
 // kernel reports TQ4_DEV_TIMEOUT.  Tensor memory is released on every path.
-#include <cuda.h>
 #include <math_constants.h>
 
 #include <cstdlib>
@@ -642,27 +641,10 @@ compress_tc16_kernel(const __grid_constant__ CompressArgs a, const int group_row
   }
 }
 
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
-                                  CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
-                                  CUtensorMapFloatOOBfill);
-EncodeTiledFn encode_fn() {
-  static EncodeTiledFn fn = nullptr;
-  static bool tried = false;
-  if (!tried) {
-    tried = true;
-    void* ptr = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(ptr);
-  }
-  return fn;
-}
 // One source as a 3-D tensor [groups][rows of a group][D] of 16-bit elements: a group is a token and its rows the heads
 // when the heads divide a tile (any token and head stride), else one row of a dense array.  Box: 128 rows x 64 columns.
 bool make_x_map(CUtensorMap* m, const CompressArgs& a, int src, int D, int group_rows) {
-  EncodeTiledFn fn = encode_fn();
+  EncodeTiledFn fn = encode_tiled_fn();
   const int64_t rows = a.n_tokens * a.num_heads;
   if (!fn || rows <= 0) return false;
   const cuuint64_t dims[3] = {(cuuint64_t)D, (cuuint64_t)group_rows, (cuuint64_t)(rows / group_rows)};
@@ -720,7 +702,7 @@ int launch_d(const CompressArgs& a, int head_dim, cudaStream_t st) {
 bool compress_tc16_eligible(const CompressArgs& a, int head_dim, int dtype) {
   static const bool disabled = getenv("TQ4_NO_TC") != nullptr || getenv("TQ4_NO_TC16") != nullptr;
   if (disabled || !supported_head_dim(head_dim) || (dtype != TQ4_F16 && dtype != TQ4_BF16)) return false;
-  if (a.n_tokens * a.num_heads >= (1ll << 31) || encode_fn() == nullptr || !tokens_uniform(a)) return false;
+  if (a.n_tokens * a.num_heads >= (1ll << 31) || encode_tiled_fn() == nullptr || !tokens_uniform(a)) return false;
   for (int s = 0; s < a.n_sources; ++s)
     if (((uintptr_t)a.x[s] & 15) || a.head_stride[s] <= 0 || a.token_stride[s] <= 0 || a.head_stride[s] % 8 || a.token_stride[s] % 8)
       return false;

@@ -28,7 +28,6 @@
 // back to per-thread cp.async of exactly the bytes each thread consumes.  Tiles are read back
 // with 16/8-byte shared loads at compile-time offsets; a token permutation plus the 64-byte TMA
 // swizzle keep them free of bank conflicts.
-#include <cuda.h>
 #include <math_constants.h>
 
 #include <cstdlib>
@@ -1572,24 +1571,6 @@ attention_mma_kernel(const AttnArgs a, const CompressArgs w, const int has_write
 }
 
 // ---- TMA tensor maps over the paged cache: dims (row bytes, tokens in a block, blocks) -----------
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                  const cuuint64_t*, const cuuint32_t*, const cuuint32_t*,
-                                  CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
-                                  CUtensorMapFloatOOBfill);
-EncodeTiledFn encode_tiled_fn() {
-  static EncodeTiledFn fn = nullptr;
-  static bool tried = false;
-  if (!tried) {
-    tried = true;
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
-        q == cudaDriverEntryPointSuccess)
-      fn = reinterpret_cast<EncodeTiledFn>(p);
-  }
-  return fn;
-}
-
 bool make_cache_map(CUtensorMap* m, const AttnArgs& a, uint32_t box_bytes, bool swizzle64) {
   EncodeTiledFn fn = encode_tiled_fn();
   if (!fn) return false;
