@@ -925,13 +925,15 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
     };
     bool ok = true;
     const bool use = n_tiles > 0 && blk < n_blk;  // (uniform per warp)
-    // the raw queries, for every live row of the CTA: waited for whether this part has keys or not
-    if (q_staged && (use || n_tiles == 0)) ok = bar_wait_own(bar(s_bars.qraw), 0u, dead);
+    // the raw queries were asked for, whether this part has keys (then the wait is below) or not.  (One wait for both
+    // here, in front of the branch, lengthens a tile by 2 %: 4977 against 4863 us at 8 x 2048 rows on 8192 cached.)
+    if (q_staged && n_tiles == 0) bar_wait_own(bar(s_bars.qraw), 0u, dead);
 
     // ---- rotate the queries -----------------------------------------------------------------------
     float qscale = 0.f;
     if (use) {
       // (code that runs once per CTA costs its instruction fetches: short rolled loops)
+      if (q_staged) ok = bar_wait_own(bar(s_bars.qraw), 0u, dead);
       auto load_q = [&](int c, float (&x)[32]) {
         if (!live) {
 #pragma unroll
