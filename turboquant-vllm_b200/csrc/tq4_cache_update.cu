@@ -8,9 +8,11 @@
 // copies into the buffers), which bounded a step by its host time.  A warp takes four vectors, a lane D / 32
 // consecutive coordinates of each; both products read Pi from shared memory (once transposed, once as
 // it is; at head_dim 256, where that does not fit, in chunks of 64 rows) and the vectors from a strip per warp.
-// A step of a few tokens is latency bound (staging Pi: 128 KB per block), so its vectors are spread over the blocks
-// first; a prompt is bound by FMA issue.
-// Measured: a generation of 8 tokens behind 4 prompts of 1100, 2 layers of 8 heads of 128, 7800 -> 357 us.
+// A step of a few tokens is bound by latency and has a kernel of its own (cache_update_tiny_kernel); a prompt is bound by
+// FMA issue and the reads of Pi.
+// The kernels' own times, against the chain's (ncu: cold, serialised; bf16, 8 heads of 128, K4 / V3): a prompt of
+// 4 x 1100 tokens 293 us in 26 launches -> 124 in two (16 of them the write kernel's), one token of each 103 us in 25
+// launches -> 11 in one.
 #include <math_constants.h>
 
 #include "tq4_common.cuh"
@@ -467,9 +469,10 @@ int launch_update(const UpdateArgs& a, cudaStream_t st) {
   return launch_update<D, 4>(a, st);
 }
 
-// The writes that the tensor cores make (dispatch_compress, head_dim 128 above kSmallRows vectors a tensor) are made by them
-// here too: the indices are the same whichever call a vector arrives in, and half of the FMAs go away
-// (the generation named above: 486 -> 452 us, then host time).
+// The compression that the tensor cores do for a tensor by itself (dispatch_compress, head_dim 128 above kSmallRows
+// vectors) is theirs here, too: the indices are those of tq4_compress of that tensor, and half of the FMAs go away (8 tokens
+// behind 4 x 1100, 2 layers: 486 -> 452 us).  A paged write counts K and V together, so between 4097 and 8192 vectors a
+// tensor its indices are the tensor cores' and may differ from these, within the write path's bound.
 bool compress_first(int batch, int heads, int n_new, int head_dim) {
   return head_dim == 128 && (int64_t)batch * heads * n_new > kSmallRows;
 }
