@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 compress_tc_kernel(const CompressArgs a, const __grid_constant__ CUtensorMap tm_x0,
                    const __grid_constant__ CUtensorMap tm_x1) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
-  __shared__ __align__(8) uint64_t s_bar[3];  // [0]: first K-step's MMAs done, [1]: tile's MMAs done, [2]: input tile landed
+  __shared__ __align__(8) uint64_t s_bar[4];  // [0]: first K-step's MMAs done, [1]: tile's, [2]: input tile landed, [3]: a dead CTA's MMAs done
   __shared__ uint32_t s_tmem;
   __shared__ int s_dead;
   __shared__ float s_bounds[2][16];
@@ -192,6 +192,7 @@ compress_tc_kernel(const CompressArgs a, const __grid_constant__ CUtensorMap tm_
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar0) : "memory");
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar1) : "memory");
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&s_bar[2])) : "memory");
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&s_bar[3])) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     s_dead = 0;
   }
@@ -235,7 +236,11 @@ compress_tc_kernel(const CompressArgs a, const __grid_constant__ CUtensorMap tm_
     tma_load_2d(base + kOffX, s_ ? &tm_x1 : &tm_x0, 0, y, bar_x);
     tma_load_2d(base + kOffX + kBlockBytes, s_ ? &tm_x1 : &tm_x0, 64, y, bar_x);
   };
-  if (XT && (int64_t)blockIdx.x < n_tiles && warp == 0 && elect_one_sync()) fetch_tile(blockIdx.x);
+  uint32_t fetched = 0;  // (the fetching thread) tiles asked for
+  if (XT && (int64_t)blockIdx.x < n_tiles && warp == 0 && elect_one_sync()) {
+    fetch_tile(blockIdx.x);
+    ++fetched;
+  }
 
   for (int64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
     int64_t row;
@@ -332,7 +337,10 @@ compress_tc_kernel(const CompressArgs a, const __grid_constant__ CUtensorMap tm_
         }
         mma_commit(step == 0 ? bar0 : bar1);
         // every thread has read its row for the last time: fetch the rows of this CTA's next tile
-        if (XT && step == 1 && tile + gridDim.x < n_tiles) fetch_tile(tile + gridDim.x);
+        if (XT && step == 1 && tile + gridDim.x < n_tiles) {
+          fetch_tile(tile + gridDim.x);
+          ++fetched;
+        }
       }
     }
     if (s_dead) break;
@@ -399,6 +407,14 @@ compress_tc_kernel(const CompressArgs a, const __grid_constant__ CUtensorMap tm_
   if (s_dead && tid == 0 && a.err_flag) atomicOr(a.err_flag, TQ4_DEV_TIMEOUT);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (s_dead && warp == 0) {  // a dead CTA waits, within a bound, for the tile and the MMAs it has in flight
+    if (elect_one_sync()) {
+      if (fetched > 0) bar_wait_bounded(bar_x, (fetched - 1) & 1u);
+      mma_commit(smem_addr(&s_bar[3]));
+      bar_wait_bounded(smem_addr(&s_bar[3]), 0u);
+    }
+    __syncwarp();
+  }
   if (warp == 0) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_d), "r"(kTmemCols) : "memory");
   }

@@ -33,7 +33,8 @@
 // against a block per vector, 16384 tokens of 4 heads of 256 894 -> 79 us (62 without the
 // second sums below; the 256 columns are split over CTAs:
 // one cannot hold Pi and two stages of vectors).
-// Every mbarrier wait is bounded; a wait that gives up marks the CTA dead, all roles drain and the
+// Every mbarrier wait is bounded; a wait that gives up marks the CTA dead, all roles drain (tiles and MMAs in flight are
+// waited for, again within a bound: they work on memory that the next CTA of the SM is given) and the
 // kernel reports TQ4_DEV_TIMEOUT.  Tensor memory is released on every path.
 #include <math_constants.h>
 
@@ -106,7 +107,7 @@ __device__ __forceinline__ void bar_init(uint32_t bar, uint32_t count) {
 __device__ __forceinline__ void bar_arrive(uint32_t bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
 }
-// Bounded wait that also gives up as soon as another role has marked the CTA dead.
+// Bounded wait that also gives up as soon as another role has marked the CTA dead (`dead` null: only at its bound).
 __device__ __forceinline__ bool bar_wait_bounded(uint32_t bar, uint32_t parity, const volatile int* dead) {
   for (int it = 0; it < (1 << 22); ++it) {
     uint32_t done;
@@ -116,7 +117,7 @@ __device__ __forceinline__ bool bar_wait_bounded(uint32_t bar, uint32_t parity, 
         "selp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(done) : "r"(bar), "r"(parity) : "memory");
     if (done) return true;
-    if ((it & 1023) == 1023 && *dead) return false;
+    if ((it & 1023) == 1023 && dead && *dead) return false;
   }
   return false;
 }
@@ -334,6 +335,7 @@ struct Bars {
   uint64_t empty[4];   // consumers -> TMA: MMAs (1 commit) and the norm readers (4 warps) are done with it
   uint64_t tfull[4];   // MMA -> epilogue: the accumulator holds the tile's product
   uint64_t tempty[4];  // epilogue (4 warps) -> MMA: the accumulator has been read
+  uint64_t drain;      // a dead CTA's last MMA is complete
 };
 
 template <typename T, int D>
@@ -370,6 +372,7 @@ compress_tc16_kernel(const __grid_constant__ CompressArgs a, const int group_row
       bar_init(smem_addr(&s_bars.tfull[s]), 1);
       bar_init(smem_addr(&s_bars.tempty[s]), 4);
     }
+    bar_init(smem_addr(&s_bars.drain), 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     s_dead = 0;
@@ -417,6 +420,7 @@ compress_tc16_kernel(const __grid_constant__ CompressArgs a, const int group_row
   const int64_t n_tiles = tiles_per_src * a.n_sources;
   const int64_t my_tiles = stream < n_tiles ? (n_tiles - stream + n_streams - 1) / n_streams : 0;
   bool ok = true;
+  int64_t fetched = 0;  // (producer) tiles asked for
 
   if (warp == 0) {
     // ================= TMA producer =================
@@ -440,6 +444,7 @@ compress_tc16_kernel(const __grid_constant__ CompressArgs a, const int group_row
           tma_load_3d(dst + kb * kBlockBytes, s_ ? &tm_x1 : &tm_x0, 64 * kb, 0, y / group_rows, bar);
       }
       __syncwarp();
+      fetched = i + 1;
     }
   } else if (warp == 1) {
     // ================= MMA issuer =================
@@ -636,6 +641,18 @@ compress_tc16_kernel(const __grid_constant__ CompressArgs a, const int group_row
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if (s_dead) {
+    if (warp == 0) {
+      for (int64_t i = fetched > STAGES ? fetched - STAGES : 0; i < fetched; ++i)
+        bar_wait_bounded(smem_addr(&s_bars.full[i % STAGES]), (uint32_t)((i / STAGES) & 1), nullptr);
+    } else if (warp == 1) {
+      if (elect_one_sync()) {
+        mma_commit(smem_addr(&s_bars.drain));
+        bar_wait_bounded(smem_addr(&s_bars.drain), 0u, nullptr);
+      }
+      __syncwarp();
+    }
+  }
   if (warp == 1) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(C::kTmemCols) : "memory");
   }

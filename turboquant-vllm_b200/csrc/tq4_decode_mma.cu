@@ -1405,6 +1405,9 @@ attention_mma_kernel(const AttnArgs a, const CompressArgs w, const int has_write
           if (!mbar_wait_bounded(bar0 + st * 8, ph)) {
             if (lane == 0 && a.err_flag) atomicOr(a.err_flag, TQ4_DEV_TIMEOUT);
             dead = true;
+            // the pairs in flight work on the ring, which the next CTA of the SM is given
+            mbar_wait_bounded(bar0 + st * 8, ph);
+            if (k + 1 < n_pairs) mbar_wait_bounded(bar0 + (st ^ 1u) * 8, ph ^ st);
             break;
           }
           if (gk == 0 && k == 0) TQ4_STAMP(5);
@@ -1491,6 +1494,8 @@ attention_mma_kernel(const AttnArgs a, const CompressArgs w, const int has_write
             if (!mbar_wait_bounded(bar0 + (use % kStages) * 8, (use / kStages) & 1u)) {
               if (lane == 0 && a.err_flag) atomicOr(a.err_flag, TQ4_DEV_TIMEOUT);
               dead = true;
+              for (uint32_t u = use; u < gk + min(n_pairs, k + kStages); ++u)  // (as above)
+                mbar_wait_bounded(bar0 + (u % kStages) * 8, (u / kStages) & 1u);
               break;
             }
           } else {

@@ -731,7 +731,9 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
         mma_commit(bar(s_bars.odone));
         if (unrotate) rotate(true, true);
       }
-      if (!ok) {  // (the CTA is dead)
+      if (ok) {  // (as the softmax warps do, unless they have given up)
+        bar_wait_own(unrotate ? bar(s_bars.rot) : bar(s_bars.odone), unrotate ? 1u : 0u, dead);
+      } else {  // (the CTA is dead)
         if (img_n != img_ph) bar_wait_own(bar(s_bars.img), img_ph & 1, dead);
         mma_commit(bar(s_bars.drain));
         bar_wait_own(bar(s_bars.drain), 0u, dead);
