@@ -190,3 +190,44 @@ def test_prefill_kernel_next_to_the_streaming_kernel(cuda_lib, d, hq, hkv, lens,
     a, b = (ops.paged_tq4_attention(*args, query_start_loc=qsl, out_dtype=torch.float32, mode=m).double() for m in (3, 2))
     tiles = -(-max(lens) // 64)
     assert (a - b).norm() / b.norm() <= 8 * tiles * 2.0**-23 + 2.0**-18
+
+
+@pytest.mark.parametrize("d,hq,hkv,v_bits", [(64, 14, 2, 4), (96, 4, 4, 4), (128, 28, 4, 3), (256, 8, 4, 4), (256, 8, 4, 3)])
+@pytest.mark.parametrize("power", [-14, -4, 0, 4, 14])
+def test_prefill_large_and_small_queries(cuda_lib, d, hq, hkv, v_bits, power):
+    """Queries times 2^power over keys times 2^-power: the scores are the same, the factor that makes them is inside the
+    range of the queries' fp16 terms, or partly outside.  Against the streaming kernel, bound as above."""
+    from turboquant_vllm.kernels import ops
+
+    pk, pv, gen = Prims(d).cuda(), Prims(d, v_bits=v_bits).cuda(), torch.Generator(device="cuda").manual_seed(1)
+    rand = lambda *shape: torch.randn(*shape, device="cuda", generator=gen)  # noqa: E731
+    n, new = 300, 150
+    cache = torch.zeros(19, 16, hkv * O.padded_slot_bytes(d), dtype=torch.uint8, device="cuda")
+    ops.tq4_write_paged(rand(n, hkv, d) * 2.0**-power, rand(n, hkv, d), cache, torch.arange(n, device="cuda"), pk["even"],
+                        pk["odd"], pk["kb"], pv["vb"])
+    table = torch.arange(19, dtype=torch.int32, device="cuda")[None]
+    q = (rand(new, hq, d) * 2.0**power).bfloat16()
+    args = (q, cache, table, torch.tensor([n], dtype=torch.int32).cuda(), pk["kc"], pv["vc"], pk["rot"], hkv, 16)
+    qsl = torch.tensor([0, new], dtype=torch.int32).cuda()
+    a, b = (ops.paged_tq4_attention(*args, query_start_loc=qsl, out_dtype=torch.float32, mode=m).double() for m in (3, 2))
+    assert (a - b).norm() / b.norm() <= 8 * 5 * 2.0**-23 + 2.0**-18
+
+
+@pytest.mark.parametrize("d,hq,hkv", [(64, 14, 2), (96, 4, 4), (128, 28, 4), (256, 8, 4)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("pad", [0, 8, 2])
+def test_prefill_16bit_rows_are_the_rounded_fp32_ones(cuda_lib, d, hq, hkv, dtype, pad):
+    """Outputs that leave through shared memory (rows on 16 bytes) or not: each the rounded fp32 result, nothing beside it."""
+    from turboquant_vllm.kernels import ops
+
+    pr = Prims(d)
+    p = pr.cuda()
+    case = build_paged_case([170, 40], hkv, d, 16, pr, seed=5, padded=True)
+    new = [99, 9]
+    q = torch.randn(sum(new), hq, d, generator=torch.Generator().manual_seed(1)).to(dtype).cuda()
+    qsl = torch.tensor([0, 99, 108], dtype=torch.int32).cuda()
+    args = (q, case["cache"].cuda(), case["block_table"].cuda(), case["seq_lens"].cuda(), p["kc"], p["vc"], p["rot"], hkv, 16)
+    want = ops.paged_tq4_attention(*args, query_start_loc=qsl, out_dtype=torch.float32, mode=3).to(dtype)
+    wide = torch.full((sum(new), hq, d + pad), 7.0, dtype=dtype, device="cuda")
+    ops.paged_tq4_attention(*args, query_start_loc=qsl, out=wide[..., :d], mode=3)
+    assert torch.equal(wide[..., :d], want) and (wide[..., d:] == 7).all()

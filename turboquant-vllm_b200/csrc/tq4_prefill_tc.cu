@@ -16,15 +16,21 @@
 //      store the caller's output.  Nothing but queries, cache and outputs touches global memory.
 //
 // Why this shape: a tile costs the tensor pipe 2 x 528 cycles per 128 rows (head_dim 128, two terms), the
-// softmax about 2 100 cycles of latency-bound CUDA-core work (a thread per row, 64 columns) and the dequantisation
-// about 700 + 700 of shared-memory traffic.  With one row block per CTA these formed one chain of 3 550 cycles a
+// softmax about 2 000 cycles of latency-bound CUDA-core work (a thread per row, 64 columns) and the dequantisation
+// about 700 + 700 of shared-memory traffic.  Two score buffers a block, sixteen softmax warps, or rows dealt over quads of lanes
+// (fewer reads of norms) were each no faster: issue, shared memory and tensor memory are all half busy, and what one of
+// these saves the next one takes.  With one row block per CTA these formed one chain of 3 550 cycles a
 // tile; with two blocks the tensor pipe works on one while the other is in its softmax, and a dequantised tile
 // serves 256 rows: 3 600 cycles for twice the rows, 58 % of them tensor work, which at 8 x 2048 rows on 8192 cached
 // tokens (32 / 8 heads) runs into the 1000 W limit.  What bounds it: the chain scores -> softmax -> P -> O and next
 // scores of a block (2 150 + 1 450).  Everything meets at mbarriers only: softmax warps (a thread per row; two at
 // head_dim 256), eight dequantising warps and one issuing thread.
 //   Code that runs once per CTA pays for its instruction fetches (the first version, unrolled, needed 62 000 cycles
-//   before its second tile, this one 30 000): set-up, rotation, masks and the new-reference path are short loops.
+//   before its second tile): set-up, rotation, masks and the new-reference path are short loops, a row's largest
+//   coordinate is found on its packed bits, the rotated row is split without looking for one, and the outputs leave a row a
+//   half-warp.  20 700 -> 15 800 cycles before the loop and 15 600 -> 13 200 after it; with the row factor inside the queries' terms
+//   and 16 columns of P a store: 8 x 2048 rows on 8192 (32 / 8 heads) 4815 -> 4690 us, 1531 rows of 28 / 4 heads with their write
+//   91 -> 81, 8 x 2048 of 8 / 4 heads of 256 in a window of 4096 1285 -> 1203 (there 5 % by one table for K and V).
 //   Tensor memory, per block: [S | P in place][Q hi][Q lo][O]: 64 + 64 + 128 columns at head_dim 128, where
 //   Q lo does not fit and sits in shared memory; at head_dim 256 there is one block of 448 columns and the 64 left
 //   hold a second S, so that the scores of the next tile are computed during the softmax of this one.
@@ -63,7 +69,8 @@ constexpr int kDeq = 256;       // warps 8-15: dequantisation
 constexpr int kThreads = kSmx + kDeq + 32;
 constexpr int kIssueWarp = (kSmx + kDeq) / 32;
 constexpr int kNormBufs = 4;
-constexpr float kHidden = 1e-31f;  // key norm in shared memory of a token whose page id is out of range
+constexpr float kHidden = 1e-33f;  // key norm in shared memory of a token whose page id is out of range
+constexpr float kQGain = 64.f;     // factor of the queries' terms, its inverse in the key norms: keeps the lo terms normal numbers
 
 template <int D>
 struct Cfg {
@@ -95,7 +102,9 @@ struct Cfg {
   static constexpr uint32_t kQPitch = 2 * D + 16;
   static constexpr uint32_t kQStage = NBLK * 128 * kQPitch, kQlo = QLO_SMEM ? NBLK * NC * 128 * 128 : 0;
   static constexpr uint32_t kOffLut = kOffQlo + (((kQStage > kQlo ? kQStage : kQlo) + 1023) & ~1023u);
-  static constexpr int kLutCopies = D == 256 ? 16 : 32;    // (16: room; every lookup is then a two-way conflict)
+  // lane copies of a table entry.  (16: room for no more of two tables; every lookup is then a two-way conflict.  K and V of one
+  // codebook share a table of 32.)
+  static constexpr int kLutCopies = D == 256 ? 16 : 32;
   static constexpr uint32_t kOffNorm = kOffLut + 2 * 256 * kLutCopies * 4;
   static constexpr uint32_t kOffXchg = kOffNorm + kNormBufs * 2 * kBN * 4;
   static constexpr uint32_t kSmem = kOffXchg + (TPR == 2 ? 2 * 2 * 128 * 4 : 0);
@@ -419,7 +428,8 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   __shared__ __align__(8) Bars s_bars;
   __shared__ uint32_t s_tmem;
-  __shared__ int s_info[3];      // sequence, first row and rows of the CTA
+  __shared__ int s_info[5];      // sequence, first row and rows of the CTA; end of the sequence's rows and its length
+  __shared__ float s_cent[2][16];  // scaled centroids of K and V
   __shared__ int s_dead, s_bad;  // a wait gave up / some page id is out of range
   const AttnShape& sh = a.sh;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -435,10 +445,12 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
     int acc = 0, found = -1, first = 0, nrows = 0;
     for (int s0 = 0; s0 < sh.num_seqs && found < 0; s0 += 32) {
       const int s = s0 + lane;
-      int q0 = 0, q1 = 0;
+      int q0 = 0, q1 = 0, q_end = 0, seq_len = 0;
       if (s < sh.num_seqs) {
-        q0 = max(a.query_start_loc[s], 0);
-        q1 = min(a.query_start_loc[s + 1], sh.rows);
+        q0 = max(__ldg(a.query_start_loc + s), 0);
+        q_end = __ldg(a.query_start_loc + s + 1);
+        seq_len = __ldg(a.seq_lens + s);
+        q1 = min(q_end, sh.rows);
       }
       const int n = q1 - q0 >= max(pa.min_rows, 1) ? (q1 - q0 + NBLK * RB - 1) / (NBLK * RB) : 0;
       int incl = n;
@@ -455,6 +467,10 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
         found = s0 + w;
         first = __shfl_sync(0xffffffffu, q0 + b * NBLK * RB, w);
         nrows = __shfl_sync(0xffffffffu, min(NBLK * RB, q1 - (q0 + b * NBLK * RB)), w);
+        if (lane == w) {
+          s_info[3] = q_end;
+          s_info[4] = seq_len;
+        }
       }
       acc += __shfl_sync(0xffffffffu, incl, 31);
     }
@@ -465,6 +481,11 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
       s_dead = 0;
       s_bad = 0;
     }
+  }
+  if (warp == 1) {
+    const int w = lane >> 4, i = lane & 15;
+    const float* cent = w ? a.v_centroids : a.k_centroids;
+    s_cent[w][i] = i < (w ? a.n_v_centroids : a.n_k_centroids) ? __fmul_rn(w ? a.lut_scale_v : a.lut_scale_k, __ldg(cent + i)) : 0.f;
   }
   if (tid == 64) {
     for (int i = 0; i < 2; ++i) {
@@ -534,18 +555,17 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_addr(&s_tmem)), "r"(512u) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
+  bool one_table = C::kLutCopies == 16;
+  if (one_table)
+    for (int i = 0; i < 16; ++i) one_table = one_table && s_cent[0][i] == s_cent[1][i];
   // byte -> half2 tables: (centroid[hi nibble], centroid[lo nibble]) scaled onto the fp16 grid, one copy per lane
   {
-    uint32_t* lut = reinterpret_cast<uint32_t*>(sm + C::kOffLut);
+    uint4* lut = reinterpret_cast<uint4*>(sm + C::kOffLut);
+#pragma unroll 4
     for (int i = tid; i < 512 * C::kLutCopies / 4; i += kThreads) {
-      const int e = i / (C::kLutCopies / 4), w = e >> 8, b = e & 255;
-      const float* cent = w ? a.v_centroids : a.k_centroids;
-      const int nc = w ? a.n_v_centroids : a.n_k_centroids;
-      const float sc = w ? a.lut_scale_v : a.lut_scale_k;
-      const float c_hi = (b >> 4) < nc ? __fmul_rn(sc, __ldg(cent + (b >> 4))) : 0.f;
-      const float c_lo = (b & 15) < nc ? __fmul_rn(sc, __ldg(cent + (b & 15))) : 0.f;
-      const uint32_t v = pack_h2(c_hi, c_lo);
-      reinterpret_cast<uint4*>(lut)[i] = make_uint4(v, v, v, v);
+      const int e = one_table ? i / 8 : i / (C::kLutCopies / 4), w = e >> 8, b = e & 255;
+      const uint32_t v = pack_h2(s_cent[w][b >> 4], s_cent[w][b & 15]);
+      lut[i] = make_uint4(v, v, v, v);
     }
   }
   pdl_trigger();
@@ -557,7 +577,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
 
   PF_STAMP(tid == 0 ? 0 : -1, 0, 5);
   // ---- keys the CTA needs: rows are in query order, their visible ranges move forward with them -----------
-  const int q_end = a.query_start_loc[seq + 1], len = clamp_seq_len(a, max(0, a.seq_lens[seq]));
+  const int q_end = s_info[3], len = clamp_seq_len(a, max(0, s_info[4]));
   auto row_keys = [&](int row, int& lo, int& hi) {  // visible keys of row `row` of the call
     const int pos = len - (q_end - row);
     hi = max(0, min(a.causal ? pos + 1 : len, len));
@@ -813,15 +833,25 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
         it[n].vn = __ldg(reinterpret_cast<const float*>(row + kn_off + vn_delta));
       }
     };
-    auto expand = [&](const uint4& pk, int which, uint32_t buf, int tok, int seg) {  // 16 bytes -> 32 fp16
-      const uint32_t* lut = reinterpret_cast<const uint32_t*>(sm + C::kOffLut) + which * 256 * C::kLutCopies + (lane & (C::kLutCopies - 1));
+    // table entry of a byte: sh bits left of it, plus the lane's copy
+    const int sh = C::kLutCopies == 32 || one_table ? 7 : 6;
+    const uint32_t lut_mask = 255u << sh;
+    uint32_t lut_k = base + C::kOffLut + (lane & ((1 << (sh - 2)) - 1)) * 4;
+    asm volatile("" : "+r"(lut_k) :: "memory");  // (no lookup before the tables are there)
+    const uint32_t lut_v = lut_k + (one_table ? 0u : 256u << sh);
+    auto look = [&](uint32_t at) -> uint32_t {
+      uint32_t y;
+      asm("ld.shared.b32 %0, [%1];" : "=r"(y) : "r"(at));
+      return y;
+    };
+    auto expand = [&](const uint4& pk, uint32_t lut, uint32_t buf, int tok, int seg) {  // 16 bytes -> 32 fp16
       const uint32_t w[4] = {pk.x, pk.y, pk.z, pk.w};
       unsigned char* dst = sm + buf + (seg >> 1) * (kBN * 128);
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
         const uint32_t x = w[c];
-        const uint4 o = make_uint4(lut[(x & 255) * C::kLutCopies], lut[((x >> 8) & 255) * C::kLutCopies],
-                                   lut[((x >> 16) & 255) * C::kLutCopies], lut[(x >> 24) * C::kLutCopies]);
+        const uint4 o = make_uint4(look(lut + ((x << sh) & lut_mask)), look(lut + ((x >> (8 - sh)) & lut_mask)),
+                                   look(lut + ((x >> (16 - sh)) & lut_mask)), look(lut + ((x >> (24 - sh)) & lut_mask)));
         *reinterpret_cast<uint4*>(dst + swz(tok, (seg & 1) * 4 + c)) = o;
       }
     };
@@ -838,10 +868,10 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
       for (int n = 0; n < NIT; ++n) {
         int tok, seg;
         if (item(n, tok, seg)) {
-          expand(it[n].k, 0, C::kOffK + b * C::kKvBuf, tok, seg);
+          expand(it[n].k, lut_k, C::kOffK + b * C::kKvBuf, tok, seg);
           if (seg == 0) {
             // (positive, so that -inf times it stays -inf)
-            ns[tok] = it[n].kn == kHidden ? kHidden : fmaxf(it[n].kn, 1e-30f);
+            ns[tok] = it[n].kn == kHidden ? kHidden : fmaxf(it[n].kn, 1e-30f) * (1.f / kQGain);
             ns[kBN + tok] = it[n].vn;
           }
         }
@@ -871,7 +901,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
 #pragma unroll
       for (int n = 0; n < NIT; ++n) {
         int tok, seg;
-        if (item(n, tok, seg)) expand(v_now[n], 1, C::kOffV + b * C::kKvBuf, tok, seg);
+        if (item(n, tok, seg)) expand(v_now[n], lut_v, C::kOffV + b * C::kKvBuf, tok, seg);
       }
       fence_async();
       __syncwarp();
@@ -932,89 +962,96 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
     if (q_staged && n_tiles == 0) bar_wait_own(bar(s_bars.qraw), 0u, dead);
 
     // ---- rotate the queries -----------------------------------------------------------------------
-    float qscale = 0.f;
+    float qexp = 1.f;  // what is left between a stored dot product and the score (1 unless the queries are very large or small)
     if (use) {
       // (code that runs once per CTA costs its instruction fetches: short rolled loops)
       if (q_staged) ok = bar_wait_own(bar(s_bars.qraw), 0u, dead);
-      auto load_q = [&](int c, float (&x)[32]) {
-        if (!live) {
-#pragma unroll
-          for (int e = 0; e < 32; ++e) x[e] = 0.f;
-        } else if (q_staged) {
-          const uint4* src = reinterpret_cast<const uint4*>(sm + q_at + 64 * c);
-          const bool f16 = a.q_dtype == TQ4_F16;
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            const uint4 r = src[e];
-            half_pair(r.x, f16, x[8 * e], x[8 * e + 1]);
-            half_pair(r.y, f16, x[8 * e + 2], x[8 * e + 3]);
-            half_pair(r.z, f16, x[8 * e + 4], x[8 * e + 5]);
-            half_pair(r.w, f16, x[8 * e + 6], x[8 * e + 7]);
-          }
-        } else {
-          load32(a.q, a.q_dtype, qi + 32 * c, q_vec, x);
+      float sc = 1.f, isc = 1.f;
+      if (q_staged) {  // 16-bit rows in shared memory: the bits without the sign are in the order of the magnitudes
+        const uint4* src = reinterpret_cast<const uint4*>(sm + q_at);
+        const bool f16 = a.q_dtype == TQ4_F16;
+        uint32_t top = 0;
+#pragma unroll 4
+        for (int i = 0; i < DPT / 8; ++i) {
+          const uint4 r = src[i];
+          top = __vmaxu2(__vmaxu2(top, r.x & 0x7FFF7FFFu), __vmaxu2(r.y & 0x7FFF7FFFu, __vmaxu2(r.z & 0x7FFF7FFFu, r.w & 0x7FFF7FFFu)));
         }
-      };
-      float amax = 0.f, sc = 1.f, isc = 1.f;
-#pragma unroll 1
-      for (int pass = 0; pass < 2; ++pass) {
+        float x0, x1;
+        half_pair(top, f16, x0, x1);
+        pow2_scale(row_reduce(live ? fmaxf(x0, x1) : 0.f, fmax_op), sc, isc);
+        if (!live) sc = 0.f;
 #pragma unroll 1
         for (int c = 0; c < DPT / 32; ++c) {
-          float x[32];
-          load_q(c, x);
-          if (pass == 0) {
+          uint32_t h[16];
 #pragma unroll
-            for (int e = 0; e < 16; ++e) amax = max3(amax, fabsf(x[2 * e]), fabsf(x[2 * e + 1]));
-          } else {
-            uint32_t h[16], l[16];
+          for (int e = 0; e < 4; ++e) {
+            const uint4 r = live ? src[4 * c + e] : make_uint4(0u, 0u, 0u, 0u);
+            const uint32_t w[4] = {r.x, r.y, r.z, r.w};
 #pragma unroll
-            for (int e = 0; e < 16; ++e) split2(x[2 * e] * sc, x[2 * e + 1] * sc, h[e], l[e]);
-            tmem_st16(tb + C::kColS + (part * DPT) / 2 + 16 * c, h);
-            if (a.q_dtype == TQ4_F32) tmem_st16(tb + C::kColQ + (part * DPT) / 2 + 16 * c, l);
+            for (int k = 0; k < 4; ++k) {
+              half_pair(w[k], f16, x0, x1);
+              h[4 * e + k] = pack_h2(x0 * sc, x1 * sc);
+            }
           }
+          tmem_st16(tb + C::kColS + (part * DPT) / 2 + 16 * c, h);
         }
-        if (pass == 0) pow2_scale(row_reduce(amax, fmax_op), sc, isc);
+      } else {
+        float amax = 0.f;
+#pragma unroll 1
+        for (int pass = 0; pass < 2; ++pass) {
+#pragma unroll 1
+          for (int c = 0; c < DPT / 32; ++c) {
+            float x[32];
+#pragma unroll
+            for (int e = 0; e < 32; ++e) x[e] = 0.f;
+            if (live) load32(a.q, a.q_dtype, qi + 32 * c, q_vec, x);
+            if (pass == 0) {
+#pragma unroll
+              for (int e = 0; e < 16; ++e) amax = max3(amax, fabsf(x[2 * e]), fabsf(x[2 * e + 1]));
+            } else {
+              uint32_t h[16], l[16];
+#pragma unroll
+              for (int e = 0; e < 16; ++e) split2(x[2 * e] * sc, x[2 * e + 1] * sc, h[e], l[e]);
+              tmem_st16(tb + C::kColS + (part * DPT) / 2 + 16 * c, h);
+              if (a.q_dtype == TQ4_F32) tmem_st16(tb + C::kColQ + (part * DPT) / 2 + 16 * c, l);
+            }
+          }
+          if (pass == 0) pow2_scale(row_reduce(amax, fmax_op), sc, isc);
+        }
       }
       tmem_st_wait();
       arrive(s_bars.aready);
       ok = __all_sync(0xffffffffu, bar_wait(bar(s_bars.rot), 0u, dead));
       fence_after();
-      // largest coordinate of the rotated row, then its terms at that scale
-      float rmax = 0.f, inv = 0.f;
+      // The rotated row (in tensor memory 2^8 sc times it), times kQGain and what makes its dot products scores in the log2 domain
+      // (before the key norm), as fp16 terms.  Its largest coordinate is between isc / sqrt(D) and 2 sqrt(D) isc: no pass looks
+      // for it, and where the factor could take the row out of fp16's range, the row keeps a power of two back.
+      float f = isc * (a.scale_log2e / a.lut_scale_k);
+      const int fe = (int)((__float_as_uint(fabsf(f)) >> 23) & 0xFFu) - 127;
+      if (f != 0.f && (fe < -6 || fe > 3)) {
+        const int ec = min(max(fe, -126), 126);
+        qexp = __uint_as_float((uint32_t)(127 + ec) << 23);
+        f *= __uint_as_float((uint32_t)(127 - ec) << 23);
+      }
+      f *= kQGain / 256.f;
 #pragma unroll 1
-      for (int pass = 0; pass < 2 && ok; ++pass) {
-#pragma unroll 1
-        for (int c = 0; c < DPT / 32; ++c) {
-          uint32_t v[32];
-          const int d0 = part * DPT + 32 * c;
-          tmem_ld_cols(tb + C::kColO + d0, v);
-          if (pass == 0) {
+      for (int c = 0; c < DPT / 32 && ok; ++c) {
+        uint32_t v[32], h[16], l[16];
+        const int d0 = part * DPT + 32 * c;
+        tmem_ld_cols(tb + C::kColO + d0, v);
 #pragma unroll
-            for (int e = 0; e < 16; ++e) rmax = max3(rmax, fabsf(__uint_as_float(v[2 * e])), fabsf(__uint_as_float(v[2 * e + 1])));
-            continue;
-          }
-          uint32_t h[16], l[16];
+        for (int e = 0; e < 16; ++e) split2(__uint_as_float(v[2 * e]) * f, __uint_as_float(v[2 * e + 1]) * f, h[e], l[e]);
+        tmem_st16(tb + C::kColQ + d0 / 2, h);
+        if (FAST) continue;
+        if (C::QLO_SMEM) {
+          unsigned char* dst = sm + C::kOffQlo + blk * (NC * 16384) + (d0 >> 6) * 16384;
 #pragma unroll
-          for (int e = 0; e < 16; ++e)
-            split2(__uint_as_float(v[2 * e]) * inv, __uint_as_float(v[2 * e + 1]) * inv, h[e], l[e]);
-          tmem_st16(tb + C::kColQ + d0 / 2, h);
-          if (FAST) continue;
-          if (C::QLO_SMEM) {
-            unsigned char* dst = sm + C::kOffQlo + blk * (NC * 16384) + (d0 >> 6) * 16384;
-#pragma unroll
-            for (int i = 0; i < 4; ++i)
-              *reinterpret_cast<uint4*>(dst + swz(m, ((d0 & 63) >> 3) + i)) = make_uint4(l[4 * i], l[4 * i + 1], l[4 * i + 2], l[4 * i + 3]);
-          } else {
-            tmem_st16(tb + C::kColQlo + d0 / 2, l);
-          }
-        }
-        if (pass == 0) {
-          rmax = row_reduce(rmax, fmax_op);
-          inv = rmax > 0.f ? 1.f / rmax : 0.f;
+          for (int i = 0; i < 4; ++i)
+            *reinterpret_cast<uint4*>(dst + swz(m, ((d0 & 63) >> 3) + i)) = make_uint4(l[4 * i], l[4 * i + 1], l[4 * i + 2], l[4 * i + 3]);
+        } else {
+          tmem_st16(tb + C::kColQlo + d0 / 2, l);
         }
       }
-      // factor between a stored dot product and the score in the log2 domain
-      qscale = fmaxf(rmax * isc * (1.f / 256.f) * (a.scale_log2e / a.lut_scale_k), 1.17549435e-38f);
       tmem_st_wait();
       fence_async();
       arrive(s_bars.qready);
@@ -1025,7 +1062,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
 
     PF_STAMP(tid == 0 ? 0 : -1, 0, 6);
     // ---- the tile loop --------------------------------------------------------------------------------
-    int kv_lo = 0, kv_hi = 0;
+    int kv_lo = 0, kv_hi = 0x7fffffff;  // (a row that is not there: zeros, nothing to mask)
     if (live) row_keys(row, kv_lo, kv_hi);
     float m_run = -CUDART_INF_F, l_run = 0.f;
     const int role = tid == 0 ? 0 : tid == 128 ? 1 : -1;  // (time stamps)
@@ -1046,8 +1083,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
         // per-element masks.  The reference is updated lazily, and looked at only after the fact: when some
         // weight exceeds 2^8 (or the row has no reference yet) the tile is done again from the scores, which stay in
         // registers, with a new one.  That saves the pass over the scores that would find the maximum first.
-        const bool inner = __all_sync(0xffffffffu, t0 >= kv_lo && t0 + CPT <= kv_hi) && !*(volatile int*)&s_bad;
-        const f2 qs2 = pack2(qscale, qscale);
+        const bool inner = __all_sync(0xffffffffu, t0 >= kv_lo && kv_hi - CPT >= t0 && qexp == 1.f) && !*(volatile int*)&s_bad;
         uint32_t v[CPT];
         tmem_ld_cols(scol, v);
         bool seen = true;  // some key of the tile is visible
@@ -1066,7 +1102,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
           }
 #pragma unroll
           for (int i = 0; i < CPT; ++i)
-            if (!((vis[i >> 5] >> (i & 31)) & 1u)) v[i] = 0xFF800000u;
+            v[i] = (vis[i >> 5] >> (i & 31)) & 1u ? __float_as_uint(__uint_as_float(v[i]) * qexp) : 0xFF800000u;
         }
         f2 ls2;
 #pragma unroll 1
@@ -1085,36 +1121,50 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
             }
           };
           load_norms(0);
-          uint32_t ph[8], pl[8];
+          f2 lsb = pack2(0.f, 0.f);
+          uint32_t w16[16];  // P of 16 columns: eight words of hi, eight of lo
 #pragma unroll
           for (int g = 0; g < CPT / 8; ++g) {
             if (g + 1 < CPT / 8) load_norms(g + 1);
+            float x[8];
+            f2 e[4];
 #pragma unroll
             for (int p = 0; p < 4; ++p) {
               const int i = 8 * g + 2 * p;
-              const f2 k2 = (p & 1) ? kn[g & 1][p >> 1].y : kn[g & 1][p >> 1].x, v2 = (p & 1) ? vn[g & 1][p >> 1].y : vn[g & 1][p >> 1].x;
-              float x0, x1;
-              unpack2(fma2(mul2(pack2(__uint_as_float(v[i]), __uint_as_float(v[i + 1])), k2), qs2, mn2), x0, x1);
-              const f2 e = pack2(ex2_approx(x0), ex2_approx(x1));
-              ls2 = add2(ls2, e);
-              unpack2(mul2(e, v2), x0, x1);
-              wmax = max3(wmax, x0, x1);
-              const int at = 4 * (g & 1) + p;
-              if (FAST) ph[at] = pack_h2(x0, x1);
-              else {
-                const __half2 h = __floats2half2_rn(x0, x1);
-                const float2 f = __half22float2(h);
-                ph[at] = *reinterpret_cast<const uint32_t*>(&h);
+              const f2 k2 = (p & 1) ? kn[g & 1][p >> 1].y : kn[g & 1][p >> 1].x;
+              unpack2(fma2(pack2(__uint_as_float(v[i]), __uint_as_float(v[i + 1])), k2, mn2), x[2 * p], x[2 * p + 1]);
+            }
+#pragma unroll
+            for (int p = 0; p < 4; ++p) e[p] = pack2(ex2_approx(x[2 * p]), ex2_approx(x[2 * p + 1]));
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {
+              f2& sum = (p & 1) ? lsb : ls2;
+              sum = add2(sum, e[p]);
+              const f2 v2 = (p & 1) ? vn[g & 1][p >> 1].y : vn[g & 1][p >> 1].x;
+              unpack2(mul2(e[p], v2), x[2 * p], x[2 * p + 1]);
+            }
+            float2 f[4];
+#pragma unroll
+            for (int p = 0; p < 4; ++p) {
+              wmax = max3(wmax, x[2 * p], x[2 * p + 1]);
+              const __half2 h = __floats2half2_rn(x[2 * p], x[2 * p + 1]);
+              w16[4 * (g & 1) + p] = *reinterpret_cast<const uint32_t*>(&h);
+              f[p] = __half22float2(h);
+            }
+            if (!FAST) {
+#pragma unroll
+              for (int p = 0; p < 4; ++p) {
                 float r0, r1;
-                unpack2(fma2(pack2(f.x, f.y), pack2(-1.f, -1.f), pack2(x0, x1)), r0, r1);
-                pl[at] = pack_h2(r0, r1);
+                unpack2(fma2(pack2(f[p].x, f[p].y), pack2(-1.f, -1.f), pack2(x[2 * p], x[2 * p + 1])), r0, r1);
+                w16[8 + 4 * (g & 1) + p] = pack_h2(r0, r1);
               }
             }
             if (g & 1) {
-              tmem_st8(scol + 8 * (g - 1), ph);
-              if (!FAST) tmem_st8(scol + 8 * (g - 1) + 8, pl);
+              if (FAST) tmem_st8(scol + 8 * (g - 1), *reinterpret_cast<const uint32_t(*)[8]>(w16));
+              else tmem_st16(scol + 8 * (g - 1), w16);
             }
           }
+          ls2 = add2(ls2, lsb);
           // (sums past 1e30: a value norm of zero hides an overflow from the weights)
           float e0, e1;
           unpack2(ls2, e0, e1);
@@ -1126,10 +1176,10 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
 #pragma unroll
           for (int i = 0; i < CPT; i += 4) {
             const float4 kn = *reinterpret_cast<const float4*>(ns + i), vn = *reinterpret_cast<const float4*>(ns + kBN + i);
-            mt = max3(mt, fmaf(__uint_as_float(v[i]) * kn.x, qscale, fmaxf(lg2_approx(vn.x), -30.f)),
-                      fmaf(__uint_as_float(v[i + 1]) * kn.y, qscale, fmaxf(lg2_approx(vn.y), -30.f)));
-            mt = max3(mt, fmaf(__uint_as_float(v[i + 2]) * kn.z, qscale, fmaxf(lg2_approx(vn.z), -30.f)),
-                      fmaf(__uint_as_float(v[i + 3]) * kn.w, qscale, fmaxf(lg2_approx(vn.w), -30.f)));
+            mt = max3(mt, fmaf(__uint_as_float(v[i]), kn.x, fmaxf(lg2_approx(vn.x), -30.f)),
+                      fmaf(__uint_as_float(v[i + 1]), kn.y, fmaxf(lg2_approx(vn.y), -30.f)));
+            mt = max3(mt, fmaf(__uint_as_float(v[i + 2]), kn.z, fmaxf(lg2_approx(vn.z), -30.f)),
+                      fmaf(__uint_as_float(v[i + 3]), kn.w, fmaxf(lg2_approx(vn.w), -30.f)));
           }
           mt = row_reduce(mt, fmax_op);
           const bool bump = need && mt > m_run;
@@ -1226,6 +1276,9 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
       }
       const float f = have && ok ? isc * (1.f / 256.f) : 0.f;
       const int64_t oi = (int64_t)row * a.out_token_stride + (int64_t)head * a.out_head_stride + part * DPT;
+      // 16-bit rows go through shared memory (where the raw queries came in), from which a warp stores whole rows: stored from
+      // here, its 16-byte pieces would fall into 32 of them
+      const bool staged = out_vec && a.out_dtype != TQ4_F32;
 #pragma unroll 1
       for (int c = 0; c < DPT / 32; ++c) {
         uint32_t v[32];
@@ -1234,7 +1287,21 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
           float y[32];
 #pragma unroll
           for (int e = 0; e < 32; ++e) y[e] = f != 0.f ? __uint_as_float(v[e]) * f : 0.f;
-          store32(a.out, a.out_dtype, oi + 32 * c, out_vec, y);
+          if (staged) store32(sm + q_at, a.out_dtype, 32 * c, true, y);
+          else store32(a.out, a.out_dtype, oi + 32 * c, out_vec, y);
+        }
+      }
+      if (staged) {
+        __syncwarp();
+        constexpr int PCS = DPT / 8;  // 16-byte pieces of a thread's part of a row
+        const unsigned char* rows = sm + C::kOffQlo + (blk * 128 + 32 * (warp & 3)) * C::kQPitch + part * DPT * 2;
+        const int64_t to = live ? oi : -1;
+#pragma unroll 4
+        for (int i = lane; i < 32 * PCS; i += 32) {
+          const int r = i / PCS, pc = i - r * PCS;
+          const int64_t at = __shfl_sync(0xffffffffu, to, r);
+          if (at >= 0)
+            *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(a.out) + at + 8 * pc) = *reinterpret_cast<const uint4*>(rows + r * C::kQPitch + 16 * pc);
         }
       }
       if (live && part == 0 && a.lse_out) a.lse_out[(int64_t)row * sh.Hq + head] = lse;
