@@ -301,23 +301,26 @@ inline bool tokens_uniform(const CompressArgs& a) {
   return true;
 }
 
-// Which kernel makes a write of so many vectors (B200, graph replays of stand-alone writes, bf16):
-//   a block per vector up to tiny_rows(): a few us plus 1.1 / 1.7 / 2.5 us per 1000 vectors of 64 / 96 / 128, against 8 - 10 us
-//     of the tensor-core kernel and 16 us of the prologue kernel at 4800 vectors of 128; at 256 it never pays
-//   the tensor-core kernel above tc_rows().  At head_dim 128 it would pay earlier (8192 vectors: 10.8 us, the prologue
-//     kernel 16, a block per vector 24), but up to kSmallRows a vector is promised the same bytes however the calls are cut,
-//     and there only the FMA kernels agree with one another bit for bit.  At 256 the prologue kernel takes 15 us at 800
+// Which kernel makes a write of so many vectors (B200, back to back, bf16):
+//   a block per vector up to tiny_rows(): a few us plus 1.1 / 1.7 / 2.5 us per 1000 vectors of 64 / 96 / 128, against 8 - 14 us
+//     of the tensor-core kernel; at 256 it never pays
+//   the tensor-core kernel above tc_rows(): 4096 vectors of 128 14.4 us either way, 5120 - 8192 14.4 against 18.5 us of the prologue
+//     kernel.  Up to kSmallRows a vector is promised the same bytes however the calls are cut, so there it sums coordinates
+//     near a boundary again the FMA kernels' way (above, at head_dim 128, its bytes are its own).  At 256 the prologue kernel
+//     takes 15 us at 800
 //   the prologue kernel in between, and up to kSmallRows for what the tensor-core kernel cannot address
 constexpr int64_t kSmallRows = 8192;
 constexpr int64_t tiny_rows(int head_dim) { return head_dim == 64 ? 6500 : head_dim == 96 ? 3000 : head_dim == 128 ? 4096 : 0; }
-constexpr int64_t tc_rows(int head_dim) { return head_dim == 128 ? kSmallRows : head_dim == 256 ? 1000 : tiny_rows(head_dim); }
+constexpr int64_t tc_rows(int head_dim) { return head_dim == 256 ? 1000 : tiny_rows(head_dim); }
 int launch_small_write(const CompressArgs& w, int head_dim, cudaStream_t st);
-int dispatch_compress(const CompressArgs& a, int head_dim, int dtype, cudaStream_t st);
+// `fma_bytes`: the bytes of the FMA kernels above kSmallRows, too
+int dispatch_compress(const CompressArgs& a, int head_dim, int dtype, cudaStream_t st, bool fma_bytes = false);
 // tensor-core (tcgen05) compress kernel for large fp32 or oddly strided inputs at head_dim 128 (tq4_compress_tc.cu)
 bool compress_tc_eligible(const CompressArgs& a, int head_dim, int dtype);
 int launch_compress_tc(const CompressArgs& a, int dtype, cudaStream_t st);
 // pipelined tcgen05 kernel for 16-bit inputs (tq4_compress_tc16.cu)
 bool compress_tc16_eligible(const CompressArgs& a, int head_dim, int dtype);
-int launch_compress_tc16(const CompressArgs& a, int head_dim, int dtype, cudaStream_t st);
+// (fma_bytes: at head_dim 128 the FMA kernels' bytes, too)
+int launch_compress_tc16(const CompressArgs& a, int head_dim, int dtype, bool fma_bytes, cudaStream_t st);
 
 }  // namespace tq4

@@ -359,14 +359,15 @@ int dispatch_dtype(const CompressArgs& a, int dtype, cudaStream_t st) {
   return TQ4_ERR_UNSUPPORTED;
 }
 
-int dispatch_compress(const CompressArgs& a, int head_dim, int dtype, cudaStream_t st) {
+int dispatch_compress(const CompressArgs& a, int head_dim, int dtype, cudaStream_t st, bool fma_bytes) {
   const int64_t vectors = a.n_tokens * a.num_heads * a.n_sources;
   if (vectors == 0) return TQ4_OK;
   const bool tiny = vectors <= tiny_rows(head_dim);  // (dispatch_dtype: a block per vector)
+  fma_bytes = fma_bytes || vectors <= kSmallRows;
   if (vectors > tc_rows(head_dim) && compress_tc16_eligible(a, head_dim, dtype))
-    return launch_compress_tc16(a, head_dim, dtype, st);
+    return launch_compress_tc16(a, head_dim, dtype, fma_bytes, st);
   if (!tiny && vectors <= kSmallRows) return launch_small_write(a, head_dim, st);
-  if (!tiny && compress_tc_eligible(a, head_dim, dtype)) return launch_compress_tc(a, dtype, st);
+  if (!tiny && !fma_bytes && compress_tc_eligible(a, head_dim, dtype)) return launch_compress_tc(a, dtype, st);
   switch (head_dim) {
     case 64: return dispatch_dtype<64>(a, dtype, st);
     case 96: return dispatch_dtype<96>(a, dtype, st);

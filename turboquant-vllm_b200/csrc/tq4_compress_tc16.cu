@@ -224,7 +224,7 @@ __device__ __forceinline__ int bucketize_reg(float y, const float (&b)[15]) {
 
 // The two roundings of a coordinate (this kernel's product, the FMA kernels' chains) lie 2e-8 apart on average; a coordinate
 // nearer than this to a boundary (about 1e-5 of them) is summed again the FMA kernels' way, so that the bytes are theirs.
-// (Not at head_dim 128, whose large writes have been the tensor cores' own for longer than there was a choice.)
+// (Not in large writes at head_dim 128, which have been the tensor cores' own for longer than there was a choice.)
 constexpr float kNear = 1.5e-7f;
 
 // The 32-cell map: cell = round(31 * sat(y * s / 31 + 16 / 31)), so y = 0 sits in the middle of cell 16 and
@@ -282,7 +282,7 @@ struct Again {
   uint8_t* dst;
   unsigned row, where;
 };
-constexpr int kAgainMax = 8;  // a warp's list
+template <int D> constexpr int kAgainMax = D == 128 ? 4 : 8;  // a warp's list (what shared memory leaves)
 
 // The chunks on a warp's list by the sums of the FMA kernels: the norm, then lane = coordinate, four quarter chains in
 // ascending k, combined as (s0 + s1) + (s2 + s3).  Kept out of the tile loop, whose code has to stay short.
@@ -338,21 +338,23 @@ struct Bars {
   uint64_t drain;      // a dead CTA's last MMA is complete
 };
 
-template <typename T, int D>
+// AGAIN: a coordinate near a boundary is summed again, see kNear
+template <typename T, int D, bool AGAIN>
 __global__ void __launch_bounds__(Cfg<D>::THREADS, 1)
 compress_tc16_kernel(const __grid_constant__ CompressArgs a, const int group_rows, const __grid_constant__ CUtensorMap tm_x0,
                      const __grid_constant__ CUtensorMap tm_x1) {
   using F = Fmt<T>;
   using C = Cfg<D>;
   constexpr int N = C::N, STAGES = C::STAGES;
-  constexpr bool kAgain = D != 128;
+  constexpr bool kAgain = AGAIN;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   __shared__ __align__(8) Bars s_bars;
   __shared__ uint32_t s_tmem;
   __shared__ int s_dead;
   __shared__ float s_bounds[2][16];
-  __shared__ Again s_again[kAgain ? kAgainMax * (C::THREADS / 32 - 2) : 1];
+  __shared__ Again s_again[kAgain ? kAgainMax<D> * (C::THREADS / 32 - 2) : 1];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  pdl_trigger();
   if (warp == 0) CT_STAMP(0, 31, 6);  // kernel entry
   const uint32_t base = (smem_addr(smem_raw) + 1023u) & ~1023u;  // swizzle atoms need 1024-byte alignment
   unsigned char* sm = smem_raw + (base - smem_addr(smem_raw));
@@ -483,7 +485,7 @@ compress_tc16_kernel(const __grid_constant__ CompressArgs a, const int group_row
     Grid grid[2];
     bool grid_ok = make_grid(s_bounds[0], grid[0], lane);
     grid_ok = make_grid(s_bounds[1], grid[1], lane) && grid_ok;
-    [[maybe_unused]] Again* my_again = s_again + (kAgain ? kAgainMax * (warp - 2) : 0);
+    [[maybe_unused]] Again* my_again = s_again + (kAgain ? kAgainMax<D> * (warp - 2) : 0);
     [[maybe_unused]] int n_again = 0;
     for (int64_t i = grp; i < my_tiles && ok; i += STAGES) {
       const int st = grp;
@@ -611,7 +613,7 @@ compress_tc16_kernel(const __grid_constant__ CompressArgs a, const int group_row
           uint32_t who = __ballot_sync(0xffffffffu, closest < kNear && dst_idx != nullptr && nrm != 0.f);
 #pragma unroll 1
           for (; who != 0; who &= who - 1) {
-            if (n_again == kAgainMax) {
+            if (n_again == kAgainMax<D>) {
               __syncwarp();
               sum_again<T, D>(reinterpret_cast<const T*>(a.x[0]), reinterpret_cast<const T*>(a.x[1]), a.rot_even, a.rot_odd, &a,
                               s_bounds, my_again, n_again, j0, lane);
@@ -684,7 +686,7 @@ int group_of(const CompressArgs& a, int D) {
   return 0;
 }
 
-template <typename T, int D>
+template <typename T, int D, bool AGAIN>
 int launch_t(const CompressArgs& a, cudaStream_t st) {
   using C = Cfg<D>;
   CUtensorMap m0, m1;
@@ -693,21 +695,21 @@ int launch_t(const CompressArgs& a, cudaStream_t st) {
   const int group = group_of(a, D);
   if (!make_x_map(&m0, a, 0, D, group) || !make_x_map(&m1, a, a.n_sources > 1 ? 1 : 0, D, group)) return TQ4_ERR_CUDA;
   const int smem = (int)C::kSmem + 1024;
-  if (!ensure_dynamic_smem<compress_tc16_kernel<T, D>>(smem)) return TQ4_ERR_CUDA;
+  if (!ensure_dynamic_smem<compress_tc16_kernel<T, D, AGAIN>>(smem)) return TQ4_ERR_CUDA;
   int64_t streams = ((a.n_tokens * a.num_heads + kRows - 1) / kRows) * a.n_sources;
   if (streams > sm_count() / C::NSPLIT) streams = sm_count() / C::NSPLIT;
-  compress_tc16_kernel<T, D><<<(unsigned)(streams * C::NSPLIT), C::THREADS, smem, st>>>(a, group, m0, m1);
+  compress_tc16_kernel<T, D, AGAIN><<<(unsigned)(streams * C::NSPLIT), C::THREADS, smem, st>>>(a, group, m0, m1);
   TQ4_CHECK_LAUNCH();
   return TQ4_OK;
 }
 
 template <typename T>
-int launch_d(const CompressArgs& a, int head_dim, cudaStream_t st) {
+int launch_d(const CompressArgs& a, int head_dim, bool fma_bytes, cudaStream_t st) {
   switch (head_dim) {
-    case 64: return launch_t<T, 64>(a, st);
-    case 96: return launch_t<T, 96>(a, st);
-    case 128: return launch_t<T, 128>(a, st);
-    case 256: return launch_t<T, 256>(a, st);
+    case 64: return launch_t<T, 64, true>(a, st);
+    case 96: return launch_t<T, 96, true>(a, st);
+    case 128: return fma_bytes ? launch_t<T, 128, true>(a, st) : launch_t<T, 128, false>(a, st);
+    case 256: return launch_t<T, 256, true>(a, st);
   }
   return TQ4_ERR_UNSUPPORTED;
 }
@@ -726,8 +728,8 @@ bool compress_tc16_eligible(const CompressArgs& a, int head_dim, int dtype) {
   return group_of(a, head_dim) != 0;
 }
 
-int launch_compress_tc16(const CompressArgs& a, int head_dim, int dtype, cudaStream_t st) {
-  return dtype == TQ4_F16 ? launch_d<__half>(a, head_dim, st) : launch_d<__nv_bfloat16>(a, head_dim, st);
+int launch_compress_tc16(const CompressArgs& a, int head_dim, int dtype, bool fma_bytes, cudaStream_t st) {
+  return dtype == TQ4_F16 ? launch_d<__half>(a, head_dim, fma_bytes, st) : launch_d<__nv_bfloat16>(a, head_dim, fma_bytes, st);
 }
 
 }  // namespace tq4
