@@ -57,3 +57,45 @@ def test_token_rows(cuda_lib, d, b, h):
         got = idx.contiguous().cpu().reshape(-1, d // 2)
         assert (O.nibble_unpack(got) != O.nibble_unpack(packed.reshape(-1, d // 2))).float().mean() <= 1e-4
         assert torch.allclose(norm.cpu().reshape(-1), norms.reshape(-1), rtol=1e-6)
+
+
+@pytest.mark.parametrize("d", [64, 96, 128])
+@pytest.mark.parametrize("b,h,n,dtype", [
+    (1, 1, 2369, torch.bfloat16),   # one vector past the line, 19 tiles a tensor, 65 vectors in the last
+    (1, 4, 640, torch.float16),     # whole tiles
+    (3, 5, 171, torch.bfloat16),    # batch and head change inside a tile
+    (5, 32, 120, torch.bfloat16),   # 300 tiles: three a CTA for some; at 128 above the line of the tensor cores' own bytes
+])
+@pytest.mark.parametrize("aligned", [True, False])
+def test_prompt_restored_by_the_tensor_cores(cuda_lib, d, b, h, n, dtype, aligned):
+    """Indices and norms of the compression by itself; the reconstruction against 64 bits: half a unit of the 16-bit type and
+    2^-19 of a vector's norm for the sums (128 terms of 22 bits, fp32); nothing beside the update's own rows."""
+    from turboquant_vllm import TurboQuantMSE
+    from turboquant_vllm import _native as nv
+    from turboquant_vllm.kernels import ops
+
+    kq, vq = TurboQuantMSE(d, 4, seed=42), TurboQuantMSE(d, 3, seed=42)
+    rot = kq.rotation.contiguous().cuda()
+    even, odd = rot.T[:, 0::2].contiguous(), rot.T[:, 1::2].contiguous()
+    kb, vb, kc, vc = (x.cuda() for x in (kq.codebook.boundaries, vq.codebook.boundaries, kq.codebook.centroids, vq.codebook.centroids))
+    k, v = _states(b, h, n, d, dtype, seed=d)
+    cap, off = n + 7, 3
+
+    def dec():  # (misaligned: the FMA kernels' turn)
+        return torch.zeros(b * h * cap * d + 1, dtype=dtype, device="cuda")[0 if aligned else 1:][: b * h * cap * d].view(b, h, cap, d)
+
+    ki, vi = (torch.zeros(b, h, cap, w, dtype=torch.uint8, device="cuda") for w in (d // 2, d))
+    kn, vn = (torch.zeros(b, h, cap, 1, device="cuda") for _ in range(2))
+    kd, vd = dec(), dec()
+    nv.host().cache_update(k, v, rot, even, odd, kb, vb, kc, vc, True, False, ki, kn, vi, vn, off, kd, vd, off)
+    for x, bounds, cents, idx, norm, out in ((k, kb, kc, torch.stack([ki >> 4, ki & 15], -1).flatten(-2), kn, kd), (v, vb, vc, vi, vn, vd)):
+        whole = d == 128 and b * h * n > 8192
+        parts = [ops.tq4_compress(p.transpose(1, 2).reshape(-1, h, d), even, odd, bounds) for p in x.split(n if whole else 5, dim=2)]
+        packed, norms = (torch.cat([p[i].view(b, -1, h, p[i].shape[-1]) for p in parts], 1).transpose(1, 2) for i in (0, 1))
+        live = slice(off, off + n)
+        assert torch.equal(idx[:, :, live], torch.stack([packed >> 4, packed & 15], -1).flatten(-2)) and torch.equal(norm[:, :, live], norms)
+        want = (cents.double()[idx[:, :, live].long()] * norms.double()) @ rot.double()
+        half = 2.0**-8 if dtype == torch.bfloat16 else 2.0**-11  # (significands of 8 and 11 bits)
+        assert ((out[:, :, live].double() - want).abs() <= half * want.abs() * (1 + 2.0**-7) + 2.0**-19 * norms.double()).all()
+        for t in (idx, norm, out):
+            assert (t[:, :, :off] == 0).all() and (t[:, :, off + n:] == 0).all()

@@ -8,34 +8,18 @@
 // copies into the buffers), which bounded a step by its host time.  A warp takes four vectors, a lane D / 32
 // consecutive coordinates of each; both products read Pi from shared memory (once transposed, once as
 // it is; at head_dim 256, where that does not fit, in chunks of 64 rows) and the vectors from a strip per warp.
-// A step of a few tokens is bound by latency and has a kernel of its own (cache_update_tiny_kernel); a prompt is bound by
-// FMA issue and the reads of Pi.
+// A step of a few tokens is bound by latency and has a kernel of its own (cache_update_tiny_kernel); a prompt of 16-bit vectors is
+// compressed by the write kernels and restored by the tensor cores (tq4_restore_tc.cu); what is left is bound by FMA issue
+// and the reads of Pi.
 // The kernels' own times, against the chain's (ncu: cold, serialised; bf16, 8 heads of 128, K4 / V3): a prompt of
-// 4 x 1100 tokens 293 us in 26 launches -> 124 in two (16 of them the write kernel's), one token of each 103 us in 25
-// launches -> 11 in one.
+// 4 x 1100 tokens 293 us in 26 launches -> 124 in two (16 of them the write kernel's; 36 with the tensor cores restoring), one token
+// of each 103 us in 25 launches -> 11 in one.
 #include <math_constants.h>
 
-#include "tq4_common.cuh"
+#include "tq4_cache_update.cuh"
 
 namespace tq4 {
 namespace {
-
-struct UpdateArgs {
-  const void* x[2];                    // K and V [B, H, S, D]
-  int64_t batch_stride[2], head_stride[2], token_stride[2];
-  const float* bounds[2];
-  const float* cents[2];
-  int n_bounds[2], n_cents[2], nibble[2];
-  uint8_t* idx[2];                     // [B, H, cap, D / 2 or D]
-  float* norms[2];                     // [B, H, cap]
-  void* dec[2];                        // [B, H, dec_cap, D] in x's type, or null
-  int64_t cap, dec_cap, offset, dec_offset;
-  int batch, heads, n_new, dtype;
-  const float* rotation;
-  const float *rot_even, *rot_odd;  // even / odd columns of Pi^T
-  const uint8_t* packed;               // DONE: the compressed vectors, K then V, [B, S, H, D / 2] and [B, S, H]
-  const float* packed_norms;
-};
 
 // two fp32 operations an instruction, each rounded as alone
 struct F2 { unsigned long long v; };
@@ -476,13 +460,23 @@ int launch_update(const UpdateArgs& a, cudaStream_t st) {
 bool compress_first(int batch, int heads, int n_new, int head_dim) {
   return head_dim == 128 && (int64_t)batch * heads * n_new > kSmallRows;
 }
+// Otherwise it pays where the tensor cores restore, too (restore_tc_kernel): once the FMA kernel would take a second pass (four vectors
+// a warp of every SM).  K and V of 8 heads, bf16, FMA kernel / compressed first: 4000 vectors of 128 20.7 / 22.7 us, 6400 35.0 / 22.7,
+// 14 400 53 / 24; of 64 12.4 / 12.9, 18.6 / 16.5, 24.7 / 16.6; of 96 16.3 / 20.6, 25.5 / 20.7, 41 / 20.7.  The indices are the FMA
+// kernels' (fma_bytes).
+bool restore_pays(int batch, int heads, int n_new, int head_dim) {
+  return head_dim <= 128 && 2 * (int64_t)batch * heads * n_new > 32 * (int64_t)sm_count();
+}
+size_t scratch_norms(int batch, int heads, int n_new) { return ((size_t)2 * batch * heads * n_new * sizeof(float) + 15) & ~(size_t)15; }
 
 }  // namespace
 }  // namespace tq4
 
 extern "C" size_t tq4_cache_update_scratch_bytes(int batch, int num_heads, int n_new, int head_dim) {
-  if (batch <= 0 || num_heads <= 0 || n_new <= 0 || !tq4::compress_first(batch, num_heads, n_new, head_dim)) return 0;
-  return (size_t)2 * batch * num_heads * n_new * (head_dim / 2 + sizeof(float));
+  using namespace tq4;
+  if (batch <= 0 || num_heads <= 0 || n_new <= 0) return 0;
+  if (!compress_first(batch, num_heads, n_new, head_dim) && !restore_pays(batch, num_heads, n_new, head_dim)) return 0;
+  return scratch_norms(batch, num_heads, n_new) + (size_t)2 * batch * num_heads * n_new * (head_dim / 2);
 }
 
 extern "C" int tq4_cache_update(const void* key, const void* value, int dtype, int batch, int num_heads, int n_new,
@@ -530,10 +524,13 @@ extern "C" int tq4_cache_update(const void* key, const void* value, int dtype, i
   a.rotation = rotation;
   a.rot_even = rot_t_even;
   a.rot_odd = rot_t_odd;
-  if (compress_first(batch, num_heads, n_new, head_dim)) {
-    if (!scratch || ((uintptr_t)scratch & 15) || scratch_bytes < tq4_cache_update_scratch_bytes(batch, num_heads, n_new, head_dim))
-      return TQ4_ERR_WORKSPACE;
-    const int64_t vectors = 2 * (int64_t)batch * num_heads * n_new;
+  const bool must = compress_first(batch, num_heads, n_new, head_dim);
+  const bool room = scratch && ((uintptr_t)scratch & 15) == 0 && scratch_bytes >= tq4_cache_update_scratch_bytes(batch, num_heads, n_new, head_dim);
+  if (must && !room) return TQ4_ERR_WORKSPACE;
+  a.packed = (const uint8_t*)scratch + scratch_norms(batch, num_heads, n_new);
+  const bool restore = room && restore_tc_eligible(a, head_dim) && (must || restore_pays(batch, num_heads, n_new, head_dim));
+  a.packed = nullptr;
+  if (must || restore) {
     CompressArgs c{};
     for (int i = 0; i < 2; ++i) {
       c.x[i] = a.x[i];
@@ -551,12 +548,13 @@ extern "C" int tq4_cache_update(const void* key, const void* value, int dtype, i
     c.rot_odd = rot_t_odd;
     c.seq = n_new;
     for (int i = 0; n_new == 1 && i < 2; ++i) c.token_stride[i] = c.batch_stride[i];  // the sequences are the tokens
-    c.norms_out = (float*)scratch;  // (the norms first: a multiple of four bytes each)
-    c.packed_out = (uint8_t*)scratch + vectors * sizeof(float);
-    const int rc = dispatch_compress(c, head_dim, dtype, (cudaStream_t)stream);
+    c.norms_out = (float*)scratch;
+    c.packed_out = (uint8_t*)scratch + scratch_norms(batch, num_heads, n_new);
+    const int rc = dispatch_compress(c, head_dim, dtype, (cudaStream_t)stream, !must);
     if (rc != TQ4_OK) return rc;
     a.packed = c.packed_out;
     a.packed_norms = c.norms_out;
+    if (restore) return launch_restore_tc(a, head_dim, (cudaStream_t)stream);
   }
   switch (head_dim) {
     case 64: return launch_update<64>(a, (cudaStream_t)stream);
