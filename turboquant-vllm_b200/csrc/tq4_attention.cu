@@ -442,146 +442,174 @@ prologue_kernel(const AttnArgs a, const CompressArgs w, const int has_attn, cons
   }
 }
 
-// The same for a step of a few vectors: a block of four warps per vector, each warp one quarter of the
-// reduction with Pi^T read straight from L1 / L2 (the caller's even / odd halves), as the write kernel for few vectors does.
-// No staging, half the code: latency is all that counts here.
-// Q_ONLY: no write, so no Pi^T from the caller: a lane reads the rows of Pi of its two coordinates, a 128-byte line of each at a
-// time (the same bytes, four k a load; the sums are the same).
-template <int D, bool Q_ONLY>
-__global__ void __launch_bounds__(128) tiny_prologue_kernel(const AttnArgs a, const CompressArgs w) {
-  constexpr int HALF = D / 2, NBL = (HALF + 31) / 32, XPL = D / 32, KQ = D / 4;
+// The same for a step of a few vectors: a block per vector, with all of its Pi (or half, at head_dim 256) asked for before
+// anything is known of the vector, so that a load's latency is paid once.
+//   A query: lanes along the rows of Pi, so a warp's load is a row (or two), a warp has D / WARPS rows, and their 32 partial sums each are
+//     folded over the lanes together.  No staging, no block barrier.
+//   A new token's vector: the arithmetic contract of the compress kernels (four quarter chains in ascending k), Pi^T from the
+//     caller's even / odd halves, a lane per column pair, warps = quarters x 32 pairs.
+// FRAG: for the kernel of small decode steps (tq4_decode_step.cu), which wants a query as fp16 hi and lo terms of y times a power of
+// two that follows from the raw vector's largest element.
+template <int D>
+struct TinyStepCfg {
+  static constexpr int HALF = D / 2, CS = (HALF + 31) / 32, WARPS = 4 * CS, THREADS = 32 * WARPS;
+  static constexpr int RPL = D == 64 ? 2 : 1;             // rows of Pi a warp's load covers
+  static constexpr int F4 = D == 256 ? 2 : 1;             // float4 a lane has of a row
+  static constexpr int NV = D / WARPS / RPL;              // rows (row pairs) of a warp
+  static constexpr int KQ = D / 4, KB = D == 256 ? 32 : KQ;
+};
+template <int D, bool WRITE, bool FRAG>
+__global__ void __launch_bounds__(TinyStepCfg<D>::THREADS) tiny_prologue_kernel(const AttnArgs a, const CompressArgs w) {
+  using C = TinyStepCfg<D>;
+  constexpr int HALF = C::HALF, XPL = D / 32, KQ = C::KQ, KB = C::KB, NV = C::NV, F4 = C::F4;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ float s_x[D];
-  __shared__ float s_part[3][2 * NBL][32];
+  __shared__ __align__(16) float s_part[4][D];
   __shared__ float s_b[16];
   pdl_trigger();
-  if (blockIdx.x == 0) {  // the planning block
+  if (!FRAG && blockIdx.x == 0) {  // the planning block
     build_plan(a, reinterpret_cast<int*>(smem_raw));
     return;
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int n_q = a.sh.rows * a.sh.Hq, vec = (int)blockIdx.x - 1;
-  const bool is_w = !Q_ONLY && vec >= n_q;
-  int src = 0, tok = 0, h = 0;
-  int64_t slot = -1, at;
-  const void* x;
-  int dt;
-  if (is_w) {
-    const int rows_per_src = (int)w.n_tokens * w.num_heads, r = vec - n_q;
-    src = r >= rows_per_src ? 1 : 0;
-    const unsigned rem = (unsigned)(r - src * rows_per_src);
-    tok = (int)(rem / (unsigned)w.num_heads);
-    h = (int)(rem - (unsigned)tok * (unsigned)w.num_heads);
-    x = w.x[src];
-    dt = w.x_dtype;
-    at = token_offset(w, src, tok) + (int64_t)h * w.head_stride[src];
-    slot = tok < w.n_slots ? write_slot(w, tok) : -1;
-    if (threadIdx.x >= 32 && threadIdx.x < 48) {
-      const int i = threadIdx.x - 32;
-      s_b[i] = i < w.n_bounds[src] ? w.bounds[src][i] : CUDART_INF_F;
-    }
-  } else {
+  const int n_q = a.sh.rows * a.sh.Hq, vec = (int)blockIdx.x - (FRAG ? 0 : 1);
+  if (!WRITE || vec < n_q) {
+    // ---- a query ----------------------------------------------------------------------------------------
+    constexpr int GL = 32 / C::RPL;                         // lanes of a row
+    const int l4 = lane % GL, first = warp * (D / C::WARPS) + lane / GL;
+    const bool act = l4 < D / 4 / F4;                       // (head_dim 96: 24 lanes)
+    float4 pi[NV][F4];
+#pragma unroll
+    for (int i = 0; i < NV; ++i)
+#pragma unroll
+      for (int f = 0; f < F4; ++f)
+        pi[i][f] = act ? __ldg(reinterpret_cast<const float4*>(a.rotation + (size_t)(first + C::RPL * i) * D) + l4 + GL * f)
+                       : make_float4(0.f, 0.f, 0.f, 0.f);
     const int row = vec / a.sh.Hq;
-    x = a.q;
-    dt = a.q_dtype;
-    at = ((int64_t)row + a.sh.row_offset) * a.q_token_stride + (int64_t)(vec - row * a.sh.Hq) * a.q_head_stride;
-  }
-  float xv[XPL], norm = 0.f;
+    const int64_t at = ((int64_t)row + a.sh.row_offset) * a.q_token_stride + (int64_t)(vec - row * a.sh.Hq) * a.q_head_stride;
+    float v[NV], top = 0.f;
 #pragma unroll
-  for (int i = 0; i < XPL; ++i) xv[i] = load_as_float(x, dt, at + lane + 32 * i);
-  float den = 1.f;
-  if (is_w) {
-    float ss = 0.f;
+    for (int i = 0; i < NV; ++i) v[i] = 0.f;
 #pragma unroll
-    for (int i = 0; i < XPL; ++i) ss = fmaf(xv[i], xv[i], ss);
-    norm = sqrtf(warp_sum(ss));
-    den = norm + 1e-10f;
-  }
-  if (warp == 0) {
+    for (int f = 0; f < F4; ++f) {
+      float x[4];
 #pragma unroll
-    for (int i = 0; i < XPL; ++i) s_x[lane + 32 * i] = is_w ? xv[i] / den : xv[i];
-  }
-  __syncthreads();
-  float acc[2 * NBL];
-#pragma unroll
-  for (int i = 0; i < 2 * NBL; ++i) acc[i] = 0.f;
-  for (int kb = 0; kb < KQ; kb += 8) {  // eight k-steps of Pi^T in flight before the first FMA of the batch
-    float pe[8][NBL], po[8][NBL];
-    if constexpr (Q_ONLY) {
-#pragma unroll
-      for (int i = 0; i < NBL; ++i) {
-        const int p = lane + 32 * i;
-#pragma unroll
-        for (int u = 0; u < 8; u += 4) {
-          const float* row = a.rotation + 2 * p * D + warp * KQ + kb + u;
-          const float4 z = make_float4(0.f, 0.f, 0.f, 0.f);
-          const float4 e = p < HALF ? __ldg(reinterpret_cast<const float4*>(row)) : z;
-          const float4 o = p < HALF ? __ldg(reinterpret_cast<const float4*>(row + D)) : z;
-          pe[u][i] = e.x; pe[u + 1][i] = e.y; pe[u + 2][i] = e.z; pe[u + 3][i] = e.w;
-          po[u][i] = o.x; po[u + 1][i] = o.y; po[u + 2][i] = o.z; po[u + 3][i] = o.w;
-        }
+      for (int e = 0; e < 4; ++e) {
+        x[e] = act ? load_as_float(a.q, a.q_dtype, at + 4 * (l4 + GL * f) + e) : 0.f;
+        top = fmaxf(top, fabsf(x[e]));
       }
+#pragma unroll
+      for (int i = 0; i < NV; ++i)
+        v[i] = fmaf(x[0], pi[i][f].x, fmaf(x[1], pi[i][f].y, fmaf(x[2], pi[i][f].z, fmaf(x[3], pi[i][f].w, v[i]))));
+    }
+    // fold: after the step of `o` lanes a lane has the sums of half as many rows
+    int n = 0;  // row of the warp that the lane ends up with (of NV, padded to a power of two)
+    constexpr int NP = NV <= 8 ? 8 : 16;
+    float t[NP];
+#pragma unroll
+    for (int i = 0; i < NP; ++i) t[i] = i < NV ? v[i] : 0.f;
+    int o = GL / 2;
+#pragma unroll
+    for (int h = NP / 2; h > 0; h >>= 1) {
+      const bool up = lane & o;
+#pragma unroll
+      for (int i = 0; i < h; ++i) {
+        const float mine = up ? t[i + h] : t[i], other = up ? t[i] : t[i + h];
+        t[i] = mine + __shfl_xor_sync(0xffffffffu, other, o);
+      }
+      n += up ? h : 0;
+      o >>= 1;
+    }
+    float y = t[0];
+#pragma unroll
+    for (; o > 0; o >>= 1) y += __shfl_xor_sync(0xffffffffu, y, o);
+    const bool mine = n < NV && (l4 & (GL / NP - 1)) == 0;  // (the lanes that are left hold the same sum)
+    const int j = first + C::RPL * n;
+    if constexpr (!FRAG) {
+      if (mine) a.plan.q_rot[(int64_t)vec * D + j] = y;
     } else {
 #pragma unroll
-      for (int u = 0; u < 8; ++u)
-#pragma unroll
-        for (int i = 0; i < NBL; ++i) {
-          const int p = lane + 32 * i, k = warp * KQ + kb + u;
-          pe[u][i] = p < HALF ? __ldg(w.rot_even + k * HALF + p) : 0.f;
-          po[u][i] = p < HALF ? __ldg(w.rot_odd + k * HALF + p) : 0.f;
-        }
-    }
-#pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const float xk = s_x[warp * KQ + kb + u];
-#pragma unroll
-      for (int i = 0; i < NBL; ++i) {
-        acc[2 * i] = fmaf(xk, pe[u][i], acc[2 * i]);
-        acc[2 * i + 1] = fmaf(xk, po[u][i], acc[2 * i + 1]);
+      for (int s = GL / 2; s > 0; s >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, s));
+      const int e = top > 0.f && top < CUDART_INF_F ? min(max((int)(__float_as_uint(top) >> 23) - 127, -100), 100) : 0;
+      const float z = y * __uint_as_float((uint32_t)(127 + 4 - e) << 23);  // (at most 2^5 sqrt(D))
+      const __half hi = __float2half_rn(z);
+      __half* dst = reinterpret_cast<__half*>(a.plan.q_rot + (int64_t)vec * D);
+      if (mine) {
+        dst[j] = hi;
+        dst[D + j] = __float2half_rn(z - __half2float(hi));
       }
+      if (threadIdx.x == 0) a.plan.part_l[vec] = __uint_as_float((uint32_t)(127 - 4 + e) << 23);
     }
-  }
-  if (warp > 0) {
-#pragma unroll
-    for (int i = 0; i < 2 * NBL; ++i) s_part[warp - 1][i][lane] = acc[i];
-  }
-  __syncthreads();
-  if (warp != 0) return;
-#pragma unroll
-  for (int i = 0; i < 2 * NBL; ++i) acc[i] = (acc[i] + s_part[0][i][lane]) + (s_part[1][i][lane] + s_part[2][i][lane]);
-  if (!is_w) {
-#pragma unroll
-    for (int i = 0; i < NBL; ++i)
-      if (lane + 32 * i < HALF)
-        *reinterpret_cast<float2*>(a.plan.q_rot + (int64_t)vec * D + 2 * (lane + 32 * i)) = make_float2(acc[2 * i], acc[2 * i + 1]);
     return;
   }
+  // ---- a vector of a new token --------------------------------------------------------------------------
+  const int rows_per_src = (int)w.n_tokens * w.num_heads, r = vec - n_q;
+  const int src = r >= rows_per_src ? 1 : 0;
+  const unsigned rem = (unsigned)(r - src * rows_per_src);
+  const int tok = (int)(rem / (unsigned)w.num_heads), h = (int)(rem - (unsigned)tok * (unsigned)w.num_heads);
+  const int q = warp & 3, p = 32 * (warp >> 2) + lane, k0 = q * KQ;
+  float pe[KB], po[KB];
+  auto load_batch = [&](int kb) {
+#pragma unroll
+    for (int u = 0; u < KB; ++u) {
+      pe[u] = p < HALF ? __ldg(w.rot_even + (k0 + kb + u) * HALF + p) : 0.f;
+      po[u] = p < HALF ? __ldg(w.rot_odd + (k0 + kb + u) * HALF + p) : 0.f;
+    }
+  };
+  load_batch(0);
+  const int64_t slot = tok < w.n_slots ? write_slot(w, tok) : -1;
+  if (threadIdx.x < 16) s_b[threadIdx.x] = threadIdx.x < w.n_bounds[src] ? w.bounds[src][threadIdx.x] : CUDART_INF_F;
+  const int64_t at = token_offset(w, src, tok) + (int64_t)h * w.head_stride[src];
+  float xv[XPL], ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < XPL; ++i) xv[i] = load_as_float(w.x[src], w.x_dtype, at + lane + 32 * i);
+#pragma unroll
+  for (int i = 0; i < XPL; ++i) ss = fmaf(xv[i], xv[i], ss);
+  const float norm = sqrtf(warp_sum(ss)), den = norm + 1e-10f;
+  if (warp == 0) {
+#pragma unroll
+    for (int i = 0; i < XPL; ++i) s_x[lane + 32 * i] = xv[i] / den;
+  }
+  __syncthreads();
+  float ae = 0.f, ao = 0.f;
+#pragma unroll
+  for (int kb = 0; kb < KQ; kb += KB) {
+    if (kb > 0) load_batch(kb);
+#pragma unroll
+    for (int u = 0; u < KB; ++u) {
+      const float xk = s_x[k0 + kb + u];
+      ae = fmaf(xk, pe[u], ae);
+      ao = fmaf(xk, po[u], ao);
+    }
+  }
+  if (p < HALF) *reinterpret_cast<float2*>(&s_part[q][2 * p]) = make_float2(ae, ao);
+  __syncthreads();
   if (slot < 0) return;
   if (slot >= w.num_cache_slots) {
-    if (lane == 0 && w.err_flag) atomicOr(w.err_flag, TQ4_DEV_BAD_SLOT);
+    if (threadIdx.x == 0 && w.err_flag) atomicOr(w.err_flag, TQ4_DEV_BAD_SLOT);
     return;
   }
   const RowLayout lay = row_layout(w.num_heads, D);
   uint8_t* rowp = w.cache + slot * w.cache_token_stride;
   uint8_t* dst = rowp + (src == 0 ? lay.k_idx : lay.v_idx) + h * HALF;
+  if (threadIdx.x < HALF) {
+    const int c = threadIdx.x;
+    float y[2];
 #pragma unroll
-  for (int i = 0; i < NBL; ++i)
-    if (lane + 32 * i < HALF)
-      dst[lane + 32 * i] = (uint8_t)((bucketize_sorted16(acc[2 * i], s_b) << 4) | bucketize_sorted16(acc[2 * i + 1], s_b));
-  if (lane == 0) *reinterpret_cast<float*>(rowp + (src == 0 ? lay.k_norm : lay.v_norm) + h * 4) = norm;
+    for (int e = 0; e < 2; ++e) y[e] = (s_part[0][2 * c + e] + s_part[1][2 * c + e]) + (s_part[2][2 * c + e] + s_part[3][2 * c + e]);
+    dst[c] = (uint8_t)((bucketize_sorted16(y[0], s_b) << 4) | bucketize_sorted16(y[1], s_b));
+  }
+  if (threadIdx.x == 0) *reinterpret_cast<float*>(rowp + (src == 0 ? lay.k_norm : lay.v_norm) + h * 4) = norm;
 }
 
-// Vectors up to which a step takes a block per vector.  One decode call, graph replay, without -> with it:
-// 36 vectors (batch 1, 28 + 4 + 4) 19.4 -> 16.3 us, 192 (batch 4) 20.9 -> 17.7, 576 (batch 32, 14 + 2 + 2, head_dim 64)
-// 23.7 -> 23.3, 768 (batch 16) 42.1 -> 40.7: every vector reads all of Pi^T, so the
-// gain shrinks as they grow in number.
-constexpr int64_t kTinyStep = 1024;
+constexpr int64_t kTinyWrites = 2 * kTinyQueries;  // new vectors beside them; more are left to the write kernels
 
-template <int D, bool Q_ONLY>
+template <int D, bool WRITE, bool FRAG>
 int launch_tiny_prologue(const AttnArgs& a, const CompressArgs& w, int64_t vectors, cudaStream_t st) {
-  const size_t smem = 2 * (size_t)a.sh.rows * sizeof(int);
+  const size_t smem = FRAG ? 0 : 2 * (size_t)a.sh.rows * sizeof(int);
   // (first kernel of an entry point: plain stream-ordered launch, see launch_prologue_jc)
-  if (launch_kernel(tiny_prologue_kernel<D, Q_ONLY>, dim3((unsigned)vectors + 1), dim3(128), smem, st, false, a, w) != cudaSuccess)
+  if (launch_kernel(tiny_prologue_kernel<D, WRITE, FRAG>, dim3((unsigned)vectors + (FRAG ? 0 : 1)), dim3(TinyStepCfg<D>::THREADS), smem,
+                    st, false, a, w) != cudaSuccess)
     return TQ4_ERR_CUDA;
   TQ4_CHECK_LAUNCH();
   return TQ4_OK;
@@ -617,13 +645,17 @@ int launch_prologue_t(const AttnArgs* a, const CompressArgs* w, cudaStream_t st)
   const int64_t n_w = w ? w->n_tokens * w->num_heads * w->n_sources : 0;
   const int64_t chunks = (n_q + VC - 1) / VC + (n_w + VC - 1) / VC;
   const int64_t blocks = (chunks + WARPS - 1) / WARPS;
-  if constexpr (D <= 128)
-    if (a && a->skip_long == 0) {
-      if (w && w->cache && n_w > 0 && n_q + n_w <= kTinyStep) return launch_tiny_prologue<D, false>(*a, *w, n_q + n_w, st);
-      // without Pi^T a block occupies its SM's load pipe for 2 us (rows of Pi across the lanes): one block an SM
-      // (32 vectors: a call 1.3 us shorter; 580: 13 us longer)
-      if (n_w == 0 && n_q <= sm_count()) return launch_tiny_prologue<D, true>(*a, CompressArgs{}, n_q, st);
+  if (a && a->skip_long == 0 && n_q <= kTinyQueries) {
+    static const CompressArgs no_write{};
+    if (w && n_w > kTinyWrites) {
+      const int rc = dispatch_compress(*w, D, w->x_dtype, st);
+      if (rc != TQ4_OK) return rc;
+      w = nullptr;
     }
+    const int64_t n = n_q + (w ? n_w : 0);
+    if (a->no_plan) return w ? launch_tiny_prologue<D, true, true>(*a, *w, n, st) : launch_tiny_prologue<D, false, true>(*a, no_write, n, st);
+    return w ? launch_tiny_prologue<D, true, false>(*a, *w, n, st) : launch_tiny_prologue<D, false, false>(*a, no_write, n, st);
+  }
   const int64_t wave = 3 * (int64_t)sm_count() / (D / 32);
   if (blocks <= wave) return launch_prologue_jc<D, 32>(a, w, st, blocks);
   // a mixed call streams few of its rows (the kernel finds out how many)
@@ -1332,6 +1364,20 @@ static int attention_impl(
   const bool want_fused = fused_env != nullptr && atoi(fused_env) != 0;
   a.fused = use_mma && query_start_loc == nullptr && num_rows <= kFusedMaxRows &&
             head_dim <= 128 && want_fused;
+
+  a.sh.rows = (int)rows_cap;
+  const int cl_shift = mode == 0 && use_mma && !use_prefill && num_rows <= kMaxRowsPerLaunch && !a.fused ? decode_step_cluster(a) : -1;
+  if (cl_shift >= 0) {
+    a.no_plan = 1;
+    prof_begin(TQ4_PROF_PROLOGUE, st);
+    int rc = launch_prologue(&a, wr, head_dim, st);
+    prof_end(TQ4_PROF_PROLOGUE, st);
+    if (rc != TQ4_OK) return rc;
+    prof_begin(TQ4_PROF_ATTENTION, st);
+    rc = launch_decode_step(a, cl_shift, st);
+    prof_end(TQ4_PROF_ATTENTION, st);
+    return rc;
+  }
 
   for (int64_t r0 = 0; use_stream && r0 < num_rows; r0 += kMaxRowsPerLaunch) {
     a.sh.rows = (int)((num_rows - r0) < kMaxRowsPerLaunch ? (num_rows - r0) : kMaxRowsPerLaunch);

@@ -97,6 +97,7 @@ struct AttnArgs {
   int out_rotated;
   int* err_flag;
   int skip_long;     // > 0: sequences with at least this many new rows are left to the prefill kernel
+  int no_plan;       // the prologue rotates (and writes) only, its queries are fp16 terms (tq4_decode_step.cu)
   int plan_records;  // the plan writes row_rec and span_rec (tensor-core kernel)
   int fused;  // tensor-core kernel: compute the tile plan and rotate the queries inside the kernel
   const CompressArgs* fused_write;  // host side only: the step's cache write, done inside the fused kernel
@@ -166,6 +167,12 @@ int launch_attention_mma(const AttnArgs& a, cudaStream_t st);  // returns TQ4_ER
 // tensor-core (tcgen05) chunked-prefill kernel (tq4_prefill_tc.cu) over the sequences with at least `min_rows`
 // new rows: rotates, attends, un-rotates and writes the output, or leaves `splits` dense partials per row
 // (normalised rotated output in part_o [splits][rows][Hq][D], natural-log LSE in part_m [splits][rows][Hq])
+// Query vectors up to which the prologue of a call takes a block per vector (whether it writes or not: its sums are folded in
+// another order than those of the prologue for many)
+constexpr int64_t kTinyQueries = 768;
+// small decode steps (tq4_decode_step.cu): log2 of the CTAs that share a (row, KV head), or -1: the streaming kernel's
+int decode_step_cluster(const AttnArgs& a);
+int launch_decode_step(const AttnArgs& a, int cl_shift, cudaStream_t st);
 bool prefill_tc_supported(const AttnArgs& a);
 int prefill_tc_splits(const AttnArgs& a, int64_t slots);
 size_t prefill_tc_image_bytes(int D);

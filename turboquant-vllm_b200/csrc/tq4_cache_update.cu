@@ -70,14 +70,16 @@ __device__ __forceinline__ void load_row(const float* p, float (&v)[NJ]) {
 // rotate back -- in batches of four rows a lane.  Bound by latency; staging Pi for four vectors a warp, as below,
 // cost 18 us for
 // a token of four sequences at head_dim 128 and 63 at 256, against 5.5 and 9.
-template <int D>
+// FEW: for so few vectors that each has an SM to itself: a warp per 32 column pairs, all of its share of Pi^T (head_dim 256: half)
+// asked for before anything is known of the vector, and all of Pi before the indices are found.
+template <int D, bool FEW>
 struct TinyCfg {
-  static constexpr int CS = D == 256 ? 2 : 1, WARPS = 4 * CS, THREADS = 32 * WARPS;
-  static constexpr int HALF = D / 2, NBL = (HALF / CS + 31) / 32, NJ = D / 32 / CS, B = 4;
+  static constexpr int CS = FEW ? (D == 96 ? 1 : D / 64) : D == 256 ? 2 : 1, WARPS = 4 * CS, THREADS = 32 * WARPS;
+  static constexpr int HALF = D / 2, NBL = (HALF / CS + 31) / 32, NJ = D / 32 / CS, B = FEW ? (D == 256 ? 32 : D / 4) : 4;
 };
-template <int D>
-__global__ void __launch_bounds__(TinyCfg<D>::THREADS) cache_update_tiny_kernel(const UpdateArgs a) {
-  using C = TinyCfg<D>;
+template <int D, bool FEW>
+__global__ void __launch_bounds__(TinyCfg<D, FEW>::THREADS) cache_update_tiny_kernel(const UpdateArgs a) {
+  using C = TinyCfg<D, FEW>;
   constexpr int HALF = C::HALF, NBL = C::NBL, NJ = C::NJ, B = C::B, XPL = D / 32, KQ = D / 4;
   static_assert(KQ % B == 0, "whole batches");
   __shared__ __align__(16) float s_part[4][D];
@@ -438,11 +440,20 @@ int launch_update(const UpdateArgs& a, cudaStream_t st) {
 // 8.8 and 10.1 us, 96 4.4 / 6.6 / 14.7 and 14.0, 128 5.4 / 8.5 / 19 and 19, 256 8.7 / 27 / 68 and 65).  Eight vectors a warp
 // (half the reads of Pi per FMA) once every warp of the GPU has that many.
 constexpr int64_t kTinyUpdate = 2800;
+// The form with all loads in flight at once up to so many vectors an SM (8 - 64 vectors / 148 / 296 / 592, without and with it: head_dim 64
+// 3.5 / 3.5 / 3.6 / 3.8 and 2.7 / 2.8 / 2.9 / 3.2 us, 96 4.5 / 4.9 / 5.0 / 5.5 and 3.2 / 3.3 / 3.8 / 4.7, 128 5.4 / 5.5 / 5.8 / 6.2 and 3.7 / 3.8 / 4.5 /
+// 7.1, 256 8.7 / 9.0 / 9.5 / 15.9 and 6.7 / 6.9 / 12.3 / 23.2).
+template <int D> constexpr int kFewUpdate = D == 256 ? 1 : D == 128 ? 2 : 4;
 template <int D>
 int launch_update(const UpdateArgs& a, cudaStream_t st) {
   const int64_t vectors = 2 * (int64_t)a.batch * a.heads * a.n_new;
+  if (vectors <= kFewUpdate<D> * (int64_t)sm_count()) {
+    cache_update_tiny_kernel<D, true><<<(unsigned)vectors, TinyCfg<D, true>::THREADS, 0, st>>>(a);
+    TQ4_CHECK_LAUNCH();
+    return TQ4_OK;
+  }
   if (vectors <= kTinyUpdate) {
-    cache_update_tiny_kernel<D><<<(unsigned)vectors, TinyCfg<D>::THREADS, 0, st>>>(a);
+    cache_update_tiny_kernel<D, false><<<(unsigned)vectors, TinyCfg<D, false>::THREADS, 0, st>>>(a);
     TQ4_CHECK_LAUNCH();
     return TQ4_OK;
   }

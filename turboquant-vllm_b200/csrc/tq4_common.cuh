@@ -302,6 +302,8 @@ inline bool tokens_uniform(const CompressArgs& a) {
 }
 
 // Which kernel makes a write of so many vectors (B200, back to back, bf16):
+//   a block per vector that asks for all of Pi at once up to few_rows(): 8 - 148 vectors of 128 2.8 - 3.0 us against 4.4 of the next one, 296
+//     3.4 / 4.6, 444 5.1 / 4.6; of 64 2.2 / 2.7, 592 2.6 / 3.0; of 96 2.7 / 4.4, 444 3.9 / 4.9, 592 5.2 / 5.0; of 256 4.7 / 11.2, 296 8.0 / 11.3
 //   a block per vector up to tiny_rows(): a few us plus 1.1 / 1.7 / 2.5 us per 1000 vectors of 64 / 96 / 128, against 8 - 14 us
 //     of the tensor-core kernel; at 256 it never pays
 //   the tensor-core kernel above tc_rows(): 4096 vectors of 128 14.4 us either way, 5120 - 8192 14.4 against 18.5 us of the prologue
@@ -311,6 +313,7 @@ inline bool tokens_uniform(const CompressArgs& a) {
 //   the prologue kernel in between, and up to kSmallRows for what the tensor-core kernel cannot address
 constexpr int64_t kSmallRows = 8192;
 constexpr int64_t tiny_rows(int head_dim) { return head_dim == 64 ? 6500 : head_dim == 96 ? 3000 : head_dim == 128 ? 4096 : 0; }
+inline int64_t few_rows(int head_dim) { return (head_dim == 64 ? 4 : head_dim == 96 ? 3 : 2) * (int64_t)sm_count(); }
 constexpr int64_t tc_rows(int head_dim) { return head_dim == 256 ? 1000 : tiny_rows(head_dim); }
 int launch_small_write(const CompressArgs& w, int head_dim, cudaStream_t st);
 // `fma_bytes`: the bytes of the FMA kernels above kSmallRows, too

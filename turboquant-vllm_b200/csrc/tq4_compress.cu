@@ -327,12 +327,104 @@ __global__ void __launch_bounds__(128, 16) compress_small_kernel(const CompressA
 }
 
 
+// The same for so few vectors that each has an SM to itself: a lane per column pair (32 of them a warp), so that all of a
+// quarter's Pi^T (head_dim 256: half) is in flight at once, before anything is known of the vector.
+template <int D>
+struct FewCfg {
+  static constexpr int HALF = D / 2, CS = (HALF + 31) / 32, THREADS = 128 * CS, KQ = D / 4, KB = D == 256 ? 32 : KQ;
+};
+template <int D, typename T, bool SEQ>
+__global__ void __launch_bounds__(FewCfg<D>::THREADS) compress_few_kernel(const CompressArgs a) {
+  using C = FewCfg<D>;
+  constexpr int HALF = C::HALF, XPL = D / 32, KQ = C::KQ, KB = C::KB;
+  __shared__ float s_x[D];
+  __shared__ __align__(16) float s_part[4][D];
+  __shared__ float s_b[16];
+  pdl_trigger();
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int q = warp & 3, p = 32 * (warp >> 2) + lane, k0 = q * KQ;
+  float pe[KB], po[KB];
+  auto load_batch = [&](int kb) {
+#pragma unroll
+    for (int u = 0; u < KB; ++u) {
+      pe[u] = p < HALF ? __ldg(a.rot_even + (k0 + kb + u) * HALF + p) : 0.f;
+      po[u] = p < HALF ? __ldg(a.rot_odd + (k0 + kb + u) * HALF + p) : 0.f;
+    }
+  };
+  load_batch(0);
+  const int64_t row = blockIdx.x;
+  const int64_t rows_per_src = a.n_tokens * a.num_heads;
+  const int src = row >= rows_per_src ? 1 : 0;
+  const unsigned rem = (unsigned)(row - (src ? rows_per_src : 0));
+  const int64_t tok = rem / (unsigned)a.num_heads;
+  const int h = (int)(rem - (unsigned)tok * (unsigned)a.num_heads);
+  if (threadIdx.x < 16) s_b[threadIdx.x] = threadIdx.x < a.n_bounds[src] ? a.bounds[src][threadIdx.x] : CUDART_INF_F;
+  const int64_t at = SEQ ? token_offset(a, src, tok) : tok * a.token_stride[src];
+  const T* xp = reinterpret_cast<const T*>(a.x[src]) + at + (int64_t)h * a.head_stride[src];
+  int64_t slot = -1;
+  if (a.cache != nullptr && tok < a.n_slots) slot = SEQ ? write_slot(a, tok) : a.slot_mapping[tok];
+  float xv[XPL], ss = 0.f;
+#pragma unroll
+  for (int i = 0; i < XPL; ++i) xv[i] = to_float<T>(xp[lane + 32 * i]);
+#pragma unroll
+  for (int i = 0; i < XPL; ++i) ss = fmaf(xv[i], xv[i], ss);
+  const float norm = sqrtf(warp_sum(ss)), den = norm + 1e-10f;
+  if (warp == 0) {
+#pragma unroll
+    for (int i = 0; i < XPL; ++i) s_x[lane + 32 * i] = xv[i] / den;
+  }
+  __syncthreads();
+  float ae = 0.f, ao = 0.f;
+#pragma unroll
+  for (int kb = 0; kb < KQ; kb += KB) {
+    if (kb > 0) load_batch(kb);
+#pragma unroll
+    for (int u = 0; u < KB; ++u) {
+      const float xk = s_x[k0 + kb + u];
+      ae = fmaf(xk, pe[u], ae);
+      ao = fmaf(xk, po[u], ao);
+    }
+  }
+  if (p < HALF) *reinterpret_cast<float2*>(&s_part[q][2 * p]) = make_float2(ae, ao);
+  __syncthreads();
+  uint8_t* dst_idx;
+  float* dst_norm;
+  if (a.cache != nullptr) {
+    if (slot < 0) return;  // (a padding token, or one without a slot)
+    if (slot >= a.num_cache_slots) {
+      if (threadIdx.x == 0 && a.err_flag) atomicOr(a.err_flag, TQ4_DEV_BAD_SLOT);
+      return;
+    }
+    const RowLayout lay = row_layout(a.num_heads, D);
+    uint8_t* rowp = a.cache + slot * a.cache_token_stride;
+    dst_idx = rowp + (src == 0 ? lay.k_idx : lay.v_idx) + h * HALF;
+    dst_norm = reinterpret_cast<float*>(rowp + (src == 0 ? lay.k_norm : lay.v_norm) + h * 4);
+  } else {
+    dst_idx = a.packed_out + row * HALF;
+    dst_norm = a.norms_out + row;
+  }
+  if (threadIdx.x < HALF) {
+    const int c = threadIdx.x;
+    float y[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) y[e] = (s_part[0][2 * c + e] + s_part[1][2 * c + e]) + (s_part[2][2 * c + e] + s_part[3][2 * c + e]);
+    dst_idx[c] = (uint8_t)((bucketize_sorted16(y[0], s_b) << 4) | bucketize_sorted16(y[1], s_b));
+  }
+  if (threadIdx.x == 0) *dst_norm = norm;
+}
+
 template <int D, typename T>
 int launch_compress(const CompressArgs& a, cudaStream_t st) {
   using Cfg = CompressCfg<D>;
   const int64_t total_rows = a.n_tokens * a.num_heads * a.n_sources;
   if (total_rows == 0) return TQ4_OK;
   if (total_rows > 0x7fffffffll) return TQ4_ERR_INVALID_ARG;  // the kernels index rows with 32 bits
+  if (total_rows <= few_rows(D)) {
+    if (a.seq) compress_few_kernel<D, T, true><<<(unsigned)total_rows, FewCfg<D>::THREADS, 0, st>>>(a);
+    else compress_few_kernel<D, T, false><<<(unsigned)total_rows, FewCfg<D>::THREADS, 0, st>>>(a);
+    TQ4_CHECK_LAUNCH();
+    return TQ4_OK;
+  }
   if (total_rows <= tiny_rows(D)) {
     if (a.seq) compress_small_kernel<D <= 128 ? D : 128, T, true><<<(unsigned)total_rows, 128, 0, st>>>(a);
     else compress_small_kernel<D <= 128 ? D : 128, T, false><<<(unsigned)total_rows, 128, 0, st>>>(a);
@@ -362,7 +454,7 @@ int dispatch_dtype(const CompressArgs& a, int dtype, cudaStream_t st) {
 int dispatch_compress(const CompressArgs& a, int head_dim, int dtype, cudaStream_t st, bool fma_bytes) {
   const int64_t vectors = a.n_tokens * a.num_heads * a.n_sources;
   if (vectors == 0) return TQ4_OK;
-  const bool tiny = vectors <= tiny_rows(head_dim);  // (dispatch_dtype: a block per vector)
+  const bool tiny = vectors <= few_rows(head_dim) || vectors <= tiny_rows(head_dim);  // (dispatch_dtype: a block per vector)
   fma_bytes = fma_bytes || vectors <= kSmallRows;
   if (vectors > tc_rows(head_dim) && compress_tc16_eligible(a, head_dim, dtype))
     return launch_compress_tc16(a, head_dim, dtype, fma_bytes, st);
