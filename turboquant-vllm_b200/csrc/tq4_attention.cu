@@ -602,7 +602,6 @@ __global__ void __launch_bounds__(TinyStepCfg<D>::THREADS) tiny_prologue_kernel(
   if (threadIdx.x == 0) *reinterpret_cast<float*>(rowp + (src == 0 ? lay.k_norm : lay.v_norm) + h * 4) = norm;
 }
 
-constexpr int64_t kTinyWrites = 2 * kTinyQueries;  // new vectors beside them; more are left to the write kernels
 
 template <int D, bool WRITE, bool FRAG>
 int launch_tiny_prologue(const AttnArgs& a, const CompressArgs& w, int64_t vectors, cudaStream_t st) {
@@ -645,9 +644,9 @@ int launch_prologue_t(const AttnArgs* a, const CompressArgs* w, cudaStream_t st)
   const int64_t n_w = w ? w->n_tokens * w->num_heads * w->n_sources : 0;
   const int64_t chunks = (n_q + VC - 1) / VC + (n_w + VC - 1) / VC;
   const int64_t blocks = (chunks + WARPS - 1) / WARPS;
-  if (a && a->skip_long == 0 && n_q <= kTinyQueries) {
+  if (a && a->skip_long == 0 && n_q <= tiny_queries(D)) {
     static const CompressArgs no_write{};
-    if (w && n_w > kTinyWrites) {
+    if (w && n_w > 2 * tiny_queries(D)) {  // (new vectors: more are left to the write kernels)
       const int rc = dispatch_compress(*w, D, w->x_dtype, st);
       if (rc != TQ4_OK) return rc;
       w = nullptr;

@@ -168,8 +168,10 @@ int launch_attention_mma(const AttnArgs& a, cudaStream_t st);  // returns TQ4_ER
 // new rows: rotates, attends, un-rotates and writes the output, or leaves `splits` dense partials per row
 // (normalised rotated output in part_o [splits][rows][Hq][D], natural-log LSE in part_m [splits][rows][Hq])
 // Query vectors up to which the prologue of a call takes a block per vector (whether it writes or not: its sums are folded in
-// another order than those of the prologue for many)
-constexpr int64_t kTinyQueries = 768;
+// another order than those of the prologue for many).  Whole steps on 3000 keys each, us without / with it: 512 + 256 vectors of 128 37.6 /
+// 35.0, 768 + 384 43.4 / 39.6; of 64 equal up to 756 + 216; of 96 384 + 768 53.4 / 51.5, 512 + 1024 61.7 / 62.0; of 256 192 + 192 49.7 / 47.3, 256 + 256
+// 57.4 / 57.1, 512 + 512 83.8 / 91.7.
+constexpr int64_t tiny_queries(int head_dim) { return head_dim == 256 ? 256 : head_dim == 96 ? 448 : 768; }
 // small decode steps (tq4_decode_step.cu): log2 of the CTAs that share a (row, KV head), or -1: the streaming kernel's
 int decode_step_cluster(const AttnArgs& a);
 int launch_decode_step(const AttnArgs& a, int cl_shift, cudaStream_t st);

@@ -498,7 +498,7 @@ int launch_step_d(const AttnArgs& a, int cl_shift, cudaStream_t st) {
 // 30.8 / 24.9; 2 x 4000 22.5 / 16.8, 2 x 8000 26.0 / 24.5; 4 x 2000 23.9 / 18.3, 4 x 4000 24.6 / 24.6; 8 x 2000 24.7 / 20.5, 8 x 4000
 // 29.0 / 33.4; 16 x 1000 28.7 / 22.6, 16 x 2000 31.0 / 36.8 us.  (The lengths are on the device: the longest counts.)
 int decode_step_cluster(const AttnArgs& a) {
-  if (a.block_size % kTileTokens != 0 || (int64_t)a.sh.rows * a.sh.Hq > kTinyQueries) return -1;
+  if (a.block_size % kTileTokens != 0 || (int64_t)a.sh.rows * a.sh.Hq > tiny_queries(a.sh.D)) return -1;
   const int64_t units = (int64_t)a.sh.rows * a.sh.Hkv * a.sh.NCH;
   const int64_t keys = a.sliding_window > 0 && a.sliding_window < a.max_keys ? a.sliding_window : a.max_keys;
   const bool two = a.sh.D * (a.sh.GC <= 4 ? 1 : 2) <= 128;

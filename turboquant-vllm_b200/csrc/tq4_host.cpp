@@ -251,7 +251,9 @@ PyObject* attention(PyObject*, PyObject* const* p, Py_ssize_t n) {
     if (have < need)
       fail(PyExc_ValueError, "workspace has " + std::to_string(have) + " bytes, " + std::to_string(need) + " needed");
     const int causal = truth(p[11]) ? 1 : 0, window = (int)int_or_zero(p[12]);
-    const int64_t max_seq_len = p[20] == Py_None ? 0 : as_int(p[20]);
+    // (the width of the table bounds it, too; the stride, which the C interface has, may be a wider one's)
+    int64_t max_seq_len = p[20] == Py_None ? 0 : as_int(p[20]);
+    if (bt.size(1) > 0 && (max_seq_len <= 0 || max_seq_len > bt.size(1) * block)) max_seq_len = bt.size(1) * block;
     const int rotated = truth(p[16]) ? 1 : 0, mode = (int)as_int(p[18]);
     int* flag = (int*)flag_of(dev).data_ptr();
     const int q_dt = dtype_code(q.scalar_type()), out_dt = dtype_code(out.scalar_type());
