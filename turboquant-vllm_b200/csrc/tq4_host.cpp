@@ -19,6 +19,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdint>
+#include <memory>
 #include <stdexcept>
 #include <string>
 #include <thread>
@@ -431,10 +432,28 @@ PyObject* append_rows(PyObject*, PyObject* const* p, Py_ssize_t n) {
   });
 }
 
+// What an in-place cache update found to fit together: the types and sizes of the states, the device's tables, and the buffers as
+// the Python objects that held them (compared by a later step: a buffer that was replaced since is noticed).
+struct UpdatePlan {
+  int64_t b, h, d, cap, dec_cap;
+  at::ScalarType dtype;
+  int dev;
+  bool k_nib, v_nib;
+  at::Tensor prims[7];             // rotation, even, odd, boundaries and centroids of K and V
+  std::vector<at::Tensor> out;     // k_idx, k_norms, v_idx, v_norms (and k_dec, v_dec)
+  std::vector<PyObject*> held;     // ... as Python objects, and the two quantisers
+  ~UpdatePlan() {
+    for (PyObject* o : held) Py_XDECREF(o);
+  }
+};
+constexpr const char* kPlanName = "tq4.update_plan";
+PyObject *g_buf_name, *g_len_name;  // interned attribute names
+
 // cache_update(key, value, rotation, rotation_T_even, rotation_T_odd, k_boundaries, v_boundaries, k_centroids, v_centroids, k_nibble, v_nibble,
-//              k_idx, k_norms, v_idx, v_norms, offset, k_dec, v_dec, dec_offset)
+//              k_idx, k_norms, v_idx, v_norms, offset, k_dec, v_dec, dec_offset[, k_quantizer, v_quantizer])
+// With the quantisers: returns the plan of the update, for cache_step.
 PyObject* cache_update(PyObject*, PyObject* const* p, Py_ssize_t n) {
-  if (!expect("cache_update", n, 19)) return nullptr;
+  if (n != 21 && !expect("cache_update", n, 19)) return nullptr;
   return guarded([&]() -> PyObject* {
     const States k(p[0], "key"), v(p[1], "value");
     const at::Tensor& rot = cuda_tensor(p[2], "rotation");
@@ -481,7 +500,103 @@ PyObject* cache_update(PyObject*, PyObject* const* p, Py_ssize_t n) {
                             dec_offset, need ? scratch.data_ptr() : nullptr, need, launch.stream);
     }
     check(st, "tq4_cache_update");
-    Py_RETURN_NONE;
+    if (n == 19) Py_RETURN_NONE;
+    auto plan = std::make_unique<UpdatePlan>();
+    plan->b = b; plan->h = h; plan->d = d;
+    plan->cap = cap;
+    plan->dec_cap = dec_cap;
+    plan->dtype = k.t.scalar_type();
+    plan->dev = device_index(k.t);
+    plan->k_nib = k_nib;
+    plan->v_nib = v_nib;
+    const at::Tensor* prims[7] = {&rot, &even, &odd, &kb, &vb, &kc, &vc};
+    for (int i = 0; i < 7; ++i) plan->prims[i] = *prims[i];
+    for (int i : {11, 12, 13, 14, 16, 17}) {
+      if (p[i] == Py_None) continue;
+      plan->out.push_back(THPVariable_Unpack(p[i]));
+      Py_INCREF(p[i]);
+      plan->held.push_back(p[i]);
+    }
+    for (int i : {19, 20}) {
+      Py_INCREF(p[i]);
+      plan->held.push_back(p[i]);
+    }
+    PyObject* c = PyCapsule_New(plan.get(), kPlanName, [](PyObject* o) { delete (UpdatePlan*)PyCapsule_GetPointer(o, kPlanName); });
+    if (!c) throw PyError{};
+    plan.release();
+    return c;
+  });
+}
+
+// cache_step(plan, groups, key, value, k_quantizer, v_quantizer): another update into the plan's buffers, which are the `buf` of the
+// groups with `len` tokens each -> (keys, values) of all tokens held, reconstructed, or True without such buffers; None, with nothing changed,
+// when the states or the groups are not those of the plan, or there is no room left.
+PyObject* cache_step(PyObject*, PyObject* const* p, Py_ssize_t n) {
+  if (!expect("cache_step", n, 6)) return nullptr;
+  return guarded([&]() -> PyObject* {
+    UpdatePlan* plan = (UpdatePlan*)PyCapsule_GetPointer(p[0], kPlanName);
+    if (!plan) throw PyError{};
+    const size_t n_out = plan->out.size();
+    if (!PyTuple_Check(p[1]) || (size_t)PyTuple_GET_SIZE(p[1]) != n_out || plan->held[n_out] != p[4] || plan->held[n_out + 1] != p[5] ||
+        !THPVariable_Check(p[2]) || !THPVariable_Check(p[3]))
+      Py_RETURN_NONE;
+    const at::Tensor &k = THPVariable_Unpack(p[2]), &v = THPVariable_Unpack(p[3]);
+    if (k.dim() != 4 || !k.is_cuda() || !v.is_cuda() || k.scalar_type() != plan->dtype || v.scalar_type() != plan->dtype || k.sizes() != v.sizes() ||
+        k.get_device() != plan->dev || v.get_device() != plan->dev || k.size(0) != plan->b || k.size(1) != plan->h || k.size(3) != plan->d ||
+        k.size(2) == 0)
+      Py_RETURN_NONE;
+    const int64_t fresh = k.size(2);
+    int64_t len[2] = {-1, 0};  // tokens held: compressed, reconstructed
+    for (size_t i = 0; i < n_out; ++i) {
+      PyObject* g = PyTuple_GET_ITEM(p[1], i);
+      PyObject* buf = PyObject_GetAttr(g, g_buf_name);
+      if (!buf) throw PyError{};
+      const bool same = buf == plan->held[i];
+      Py_DECREF(buf);
+      if (!same) Py_RETURN_NONE;
+      PyObject* l = PyObject_GetAttr(g, g_len_name);
+      if (!l) throw PyError{};
+      const long long x = PyLong_AsLongLong(l);
+      Py_DECREF(l);
+      if (x == -1 && PyErr_Occurred()) throw PyError{};
+      int64_t& want = len[i < 4 ? 0 : 1];
+      if (i == 0 || i == 4) want = x;
+      else if (x != want) Py_RETURN_NONE;
+    }
+    if (len[0] < 0 || len[1] < 0 || len[0] + fresh > plan->cap || (n_out == 6 && len[1] + fresh > plan->dec_cap)) Py_RETURN_NONE;
+    const States ks(p[2], "key"), vs(p[3], "value");
+    Launch launch(plan->dev);
+    const size_t need = tq4_cache_update_scratch_bytes((int)plan->b, (int)plan->h, (int)fresh, (int)plan->d);
+    at::Tensor scratch;
+    if (need) scratch = at::empty({(int64_t)need}, k.options().dtype(at::kByte).requires_grad(false));
+    auto f = [&](int i) { return (const float*)plan->prims[i].data_ptr(); };
+    int st;
+    {
+      const NoGil no_gil;
+      st = tq4_cache_update(ks.t.data_ptr(), vs.t.data_ptr(), dtype_code(plan->dtype), (int)plan->b, (int)plan->h, (int)fresh, (int)plan->d,
+                            ks.strides, vs.strides, f(0), f(1), f(2), f(3), (int)plan->prims[3].numel(), f(4), (int)plan->prims[4].numel(), f(5),
+                            (int)plan->prims[5].numel(), f(6), (int)plan->prims[6].numel(), plan->k_nib, plan->v_nib,
+                            (uint8_t*)plan->out[0].data_ptr(), (float*)plan->out[1].data_ptr(), (uint8_t*)plan->out[2].data_ptr(),
+                            (float*)plan->out[3].data_ptr(), plan->cap, len[0], n_out == 6 ? plan->out[4].data_ptr() : nullptr,
+                            n_out == 6 ? plan->out[5].data_ptr() : nullptr, plan->dec_cap, len[1], need ? scratch.data_ptr() : nullptr, need,
+                            launch.stream);
+    }
+    check(st, "tq4_cache_update");
+    for (int part = 0; part < (n_out == 6 ? 2 : 1); ++part) {
+      PyObject* l = PyLong_FromLongLong(len[part] + fresh);
+      if (!l) throw PyError{};
+      for (size_t i = part ? 4 : 0; i < (part ? n_out : 4); ++i)
+        if (PyObject_SetAttr(PyTuple_GET_ITEM(p[1], i), g_len_name, l) < 0) {
+          Py_DECREF(l);
+          throw PyError{};
+        }
+      Py_DECREF(l);
+    }
+    if (n_out == 4) Py_RETURN_TRUE;
+    PyObject* kv = PyTuple_New(2);
+    if (!kv) throw PyError{};
+    for (int i = 0; i < 2; ++i) PyTuple_SET_ITEM(kv, i, THPVariable_Wrap(plan->out[4 + i].narrow(2, 0, len[1] + fresh)));
+    return kv;
   });
 }
 
@@ -501,10 +616,16 @@ PyMethodDef kMethods[] = {
     {"attend_rows", (PyCFunction)(void (*)(void))attend_rows, METH_FASTCALL, "Attention of one query row per sequence over token rows."},
     {"append_rows", (PyCFunction)(void (*)(void))append_rows, METH_FASTCALL, "Compress K and V into token rows of a batch."},
     {"cache_update", (PyCFunction)(void (*)(void))cache_update, METH_FASTCALL, "Compress, store and reconstruct an update."},
+    {"cache_step", (PyCFunction)(void (*)(void))cache_step, METH_FASTCALL, "An update by a plan."},
     {"error_flag", (PyCFunction)(void (*)(void))error_flag, METH_FASTCALL, "Device error flag."},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_tq4_host", nullptr, -1, kMethods, nullptr, nullptr, nullptr, nullptr};
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__tq4_host(void) { return PyModule_Create(&kModule); }
+PyMODINIT_FUNC PyInit__tq4_host(void) {
+  g_buf_name = PyUnicode_InternFromString("buf");
+  g_len_name = PyUnicode_InternFromString("len");
+  if (!g_buf_name || !g_len_name) return nullptr;
+  return PyModule_Create(&kModule);
+}

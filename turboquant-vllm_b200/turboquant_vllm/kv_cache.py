@@ -59,7 +59,7 @@ class _GrowBuffer:
     def __init__(self) -> None:
         self.buf: torch.Tensor | None = None
         self.len = 0
-        self.fit = None  # (first buffer of a layer) what the last in-place update found to fit together
+        self.fit = None  # (first buffer of a layer) plan of the last in-place update, see CompressedDynamicCache._step
 
     def reserve(self, b: int, h: int, n: int, w: int, dtype: torch.dtype, device: torch.device) -> torch.Tensor:
         """The buffer with room for ``n`` more tokens of ``[b, h, ., w]``; a new one if it held another shape."""
@@ -356,6 +356,9 @@ class CompressedDynamicCache:
     # ----- the patched cache methods ----------------------------------------------------------------
     def _compressed_update(self, key_states, value_states, layer_idx: int, cache_kwargs=None):
         """Compress the new tokens, append, return K/V for attention (or placeholders in fused mode)."""
+        kv = self._step(key_states, value_states, layer_idx)
+        if kv is not None:
+            return kv
         if not self.enabled:
             return self._original_update(key_states, value_states, layer_idx, cache_kwargs)
         if layer_idx in self._full_attn_bypass:
@@ -408,6 +411,36 @@ class CompressedDynamicCache:
         layer.keys, layer.values = dec[0].view(), dec[1].view()
         return layer.keys, layer.values
 
+    def _step(self, key_states, value_states, layer_idx: int):
+        """An update like the one before of its layer, which is most of a generation: what it returns, or ``None`` (nothing
+        changed) for the whole way round.  The native part compares what the earlier update found with what is there now."""
+        if not self.enabled or layer_idx >= len(self._k_store) or layer_idx >= len(self.cache.layers):
+            return None
+        ks = self._k_store[layer_idx]
+        layer = self.cache.layers[layer_idx]
+        if ks is None or layer_idx in self._full_attn_bypass or not layer.is_initialized:
+            return None
+        dim = key_states.shape[-1]
+        k_comp, v_comp = self._key_compressors.get(dim), self._value_compressors.get(dim)
+        if k_comp is None or v_comp is None:
+            return None
+        rows, kv = self._rows[layer_idx], True
+        if self.fused_mode and self._k_nibble_packed and self._v_nibble_packed:
+            if rows is None or dim != self.head_dim or not rows.append_like(
+                    key_states, value_states, k_comp.quantizer, v_comp.quantizer):
+                return None
+        else:
+            dec = () if self.fused_mode else (self._dec_k[layer_idx], self._dec_v[layer_idx])
+            if rows is not None or ks[0].fit is None or None in dec or self.fused_mode and dim != self.head_dim:
+                return None
+            kv = nv.host().cache_step(ks[0].fit, (*ks, *self._v_store[layer_idx], *dec), key_states, value_states,
+                                      k_comp.quantizer, v_comp.quantizer)
+            if kv is None:
+                return None
+        layer.keys, layer.values = (key_states, value_states) if kv is True else kv  # (fused mode: placeholders)
+        self._original_dtype = key_states.dtype
+        return layer.keys, layer.values
+
     def _update_in_place(self, key_states, value_states, store, dec, k_quant, v_quant) -> bool:
         """Compress, store and (``dec``) reconstruct the new tokens in one launch behind the tokens held.
 
@@ -419,22 +452,6 @@ class CompressedDynamicCache:
                 or dev != value_states.device or not key_states.is_cuda or dtype not in _UPDATE_DTYPES):
             return False
         b, h, n, d = key_states.shape
-        groups, first = store + dec, store[0]
-        fit = first.fit
-        if fit is not None and n and fit[0] == (b, h, d, dtype, dev, k_quant, v_quant, len(dec)):
-            # the buffers of the update before, with room for this one
-            _, prims, out = fit
-            held, at = first.len, dec[0].len if dec else 0
-            if held + n <= out[0].shape[2] and (not dec or at + n <= out[4].shape[2]):
-                for g, t, want in zip(groups, out, (held, held, held, held, at, at)):
-                    if g.buf is not t or g.len != want:
-                        break
-                else:
-                    nv.host().cache_update(key_states, value_states, *prims, self._k_nibble_packed, self._v_nibble_packed,
-                                           *out[:4], held, *(out[4:] or (None, None)), at)
-                    for g in groups:
-                        g.len += n
-                    return True
         if n == 0 or d not in _UPDATE_DIMS or k_quant.bits > 4 or v_quant.bits > 4:
             return False
         rot, even, odd, k_cents, k_bounds = k_quant.device_primitives(dev)
@@ -453,13 +470,12 @@ class CompressedDynamicCache:
                     return False
                 bufs.append((g, w, t))
         # nothing here may hold the old buffers: each goes when its copy is made, not when all six have grown
-        store[0].fit = fit = out = buf = t = None
+        store[0].fit = out = buf = t = None
         out = [g.reserve(b, h, n, w, t, dev) for g, w, t in bufs]
         prims = (rot, even, odd, k_bounds, v_bounds, k_cents, v_cents)
-        nv.host().cache_update(
+        store[0].fit = nv.host().cache_update(
             key_states, value_states, *prims, self._k_nibble_packed, self._v_nibble_packed, *out[:4], store[0].len,
-            *(out[4:] or (None, None)), dec[0].len if dec else 0)
-        store[0].fit = ((b, h, d, dtype, dev, k_quant, v_quant, len(dec)), prims, out)
+            *(out[4:] or (None, None)), dec[0].len if dec else 0, k_quant, v_quant)
         for g, _, _ in bufs:
             g.len += n
         return True

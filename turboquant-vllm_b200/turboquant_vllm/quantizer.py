@@ -99,8 +99,10 @@ class TurboQuantMSE:
 
     def device_primitives(self, device: torch.device):
         """(rotation, rot_T_even, rot_T_odd, centroids, boundaries) resident on ``device``."""
-        device = torch.device(device)
         prim = self._dev.get(device)
+        if prim is None:
+            device = torch.device(device)
+            prim = self._dev.get(device)
         if prim is None:
             def rotation():
                 rot_t = self.rotation.T.contiguous()

@@ -106,6 +106,18 @@ class TokenRowStore:
         nv.host().append_rows(key_states, value_states, self.rows, self.len, even, odd, k_bounds, v_bounds)
         self.len += s
 
+    def append_like(self, key_states, value_states, k_quantizer, v_quantizer) -> bool:
+        """:meth:`append` where there is room and the states are like the store; else ``False``, nothing changed."""
+        b, h, s, d = shape = key_states.shape
+        if (b != self.batch or h != self.heads or d != self.dim or value_states.shape != shape or s == 0
+                or self.len + s > self._capacity or key_states.device != self.device):
+            return False
+        _, even, odd, _, k_bounds = k_quantizer.device_primitives(self.device)
+        v_bounds = v_quantizer.device_primitives(self.device)[4]
+        nv.host().append_rows(key_states, value_states, self.rows, self.len, even, odd, k_bounds, v_bounds)
+        self.len += s
+        return True
+
     @classmethod
     def from_tensors(cls, k_packed: torch.Tensor, k_norms: torch.Tensor, v_packed: torch.Tensor,
                      v_norms: torch.Tensor) -> "TokenRowStore":
