@@ -487,20 +487,19 @@ __global__ void __launch_bounds__(TinyStepCfg<D>::THREADS) tiny_prologue_kernel(
                        : make_float4(0.f, 0.f, 0.f, 0.f);
     const int row = vec / a.sh.Hq;
     const int64_t at = ((int64_t)row + a.sh.row_offset) * a.q_token_stride + (int64_t)(vec - row * a.sh.Hq) * a.q_head_stride;
+    uint4 raw[F4];
+#pragma unroll
+    for (int f = 0; f < F4; ++f) raw[f] = act ? load4_raw(a.q, a.q_dtype, at + 4 * (l4 + GL * f)) : make_uint4(0u, 0u, 0u, 0u);
     float v[NV], top = 0.f;
 #pragma unroll
     for (int i = 0; i < NV; ++i) v[i] = 0.f;
 #pragma unroll
     for (int f = 0; f < F4; ++f) {
-      float x[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        x[e] = act ? load_as_float(a.q, a.q_dtype, at + 4 * (l4 + GL * f) + e) : 0.f;
-        top = fmaxf(top, fabsf(x[e]));
-      }
+      const float4 x = raw_as_float4(raw[f], a.q_dtype);
+      top = fmaxf(top, fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))));
 #pragma unroll
       for (int i = 0; i < NV; ++i)
-        v[i] = fmaf(x[0], pi[i][f].x, fmaf(x[1], pi[i][f].y, fmaf(x[2], pi[i][f].z, fmaf(x[3], pi[i][f].w, v[i]))));
+        v[i] = fmaf(x.x, pi[i][f].x, fmaf(x.y, pi[i][f].y, fmaf(x.z, pi[i][f].z, fmaf(x.w, pi[i][f].w, v[i]))));
     }
     // fold: after the step of `o` lanes a lane has the sums of half as many rows
     int n = 0;  // row of the warp that the lane ends up with (of NV, padded to a power of two)
@@ -1368,12 +1367,15 @@ static int attention_impl(
   const int cl_shift = mode == 0 && use_mma && !use_prefill && num_rows <= kMaxRowsPerLaunch && !a.fused ? decode_step_cluster(a) : -1;
   if (cl_shift >= 0) {
     a.no_plan = 1;
-    prof_begin(TQ4_PROF_PROLOGUE, st);
-    int rc = launch_prologue(&a, wr, head_dim, st);
-    prof_end(TQ4_PROF_PROLOGUE, st);
-    if (rc != TQ4_OK) return rc;
+    const bool rotate = !wr && decode_step_rotates(a);
+    if (!rotate) {
+      prof_begin(TQ4_PROF_PROLOGUE, st);
+      const int rc = launch_prologue(&a, wr, head_dim, st);
+      prof_end(TQ4_PROF_PROLOGUE, st);
+      if (rc != TQ4_OK) return rc;
+    }
     prof_begin(TQ4_PROF_ATTENTION, st);
-    rc = launch_decode_step(a, cl_shift, st);
+    const int rc = launch_decode_step(a, cl_shift, rotate, st);
     prof_end(TQ4_PROF_ATTENTION, st);
     return rc;
   }

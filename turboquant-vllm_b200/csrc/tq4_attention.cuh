@@ -174,7 +174,8 @@ int launch_attention_mma(const AttnArgs& a, cudaStream_t st);  // returns TQ4_ER
 constexpr int64_t tiny_queries(int head_dim) { return head_dim == 256 ? 256 : head_dim == 96 ? 448 : 768; }
 // small decode steps (tq4_decode_step.cu): log2 of the CTAs that share a (row, KV head), or -1: the streaming kernel's
 int decode_step_cluster(const AttnArgs& a);
-int launch_decode_step(const AttnArgs& a, int cl_shift, cudaStream_t st);
+bool decode_step_rotates(const AttnArgs& a);  // it can rotate the queries itself (`rotate`: they are not yet)
+int launch_decode_step(const AttnArgs& a, int cl_shift, bool rotate, cudaStream_t st);
 bool prefill_tc_supported(const AttnArgs& a);
 int prefill_tc_splits(const AttnArgs& a, int64_t slots);
 size_t prefill_tc_image_bytes(int D);

@@ -133,6 +133,35 @@ __device__ __forceinline__ void store4(void* p, int dtype, int64_t i, const floa
   }
 }
 
+// four consecutive elements of a typed array as they are, in one load where their address allows it, and as floats: the loads of
+// several can be in flight before the first is converted
+__device__ __forceinline__ uint4 load4_raw(const void* p, int dtype, int64_t i) {
+  uint4 r = make_uint4(0u, 0u, 0u, 0u);
+  if (dtype == TQ4_F32) {
+    const uint32_t* s = reinterpret_cast<const uint32_t*>(p) + i;
+    if (((uintptr_t)s & 15) == 0) return __ldg(reinterpret_cast<const uint4*>(s));
+    r.x = __ldg(s); r.y = __ldg(s + 1); r.z = __ldg(s + 2); r.w = __ldg(s + 3);
+  } else {
+    const uint16_t* s = reinterpret_cast<const uint16_t*>(p) + i;
+    if (((uintptr_t)s & 7) == 0) {
+      const uint2 t = __ldg(reinterpret_cast<const uint2*>(s));
+      r.x = t.x; r.y = t.y;
+    } else {
+      r.x = __ldg(s) | (uint32_t)__ldg(s + 1) << 16;
+      r.y = __ldg(s + 2) | (uint32_t)__ldg(s + 3) << 16;
+    }
+  }
+  return r;
+}
+__device__ __forceinline__ float4 raw_as_float4(const uint4& r, int dtype) {
+  if (dtype == TQ4_F32) return make_float4(__uint_as_float(r.x), __uint_as_float(r.y), __uint_as_float(r.z), __uint_as_float(r.w));
+  if (dtype == TQ4_F16) {
+    const float2 a = __half22float2(*reinterpret_cast<const __half2*>(&r.x)), b = __half22float2(*reinterpret_cast<const __half2*>(&r.y));
+    return make_float4(a.x, a.y, b.x, b.y);
+  }
+  return make_float4(__uint_as_float(r.x << 16), __uint_as_float(r.x & 0xFFFF0000u), __uint_as_float(r.y << 16), __uint_as_float(r.y & 0xFFFF0000u));
+}
+
 // N = 1, 2 or 4 consecutive floats at an address aligned to their size
 template <int N>
 __device__ __forceinline__ void load_n(const float* p, float (&v)[N]) {
