@@ -289,7 +289,7 @@ template <int D> constexpr int kAgainMax = D == 128 ? 4 : 8;  // a warp's list (
 template <typename T, int D>
 __device__ __noinline__ void sum_again(const T* x0, const T* x1, const float* even, const float* odd, const CompressArgs* a,
                                        const float (*bounds)[16], const Again* list, int n, int j0, int lane) {
-  constexpr int XPL = D / 32, KQ = D / 4, B = D == 128 ? 16 : 8, STEP = D == 256 ? 32 : B;  // (STEP: from one register of the row)
+  constexpr int XPL = D / 32, KQ = D / 4, B = 8, STEP = D == 256 ? 32 : B;  // (STEP: from one register of the row)
   static_assert(KQ % STEP == 0, "whole batches");
   for (int m = 0; m < n; ++m) {
     const Again e = list[m];
@@ -307,7 +307,7 @@ __device__ __noinline__ void sum_again(const T* x0, const T* x1, const float* ev
     for (int i = 0; i < XPL; ++i) xs[i] = xs[i] / den;
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-    for (int o = 0; o < KQ; o += STEP) {  // the four quarters side by side: 32 or 64 loads in flight
+    for (int o = 0; o < KQ; o += STEP) {  // the four quarters side by side: 32 loads in flight
 #pragma unroll 1
       for (int l = 0; l < STEP; l += B) {
         float p[4][B];
