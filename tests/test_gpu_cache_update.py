@@ -99,3 +99,27 @@ def test_prompt_restored_by_the_tensor_cores(cuda_lib, d, b, h, n, dtype, aligne
         assert ((out[:, :, live].double() - want).abs() <= half * want.abs() * (1 + 2.0**-7) + 2.0**-19 * norms.double()).all()
         for t in (idx, norm, out):
             assert (t[:, :, :off] == 0).all() and (t[:, :, off + n:] == 0).all()
+
+
+@pytest.mark.parametrize("fused", [False, True])
+def test_a_copied_cache_goes_its_own_way(cuda_lib, fused):
+    """A copy made in the middle of a generation (a shared prompt, a file): takes its next update, and neither sees the other's."""
+    import copy
+    import pickle
+
+    from transformers import DynamicCache
+    from turboquant_vllm import CompressedDynamicCache
+
+    d, b, h = 128, 2, 2
+    cc = CompressedDynamicCache(DynamicCache(), d, k_bits=4, v_bits=4)
+    cc.fused_mode = fused
+    steps = [_states(b, h, n, d, torch.bfloat16, seed=i) for i, n in enumerate((20, 1, 1, 1, 1))]
+    for kv in steps[:3]:
+        cc.cache.update(*kv, 0)
+    twins = [copy.deepcopy(cc), pickle.loads(pickle.dumps(cc))]
+    for w, kv in zip([*twins, cc], (steps[3], steps[4], steps[4])):
+        w.cache.update(*kv, 0)
+    got = [w.get_compressed(0) for w in (*twins, cc)]
+    assert all(t.shape[2] == 23 for g in got for t in g)
+    assert all(torch.equal(x, y) for x, y in zip(got[1], got[2]))
+    assert all(torch.equal(x[:, :, :22], y[:, :, :22]) and not torch.equal(x, y) for x, y in zip(got[0], got[2]))

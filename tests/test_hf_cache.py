@@ -301,3 +301,25 @@ def test_fused_backend_install_and_fallthrough_cpu():
     got, _ = triton_fa_tq4_kv_forward(attn, q, k, k, None, scaling=0.2)
     want, _ = sdpa_attention_forward(attn, q, k, k, None, scaling=0.2)
     assert torch.equal(got, want)
+
+
+def test_a_layers_plan_stays_with_its_buffers():
+    """The native plan of an update is of these very buffers: no copy, file or new buffer takes it along."""
+    import copy
+    import pickle
+    from _datetime import datetime_CAPI as capsule  # (what cannot be copied, as the plan)
+
+    from turboquant_vllm.kv_cache import _GrowBuffer
+
+    g = _GrowBuffer()
+    g.append(torch.ones(1, 2, 40, 4))
+    g.fit = capsule
+    for twin in (copy.deepcopy(g), copy.copy(g), pickle.loads(pickle.dumps(g))):
+        assert twin.fit is None and twin.len == 40 and torch.equal(twin.view(), g.view())
+    g.append(torch.ones(1, 2, 20, 4))
+    assert g.fit is capsule
+    g.append(torch.ones(1, 2, 20, 4))  # a larger buffer
+    assert g.fit is None
+    g.fit = capsule
+    g.append(torch.ones(2, 2, 3, 4))  # another shape
+    assert g.fit is None

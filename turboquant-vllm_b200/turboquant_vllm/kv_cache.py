@@ -56,10 +56,15 @@ class _CompressedLayer:
 class _GrowBuffer:
     """A ``[B, H, capacity, W]`` tensor that is appended to along dim 2 with amortised O(1) copies."""
 
+    fit = None  # (first buffer of a layer) plan of the last in-place update, see CompressedDynamicCache._step
+
     def __init__(self) -> None:
         self.buf: torch.Tensor | None = None
         self.len = 0
-        self.fit = None  # (first buffer of a layer) plan of the last in-place update, see CompressedDynamicCache._step
+
+    def __getstate__(self) -> dict:
+        """What a copy or a file takes along: not the plan, which is of these buffers."""
+        return {k: v for k, v in self.__dict__.items() if k != "fit"}
 
     def reserve(self, b: int, h: int, n: int, w: int, dtype: torch.dtype, device: torch.device) -> torch.Tensor:
         """The buffer with room for ``n`` more tokens of ``[b, h, ., w]``; a new one if it held another shape."""
@@ -68,11 +73,13 @@ class _GrowBuffer:
             cap = max(64, 1 << (max(n, 1) - 1).bit_length())
             self.buf = torch.empty(b, h, cap, w, dtype=dtype, device=device)
             self.len = 0
+            self.fit = None
         elif self.len + n > buf.shape[2]:
             cap = max(2 * buf.shape[2], 1 << (self.len + n - 1).bit_length())
             grown = torch.empty(b, h, cap, w, dtype=dtype, device=device)
             grown[:, :, : self.len] = buf[:, :, : self.len]
             self.buf = grown
+            self.fit = None
         return self.buf
 
     def append(self, x: torch.Tensor) -> torch.Tensor:
