@@ -124,7 +124,7 @@ int tq4_append_rows(const void* key, const void* value, int kv_dtype, int batch,
                     uint8_t* rows, int64_t row_bytes, int64_t capacity, int64_t offset, void* stream);
 
 /*
- * One update of a HuggingFace-style cache layer in one launch: key / value [batch, heads, n_new, D] (element
+ * One update of a HuggingFace-style cache layer in one launch (a prompt's in two): key / value [batch, heads, n_new, D] (element
  * strides {batch, head, token}) are compressed into the index and norm buffers [batch, heads, capacity, D/2 or
  * D] / [batch, heads, capacity] behind `offset` tokens (k_nibble / v_nibble: two indices a byte, else one), and
  * the reconstructed vectors centroids[idx] * norm * Pi are stored in key's type into k_dec / v_dec

@@ -490,7 +490,7 @@ class CompressedDynamicCache:
     # ----- token-row storage (fused mode) -------------------------------------------------------------
     def _append_rows(self, layer_idx: int, key_states, value_states, k_comp, v_comp) -> None:
         """Fused-mode update: compress and store the new tokens as token rows, one kernel launch."""
-        b, h, _, d = key_states.shape
+        b, h, n, d = key_states.shape
         store = self._rows[layer_idx]
         if store is None or not store.matches(b, h, d, key_states.device):
             held = self._k_store[layer_idx]
@@ -499,7 +499,7 @@ class CompressedDynamicCache:
                 ks, vs = held, self._v_store[layer_idx]
                 store = TokenRowStore.from_tensors(ks[0].view(), ks[1].view(), vs[0].view(), vs[1].view())
             else:
-                store = TokenRowStore(b, h, d, key_states.device)
+                store = TokenRowStore(b, h, d, key_states.device, n)  # (with room for these at once: no second buffer and table)
             self._rows[layer_idx] = store
             self._k_store[layer_idx] = (_RowsField(store, 0), _RowsField(store, 1))
             self._v_store[layer_idx] = (_RowsField(store, 2), _RowsField(store, 3))
