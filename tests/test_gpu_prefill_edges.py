@@ -231,3 +231,27 @@ def test_prefill_16bit_rows_are_the_rounded_fp32_ones(cuda_lib, d, hq, hkv, dtyp
     wide = torch.full((sum(new), hq, d + pad), 7.0, dtype=dtype, device="cuda")
     ops.paged_tq4_attention(*args, query_start_loc=qsl, out=wide[..., :d], mode=3)
     assert torch.equal(wide[..., :d], want) and (wide[..., d:] == 7).all()
+
+
+@pytest.mark.parametrize("d,hq,hkv", [(128, 40, 40), (64, 66, 33), (256, 32, 32)])
+def test_more_row_blocks_and_heads_than_sms(cuda_lib, d, hq, hkv):
+    """More CTAs than fit at once, spare ones and rows of no sequence among them: every (row, head) by its own CTA."""
+    from turboquant_vllm.kernels import ops
+
+    pr, lens, new, rows = Prims(d), [90, 300, 20], [70, 261, 20], 400
+    p = pr.cuda()
+    case = build_paged_case(lens, hkv, d, 16, pr, seed=6, padded=True)
+    q = torch.randn(rows, hq, d, generator=torch.Generator().manual_seed(2)).bfloat16()
+    qsl = torch.tensor(np.concatenate([[0], np.cumsum(new)]), dtype=torch.int32)
+    args = (case["cache"].cuda(), case["block_table"].cuda(), case["seq_lens"].cuda(), p["kc"], p["vc"], p["rot"], hkv, 16)
+    outs, lses = zip(*((torch.full((rows, hq, d), 7.0, device="cuda"), torch.full((rows, hq), 7.0, device="cuda")) for _ in range(2)))
+    for mode, out, lse in zip((3, 2), outs, lses):
+        ops.paged_tq4_attention(q.cuda(), *args, query_start_loc=qsl.cuda(), mode=mode, out=out, lse_out=lse)
+    n = sum(new)
+    (got, want), (lse, want_lse) = outs, lses
+    # the two kernels share their tables; the sums of at most five 64-key tiles, their order, and the split terms are what differs
+    assert (got[:n] - want[:n]).norm() <= (8 * 5 * 2.0**-23 + 2.0**-18) * want[:n].norm()
+    assert ((got[:n] - want[:n]).norm(dim=-1) <= 2.0**-10 * want[:n].norm(dim=-1)).all()  # (a vector from elsewhere would be 1 away)
+    assert torch.allclose(lse[:n], want_lse[:n], atol=1e-3, rtol=1e-4)
+    assert (got[n:] == 0).all() and (lse[n:] == -torch.inf).all()
+    assert ops.read_and_clear_errors(torch.device("cuda")) == 0

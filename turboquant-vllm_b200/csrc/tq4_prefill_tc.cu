@@ -55,7 +55,7 @@ namespace tq4 {
 __device__ long long g_ptrace[4][64][8];
 #define PF_STAMP(role, j, e)                                                                            \
   do {                                                                                                  \
-    if (blockIdx.x == gridDim.x / 2 && blockIdx.y == 0 && blockIdx.z == 0 && (role) >= 0 && (j) < 64)   \
+    if (blockIdx.x == gridDim.x / 2 && blockIdx.z == 0 && (role) >= 0 && (j) < 64)   \
       g_ptrace[(role) & 3][j][e] = clock64();                                                           \
   } while (0)
 #else
@@ -122,6 +122,7 @@ struct PrefillArgs {
   int to_parts;          // leave partials for the merge kernel instead of writing the output
   float* part_o;         // [splits][rows][Hq][D] normalised, rotated
   float* part_m;         // [splits][rows][Hq] natural-log LSE
+  bool heads_first = false;  // blockIdx.x: KV heads fastest, else row blocks (launch_t)
 };
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -433,7 +434,8 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
   __shared__ int s_dead, s_bad;  // a wait gave up / some page id is out of range
   const AttnShape& sh = a.sh;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int kvh = blockIdx.y, G = sh.G, RB = 128 / G;
+  const int inner = pa.heads_first ? sh.Hkv : (int)gridDim.x / sh.Hkv, outer = (int)blockIdx.x / inner, rest = (int)blockIdx.x - outer * inner;
+  const int rowblk = pa.heads_first ? outer : rest, kvh = pa.heads_first ? rest : outer, G = sh.G, RB = 128 / G;
   volatile int* dead = &s_dead;
   auto bar = [](const uint64_t& b) { return smem_addr(&b); };
   const uint32_t base = (smem_addr(smem_raw) + 1023u) & ~1023u;
@@ -459,7 +461,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
         const int up = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += up;
       }
-      const int x = (int)blockIdx.x - acc;
+      const int x = rowblk - acc;
       const unsigned m = __ballot_sync(0xffffffffu, x < incl);
       if (m) {
         const int w = __ffs(m) - 1;
@@ -476,8 +478,8 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
     }
     if (lane == 0) {
       s_info[0] = found;
-      s_info[1] = found < 0 ? (int)blockIdx.x - acc : first;  // (without rows: which of the spare CTAs, and how many)
-      s_info[2] = found < 0 ? (int)gridDim.x - acc : nrows;
+      s_info[1] = found < 0 ? rowblk - acc : first;  // (without rows: which of the spare CTAs, and how many)
+      s_info[2] = found < 0 ? (int)gridDim.x / sh.Hkv - acc : nrows;
       s_dead = 0;
       s_bad = 0;
     }
@@ -1317,7 +1319,7 @@ __global__ void __launch_bounds__(kThreads, 1) prefill_tc_kernel(const AttnArgs 
 }
 
 template <int D, bool FAST>
-int launch_t(const AttnArgs& a, const PrefillArgs& pa, cudaStream_t st) {
+int launch_t(const AttnArgs& a, PrefillArgs pa, cudaStream_t st) {
   using C = Cfg<D>;
   constexpr int smem = (int)C::kSmem + 1024;
   static_assert(smem + 2048 <= 227 * 1024, "shared memory");
@@ -1327,8 +1329,15 @@ int launch_t(const AttnArgs& a, const PrefillArgs& pa, cudaStream_t st) {
   if (!ensure_dynamic_smem<prefill_tc_kernel<D, FAST>>(ask)) return TQ4_ERR_CUDA;
   const int per_cta = C::NBLK * (128 / a.sh.G);
   const unsigned blocks = (unsigned)((a.sh.rows + per_cta - 1) / per_cta + a.sh.num_seqs);  // upper bound
-  if (launch_kernel(prefill_tc_kernel<D, FAST>, dim3(blocks, (unsigned)a.sh.Hkv, (unsigned)pa.splits), dim3(kThreads),
-                    (size_t)ask, st, true, a, pa) != cudaSuccess)
+  // More CTAs than fit at once: the KV heads run fastest, so that all heads of a sequence's last rows (the longest) start before any of
+  // its first and those left for the end are short.  Rows fastest / heads fastest, us: 2048 rows of 32 / 8 heads of 128 146 / 111, 6000
+  // 632 / 572, 4000 of 32 / 32 of 96 362 / 308, 2 x 1500 of 8 / 4 of 256 139 / 113, 8 x 2048 on 8192 4690 / 4605.  One wave: nothing waits, and a
+  // head's CTAs next to one another are better off (4 x 500 on 3000, 14 / 2 heads of 64: 129 / 141).
+  const int64_t grid = (int64_t)blocks * a.sh.Hkv;
+  if (grid > 0x7fffffff) return TQ4_ERR_UNSUPPORTED;
+  pa.heads_first = grid * pa.splits > sm_count();
+  if (launch_kernel(prefill_tc_kernel<D, FAST>, dim3((unsigned)grid, 1, (unsigned)pa.splits), dim3(kThreads), (size_t)ask, st, true, a,
+                    pa) != cudaSuccess)
     return TQ4_ERR_CUDA;
   TQ4_CHECK_LAUNCH();
   return TQ4_OK;
