@@ -101,6 +101,35 @@ def test_prompt_restored_by_the_tensor_cores(cuda_lib, d, b, h, n, dtype, aligne
             assert (t[:, :, :off] == 0).all() and (t[:, :, off + n:] == 0).all()
 
 
+def test_prompt_without_tensor_cores(cuda_lib):
+    """TQ4_NO_TC (read once a process): a prompt past the line is neither compressed nor restored by a tcgen05 kernel."""
+    import os
+    import subprocess
+    import sys
+
+    prog = """
+import sys
+sys.path.insert(0, {pkg!r})
+import torch
+from torch.profiler import ProfilerActivity, profile
+from transformers import DynamicCache
+from turboquant_vllm import CompressedDynamicCache
+
+cc = CompressedDynamicCache(DynamicCache(), 128, k_bits=4, v_bits=4)
+k, v = (torch.randn(1, 8, 700, 128, generator=torch.Generator().manual_seed(i)).cuda().bfloat16() for i in range(2))
+with profile(activities=[ProfilerActivity.CUDA]) as p:
+    cc.cache.update(k, v, 0)
+    torch.cuda.synchronize()
+print([e.key for e in p.key_averages() if "tq4::" in e.key])
+"""
+    pkg = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "turboquant-vllm_b200")
+    for env, tensor_cores in (({}, True), ({"TQ4_NO_TC": "1"}, False)):
+        done = subprocess.run([sys.executable, "-c", prog.format(pkg=pkg)], capture_output=True, text=True, timeout=300,
+                              env={**{k: v for k, v in os.environ.items() if k != "TQ4_NO_TC"}, **env})
+        assert done.returncode == 0, done.stderr[-2000:]
+        assert "tq4::" in done.stdout and ("_tc" in done.stdout) == tensor_cores, done.stdout
+
+
 @pytest.mark.parametrize("fused", [False, True])
 def test_a_copied_cache_goes_its_own_way(cuda_lib, fused):
     """A copy made in the middle of a generation (a shared prompt, a file): takes its next update, and neither sees the other's."""

@@ -14,6 +14,8 @@
 // Waits are bounded: a wait that gives up leaves NaN in the vectors that it should have brought.
 #include <math_constants.h>
 
+#include <cstdlib>
+
 #include "tq4_cache_update.cuh"
 
 namespace tq4 {
@@ -331,6 +333,8 @@ int launch_t(const UpdateArgs& a, cudaStream_t st) {
 }  // namespace
 
 bool restore_tc_eligible(const UpdateArgs& a, int head_dim) {
+  static const bool disabled = getenv("TQ4_NO_TC") != nullptr;
+  if (disabled) return false;
   if ((a.dtype != TQ4_F16 && a.dtype != TQ4_BF16) || head_dim > 128 || a.dec[0] == nullptr || (uintptr_t)a.packed % 16) return false;
   for (int s = 0; s < 2; ++s)
     if ((uintptr_t)a.idx[s] % 16 || (uintptr_t)a.dec[s] % 16) return false;
