@@ -48,3 +48,21 @@ def test_paged_write_tiles(cuda_lib, d, n_tok, h, dtype, strided):
             ops.tq4_write_paged(kc[i:i + 32], vc[i:i + 32], parts, slots[i:i + 32].cuda(), p["even"], p["odd"], p["kb"], p["vb"])
         assert torch.equal(cache, parts)
     assert ops.read_and_clear_errors(torch.device("cuda")) == 0
+
+
+@pytest.mark.parametrize("d,dtype", [(64, torch.float16), (96, torch.float16), (128, torch.float16), (256, torch.float16), (256, torch.bfloat16)])
+def test_coordinates_on_a_boundary(cuda_lib, golden, d, dtype):
+    """Vectors with a coordinate whose two sums, the tensor cores' and the FMA chain's, lie 1.6e-7 - 2.4e-7 apart on either side of
+    a boundary (found among 2.5e12 coordinates of vectors that few coordinates dominate): the bytes are the FMA kernels'."""
+    from turboquant_vllm.kernels import ops
+
+    pr = Prims(d)
+    p = pr.cuda()
+    hard = torch.from_numpy(golden("near_boundary.npz")[f"d{d}_{str(dtype)[6:]}"]).view(dtype).cuda()
+    few, few_norms = ops.tq4_compress(hard[:, None].contiguous(), p["even"], p["odd"], p["kb"])
+    n = {64: 6601, 96: 3101, 128: 4801, 256: 1101}[d]  # the tensor-core kernel's turn
+    x = torch.randn(n, d, generator=torch.Generator().manual_seed(d)).to(dtype).cuda()
+    at = torch.arange(0, n, 5, device="cuda")  # (six rows of a warp: its list runs full)
+    x[at] = hard[at // 5 % len(hard)]
+    packed, norms = ops.tq4_compress(x[:, None].contiguous(), p["even"], p["odd"], p["kb"])
+    assert torch.equal(packed[at], few[at // 5 % len(hard)]) and torch.equal(norms[at], few_norms[at // 5 % len(hard)])

@@ -335,10 +335,10 @@ inline bool tokens_uniform(const CompressArgs& a) {
 //     3.4 / 4.6, 444 5.1 / 4.6; of 64 2.2 / 2.7, 592 2.6 / 3.0; of 96 2.7 / 4.4, 444 3.9 / 4.9, 592 5.2 / 5.0; of 256 4.7 / 11.2, 296 8.0 / 11.3
 //   a block per vector up to tiny_rows(): a few us plus 1.1 / 1.7 / 2.5 us per 1000 vectors of 64 / 96 / 128, against 8 - 14 us
 //     of the tensor-core kernel; at 256 it never pays
-//   the tensor-core kernel above tc_rows().  Up to kSmallRows a vector is promised the same bytes however the calls are cut, so
-//     there it sums coordinates near a boundary again the FMA kernels' way (above, at head_dim 128, its bytes are its own), which
-//     at 128 is 2 us for each that a warp has: 14.4 - 18.8 us at 4800 - 8192 vectors against 16.5 of the prologue kernel's one wave up
-//     to 4736 and 18.5 above.  At 256 the prologue kernel takes 15 us at 800
+//   the tensor-core kernel above tc_rows().  Up to kSmallRows a vector is to have the same bytes however the calls are cut, so
+//     there it sums coordinates near a boundary again the FMA kernels' way, within a margin that no sum seen has left
+//     (Fmt<T>::kNear; above, at head_dim 128, its bytes are its own).  At 128 that is 2 us for each that a warp has: 15.1 - 17.4 us at
+//     4800 - 8192 vectors against 16.5 of the prologue kernel's one wave up to 4736 and 18.5 above.  At 256 the prologue kernel takes 15 us at 800
 //   the prologue kernel in between, and up to kSmallRows for what the tensor-core kernel cannot address
 constexpr int64_t kSmallRows = 8192;
 constexpr int64_t tiny_rows(int head_dim) { return head_dim == 64 ? 6500 : head_dim == 96 ? 3000 : head_dim == 128 ? 4096 : 0; }

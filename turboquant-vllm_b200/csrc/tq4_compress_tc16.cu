@@ -30,7 +30,7 @@
 // (lane c holds cell c's boundary and the index below it), one compare, one add.  The comparison is the
 // search's own, against the same fp32 boundary, so the indices are the same.  Measured (bf16 cache write, K and
 // V): 16384 tokens of 8 heads of 128 48.6 -> 31.1 us (2.7 TB/s), 8208 vectors 24 -> 11.1 us
-// against a block per vector, 16384 tokens of 4 heads of 256 894 -> 79 us (62 without the
+// against a block per vector, 16384 tokens of 4 heads of 256 894 -> 91 us (62 without the
 // second sums below; the 256 columns are split over CTAs:
 // one cannot hold Pi and two stages of vectors).
 // Every mbarrier wait is bounded; a wait that gives up marks the CTA dead, all roles drain (tiles and MMAs in flight are
@@ -155,6 +155,7 @@ template <>
 struct Fmt<__half> {
   static constexpr int kTerms = 2;
   static constexpr uint32_t kCode = 0;
+  static constexpr float kNear = 4e-7f;
   static constexpr float kScale = 256.f;  // keeps the lo term of small entries a normal fp16 number
   static __device__ __forceinline__ uint16_t term(float& rest) {
     const __half h = __float2half_rn(rest);
@@ -166,6 +167,7 @@ template <>
 struct Fmt<__nv_bfloat16> {
   static constexpr int kTerms = 3;
   static constexpr uint32_t kCode = 1;
+  static constexpr float kNear = 3.4e-7f;
   static constexpr float kScale = 1.f;
   static __device__ __forceinline__ uint16_t term(float& rest) {
     const __nv_bfloat16 h = __float2bfloat16_rn(rest);
@@ -222,10 +224,14 @@ __device__ __forceinline__ int bucketize_reg(float y, const float (&b)[15]) {
   return (c1 ? 8 : 0) + (c2 ? 4 : 0) + (c3 ? 2 : 0) + (c4 ? 1 : 0);
 }
 
-// The two roundings of a coordinate (this kernel's product, the FMA kernels' chains) lie 2e-8 apart on average; a coordinate
-// nearer than this to a boundary (about 1e-5 of them) is summed again the FMA kernels' way, so that the bytes are theirs.
+// The two roundings of a coordinate (this kernel's product, the FMA kernels' chains) lie 1 - 2e-8 apart on average; a coordinate
+// nearer than Fmt<T>::kNear to a boundary (about 3e-5 of them) is summed again the FMA kernels' way, so that the bytes are theirs.
+// That is a margin, not a bound.  Among 2.5e12 coordinates, two thirds of them of vectors that one, two or sixteen coordinates dominate
+// (the rounding errors are then as large as the result allows), the largest distance was 3.1e-7 for bf16 and 3.6e-7 for fp16,
+// whose Pi has 22 bits; with a margin of 1.5e-7 79 indices differed, from 3.2e-7 on none.  Half a unit a step of the FMA chains and a
+// unit an accumulation, at the size of the outermost boundary, would add up to 1.3e-6 at head_dim 128.  Margins of 1.5e-7 / these / 5e-7
+// cost a write of 16384 x 4 bf16 vectors of 256 82 / 91 / 96 us, of 512 x 8 of 128 15.3 / 17.4 / 17.5, of 4000 x 32 of 96 33.0 / 35.4 / 36.2.
 // (Not in large writes at head_dim 128, which have been the tensor cores' own for longer than there was a choice.)
-constexpr float kNear = 1.5e-7f;
 
 // The 32-cell map: cell = round(31 * sat(y * s / 31 + 16 / 31)), so y = 0 sits in the middle of cell 16 and
 // everything past the ends in the end cells.  `scale` = s / 31; lane c: the boundary inside cell c (+inf: none) and the
@@ -338,7 +344,7 @@ struct Bars {
   uint64_t drain;      // a dead CTA's last MMA is complete
 };
 
-// AGAIN: a coordinate near a boundary is summed again, see kNear
+// AGAIN: a coordinate near a boundary (Fmt<T>::kNear) is summed again
 template <typename T, int D, bool AGAIN>
 __global__ void __launch_bounds__(Cfg<D>::THREADS, 1)
 compress_tc16_kernel(const __grid_constant__ CompressArgs a, const int group_rows, const __grid_constant__ CUtensorMap tm_x0,
@@ -597,7 +603,7 @@ compress_tc16_kernel(const __grid_constant__ CompressArgs a, const int group_row
             for (int e = 0; e < 8; ++e) {
               const float y = __uint_as_float(v[8 * w + e]) * scale;
               const int idx = bucketize_reg(y, b);
-              if (kAgain && bucketize_reg(y - kNear, b) != bucketize_reg(y + kNear, b)) closest = 0.f;
+              if (kAgain && bucketize_reg(y - F::kNear, b) != bucketize_reg(y + F::kNear, b)) closest = 0.f;
               word[w] += (uint32_t)idx << (8 * (e >> 1) + ((e & 1) ? 0 : 4));
             }
           }
@@ -610,7 +616,7 @@ compress_tc16_kernel(const __grid_constant__ CompressArgs a, const int group_row
         }
         if constexpr (kAgain) {
           // (a zero vector is zero either way)
-          uint32_t who = __ballot_sync(0xffffffffu, closest < kNear && dst_idx != nullptr && nrm != 0.f);
+          uint32_t who = __ballot_sync(0xffffffffu, closest < F::kNear && dst_idx != nullptr && nrm != 0.f);
 #pragma unroll 1
           for (; who != 0; who &= who - 1) {
             if (n_again == kAgainMax<D>) {
