@@ -94,6 +94,27 @@ def test_contiguous_kv_matches_oracle(cuda_lib, b, hq, hkv, sq, skv, d, causal, 
     torch.testing.assert_close(out.float().cpu(), expected, atol=1.2e-2, rtol=1.6e-2)
 
 
+@pytest.mark.parametrize(("b", "sq", "held", "room"), [(1, 1, 5000, 10240), (1, 1, 0, 10240), (2, 1, 1300, 8192), (1, 300, 300, 8192)])
+def test_kernels_by_tokens_held(cuda_lib, b, sq, held, room):
+    """Which kernels run, and with them every bit of the result, does not depend on the room that the rows have for more tokens."""
+    from turboquant_vllm import _native as nv
+    from turboquant_vllm.token_rows import TokenRowStore
+
+    qz, rot, cents, _ = _prims(128)
+    q = torch.randn(b, 32, sq, 128, generator=torch.Generator().manual_seed(1)).bfloat16().cuda()
+    k, v = (_kv(b, 8, held, 128, i, torch.bfloat16).cuda() for i in (2, 3))
+    got = []
+    for tokens in (held, room):
+        store = TokenRowStore(b, 8, 128, torch.device("cuda"), min_tokens=tokens)
+        store.append(k, v, qz, qz)
+        nv.profile_start(8)
+        out = store.attention(q, cents.cuda(), cents.cuda(), rot.cuda(), is_causal=True, out_dtype=torch.float32)
+        got.append((out, len(nv.profile_read(nv.PROF_COMBINE, 8))))
+        nv.profile_stop()
+    (a, merges), (w, merges_w) = got
+    assert merges == merges_w and (sq > 1 or merges == 0) and torch.equal(a, w)
+
+
 def test_fused_mode_cache_rows_and_forward(cuda_lib):
     from transformers import DynamicCache
 

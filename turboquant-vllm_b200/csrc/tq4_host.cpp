@@ -393,10 +393,12 @@ PyObject* attend_rows(PyObject*, PyObject* const* p, Py_ssize_t n) {
     int st;
     {
       const NoGil no_gil;
-      st = tq4_paged_attention(
-          q.data_ptr(), q_dt, b, (int)b, (int)hq, (int)hkv, (int)d, q.stride(0), q.stride(1), (const uint8_t*)rows.data_ptr(),
-          page * rows.size(2), rows.size(2), b * (rows.size(1) / page), (int)page, (const int32_t*)bt.data_ptr(), bt.size(1),
-          (const int32_t*)lens.data_ptr() + len * b, nullptr, (const float*)kc.data_ptr(), (int)kc.numel(),
+      // (the kernels are chosen by the tokens held, not by the room for more)
+      st = tq4_attention_step(
+          nullptr, nullptr, q_dt, 0, 0, 0, 0, 0, nullptr, 0, nullptr, nullptr, nullptr, 0, nullptr, 0, q.data_ptr(), q_dt, b, (int)b,
+          (int)hq, (int)hkv, (int)d, q.stride(0), q.stride(1), (uint8_t*)rows.data_ptr(), page * rows.size(2), rows.size(2),
+          b * (rows.size(1) / page), (int)page, (const int32_t*)bt.data_ptr(), bt.size(1),
+          (const int32_t*)lens.data_ptr() + len * b, nullptr, len > 0 ? len : 1, (const float*)kc.data_ptr(), (int)kc.numel(),
           (const float*)vc.data_ptr(), (int)vc.numel(), (const float*)rot.data_ptr(), scale, 0, 0, out.data_ptr(), out_dt,
           out.stride(0), out.stride(2), nullptr, 0, ws.data_ptr(), (size_t)ws.numel() * ws.element_size(), 0, flag, launch.stream);
     }

@@ -186,7 +186,8 @@ class TokenRowStore:
             qsl = None if sq == 1 else torch.arange(0, (b + 1) * sq, sq, dtype=torch.int32, device=dev)
         out = paged_tq4_attention(
             q_rows, self.paged_cache(), table, lens, k_centroids, v_centroids, rotation, self.heads,
-            PAGE_TOKENS, sm_scale, query_start_loc=qsl, causal=causal, out_dtype=out_dtype)
+            PAGE_TOKENS, sm_scale, query_start_loc=qsl, causal=causal, out_dtype=out_dtype,
+            max_seq_len=max(self.len, 1))  # (the tokens held choose the kernels, not the room for more)
         return out.view(b, sq, hq, d)
 
 
