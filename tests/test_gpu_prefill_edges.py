@@ -214,6 +214,28 @@ def test_prefill_large_and_small_queries(cuda_lib, d, hq, hkv, v_bits, power):
 
 
 @pytest.mark.parametrize("d,hq,hkv", [(64, 14, 2), (96, 4, 4), (128, 28, 4), (256, 8, 4)])
+@pytest.mark.parametrize("power", [-9, 9])
+def test_prefill_some_rows_large_or_small(cuda_lib, d, hq, hkv, power):
+    """Some rows of a warp outside the range of the queries' terms, some inside; tiles that all rows see whole, and others.
+    Bound as above (the scores of the rows that are not scaled are 2^9 times smaller or larger: of the smaller of the two)."""
+    from turboquant_vllm.kernels import ops
+
+    p, gen = Prims(d).cuda(), torch.Generator(device="cuda").manual_seed(1)
+    rand = lambda *shape: torch.randn(*shape, device="cuda", generator=gen)  # noqa: E731
+    n, new = 300, 150
+    cache = torch.zeros(19, 16, hkv * O.padded_slot_bytes(d), dtype=torch.uint8, device="cuda")
+    ops.tq4_write_paged(rand(n, hkv, d) * min(1.0, 2.0**-power), rand(n, hkv, d), cache, torch.arange(n, device="cuda"), p["even"],
+                        p["odd"], p["kb"], p["vb"])
+    table = torch.arange(19, dtype=torch.int32, device="cuda")[None]
+    q = rand(new, hq, d)
+    q[::5] *= 2.0**power
+    args = (q, cache, table, torch.tensor([n], dtype=torch.int32).cuda(), p["kc"], p["vc"], p["rot"], hkv, 16)
+    qsl = torch.tensor([0, new], dtype=torch.int32).cuda()
+    a, b = (ops.paged_tq4_attention(*args, query_start_loc=qsl, out_dtype=torch.float32, mode=m).double() for m in (3, 2))
+    for rows in (slice(0, None, 5), slice(1, None, 5)):
+        assert (a[rows] - b[rows]).norm() / b[rows].norm() <= 8 * 5 * 2.0**-23 + 2.0**-18
+
+@pytest.mark.parametrize("d,hq,hkv", [(64, 14, 2), (96, 4, 4), (128, 28, 4), (256, 8, 4)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("pad", [0, 8, 2])
 def test_prefill_16bit_rows_are_the_rounded_fp32_ones(cuda_lib, d, hq, hkv, dtype, pad):
