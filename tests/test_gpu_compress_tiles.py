@@ -42,7 +42,7 @@ def test_paged_write_tiles(cuda_lib, d, n_tok, h, dtype, strided):
         x, y = (t[:, a:a + 4 * h].contiguous().view(torch.float32) + 1e-30 for t in (got, want))
         assert ulp_diff(x, y).max() <= 4
     assert torch.equal(got[:, end:], want[:, end:])
-    if d != 128:  # coordinates on a boundary are summed again: the bytes are those of the kernels for few vectors
+    if d != 128 or 2 * n_tok * h <= 8192:  # coordinates on a boundary are summed again: the bytes are those of the kernels for few vectors
         parts = torch.zeros_like(cache)
         for i in range(0, n_tok, 32):
             ops.tq4_write_paged(kc[i:i + 32], vc[i:i + 32], parts, slots[i:i + 32].cuda(), p["even"], p["odd"], p["kb"], p["vb"])
