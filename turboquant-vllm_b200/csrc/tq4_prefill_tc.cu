@@ -1340,7 +1340,10 @@ int launch_t(const AttnArgs& a, PrefillArgs pa, cudaStream_t st) {
   // More CTAs than fit at once: the KV heads run fastest, so that all heads of a sequence's last rows (the longest) start before any of
   // its first and those left for the end are short.  Rows fastest / heads fastest, us: 2048 rows of 32 / 8 heads of 128 146 / 111, 6000
   // 632 / 572, 4000 of 32 / 32 of 96 362 / 308, 2 x 1500 of 8 / 4 of 256 139 / 113, 8 x 2048 on 8192 4690 / 4605.  One wave: nothing waits, and a
-  // head's CTAs next to one another are better off (4 x 500 on 3000, 14 / 2 heads of 64: 129 / 141).
+  // head's CTAs next to one another are better off (4 x 500 on 3000, 14 / 2 heads of 64: 129 / 141).  Counted with the spare row blocks
+  // of the upper bound, which the SMs go through as well: heads fastest, they come behind all others (480 rows beside 32 running
+  // sequences 206 / 201, 256 beside 60, 28 / 4 heads, 145 / 134).  Where only the spare ones make it more than a wave (10 - 64 prompts of
+  // 30 - 190 rows on 2000 - 3000, 14 / 2 of 64 and 4 / 1 of 128) the two orders are within 0.6 %.
   const int64_t grid = (int64_t)blocks * a.sh.Hkv;
   if (grid > 0x7fffffff) return TQ4_ERR_UNSUPPORTED;
   pa.heads_first = grid * pa.splits > sm_count();
