@@ -164,9 +164,6 @@ inline size_t carve_plan(AttnPlan& p, void* ws, int64_t rows, int Hq, int D, int
 // Launchers implemented in tq4_attention.cu / tq4_decode_mma.cu.
 int launch_attention_fp32(const AttnArgs& a, cudaStream_t st);
 int launch_attention_mma(const AttnArgs& a, cudaStream_t st);  // returns TQ4_ERR_UNSUPPORTED if shape not covered
-// tensor-core (tcgen05) chunked-prefill kernel (tq4_prefill_tc.cu) over the sequences with at least `min_rows`
-// new rows: rotates, attends, un-rotates and writes the output, or leaves `splits` dense partials per row
-// (normalised rotated output in part_o [splits][rows][Hq][D], natural-log LSE in part_m [splits][rows][Hq])
 // Query vectors up to which the prologue of a call takes a block per vector (whether it writes or not: its sums are folded in
 // another order than those of the prologue for many).  Whole steps on 3000 keys each, us without / with it: 512 + 256 vectors of 128 37.6 /
 // 35.0, 768 + 384 43.4 / 39.6; of 64 equal up to 756 + 216; of 96 384 + 768 53.4 / 51.5, 512 + 1024 61.7 / 62.0; of 256 192 + 192 49.7 / 47.3, 256 + 256
@@ -176,6 +173,9 @@ constexpr int64_t tiny_queries(int head_dim) { return head_dim == 256 ? 256 : he
 int decode_step_cluster(const AttnArgs& a);
 bool decode_step_rotates(const AttnArgs& a);  // it can rotate the queries itself (`rotate`: they are not yet)
 int launch_decode_step(const AttnArgs& a, int cl_shift, bool rotate, cudaStream_t st);
+// tensor-core (tcgen05) chunked-prefill kernel (tq4_prefill_tc.cu) over the sequences with at least `min_rows`
+// new rows: rotates, attends, un-rotates and writes the output, or leaves `splits` dense partials per row
+// (normalised rotated output in part_o [splits][rows][Hq][D], natural-log LSE in part_m [splits][rows][Hq])
 bool prefill_tc_supported(const AttnArgs& a);
 int prefill_tc_splits(const AttnArgs& a, int64_t slots);
 size_t prefill_tc_image_bytes(int D);

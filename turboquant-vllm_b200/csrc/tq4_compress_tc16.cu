@@ -229,8 +229,9 @@ __device__ __forceinline__ int bucketize_reg(float y, const float (&b)[15]) {
 // That is a margin, not a bound.  Among 2.5e12 coordinates, two thirds of them of vectors that one, two or sixteen coordinates dominate
 // (the rounding errors are then as large as the result allows), the largest distance was 3.1e-7 for bf16 and 3.6e-7 for fp16,
 // whose Pi has 22 bits; with a margin of 1.5e-7 79 indices differed, from 3.2e-7 on none.  Half a unit a step of the FMA chains and a
-// unit an accumulation, at the size of the outermost boundary, would add up to 1.3e-6 at head_dim 128.  Margins of 1.5e-7 / these / 5e-7
-// cost a write of 16384 x 4 bf16 vectors of 256 82 / 91 / 96 us, of 512 x 8 of 128 15.3 / 17.4 / 17.5, of 4000 x 32 of 96 33.0 / 35.4 / 36.2.
+// unit an accumulation, at the size of the outermost boundary, would add up to 1.3e-6 at head_dim 128.  With margins of 1.5e-7 / these /
+// 1.3e-6 a write of K and V takes, us (bf16): 16384 tokens x 4 heads of 256 82 / 91 / 147, 512 x 8 of 128 15.3 / 17.4 / 20.0 (18.5 by the
+// FMA kernels), 4000 x 32 of 96 33.0 / 35.4 / 39.9, 16384 x 2 of 64 14.5 / 14.5 / 16.4.
 // (Not in large writes at head_dim 128, which have been the tensor cores' own for longer than there was a choice.)
 
 // The 32-cell map: cell = round(31 * sat(y * s / 31 + 16 / 31)), so y = 0 sits in the middle of cell 16 and
