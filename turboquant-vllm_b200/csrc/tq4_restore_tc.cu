@@ -10,9 +10,9 @@
 // to the cache's buffers on the way.  The 70 400 vectors of 128 of a prompt of 4 x 1100 tokens (8 heads): 97 us by the FMA kernel that
 // did this (bound by FMA issue and the reads of Pi), 20 here; what bounds it is the lookups (8192 a tile, and their operand
 // stores) and, for few tiles a CTA, the preparation of Pi.
-// The FMA kernel's operands had 24 bits, these have 22.  Of the values as rounded to 16 bits, against the rounded 64-bit result (8000 vectors x 6 rotations, K4/V3 and K2/V4), so many differ, here / FMA kernel: bf16 1.4 - 2.0 /
-// 1.8 - 2.3 in 10^4 at head_dim 64 and 96, 1.9 - 2.2 / 2.2 - 2.5 at 128; fp16 0.9 - 1.3 / 1.2 - 1.5 in 10^3 and 1.3 - 1.4 / 1.5 - 1.6; the 2-norm of
-// the error is the same to six figures.
+// The FMA kernel's operands had 24 bits, these have 22.  Of the values as rounded to 16 bits so many are not the rounded 64-bit
+// result (8000 vectors x 6 rotations, K4/V3 and K2/V4), here / FMA kernel: bf16 1.4 - 2.0 / 1.8 - 2.3 in 10^4 at head_dim 64 and 96, 1.9 - 2.2
+// / 2.2 - 2.5 at 128; fp16 0.9 - 1.3 / 1.2 - 1.5 in 10^3 and 1.3 - 1.4 / 1.5 - 1.6; the 2-norm of the error is the same to six figures.
 // Waits are bounded: a wait that gives up leaves NaN in the vectors that it should have brought.
 #include <math_constants.h>
 
