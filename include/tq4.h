@@ -65,7 +65,7 @@ const char* tq4_status_string(int status);
  * end to end a coordinate within ~1e-7 of a boundary may land in the neighbouring bucket, because
  * the rotation's summation order differs from the reference's matmul: at most 1e-4 of the indices
  * (measured 6e-7 on the FFMA kernels, 5e-7 on the tensor-core kernels that take 16-bit inputs of more
- * than 6500 / 3000 / 8192 / 1000 vectors at head_dim 64 / 96 / 128 / 256 and fp32 ones above 8192 at 128; setting
+ * than 6500 / 3000 / 4736 / 1000 vectors at head_dim 64 / 96 / 128 / 256 and fp32 ones above 8192 at 128; setting
  * TQ4_NO_TC in the environment keeps every input on the FFMA kernels).  Norms are within 3 ulp of a CPU torch.norm and identical across all kernels here.
  * Replaces: tq4_compress() + _tq4_compress_kernel, src/turboquant_vllm/triton/tq4_compress.py:46-148,173-245
  *           (arithmetic contract = its PyTorch path, :248-295 / quantizer.py:112-151).
